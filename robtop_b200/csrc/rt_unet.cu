@@ -242,13 +242,8 @@ static int unet_conv_bwd(rt_unet* u, int li, int lvl, const __nv_bfloat16* in, i
         rtu::k_bias_grad<<<(unsigned)std::min<long>((V + 63) / 64, 1024), 256, 0, c->stream>>>(u->gpre, l.cout, V,
                                                                                                u->G + l.boff);
     }));
-    const long nw = 27L * l.cin * l.cout;
-    const long chunk = 4096;
-    const dim3 gdw((unsigned)((nw + 255) / 256), (unsigned)((V + chunk - 1) / chunk));
-    RT_CHECK(rt_launch(c, "unet_conv3_dw", [&] {
-        rtu::k_conv3_dw<<<gdw, 256, 0, c->stream>>>(in, in_stride, l.cin, u->gpre, l.cout, u->X[lvl], u->Y[lvl],
-                                                    u->Z[lvl], chunk, u->G + l.woff);
-    }));
+    RT_CHECK(rtu::conv3_dw(c, in, in_stride, l.cin, u->gpre, l.cout, u->X[lvl], u->Y[lvl], u->Z[lvl], u->G + l.woff,
+                           u->err));
     if (!gin) return RT_OK;
     rtu::ConvArgs a;
     a.in = u->gpre;

@@ -28,6 +28,8 @@ struct ConvArgs {
 
 int conv3_init(rt_ctx* c);
 int conv3(rt_ctx* c, const ConvArgs& a);
+int conv3_dw(rt_ctx* c, const __nv_bfloat16* in, int in_stride, int cin, const __nv_bfloat16* gpre, int cout, int X,
+             int Y, int Z, float* dw, int* err);
 size_t conv3_smem_bytes(int cin, int cout);
 void conv3_set_variant(int v);  // 1: halo tile (default), 0: per-tap gather
 
@@ -43,8 +45,6 @@ __global__ void k_up2_bwd(const float* gout, int gout_stride, int C, int X, int 
 __global__ void k_relu_bwd(const float* g, int g_stride, const __nv_bfloat16* y, int y_stride, int C, long V, int relu,
                            __nv_bfloat16* gpre);
 __global__ void k_bias_grad(const __nv_bfloat16* gpre, int C, long V, float* db);
-__global__ void k_conv3_dw(const __nv_bfloat16* in, int in_stride, int cin, const __nv_bfloat16* gpre, int cout, int X,
-                           int Y, int Z, long chunk, float* dw);
 __global__ void k_weights_bf16(const float* w, int cin, int cout, __nv_bfloat16* w16, __nv_bfloat16* w16t);
 __global__ void k_adam(long n, float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float c1,
                        float c2, float eps);

@@ -324,6 +324,10 @@ static int halo_plan(int cin, int cout, int* G, size_t* smem) {
     return 0;
 }
 
+__global__ void k_conv3_dw_tc(const __nv_bfloat16* __restrict__ in, int in_stride, int cin,
+                              const __nv_bfloat16* __restrict__ gpre, int cout, int X, int Y, int Z, int P, int TG,
+                              float* __restrict__ dw, int* err);
+
 static int g_conv_variant = 1;  // 1: halo tile (default), 0: per-tap gather
 
 size_t conv3_smem_bytes(int cin, int cout) {
@@ -339,6 +343,8 @@ int conv3_init(rt_ctx* c) {
     cudaError_t e = cudaFuncSetAttribute(k_conv3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_conv3_halo, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_conv3_dw_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return rt_fail(c, RT_ECUDA, "conv3 smem attribute: %s", cudaGetErrorString(e));
     return RT_OK;
 }
@@ -362,6 +368,139 @@ int conv3(rt_ctx* c, const ConvArgs& a) {
     const unsigned blocks = (unsigned)((V + CONV_TM - 1) / CONV_TM);
     const size_t smem = conv3_smem_bytes(a.cin, a.cout);
     return rt_launch(c, "unet_conv3_tc", [&] { k_conv3_tc<<<blocks, CONV_THREADS, smem, c->stream>>>(a); });
+}
+
+// ---------------------------------------------------------------------------
+// k_conv3_dw_tc: weight gradient dW[n][tap][c] += sum_v gpre[v][n] in[v + off(tap)][c] as 27 GEMMs with K = voxels:
+// D[n x c] in TMEM += A[n x 16 voxels] B[c x 16 voxels]^T.  Both operands are MN-major (channels-last voxels hold 8
+// channels per 16 bytes), so the halo of k_conv3_halo is already the B operand of every tap: 8 voxels of a patch
+// row are one core matrix, the next row (LBO) is 160 B on, the next 8 channels (SBO) one chunk plane, and a tap
+// moves the start address.  A is the patch of the gradient, [8-channel chunk][plane][y][x]; it has M = 128 rows,
+// and the rows past cout read whatever follows in shared memory and are dropped.  A CTA owns TG taps (blockIdx.y)
+// and walks the patches blockIdx.x, + gridDim.x, ... with its TG x cin accumulator columns kept in TMEM, then adds
+// them to dW.  It replaces a CUDA-core loop over the voxels per weight (21.7 of the 23.2 ms of a 33^3 sample's
+// gradients).  Waits are bounded as in the convolution.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(CONV_THREADS) k_conv3_dw_tc(const __nv_bfloat16* __restrict__ in, int in_stride,
+                                                              int cin, const __nv_bfloat16* __restrict__ gpre,
+                                                              int cout, int X, int Y, int Z, int P, int TG,
+                                                              float* __restrict__ dw, int* err) {
+    extern __shared__ __align__(128) uint8_t sm[];
+    const int kchI = cin / 8, kchG = cout / 8, npl = P + 2;
+    const uint32_t plane_b = HALO_V * 16, sboB = (uint32_t)npl * plane_b, sboA = (uint32_t)P * CONV_TM * 16;
+    uint8_t* sG = sm + 128;
+    uint8_t* sH = sG + (uint32_t)kchG * sboA;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int t0 = blockIdx.y * TG, t1 = min(27, t0 + TG);
+    const int npx = (X + 7) / 8, npy = (Y + 15) / 16, npz = (Z + P - 1) / P;
+    const int npatch = npx * npy * npz;
+    const uint32_t ncols = rttc::tmem_cols(TG * cin);
+    if (tid == 0) {
+        rttc::mbar_init(bar, 1);
+        rttc::fence_mbar_init();
+    }
+    if (warp == 0) rttc::tmem_alloc(tslot, ncols);
+    rttc::tc_fence_before();
+    __syncthreads();
+    rttc::tc_fence_after();
+    const uint32_t tmem = *tslot;
+    const uint32_t idesc = rttc::idesc_bf16(CONV_TM, cin, 1, 1);
+    bool ok = true;
+    uint32_t phase = 0;
+    for (int pt = blockIdx.x; pt < npatch; pt += gridDim.x) {
+        const int x0 = (pt % npx) * 8, y0 = (pt / npx % npy) * 16, z0 = (pt / (npx * npy)) * P;
+        for (int pr = tid; pr < npl * HALO_V; pr += CONV_THREADS) {
+            const int pl = pr / HALO_V, hv = pr - pl * HALO_V;
+            const int hy = hv / HALO_X, hx = hv - hy * HALO_X;
+            const int gx = x0 - 1 + hx, gy = y0 - 1 + hy, gz = z0 - 1 + pl;
+            const bool inb = gx >= 0 && gx < X && gy >= 0 && gy < Y && gz >= 0 && gz < Z;
+            const __nv_bfloat16* src = inb ? in + ((long)gx + (long)X * (gy + (long)Y * gz)) * in_stride : in;
+            uint8_t* dst = sH + (uint32_t)pr * 16;
+            for (int j = 0; j < kchI; j++) rttc::cp_async16(dst + j * sboB, src + (inb ? j * 8 : 0), inb ? 16u : 0u);
+        }
+        for (int p = 0; p < P; p++) {
+            const int gx = x0 + (tid & 7), gy = y0 + (tid >> 3), gz = z0 + p;
+            const bool inb = gx < X && gy < Y && gz < Z;
+            const __nv_bfloat16* src = inb ? gpre + ((long)gx + (long)X * (gy + (long)Y * gz)) * cout : gpre;
+            uint8_t* dst = sG + (uint32_t)(p * CONV_TM + tid) * 16;
+            for (int j = 0; j < kchG; j++) rttc::cp_async16(dst + j * sboA, src + (inb ? j * 8 : 0), inb ? 16u : 0u);
+        }
+        rttc::cp_async_commit();
+        rttc::cp_async_wait_all();
+        rttc::fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            rttc::tc_fence_after();
+            const uint64_t ad0 = rttc::sdesc(rttc::smem_u32(sG), 128, sboA);
+            const uint64_t bd0 = rttc::sdesc(rttc::smem_u32(sH), HALO_X * 16, sboB);
+            for (int t = t0; t < t1; t++) {
+                const int dx = t % 3, dy = (t / 3) % 3, dz = t / 9;  // offsets + 1
+                const uint32_t dcol = tmem + (uint32_t)((t - t0) * cin);
+                for (int p = 0; p < P; p++)
+                    for (int y = 0; y < 16; y += 2)  // K = 16: the voxels of rows y, y + 1
+                        rttc::mma_bf16(dcol, ad0 + (uint32_t)(p * CONV_TM + y * 8),
+                                       bd0 + (uint32_t)((p + dz) * HALO_V + (y + dy) * HALO_X + dx), idesc,
+                                       (pt != (int)blockIdx.x || p > 0 || y > 0) ? 1u : 0u);
+            }
+            rttc::mma_commit(bar);
+        }
+        // the operands are overwritten by the next patch once these MMAs have finished
+        const bool wt = rttc::mbar_wait(bar, phase);
+        phase ^= 1u;
+        if (!__syncthreads_and(wt)) {
+            ok = false;
+            break;
+        }
+    }
+    if (!ok) {
+        if (tid == 0 && err) atomicExch(err, 1);
+    } else if ((int)blockIdx.x < npatch && warp * 32 < cout) {
+        rttc::tc_fence_after();
+        for (int t = t0; t < t1; t++)
+            for (int c0 = 0; c0 < cin; c0 += 16) {
+                float v[16];
+                rttc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((t - t0) * cin + c0), v);
+                if (tid < cout) {
+                    float4* o = reinterpret_cast<float4*>(dw + ((long)tid * 27 + t) * cin + c0);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        atomicAdd(o + q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+                }
+            }
+    }
+    rttc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) rttc::tmem_dealloc(tmem, ncols);
+}
+
+// dW += the weight gradient of one convolution; dw on a 16-byte boundary, channel counts multiples of 16
+int conv3_dw(rt_ctx* c, const __nv_bfloat16* in, int in_stride, int cin, const __nv_bfloat16* gpre, int cout, int X,
+             int Y, int Z, float* dw, int* err) {
+    if (cin % 16 || cout % 16 || cin > 128 || cout > 128 || in_stride % 8)
+        return rt_fail(c, RT_EINVAL, "conv3_dw: channel counts must be multiples of 16 in [16, 128]");
+    // taps per CTA: at most 256 accumulator columns, so that two CTAs share an SM's TMEM
+    const int TG = 256 / cin < 9 ? 256 / cin : 9, groups = (27 + TG - 1) / TG;
+    // planes per patch: the most that let two CTAs share the shared memory (one loads while the other multiplies),
+    // fewer where that would leave SMs without a patch
+    int P = 4;
+    size_t smem = 0;
+    for (; P >= 1; P /= 2) {
+        size_t op = (size_t)(cout / 8) * P * CONV_TM * 16 + (size_t)(P + 2) * HALO_V * 16 * (cin / 8);
+        const size_t rows = (size_t)16 * P * CONV_TM * 16;  // the 128-row A operand stays inside the allocation
+        smem = 128 + (op > rows ? op : rows);
+        const long np = (long)((X + 7) / 8) * ((Y + 15) / 16) * ((Z + P - 1) / P);
+        if (P == 1 || (smem <= 113 * 1024 && np * groups >= c->sm_count)) break;
+    }
+    const size_t floor_b = 233472 / (512 / rttc::tmem_cols(TG * cin) + 1);  // no more CTAs than TMEM serves
+    if (smem < floor_b) smem = floor_b;
+    const long np = (long)((X + 7) / 8) * ((Y + 15) / 16) * ((Z + P - 1) / P);
+    const long want = (2L * c->sm_count + groups - 1) / groups;
+    const dim3 grid((unsigned)(np < want ? np : want), (unsigned)groups);
+    return rt_launch(c, "unet_conv3_dw", [&] {
+        k_conv3_dw_tc<<<grid, CONV_THREADS, smem, c->stream>>>(in, in_stride, cin, gpre, cout, X, Y, Z, P, TG, dw, err);
+    });
 }
 
 }  // namespace rtu
@@ -531,30 +670,6 @@ __global__ void k_bias_grad(const __nv_bfloat16* __restrict__ gpre, int C, long 
     if (r0 < rows_per_pass) atomicAdd(&sh[c], s);
     __syncthreads();
     for (int q = threadIdx.x; q < C; q += blockDim.x) atomicAdd(&db[q], sh[q]);
-}
-
-// dW[n][tap][c] += sum_v gpre[v][n] * in[v + off(tap)][c]: thread per (n, tap, c) over a voxel chunk
-__global__ void k_conv3_dw(const __nv_bfloat16* __restrict__ in, int in_stride, int cin,
-                           const __nv_bfloat16* __restrict__ gpre, int cout, int X, int Y, int Z, long chunk,
-                           float* __restrict__ dw) {
-    const long nw = (long)cout * 27 * cin;
-    const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (idx >= nw) return;
-    const int c = (int)(idx % cin);
-    const int tap = (int)((idx / cin) % 27);
-    const int n = (int)(idx / (27L * cin));
-    const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-    const long V = (long)X * Y * Z;
-    const long v0 = blockIdx.y * chunk, v1 = min(V, v0 + chunk);
-    float s = 0.f;
-    for (long v = v0; v < v1; v++) {
-        const int x = (int)(v % X), y = (int)((v / X) % Y), z = (int)(v / ((long)X * Y));
-        const int xn = x + dx, yn = y + dy, zn = z + dz;
-        if (xn < 0 || xn >= X || yn < 0 || yn >= Y || zn < 0 || zn >= Z) continue;
-        const float gv = bf(gpre[v * cout + n]);
-        if (gv != 0.f) s += gv * bf(in[((long)xn + (long)X * (yn + (long)Y * zn)) * in_stride + c]);
-    }
-    atomicAdd(&dw[idx], s);
 }
 
 // bf16 weights for the forward pass and tap-flipped transposed weights for the input gradient:

@@ -350,7 +350,7 @@ static void free_hier(rt_hier* h) {
     cudaFree(h->sens); cudaFree(h->ftmp); cudaFree(h->eshell); cudaFree(h->load_nodes); cudaFree(h->load_normal);
     cudaFree(h->Rd); cudaFree(h->Ru); cudaFree(h->fs); cudaFree(h->fs_old); cudaFree(h->x); cudaFree(h->rr);
     cudaFree(h->z); cudaFree(h->p); cudaFree(h->q); cudaFree(h->rold); cudaFree(h->Q); cudaFree(h->partials);
-    cudaFree(h->scal); cudaFree(h->Qgal); cudaFree(h->dinv64); cudaFree(h->dinv32);
+    cudaFree(h->scal); cudaFree(h->Qgal); cudaFree(h->dinv64); cudaFree(h->dinv32); cudaFree(h->ncode);
     if (h->pcg_exec) cudaGraphExecDestroy(h->pcg_exec);
     if (h->pcg_graph) cudaGraphDestroy(h->pcg_graph);
     if (h->pcg_exec_alt) cudaGraphExecDestroy(h->pcg_exec_alt);
@@ -373,7 +373,7 @@ static void ws_sync(rt_hier* w) {
     memcpy(w->st_variant, p->st_variant, sizeof(w->st_variant));
     w->cheby_fused = p->cheby_fused;
     w->cheby_stream = p->cheby_stream;
-    w->dinv64 = p->dinv64; w->dinv32 = p->dinv32;
+    w->dinv64 = p->dinv64; w->dinv32 = p->dinv32; w->ncode = p->ncode;
     for (size_t i = 0; i < w->L.size(); i++) {
         rt_level& a = w->L[i];
         const rt_level& b = p->L[i];
@@ -515,11 +515,9 @@ static int build_hier(rt_ctx* c, const rt_params* p, int nx, int ny, int nz, uin
     RT_CHECK(dalloc(c, &h->KE32_dev, 576));
     RT_CHECK(dalloc(c, &h->dinv64, 6 * (size_t)L0.nv));
     RT_CHECK(dalloc(c, &h->dinv32, 6 * (size_t)L0.nv));
-    {
-        const int zc = rtk::tile_zchunk_default(c, L0.vx, L0.vy, L0.vz);
-        for (int pr = 0; pr < 2; pr++)
-            for (int m = 0; m < 4; m++) h->tune[pr][m] = rt_tile_cfg{1, 4, zc};
-    }
+    RT_CHECK(dalloc(c, &h->ncode, (size_t)L0.nv));
+    for (int pr = 0; pr < 2; pr++)
+        for (int m = 0; m < 4; m++) h->tune[pr][m] = rtk::face_default(c, pr == 1, m, L0.vx, L0.vy, L0.vz);
     RT_CHECK(dalloc(c, &h->rho, L0.ne));
     RT_CHECK(dalloc(c, &h->w, L0.ne));
     RT_CHECK(dalloc(c, &h->vfix, L0.nv));
@@ -1019,13 +1017,26 @@ extern "C" int rt_init_density(rt_hier* h, float rho) {
 // ---------------------------------------------------------------------------
 static int estimate_lmax(rt_hier* h, int lvl);
 
-// element weights rho^p and the inverted diagonal blocks of the finest level
+// the marching kernels (variants 1, 2) smooth with stored inverted diagonal blocks; the others form them
+static bool reads_dinv(const rt_hier* h) {
+    for (int pr = 0; pr < 2; pr++)
+        for (int m = 2; m < 4; m++)
+            if (h->tune[pr][m].variant == 1 || h->tune[pr][m].variant == 2) return true;
+    return false;
+}
+
+// element weights rho^p, node codes and (where a chosen kernel reads them) the inverted diagonal blocks of
+// the finest level
 static int refresh_fine(rt_hier* h) {
     if (h->parent) {  // weights and diagonal blocks belong to the parent (refreshed by its own calls)
         ws_sync(h);
         return RT_OK;
     }
     RT_CHECK(rtk::penalty_weights(h));
+    RT_CHECK(rtk::node_codes(h));
+    h->dinv_ready = false;
+    if (!reads_dinv(h)) return RT_OK;
+    h->dinv_ready = true;
     return rtk::fine_dinv(h);
 }
 
@@ -2485,32 +2496,24 @@ extern "C" int rt_autotune(rt_hier* h, int reps) {
     RT_CUDA(c, cudaMemsetAsync(h->p, 0, sizeof(double) * n, c->stream));
     RT_CUDA(c, cudaMemsetAsync(L.d32, 0, sizeof(float) * n, c->stream));
     if (!h->stencil_ready) RT_CHECK(spare_cheby_table(h));
+    // the face-carrying march, and the tile kernels that were the fastest before it (511x256x256, 255x256x128,
+    // 129x97x85 and 64x32x32: the march won every kernel there, by 1.1 to 2.5 times)
     std::vector<rt_tile_cfg> cands;
-    for (int ty : {2, 4, 8})
-        for (int zc : {4, 8, 16, 32, 64}) cands.push_back(rt_tile_cfg{1, ty, zc});
-    for (int ty : {2, 4})
-        for (int zc : {8, 16, 32}) cands.push_back(rt_tile_cfg{2, ty, zc});
-    for (int ty : {2, 4, 8})
-        for (int zc : {8, 16, 32}) cands.push_back(rt_tile_cfg{0, ty, zc});
-    for (int ty : {2, 4, 8})
-        for (int zc : {8, 16, 32, 64}) cands.push_back(rt_tile_cfg{3, ty, zc});
-    for (int ty : {2, 4, 8})
-        for (int zc : {8, 16, 32, 64}) cands.push_back(rt_tile_cfg{4, ty, zc});  // FP32 only
-    for (int ty : {4, 8, 16})
-        for (int zc : {16, 32, 64}) cands.push_back(rt_tile_cfg{5, ty, zc});  // ty 16: FP32 only
-    if (h->L[0].vx % 16 == 0)  // TMA-staged node layers: the flags' row pitch must be a multiple of 16 bytes
-        for (int v : {6, 7})
-            for (int ty : {4, 6, 8})
-                for (int zc : {8, 16, 32, 64})
-                    if (ty != 6 || v == 7) cands.push_back(rt_tile_cfg{v, ty, zc});
+    for (int ty : {1, 2})  // 2: FP32 only
+        for (int zc : {2, 4, 8, 16, 32, 64}) cands.push_back(rt_tile_cfg{8, ty, zc});
+    cands.push_back(rt_tile_cfg{0, 4, 8});
+    cands.push_back(rt_tile_cfg{3, 8, 16});
+    if (h->L[0].vx % 16 == 0) {  // TMA-staged node layers: the flags' row pitch must be a multiple of 16 bytes
+        cands.push_back(rt_tile_cfg{7, 8, 32});
+        cands.push_back(rt_tile_cfg{7, 6, 64});
+    }
     for (int prec = 0; prec < 2; prec++)
         for (int mode = 0; mode < 4; mode++) {
             rt_tile_cfg best_cfg = h->tune[prec][mode];
             double best = 1e30;
             for (const rt_tile_cfg& cfg : cands) {
                 if (cfg.zchunk > 2 * L.vz && cfg.zchunk != 4) continue;
-                if (cfg.variant == 4 && prec == 1) continue;
-                if (cfg.variant == 5 && cfg.ty == 16 && prec == 1) continue;
+                if (cfg.variant == 8 && cfg.ty == 2 && prec == 1) continue;
                 h->tune[prec][mode] = cfg;
                 const double t = time_fine_kernel(h, prec, mode, reps);
                 if (t < best) { best = t; best_cfg = cfg; }
@@ -2537,11 +2540,14 @@ extern "C" int rt_tuning_info(rt_hier* h, int precision, int mode, int* variant,
 }
 
 extern "C" int rt_set_tuning(rt_hier* h, int precision, int mode, int variant, int ty, int zchunk) {
-    if (!h || precision < 0 || precision > 1 || mode < 0 || mode > 3 || variant < 0 || variant > 7 || zchunk < 1)
+    if (!h || precision < 0 || precision > 1 || mode < 0 || mode > 3 || variant < 0 || variant > 8 || zchunk < 1)
         return RT_EINVAL;
     RT_NOT_WORKSPACE(h);
     if (variant == 4 && precision == RT_FP64) return rt_fail(h->ctx, RT_EINVAL, "variant 4 (packed FP32 pairs) is FP32 only");
-    if (variant == 5) {
+    if (variant == 8) {
+        if (ty != 1 && !(ty == 2 && precision != RT_FP64))
+            return rt_fail(h->ctx, RT_EINVAL, "face-march element rows per warp must be 1 or (FP32) 2");
+    } else if (variant == 5) {
         if (ty != 4 && ty != 8 && ty != 16) return rt_fail(h->ctx, RT_EINVAL, "sum-factorised rows per tile must be 4, 8 or 16");
     } else if (variant == 6 || variant == 7) {
         if (ty != 4 && ty != 8 && !(variant == 7 && ty == 6))
@@ -2553,6 +2559,10 @@ extern "C" int rt_set_tuning(rt_hier* h, int precision, int mode, int variant, i
     if (variant == 2 && ty != 2 && ty != 4) return rt_fail(h->ctx, RT_EINVAL, "prefetching rows per tile must be 2 or 4");
     h->tune[pr][mode] = rt_tile_cfg{variant, ty, zchunk};
     h->graph_epoch++;
+    if (!h->dinv_ready && reads_dinv(h)) {  // the weights' last refresh had no reader for them
+        h->dinv_ready = true;
+        RT_CHECK(rtk::fine_dinv(h));
+    }
     return RT_OK;
 }
 

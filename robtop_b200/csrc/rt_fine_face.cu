@@ -1,0 +1,364 @@
+// rt_fine_face.cu — finest-level operator marching element columns through z, with the transforms of the
+// element vectors shared between neighbours and their partial results carried in registers.
+//
+// Same operators as rt_fine_tile.cu (residual, applyK, damped block Jacobi, Chebyshev step;
+// grid/Grid.cu:1450-1557, 2439-2517).  The operator has few flops per byte, but the tile kernels spend
+// ~880 thread-instructions per node on it (24 shared loads, 24 shared stores and two full 24-point butterflies
+// per element, 24 shared loads per node), and the issue slots bound them, at a third of the HBM rate.  Here:
+//
+//  * The 8-vertex Hadamard transform (KE = T Kt T^T / 64, see rt_element.cuh) is done one axis at a time.  The
+//    x stage of an edge serves 4 elements, the y stage of a face 2 (the element below keeps it in registers for
+//    the element above), only the z stage is per element: 6 + 12 + 24 adds instead of 72, and the same on the
+//    way back, where neighbours' results are added between the stages, so that no scatter remains.
+//  * A lane owns element column X0 - 1 + lane and node column X0 - 1 + lane, a warp R consecutive element rows.
+//    x neighbours meet by shuffles, the rows of a warp in registers.  Only the upper edge of a warp's last row
+//    crosses warps, 6 values (and 2 weight sums) per lane and layer through shared memory, with one barrier per
+//    layer.  Lanes 1..30 finish nodes; a block of W warps finishes 30 x (W R - 1) nodes per layer.
+//  * The loads of the next layer and of this layer's output stage are issued before the arithmetic.
+//  * The 3x3 diagonal block of a node needs four signed sums of its 8 weights, factorised the same way.
+//
+// Fixed and inactive nodes enter the element products as zero (the reference's WS rule); out[] follows
+// rt_fine_tile.cu's rules for them.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "rt_element.cuh"
+#include "rt_internal.h"
+
+namespace {
+
+constexpr int FACE_NX = 30;  // node columns a warp finishes (lanes 1..30)
+
+constexpr int face_warps(bool f64, int mode, int rows) { return f64 ? (mode < 2 ? 12 : 8) : rows == 1 ? 8 : 4; }
+
+template <typename T>
+__device__ __forceinline__ T face_rcp(T x) {
+    if constexpr (sizeof(T) == 4) return __frcp_rn(x);
+    else return T(1) / x;
+}
+
+// MODE 0: r = f - K u (fixed rows: r = f)     MODE 1: out = K u (fixed rows: u)
+// MODE 2: unew = u + omega D^-1 (f - K u)     MODE 3: Chebyshev step kstep: d = a_k d + b_k D^-1 (f - K u), unew = u + d
+// (fixed nodes in MODE 2/3: unew = f / n_e, d = 0; inactive nodes: 0)
+// code: per node, bit 0 active, bit 1 fixed (supports), for fixed nodes n_e << 2
+template <typename T, bool WS, int MODE, int R, int W, int MINB>
+__global__ void __launch_bounds__(32 * W, MINB)
+    k_fine_face(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code, const float* __restrict__ wgt,
+                const rte::KtVals<T> kt, const T* __restrict__ u, const T* __restrict__ f, T* __restrict__ out, T omega,
+                T* __restrict__ dvec, const double* __restrict__ coef, int kstep) {
+    constexpr int NX = MODE >= 2 ? 8 : 6;  // values handed to the next warp
+    __shared__ T S[2][W][NX][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    T cheb_a = T(0), cheb_b = T(0);
+    if (MODE == 3) {
+        cheb_a = (T)coef[2 * kstep];
+        cheb_b = (T)coef[2 * kstep + 1];
+    }
+    const int vx = nx + 1, vy = ny + 1, vz = nz + 1;
+    const int nv = vx * vy * vz, plane = vx * vy, eplane = nx * ny;  // 3 nv < 2^31 (launch_face checks)
+    const int ci = blockIdx.x * FACE_NX - 1 + lane;
+    const int rb = blockIdx.y * (W * R - 1) - 1 + w * R;  // the warp's first element row = first node row
+    const int Z0 = blockIdx.z * zchunk, Z1 = min(Z0 + zchunk, vz);
+    const bool own_col = lane >= 1 && lane <= FACE_NX && ci < vx;
+    bool n_ok[R + 1], e_ok[R];
+#pragma unroll
+    for (int r = 0; r <= R; r++) n_ok[r] = ci >= 0 && ci < vx && rb + r >= 0 && rb + r < vy;
+#pragma unroll
+    for (int r = 0; r < R; r++) e_ok[r] = ci >= 0 && ci < nx && rb + r >= 0 && rb + r < ny;
+
+    T pu[R + 1][3];    // u of the next node layer, as stored
+    uint32_t pc[R + 1];  // its node codes
+    float pw[R];       // weights of the element layer below it
+    // node layer L (index vn of the lane's first node) and element layer L - 1 (index en)
+    auto fetch = [&](int L, int vn, int en) {
+        const bool zn = L >= 0 && L < vz, ze = L >= 1 && L <= nz;
+#pragma unroll
+        for (int r = 0; r <= R; r++) {
+            const int v = vn + r * vx;
+            pc[r] = 0;
+            if (zn && n_ok[r]) {
+                pc[r] = code[v];
+                pu[r][0] = u[v];
+                pu[r][1] = u[nv + v];
+                pu[r][2] = u[2 * nv + v];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) pw[r] = ze && e_ok[r] ? wgt[en + r * nx] : 0.f;
+    };
+    // x stage of node row r: sums and differences along the edge to the next column (active free nodes only)
+    auto x_stage = [&](const T (&p)[3], uint32_t c, T (&E)[6]) {
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const T un = c == 1u ? p[q] : T(0);
+            const T nb = __shfl_down_sync(0xffffffffu, un, 1);
+            E[q] = un + nb;
+            E[3 + q] = un - nb;
+        }
+    };
+
+    T F[R][12];  // forward face data of node layer t
+    T G[R][12];  // inverse z output of element layer t - 1 toward node layer t
+    uint32_t co[R];
+    T Qp[R][4];  // signed weight sums of element layer t - 1
+    int vn = ci + vx * rb + plane * (Z0 - 1);  // node (ci, rb) of layer t
+    int en = ci + nx * rb + eplane * (Z0 - 1);
+    fetch(Z0 - 1, vn, en - eplane);
+    {
+        T E0[6], E1[6];
+        x_stage(pu[0], pc[0], E0);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            x_stage(pu[r + 1], pc[r + 1], E1);
+#pragma unroll
+            for (int q = 0; q < 6; q++) {
+                F[r][q] = E0[q] + E1[q];
+                F[r][6 + q] = E0[q] - E1[q];
+                E0[q] = E1[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 12; q++) G[r][q] = T(0);
+#pragma unroll
+            for (int q = 0; q < 4; q++) Qp[r][q] = T(0);
+            co[r] = 0;
+        }
+    }
+    fetch(Z0, vn + plane, en);
+
+    for (int t = Z0 - 1; t < Z1; t++, vn += plane, en += eplane) {
+        // ---- node layer t + 1 into the x stage, then the loads of layer t + 2
+        T E[R + 1][6];
+        uint32_t cn[R];
+        T wv[R];
+#pragma unroll
+        for (int r = 0; r <= R; r++) x_stage(pu[r], pc[r], E[r]);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            cn[r] = pc[r];
+            wv[r] = (T)pw[r];
+        }
+        if (t + 1 < Z1) fetch(t + 2, vn + 2 * plane, en + eplane);
+        const bool lay = t >= Z0;
+        // ---- element layer t, last row first: X[r] collects the x-edge data of node row r
+        T X[R][6], wa[R], wb[R];
+#pragma unroll
+        for (int r = R - 1; r >= 0; r--) {
+            if (MODE >= 2) {
+                const T wl = __shfl_up_sync(0xffffffffu, wv[r], 1);
+                wa[r] = wv[r] + wl;
+                wb[r] = wv[r] - wl;
+            }
+            T h[24], z[24], Ft[12];
+#pragma unroll
+            for (int q = 0; q < 12; q++) {
+                const T hi = q < 6 ? E[r][q] + E[r + 1][q] : E[r][q - 6] - E[r + 1][q - 6];
+                h[q] = F[r][q] + hi;
+                h[12 + q] = F[r][q] - hi;
+                F[r][q] = hi;
+            }
+            // rows 0..2 of Kt (the rigid translations) are empty; a row's first product initialises it
+#pragma unroll
+            for (int k = 0; k < 45; k++) {
+                if (k == 0 || rte::KT_R[k - 1] != rte::KT_R[k]) z[rte::KT_R[k]] = kt.v[k] * h[rte::KT_C[k]];
+                else z[rte::KT_R[k]] += kt.v[k] * h[rte::KT_C[k]];
+            }
+#pragma unroll
+            for (int q = 0; q < 12; q++) {
+                const T s = q < 3 ? z[12 + q] : z[q] + z[12 + q], d = q < 3 ? -z[12 + q] : z[q] - z[12 + q];
+                Ft[q] = G[r][q] + wv[r] * s;  // toward node layer t, with element layer t - 1's part
+                G[r][q] = wv[r] * d;          // toward node layer t + 1
+            }
+#pragma unroll
+            for (int q = 0; q < 6; q++) {
+                const T up = Ft[q] - Ft[6 + q];
+                X[r][q] = Ft[q] + Ft[6 + q];
+                if (r + 1 < R) X[r + 1 < R ? r + 1 : 0][q] += up;
+                else S[t & 1][w][q][lane] = up;
+            }
+        }
+        // ---- output-stage inputs of node layer t
+        T fv[R][3], dv[R][3], uo[R][3];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int v = vn + r * vx;
+            const bool ld = lay && own_col && co[r] != 0 && (r > 0 || w > 0);
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                fv[r][c] = (MODE != 1 && ld) ? f[c * nv + v] : T(0);
+                dv[r][c] = (MODE == 3 && ld && kstep > 0) ? dvec[c * nv + v] : T(0);
+                uo[r][c] = ((MODE >= 2 || (WS && MODE == 1 && co[r] > 1u)) && ld) ? u[c * nv + v] : T(0);  // in L1: layer t was fetched two layers ago
+            }
+        }
+        if (MODE >= 2) {
+            S[t & 1][w][NX - 2][lane] = wa[R - 1];
+            S[t & 1][w][NX - 1][lane] = wb[R - 1];
+        }
+        __syncthreads();
+        // the other buffer is written in the next iteration; this one again only after that one's barrier
+        T wa_b = T(0), wb_b = T(0);
+        if (w > 0) {
+#pragma unroll
+            for (int q = 0; q < 6; q++) X[0][q] += S[t & 1][w > 0 ? w - 1 : 0][q][lane];
+            if (MODE >= 2) {
+                wa_b = S[t & 1][w > 0 ? w - 1 : 0][NX - 2][lane];
+                wb_b = S[t & 1][w > 0 ? w - 1 : 0][NX - 1][lane];
+            }
+        }
+        // ---- node layer t
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            T acc[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                acc[c] = X[r][c] + X[r][3 + c] + __shfl_up_sync(0xffffffffu, X[r][c] - X[r][3 + c], 1);
+            T Q[4];
+            if (MODE >= 2) {
+                const T ab = r > 0 ? wa[r > 0 ? r - 1 : 0] : wa_b, bb = r > 0 ? wb[r > 0 ? r - 1 : 0] : wb_b;
+                Q[0] = wa[r] + ab;  // sum w
+                Q[1] = wb[r] - bb;  // sum w sx sy
+                Q[2] = wa[r] - ab;  // sum w sy
+                Q[3] = wb[r] + bb;  // sum w sx
+            }
+            if (lay && own_col && n_ok[r] && (r > 0 || w > 0)) {
+                const int v = vn + r * vx;
+                const bool act = co[r] != 0, fixed = WS && co[r] > 1u;
+                T o[3] = {T(0), T(0), T(0)}, dn[3] = {T(0), T(0), T(0)};
+                if (MODE == 0) {
+#pragma unroll
+                    for (int c = 0; c < 3; c++) o[c] = act ? (fixed ? fv[r][c] : fv[r][c] - acc[c]) : T(0);
+                } else if (MODE == 1) {
+#pragma unroll
+                    for (int c = 0; c < 3; c++) o[c] = act ? (fixed ? uo[r][c] : acc[c]) : T(0);
+                } else if (fixed) {
+#pragma unroll
+                    for (int c = 0; c < 3; c++) o[c] = fv[r][c] / T(co[r] >> 2);
+                } else if (act) {
+                    const T sw = Q[0] + Qp[r][0], sxy = Q[1] + Qp[r][1], sxz = Q[3] - Qp[r][3], syz = Q[2] - Qp[r][2];
+                    const T A = kt.diag_a * sw, bxy = kt.diag_b * sxy, bxz = kt.diag_b * sxz, byz = kt.diag_b * syz;
+                    // inverse of [[A,bxy,bxz],[bxy,A,byz],[bxz,byz,A]]
+                    const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
+                    const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
+                    const T id = face_rcp(A * c00 + bxy * c01 + bxz * c02);
+                    T rr[3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) rr[c] = fv[r][c] - acc[c];
+                    const T zz[3] = {id * (c00 * rr[0] + c01 * rr[1] + c02 * rr[2]),
+                                     id * (c01 * rr[0] + c11 * rr[1] + c12 * rr[2]),
+                                     id * (c02 * rr[0] + c12 * rr[1] + c22 * rr[2])};
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        if (MODE == 2) {
+                            o[c] = uo[r][c] + omega * zz[c];
+                        } else {
+                            dn[c] = cheb_a * dv[r][c] + cheb_b * zz[c];  // dv = 0 in step 0
+                            o[c] = uo[r][c] + dn[c];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) out[c * nv + v] = o[c];
+                if (MODE == 3)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) dvec[c * nv + v] = dn[c];
+            }
+            if (MODE >= 2)
+#pragma unroll
+                for (int q = 0; q < 4; q++) Qp[r][q] = Q[q];
+            co[r] = cn[r];
+        }
+    }
+}
+
+// node codes read by k_fine_face: bit 0 active, bit 1 fixed, bits 2.. the number of elements of non-zero weight
+// around a fixed node (its smoothing rule f / n_e)
+__global__ void k_node_code(int nx, int ny, int nz, const uint8_t* __restrict__ vact, const uint8_t* __restrict__ vfix,
+                            const float* __restrict__ w, uint8_t* __restrict__ code) {
+    const int vx = nx + 1, vy = ny + 1;
+    const long nv = (long)vx * vy * (nz + 1);
+    for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += (long)gridDim.x * blockDim.x) {
+        uint8_t c = vact[v] ? 1 : 0;
+        if (c && vfix != nullptr && vfix[v]) {
+            const int x = (int)(v % vx), y = (int)((v / vx) % vy), z = (int)(v / ((long)vx * vy));
+            int ne = 0;
+            for (int i = 0; i < 8; i++) {
+                const int ex = x - 1 + (i & 1), ey = y - 1 + ((i >> 1) & 1), ez = z - 1 + (i >> 2);
+                if (ex >= 0 && ey >= 0 && ez >= 0 && ex < nx && ey < ny && ez < nz &&
+                    w[ex + (long)nx * (ey + (long)ny * ez)] != 0.f)
+                    ne++;
+            }
+            c = (uint8_t)(3 | (ne << 2));
+        }
+        code[v] = c;
+    }
+}
+
+template <typename T, bool WS, int MODE, int R, int W, int MINB>
+int launch_face_rw(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
+                   const double* coef, int kstep) {
+    rt_level& L = h->L[0];
+    const int zc = h->tune[sizeof(T) == 8 ? 1 : 0][MODE].zchunk;
+    const dim3 grid((L.vx + FACE_NX - 1) / FACE_NX, (L.vy + W * R - 2) / (W * R - 1), (L.vz + zc - 1) / zc);
+    const rte::KtVals<T> kt = rte::make_kt<T>(h);
+    return rt_launch(h->ctx, name, [&] {
+        k_fine_face<T, WS, MODE, R, W, MINB><<<grid, 32 * W, 0, h->ctx->stream>>>(
+            L.nx, L.ny, L.nz, zc, h->ncode, h->w, kt, u, f, out, (T)omega, dvec, coef, kstep);
+    });
+}
+
+}  // namespace
+
+namespace rtk {
+
+int node_codes(rt_hier* h) {
+    rt_level& L = h->L[0];
+    return rt_launch(h->ctx, "node_codes", [&] {
+        k_node_code<<<(unsigned)std::min<long>((L.nv + 255) / 256, (long)h->ctx->sm_count * 16), 256, 0,
+                      h->ctx->stream>>>(L.nx, L.ny, L.nz, L.vact, h->has_support ? h->vfix : nullptr, h->w, h->ncode);
+    });
+}
+
+// the block shape of ty element rows per warp (measured on 511x256x256, where a spill costs more than a block):
+// FP32 1 row 8 warps, 2 rows 4 warps; FP64 1 row, 12 warps in one block per SM, 8 where the smoothing step needs
+// the registers (845 us residual and 1526 us Chebyshev step; two blocks of 8 warps with spills: 1287 and 2431 us)
+template <typename T, bool WS, int MODE>
+int launch_face(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
+                const double* coef, int kstep) {
+    if constexpr (sizeof(T) == 8) {
+        constexpr int W = face_warps(true, MODE, 1);
+        return launch_face_rw<T, WS, MODE, 1, W, 1>(h, u, f, out, omega, name, dvec, coef, kstep);
+    } else {
+        if (h->tune[0][MODE].ty == 1)
+            return launch_face_rw<T, WS, MODE, 1, 8, 3>(h, u, f, out, omega, name, dvec, coef, kstep);
+        return launch_face_rw<T, WS, MODE, 2, 4, 4>(h, u, f, out, omega, name, dvec, coef, kstep);
+    }
+}
+
+// the launch shape used before rt_autotune ran: the z-chunk whose waves of blocks march through the fewest layers
+// (a chunk of zc layers takes zc + 2 steps).  64x32x32: 2, 129x97x85: 16, 255x256x128: 16, as the sweep found best
+// or within 5 %
+rt_tile_cfg face_default(rt_ctx* c, bool f64, int mode, int vx, int vy, int vz) {
+    const int r = f64 || mode == 0 ? 1 : 2, w = face_warps(f64, mode, r);
+    const long slots = (long)c->sm_count * (f64 ? 1 : r == 1 ? 3 : 4);
+    const long xy = (long)((vx + FACE_NX - 1) / FACE_NX) * ((vy + w * r - 2) / (w * r - 1));
+    rt_tile_cfg best{8, r, 2};
+    long cost = -1;
+    for (int zc = 2; zc <= 64; zc *= 2) {
+        const long waves = (xy * ((vz + zc - 1) / zc) + slots - 1) / slots, cz = waves * (zc + 2);
+        if (cost < 0 || cz < cost) {
+            cost = cz;
+            best.zchunk = zc;
+        }
+    }
+    return best;
+}
+
+#define RT_INST_FACE(T, WS, M) \
+    template int launch_face<T, WS, M>(rt_hier*, const T*, const T*, T*, double, const char*, T*, const double*, int);
+#define RT_INST_FACE_T(T)                                                                                          \
+    RT_INST_FACE(T, false, 0) RT_INST_FACE(T, false, 1) RT_INST_FACE(T, false, 2) RT_INST_FACE(T, false, 3)        \
+    RT_INST_FACE(T, true, 0) RT_INST_FACE(T, true, 1) RT_INST_FACE(T, true, 2) RT_INST_FACE(T, true, 3)
+RT_INST_FACE_T(float)
+RT_INST_FACE_T(double)
+
+}  // namespace rtk

@@ -1225,11 +1225,15 @@ int launch_pair_ty(rt_hier* h, const float* u, const float* f, float* out, doubl
 // variant 0: two barriers per element layer; 3: software-pipelined, one barrier per layer;
 // 4 (FP32): pipelined with element pairs in packed FP32; 5: sum-factorised row marching (rt_fine_sf.cu);
 // 6: variant 3 with its node layers staged by TMA (node boxes whose x extent is a multiple of 16);
-// 7: variant 6 on 31-node-wide tiles (element rows of 32: whole warps)
+// 7: variant 6 on 31-node-wide tiles (element rows of 32: whole warps); 8: face-carrying column march
+// (rt_fine_face.cu)
 template <typename T, bool WS, int MODE>
 int launch_tile(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec = nullptr,
                 const double* coef = nullptr, int kstep = 0) {
     const rt_tile_cfg& tn = h->tune[sizeof(T) == 8 ? 1 : 0][MODE];
+    // 32-bit node indices: larger boxes take the plain tile below
+    if (tn.variant == 8 && 3 * h->L[0].nv < (1L << 31))
+        return rtk::launch_face<T, WS, MODE>(h, u, f, out, omega, name, dvec, coef, kstep);
     if (tn.variant == 5) return rtk::launch_sf<T, WS, MODE>(h, u, f, out, omega, name, dvec, coef, kstep);
     if ((tn.variant == 6 || tn.variant == 7) && h->L[0].vx % 16 == 0) {
         bool done = false;
@@ -1353,20 +1357,10 @@ int init_tile_kernels(rt_ctx* c) {
     return RT_OK;
 }
 
-// default launch shape (rt_autotune refines it): enough z-chunks for ~4 tiles per SM
-int tile_zchunk_default(rt_ctx* c, int vx, int vy, int vz) {
-    const long tiles = (long)((vx + 29) / 30) * ((vy + 3) / 4);
-    const long target = (long)c->sm_count * 16;  // marching kernel: 4 warps per CTA, ~16 warps per SM
-    long chunks = (target + tiles - 1) / tiles;
-    if (chunks < 1) chunks = 1;
-    int zc = (int)((vz + chunks - 1) / chunks);
-    return zc < 8 ? 8 : zc;
-}
-
 template <typename T>
 static bool use_march(rt_hier* h, int mode) {
     const int v = h->tune[sizeof(T) == 8 ? 1 : 0][mode].variant;
-    return v == 1 || v == 2;  // 1: marching, 2: marching with prefetch (0, 3, 4: tile kernels)
+    return v == 1 || v == 2;  // 1: marching, 2: marching with prefetch (the others: launch_tile)
 }
 
 template <typename T>

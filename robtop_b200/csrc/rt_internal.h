@@ -84,7 +84,8 @@ struct rt_level {
 
 // launch shape of a finest-level operator kernel (chosen by rt_autotune)
 struct rt_tile_cfg {
-    int variant = 1;  // 0: shared-memory element tile (rt_fine_tile.cu), 1: register marching (rt_fine_march.cu),
+    int variant = 8;  // 8: face-carrying column march (rt_fine_face.cu; ty = element rows per warp),
+                      // 0: shared-memory element tile (rt_fine_tile.cu), 1: register marching (rt_fine_march.cu),
                       // 5: sum-factorised row marching (rt_fine_sf.cu; ty = node rows 4, 8 or 16),
                       // 2: register marching with the output-stage loads issued ahead
     int ty = 4;       // node rows per warp tile (marching kernel: 2, 4 or 8)
@@ -112,6 +113,8 @@ struct rt_hier {
     double fused_us[15][2] = {};
     double* dinv64 = nullptr;        // [6][nv] inverted diagonal blocks of the finest level
     float* dinv32 = nullptr;
+    bool dinv_ready = false;         // the diagonal blocks match the weights (made only for kernels that read them)
+    uint8_t* ncode = nullptr;        // [nv] node codes of the finest level: bit 0 active, bit 1 fixed
     std::vector<rt_level> L;
     double KE[576];
     double* KE_dev = nullptr;
@@ -280,9 +283,13 @@ int launch_sf(rt_hier* h, const T* u, const T* f, T* out, double omega, const ch
               int kstep);
 int init_stencil_kernels(rt_ctx* c);
 int fine_dinv(rt_hier* h);
+int node_codes(rt_hier* h);
+template <typename T, bool WS, int MODE>
+int launch_face(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec, const double* coef,
+                int kstep);
 template <typename T, int MODE>
 int fine_march(rt_hier* h, const T* u, const T* f, T* out, double omega, T* dvec, const double* coef, int kstep);
-int tile_zchunk_default(rt_ctx* c, int vx, int vy, int vz);
+rt_tile_cfg face_default(rt_ctx* c, bool f64, int mode, int vx, int vy, int vz);
 // stencil levels
 template <typename T>
 int st_residual(rt_hier* h, int lvl, const T* u, const T* f, T* r);

@@ -7,7 +7,72 @@ pytestmark = pytest.mark.gpu
 if not torch.cuda.is_available():
     pytest.skip("needs a GPU", allow_module_level=True)
 
+import oracle as O  # noqa: E402
 import robtop_b200 as rb  # noqa: E402
+from gpu_common import E, NU, P, rel_err  # noqa: E402
+
+
+def _perforated(nx, ny, nz, seed, sup):
+    """A box with voids and scattered supports, and its oracle hierarchy."""
+    r = np.random.default_rng(seed)
+    eact = (r.random((nz, ny, nx)) < 0.85).astype(np.uint8)
+    rho = ((0.1 + 0.9 * r.random(eact.shape)) * eact).astype(np.float32)
+    vfix = np.zeros((nz + 1, ny + 1, nx + 1), np.uint8)
+    if sup:
+        vfix[0] = 1
+        vfix[r.random(vfix.shape) < 0.03] = 1
+    ctx = rb.Context(0)
+    G = rb.HierarchyGrid(ctx, rb.default_params(mode=rb.MODE_WSFF if sup else rb.MODE_NSFF, youngs_modulus=E,
+                                                poisson_ratio=NU, power_penalty=P))
+    G.genFromBox(eact)
+    G[0].setRho(rho.ravel())
+    G.set_support(vfix)
+    H = O.Hierarchy(eact, rho, vfix if sup else None, p=P, E=E, nu=NU, no_support=not sup)
+    G.update_stencil()
+    H.update_stencil()
+    return ctx, G, H, r
+
+
+# node columns finished per warp 30, node rows per block 7 (FP32, and FP64 smoothing), 11 (FP64): boxes one below,
+# at and above these, and z-chunks that end inside the box, at its end and beyond it
+@pytest.mark.parametrize("nx,ny,nz,rows,zc", [(29, 6, 9, 1, 1), (30, 7, 16, 1, 2), (31, 13, 8, 2, 3), (59, 10, 7, 2, 64),
+                                              (60, 11, 15, 1, 16), (12, 21, 17, 2, 5), (95, 8, 8, 2, 4)])
+@pytest.mark.parametrize("sup", [True, False])
+def test_face_march_edges(nx, ny, nz, rows, zc, sup):
+    ctx, G, H, r = _perforated(nx, ny, nz, nx + ny, sup)
+    L = rb.lib()
+    for prec in (rb.FP64, rb.FP32):
+        for m in range(4):
+            rb._capi.check(L.rt_set_tuning(G.handle, prec, m, 8, 1 if prec == rb.FP64 else rows, zc), ctx.handle)
+    act = np.tile(G[0].getVact(), 3).astype(bool)
+    u = r.standard_normal(3 * G[0].nv)
+    u[~act] = np.nan  # values of nodes without elements are not read into any result
+    f = r.standard_normal(3 * G[0].nv) * act
+    uo = np.where(act, u, 0.0)
+    G[0].setDisplacement(u)
+    G[0].setForce(f)
+    G[0].update_residual()
+    want = [np.zeros_like(u) for _ in range(4)]
+    O.lib().or_fine_residual(H.lv(0), O.ptr(H.KE), O.ptr(uo), O.ptr(f), O.ptr(want[0]))
+    want[1] = H.applyK(uo)
+    ujac, tmp = uo.copy(), np.zeros_like(u)
+    O.lib().or_fine_jacobi(H.lv(0), O.ptr(H.KE), O.ptr(ujac), O.ptr(f), 0.6, O.ptr(tmp))
+    H.set_lmax([G.smoother_lmax(i) for i in range(H.nlev - 1)])
+    d = np.zeros_like(u)
+    O.lib().or_fine_cheby(H.lv(0), O.ptr(H.KE), O.ptr(uo), O.ptr(f), O.ptr(want[3]), O.ptr(d), 0)
+    # FP64: the sums of 8 elements in another order; FP32: the tolerance of the other FP32 kernels' tests
+    assert rel_err(G[0].getResidual(), want[0]) < 1e-11
+    assert rel_err(G[0].applyK(u), want[1]) < 1e-11
+    for smoother, w in ((rb.SMOOTH_JACOBI, ujac), (rb.SMOOTH_CHEBY, want[3])):
+        G[0].setDisplacement(u)
+        G[0].smooth(smoother, 1, 0.6)
+        assert rel_err(G[0].getDisplacement(), w) < 1e-10
+    G[0].setDisplacement(u)
+    for m, w in ((0, want[0]), (1, want[1]), (2, ujac), (3, want[3])):
+        rb._capi.check(L.rt_fine_kernel_f32(G.handle, m, 0.6), ctx.handle)
+        assert rel_err(G[0].getResidual(), w) < 2e-6
+    G.close()
+    ctx.close()
 
 
 # the weight-gradient patches are 8 x 16 voxels by 1 to 4 planes: remainders in each axis, one voxel past a patch,

@@ -36,7 +36,7 @@ REFERENCE_TREE = os.environ.get("ROBTOP_REFERENCE", "/root/reference")
 
 def build() -> bool:
     """Build oracle/_ref/ when the reference tree is present; True if both libraries exist."""
-    if os.path.isdir(REFERENCE_TREE):
+    if os.path.exists(os.path.join(REFERENCE_TREE, "element", "templateMatrix.cpp")):
         subprocess.check_call(["make", "-s", "-C", _HERE, "ref", f"REF={REFERENCE_TREE}"])
     return os.path.exists(KE_LIB) and os.path.exists(KERNELS_LIB)
 

@@ -1150,7 +1150,8 @@ static int estimate_lmax(rt_hier* h, int lvl) {
         return lvl == 0 ? rtk::fine_residual<double>(h, x, zero, out) : rtk::st_residual<double>(h, lvl, x, zero, out);
     };
     auto jacobi = [&](const double* f, double* out) {
-        return lvl == 0 ? rtk::fine_jacobi<double>(h, zero, f, out, 1.0) : rtk::st_jacobi<double>(h, lvl, zero, f, out, 1.0);
+        return lvl == 0 ? rtk::fine_smooth0<double>(h, f, out, 1.0, nullptr, nullptr)
+                        : rtk::st_smooth0<double>(h, lvl, f, out, 1.0, nullptr, nullptr);
     };
     RT_CUDA(c, cudaMemsetAsync(zero, 0, sizeof(double) * n, c->stream));
     RT_CUDA(c, cudaMemsetAsync(vp, 0, sizeof(double) * n, c->stream));
@@ -1187,8 +1188,10 @@ static int level_residual(rt_hier* h, int lvl) {
     return rtk::st_residual<T>(h, lvl, LvlVec<T>::u(L), LvlVec<T>::f(L), LvlVec<T>::r(L));
 }
 
+// zero: u is zero on entry and need not be (it is not read): the first Jacobi or Chebyshev step is D^-1 f alone
 template <typename T>
-static int level_smooth(rt_hier* h, int lvl, int smoother, int sweeps, double omega, bool backward) {
+static int level_smooth(rt_hier* h, int lvl, int smoother, int sweeps, double omega, bool backward,
+                        bool zero = false) {
     rt_level& L = h->L[lvl];
     T* u = LvlVec<T>::u(L);
     T* f = LvlVec<T>::f(L);
@@ -1196,18 +1199,31 @@ static int level_smooth(rt_hier* h, int lvl, int smoother, int sweeps, double om
     const double* coef = cheby_table(h, lvl);
     if (smoother == RT_SMOOTH_CHEBY && sweeps > RT_CHEBY_MAXK)
         return rt_fail(h->ctx, RT_EINVAL, "Chebyshev smoothing takes at most 16 steps");
-    if constexpr (sizeof(T) == 4) {
-        // all steps in one cooperative launch where rt_autotune found that faster (not inside a
-        // batched graph, whose instances run concurrently)
-        if (smoother == RT_SMOOTH_CHEBY && lvl > 0 && sweeps > 0 && ((h->cheby_fused >> lvl) & 1u) &&
-            !h->ctx->batch_capture)
-            return rtk::st_cheby_fused(h, lvl, u, f, tmp, LvlVec<T>::d(L), coef, sweeps);
+    // all steps in one cooperative launch where rt_autotune found that faster (not inside a
+    // batched graph, whose instances run concurrently)
+    const bool fused = sizeof(T) == 4 && smoother == RT_SMOOTH_CHEBY && lvl > 0 && sweeps > 0 &&
+                       ((h->cheby_fused >> lvl) & 1u) && !h->ctx->batch_capture;
+    const bool pointwise = smoother == RT_SMOOTH_JACOBI || smoother == RT_SMOOTH_CHEBY;
+    if (zero && (fused || !pointwise || sweeps == 0)) {
+        RT_CUDA(h->ctx, cudaMemsetAsync(u, 0, sizeof(T) * 3 * L.nv, h->ctx->stream));
+        zero = false;
     }
+    if constexpr (sizeof(T) == 4) {
+        if (fused) return rtk::st_cheby_fused(h, lvl, u, f, tmp, LvlVec<T>::d(L), coef, sweeps);
+    }
+    // from zero the first step may write either vector: the one that leaves the result in u
+    const bool swap = zero && sweeps % 2 == 1;
     for (int s = 0; s < sweeps; s++) {
-        if (smoother == RT_SMOOTH_JACOBI || smoother == RT_SMOOTH_CHEBY) {
+        if (pointwise) {
             // ping-pong u -> tmp -> u
-            const T* src = (s % 2 == 0) ? u : tmp;
-            T* dst = (s % 2 == 0) ? tmp : u;
+            const T* src = ((s % 2 == 0) != swap) ? u : tmp;
+            T* dst = ((s % 2 == 0) != swap) ? tmp : u;
+            if (zero && s == 0) {
+                const double* c0 = smoother == RT_SMOOTH_CHEBY ? coef : nullptr;
+                RT_CHECK(lvl == 0 ? rtk::fine_smooth0<T>(h, f, dst, omega, LvlVec<T>::d(L), c0)
+                                  : rtk::st_smooth0<T>(h, lvl, f, dst, omega, LvlVec<T>::d(L), c0));
+                continue;
+            }
             if (smoother == RT_SMOOTH_CHEBY) {
                 T* d = LvlVec<T>::d(L);
                 if (lvl == 0) RT_CHECK(rtk::fine_cheby<T>(h, src, f, dst, d, coef, s));
@@ -1221,31 +1237,30 @@ static int level_smooth(rt_hier* h, int lvl, int smoother, int sweeps, double om
             else RT_CHECK(rtk::st_gs<T>(h, lvl, u, f, backward));
         }
     }
-    if ((smoother == RT_SMOOTH_JACOBI || smoother == RT_SMOOTH_CHEBY) && (sweeps % 2) == 1)
+    if (pointwise && (sweeps % 2) == 1 && !swap)
         RT_CUDA(h->ctx, cudaMemcpyAsync(u, tmp, sizeof(T) * 3 * L.nv, cudaMemcpyDeviceToDevice, h->ctx->stream));
     return RT_OK;
 }
 
-// the multigrid cycle from level i down (level i's u is the caller's initial guess): smoothing,
+// the multigrid cycle from level i down (level i's u is the caller's initial guess, or zero and not
+// yet written): smoothing,
 // the coarse correction (cycle_gamma times on levels 1 .. cycle_gamma_levels (all when 0) unless
 // the next level is the coarsest, whose solve is exact: gamma = 2 is the W-cycle), smoothing;
 // pre/post mirror each other, so the
 // cycle is symmetric when the smoother is (SGS, Jacobi, Chebyshev)
 template <typename T>
-static int mg_cycle(rt_hier* h, int i, int smoother, int pre, int post, double omega) {
+static int mg_cycle(rt_hier* h, int i, int smoother, int pre, int post, double omega, bool zero) {
     const int nl = (int)h->L.size();
     if (i == nl - 1) return rtk::coarsest_solve<T>(h, LvlVec<T>::f(h->L[i]), LvlVec<T>::u(h->L[i]));
     const int cs = h->P.coarse_sweeps;
     const int npre = (i > 0 && cs > 0) ? cs : pre, npost = (i > 0 && cs > 0) ? cs : post;
-    RT_CHECK(level_smooth<T>(h, i, smoother, npre, omega, false));
+    RT_CHECK(level_smooth<T>(h, i, smoother, npre, omega, false, zero));
     const int gl = h->P.cycle_gamma_levels;
     const int reps = (i > 0 && i + 1 < nl - 1 && h->P.cycle_gamma > 1 && (gl <= 0 || i <= gl)) ? h->P.cycle_gamma : 1;
     for (int g = 0; g < reps; g++) {
         RT_CHECK(level_residual<T>(h, i));
         RT_CHECK(rtk::restrict_<T>(h, i + 1, LvlVec<T>::r(h->L[i]), LvlVec<T>::f(h->L[i + 1])));
-        RT_CUDA(h->ctx,
-                cudaMemsetAsync(LvlVec<T>::u(h->L[i + 1]), 0, sizeof(T) * 3 * h->L[i + 1].nv, h->ctx->stream));
-        RT_CHECK(mg_cycle<T>(h, i + 1, smoother, pre, post, omega));
+        RT_CHECK(mg_cycle<T>(h, i + 1, smoother, pre, post, omega, true));
         RT_CHECK(rtk::prolong_add<T>(h, i, LvlVec<T>::u(h->L[i + 1]), LvlVec<T>::u(h->L[i])));
     }
     return level_smooth<T>(h, i, smoother, npost, omega, smoother == RT_SMOOTH_SGS);
@@ -1253,8 +1268,8 @@ static int mg_cycle(rt_hier* h, int i, int smoother, int pre, int post, double o
 
 // HierarchyGrid::v_cycle (grid/Grid.cpp:1068-1113) over levels l0 .. coarsest
 template <typename T>
-static int vcycle_T(rt_hier* h, int smoother, int pre, int post, double omega, int l0 = 0) {
-    return mg_cycle<T>(h, l0, smoother, pre, post, omega);
+static int vcycle_T(rt_hier* h, int smoother, int pre, int post, double omega, int l0 = 0, bool zero = false) {
+    return mg_cycle<T>(h, l0, smoother, pre, post, omega, zero);
 }
 
 static int read_scalars(rt_hier* h, int first, int count, double* out) {
@@ -1534,8 +1549,7 @@ static int precondition(rt_hier* h, const double* r, double* z, const double* rr
     if (dots_done) *dots_done = false;
     if (h->P.precision == RT_FP32) {
         if (!f32_ready) RT_CHECK(rtk::d2f_scaled(h, n, r, L.f32, rr_dev));
-        RT_CUDA(h->ctx, cudaMemsetAsync(L.u32, 0, sizeof(float) * n, h->ctx->stream));
-        RT_CHECK(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega));
+        RT_CHECK(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 0, true));
         if (dots) {
             RT_CHECK(rtk::f2d_scaled_dot2(h, n, L.u32, z, rr_dev, r, h->rold, dots));
             *dots_done = true;
@@ -1552,14 +1566,11 @@ static int precondition(rt_hier* h, const double* r, double* z, const double* rr
         rt_level& L1 = h->L[1];
         int s = RT_OK;
         auto step = [&](int st) { if (s == RT_OK) s = st; };
-        if (cudaMemsetAsync(z, 0, sizeof(double) * n, h->ctx->stream) != cudaSuccess) s = RT_ECUDA;
-        step(level_smooth<double>(h, 0, h->P.smoother, h->P.pre_sweeps, h->P.jacobi_omega, false));
+        step(level_smooth<double>(h, 0, h->P.smoother, h->P.pre_sweeps, h->P.jacobi_omega, false, true));
         step(level_residual<double>(h, 0));
         step(rtk::d2f_scaled(h, n, L.r, L.r32, rr_dev));
         step(rtk::restrict_<float>(h, 1, L.r32, L1.f32));
-        if (s == RT_OK && cudaMemsetAsync(L1.u32, 0, sizeof(float) * 3 * L1.nv, h->ctx->stream) != cudaSuccess)
-            s = RT_ECUDA;
-        step(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 1));
+        step(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 1, true));
         if (s == RT_OK && cudaMemsetAsync(L.u32, 0, sizeof(float) * n, h->ctx->stream) != cudaSuccess) s = RT_ECUDA;
         step(rtk::prolong_add<float>(h, 0, L1.u32, L.u32));
         step(rtk::f2d_scaled_add(h, n, L.u32, z, rr_dev));
@@ -1575,8 +1586,7 @@ static int precondition(rt_hier* h, const double* r, double* z, const double* rr
         double* saved_u = L.u;
         L.f = const_cast<double*>(r);
         L.u = z;
-        RT_CUDA(h->ctx, cudaMemsetAsync(z, 0, sizeof(double) * n, h->ctx->stream));
-        int s = vcycle_T<double>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega);
+        int s = vcycle_T<double>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 0, true);
         L.f = saved_f;
         L.u = saved_u;
         RT_CHECK(s);
@@ -1804,8 +1814,7 @@ static int pcg32_body(rt_hier* h, cudaGraphConditionalHandle cond, int use_cond)
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
     rt_ctx* c = h->ctx;
-    RT_CUDA(c, cudaMemsetAsync(L.u32, 0, sizeof(float) * n, c->stream));
-    RT_CHECK(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega));
+    RT_CHECK(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 0, true));
     RT_CHECK(rtk::dot32_2(h, n, L.u32, L.f32, h->ro32k, h->scal + 10));
     RT_CHECK(rtk::pcg32_update_p(h, n, h->scal + 10, h->scal + 24, h->p32k, L.u32));
     RT_CHECK(rtk::fine_applyK<float>(h, h->p32k, h->q32k));

@@ -215,6 +215,37 @@ __global__ void __launch_bounds__(ST_BS, sizeof(T) == 8 ? 1 : 3) k_st_split4(int
     }
 }
 
+// one smoothing step from u = 0: out = omega D^-1 f (MODE 2) or out = d = b_0 D^-1 f (MODE 3), D the centre block;
+// it reads 9 of the 243 stencil rows
+template <typename T, int MODE, typename S = T>
+__global__ void __launch_bounds__(128) k_st_diag(long nv, const uint8_t* __restrict__ vact, const S* __restrict__ st,
+                                                 const T* __restrict__ f, T* __restrict__ out, T* __restrict__ d,
+                                                 T omega, const double* __restrict__ coef) {
+    const T scale = MODE == 3 ? (T)coef[1] : omega;
+    const long rs = StAddr<S>::stride(nv);
+    for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += (long)gridDim.x * blockDim.x) {
+        const bool act = vact[v];
+        const S* sb = st + StAddr<S>::base(v);
+        T m[9];
+#pragma unroll
+        for (int i = 0; i < 9; i++) m[i] = st_centre<T>(sb, rs, i);
+        const T f0 = f[v], f1 = f[nv + v], f2 = f[2 * nv + v];
+        T o[3] = {T(0), T(0), T(0)};
+        if (act) {
+            const T A = m[4] * m[8] - m[5] * m[7], B = m[5] * m[6] - m[3] * m[8], Cc = m[3] * m[7] - m[4] * m[6];
+            const T id = T(1) / (m[0] * A + m[1] * B + m[2] * Cc) * scale;
+            o[0] = id * (A * f0 + (m[2] * m[7] - m[1] * m[8]) * f1 + (m[1] * m[5] - m[2] * m[4]) * f2);
+            o[1] = id * (B * f0 + (m[0] * m[8] - m[2] * m[6]) * f1 + (m[2] * m[3] - m[0] * m[5]) * f2);
+            o[2] = id * (Cc * f0 + (m[1] * m[6] - m[0] * m[7]) * f1 + (m[0] * m[4] - m[1] * m[3]) * f2);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            out[q * nv + v] = o[q];
+            if (MODE == 3) d[q * nv + v] = o[q];
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Fused Chebyshev sweeps of a small stencil level: all nsteps steps in one cooperative
 // launch, the steps separated by a grid barrier instead of a kernel boundary.  The coarse
@@ -1090,6 +1121,27 @@ int st_cheby(rt_hier* h, int lvl, const T* u, const T* f, T* unew, T* d, const d
             L.nx, L.ny, L.nz, L.vact, stp<T>(L), u, f, unew, d, T(0), coef, kstep);
     });
 }
+template <typename T>
+int st_smooth0(rt_hier* h, int lvl, const T* f, T* out, double omega, T* d, const double* coef) {
+    rt_level& L = h->L[lvl];
+    const unsigned g = grid_for(h->ctx, L.nv, 128);
+    return rt_launch(h->ctx, sizeof(T) == 8 ? "st_smooth0_f64" : "st_smooth0_f32", [&] {
+        cudaStream_t s = h->ctx->stream;
+        if (use_bf16<T>(h, L)) {
+            if constexpr (sizeof(T) == 4) {
+                if (coef) k_st_diag<T, 3, uint16_t><<<g, 128, 0, s>>>(L.nv, L.vact, L.st16, f, out, d, T(0), coef);
+                else k_st_diag<T, 2, uint16_t><<<g, 128, 0, s>>>(L.nv, L.vact, L.st16, f, out, d, (T)omega, nullptr);
+            }
+        } else if (coef) {
+            k_st_diag<T, 3><<<g, 128, 0, s>>>(L.nv, L.vact, stp<T>(L), f, out, d, T(0), coef);
+        } else {
+            k_st_diag<T, 2><<<g, 128, 0, s>>>(L.nv, L.vact, stp<T>(L), f, out, d, (T)omega, nullptr);
+        }
+    });
+}
+template int st_smooth0<double>(rt_hier*, int, const double*, double*, double, double*, const double*);
+template int st_smooth0<float>(rt_hier*, int, const float*, float*, double, float*, const double*);
+
 // co-resident blocks per SM of the fused kernels (queried once per context): the streaming form
 // in coop_blocks_per_sm, the resident form (RES_SMEM of shared memory per block) in res_blocks_per_sm
 static int coop_blocks(rt_hier* h, bool resident = false) {

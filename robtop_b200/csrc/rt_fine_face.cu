@@ -270,6 +270,65 @@ __global__ void __launch_bounds__(32 * W, MINB)
     }
 }
 
+// The smoothing step from u = 0, where K u needs no evaluation: out = omega D^-1 f (MODE 2) or out = d = b_0 D^-1 f
+// (MODE 3), fixed nodes f / n_e (d = 0).  A thread marches one node column through a z-chunk with the weight sums of
+// the element layer below; 33 B (MODE 2) or 45 B per node in FP32 instead of the full step's 66.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code,
+                                                   const float* __restrict__ wgt, T diag_a, T diag_b,
+                                                   const T* __restrict__ f, T* __restrict__ out, T omega,
+                                                   T* __restrict__ dvec, const double* __restrict__ coef) {
+    const int vx = nx + 1, vy = ny + 1, vz = nz + 1;
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
+    if (x >= vx || y >= vy) return;
+    const T scale = MODE == 3 ? (T)coef[1] : omega;
+    const int Z0 = blockIdx.z * zchunk, Z1 = min(Z0 + zchunk, vz);
+    const long plane = (long)vx * vy, nv = plane * vz, eplane = (long)nx * ny;
+    const long col = x + (long)vx * y, ecol = x + (long)nx * y;
+    const bool x0 = x > 0, x1 = x < nx, y0 = y > 0, y1 = y < ny;
+    T Qp[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 2
+    for (int t = Z0 - 1; t < Z1; t++) {
+        T w00 = T(0), w10 = T(0), w01 = T(0), w11 = T(0);  // element (x - 1 + i, y - 1 + j) of layer t
+        if (t >= 0 && t < nz) {
+            const float* we = wgt + ecol + eplane * t;
+            if (x0 && y0) w00 = (T)we[-1 - nx];
+            if (x1 && y0) w10 = (T)we[-nx];
+            if (x0 && y1) w01 = (T)we[-1];
+            if (x1 && y1) w11 = (T)we[0];
+        }
+        const T a0 = w10 + w00, b0 = w10 - w00, a1 = w11 + w01, b1 = w11 - w01;
+        const T Q[4] = {a1 + a0, b1 - b0, a1 - a0, b1 + b0};  // sums of w, w sx sy, w sy, w sx
+        if (t >= Z0) {
+            const long v = col + plane * t;
+            const uint32_t c = code[v];
+            const T f0 = f[v], f1 = f[nv + v], f2 = f[2 * nv + v];
+            T o[3] = {T(0), T(0), T(0)};
+            if (c == 1u) {
+                const T sw = Q[0] + Qp[0], sxy = Q[1] + Qp[1], sxz = Q[3] - Qp[3], syz = Q[2] - Qp[2];
+                const T A = diag_a * sw, bxy = diag_b * sxy, bxz = diag_b * sxz, byz = diag_b * syz;
+                const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
+                const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
+                const T id = face_rcp(A * c00 + bxy * c01 + bxz * c02) * scale;
+                o[0] = id * (c00 * f0 + c01 * f1 + c02 * f2);
+                o[1] = id * (c01 * f0 + c11 * f1 + c12 * f2);
+                o[2] = id * (c02 * f0 + c12 * f1 + c22 * f2);
+            } else if (c > 1u) {
+                o[0] = f0 / T(c >> 2);
+                o[1] = f1 / T(c >> 2);
+                o[2] = f2 / T(c >> 2);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                out[q * nv + v] = o[q];
+                if (MODE == 3) dvec[q * nv + v] = c == 1u ? o[q] : T(0);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) Qp[q] = Q[q];
+    }
+}
+
 // node codes read by k_fine_face: bit 0 active, bit 1 fixed, bits 2.. the number of elements of non-zero weight
 // around a fixed node (its smoothing rule f / n_e)
 __global__ void k_node_code(int nx, int ny, int nz, const uint8_t* __restrict__ vact, const uint8_t* __restrict__ vfix,
@@ -317,6 +376,26 @@ int node_codes(rt_hier* h) {
                       h->ctx->stream>>>(L.nx, L.ny, L.nz, L.vact, h->has_support ? h->vfix : nullptr, h->w, h->ncode);
     });
 }
+
+// one smoothing step from u = 0: Jacobi (coef null) or the first Chebyshev step
+template <typename T>
+int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const double* coef) {
+    rt_level& L = h->L[0];
+    int zc = 32;  // 1/32 of the weight layers read twice; shorter chunks where blocks are few
+    const long xy = (long)((L.vx + 31) / 32) * ((L.vy + 7) / 8);
+    while (zc > 4 && xy * ((L.vz + zc - 1) / zc) < 8L * h->ctx->sm_count) zc /= 2;
+    const dim3 grid((L.vx + 31) / 32, (L.vy + 7) / 8, (L.vz + zc - 1) / zc);
+    return rt_launch(h->ctx, sizeof(T) == 8 ? "fine_smooth0_f64" : "fine_smooth0_f32", [&] {
+        if (coef)
+            k_fine_diag<T, 3><<<grid, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, zc, h->ncode, h->w, (T)h->KE[0],
+                                                                (T)h->KE[1], f, out, T(0), dvec, coef);
+        else
+            k_fine_diag<T, 2><<<grid, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, zc, h->ncode, h->w, (T)h->KE[0],
+                                                                (T)h->KE[1], f, out, (T)omega, nullptr, nullptr);
+    });
+}
+template int fine_smooth0<double>(rt_hier*, const double*, double*, double, double*, const double*);
+template int fine_smooth0<float>(rt_hier*, const float*, float*, double, float*, const double*);
 
 // the block shape of ty element rows per warp (measured on 511x256x256, where a spill costs more than a block):
 // FP32 1 row 8 warps, 2 rows 4 warps; FP64 1 row, 12 warps in one block per SM, 8 where the smoothing step needs

@@ -98,3 +98,42 @@ def test_unet_weight_gradient_edges(dims):
     assert np.linalg.norm(got - want) / np.linalg.norm(want) < 5e-2 and cos > 0.999
     net.close()
     ctx.close()
+
+
+def _hier(nx, ny, nz, seed, sup=True, skip=1, **kw):
+    """A box with random densities and a clamped face, no oracle level beyond the occupancy."""
+    r = np.random.default_rng(seed)
+    eact = np.ones((nz, ny, nx), np.uint8)
+    rho = (0.1 + 0.9 * r.random(eact.shape)).astype(np.float32)
+    vfix = np.zeros((nz + 1, ny + 1, nx + 1), np.uint8)
+    if sup:
+        vfix[:, :, 0] = 1
+    ctx = rb.Context(0)
+    G = rb.HierarchyGrid(ctx, rb.default_params(mode=rb.MODE_WSFF, youngs_modulus=E, poisson_ratio=NU,
+                                                power_penalty=P, skip_layer1=skip, **kw))
+    G.genFromBox(eact)
+    G[0].setRho(rho.ravel())
+    G.set_support(vfix)
+    return ctx, G, eact, rho, vfix, r
+
+
+# the ratio-4 restriction's block owns 31 coarse columns (124 fine) and 4 rows, and several coarse planes per block
+# once the blocks fill the GPU (the last box); the prolongation marches several cells there
+@pytest.mark.parametrize("dims", [(123, 9, 9), (125, 17, 5), (249, 13, 30), (250, 180, 130)])
+def test_transfer_edges(dims):
+    ctx, G, eact, rho, vfix, r = _hier(*dims, seed=dims[0], sup=False)
+    H = O.Hierarchy(eact, rho, None, p=P, E=E, nu=NU, no_support=True)
+    rf = r.standard_normal(3 * G[0].nv)
+    G[0].setResidual(rf)
+    G[1].restrict_residual()
+    fc = np.zeros(3 * G[1].nv)
+    O.lib().or_restrict(H.lv(0), H.lv(1), O.ptr(rf), O.ptr(fc))
+    assert rel_err(G[1].getForce(), fc) < 1e-13
+    uc, uf = r.standard_normal(3 * G[1].nv), r.standard_normal(3 * G[0].nv)
+    G[1].setDisplacement(uc)
+    G[0].setDisplacement(uf)
+    G[0].prolongate_correction()
+    O.lib().or_prolong_add(H.lv(0), H.lv(1), O.ptr(uc), O.ptr(uf))
+    assert rel_err(G[0].getDisplacement(), uf) < 1e-13
+    G.close()
+    ctx.close()

@@ -58,56 +58,61 @@ __device__ __forceinline__ T st_centre(const S* sb, long rs, int rc) {
     return x;
 }
 
-// sum over the 27 neighbours of A_vk u_k (SKIPSELF: without the centre block)
-template <typename T, typename S, bool SKIPSELF>
-__device__ __forceinline__ void st_node_sum(int x, int y, int z, int vx, int vy, int vz, long nv,
-                                            const S* __restrict__ st, const T* __restrict__ u, long v, T Au[3]) {
-    Au[0] = Au[1] = Au[2] = T(0);
-    const long rs = StAddr<S>::stride(nv);
-    const S* sb = st + StAddr<S>::base(v);
-#pragma unroll
-    for (int k = 0; k < 27; k++) {
-        if (SKIPSELF && k == 13) continue;
-        const int jx = x + k % 3 - 1, jy = y + (k / 3) % 3 - 1, jz = z + k / 9 - 1;
-        if (jx < 0 || jy < 0 || jz < 0 || jx >= vx || jy >= vy || jz >= vz) continue;
-        const long nj = jx + (long)vx * (jy + (long)vy * jz);
-        const T u0 = u[nj], u1 = u[nv + nj], u2 = u[2 * nv + nj];
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            T a0, a1, a2;
-            if (k == 13) {
-                a0 = st_centre<T>(sb, rs, 3 * r); a1 = st_centre<T>(sb, rs, 3 * r + 1); a2 = st_centre<T>(sb, rs, 3 * r + 2);
-            } else {
-                const S* s = sb + (long)(k * 9 + 3 * r) * rs;
-                a0 = (T)st_val(s); a1 = (T)st_val(s + rs); a2 = (T)st_val(s + 2 * rs);
-            }
-            Au[r] += a0 * u0 + a1 * u1 + a2 * u2;
-        }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(ST_BS) k_st_gs(int nx, int ny, int nz, int color, bool backward,
-                                                  const uint8_t* __restrict__ vact, const T* __restrict__ st,
-                                                  T* __restrict__ u, const T* __restrict__ f) {
-    const int vx = nx + 1, vy = ny + 1, vz = nz + 1;
+// one colour of the point-block GS on a stencil level, LPN lanes per node: lane q sums neighbours k = q, q + LPN, ...
+// (the low lane bits count nodes, so that neighbouring lanes read neighbouring columns).  A colour of the levels below
+// the first has tens to hundreds of nodes, where a thread's 27 x 12 loads one after another took 16 us; 4 lanes where
+// the colour's nodes fill the GPU, a warp per node below that: 5 us.
+template <typename T, int LPN>
+__global__ void __launch_bounds__(128) k_st_gs(int vx, int vy, int vz, int color, bool backward,
+                                               const uint8_t* __restrict__ vact, const T* __restrict__ st,
+                                               T* __restrict__ u, const T* __restrict__ f) {
+    constexpr int NPW = 32 / LPN;  // nodes per warp
     const long nv = (long)vx * vy * vz;
     const long rs = StAddr<T>::stride(nv);
     const int px = color & 1, py = (color >> 1) & 1, pz = (color >> 2) & 1;
     const int cx = (vx - px + 1) / 2, cy = (vy - py + 1) / 2, cz = (vz - pz + 1) / 2;
-    const long nc = (long)cx * cy * cz;
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < nc; t += (long)gridDim.x * blockDim.x) {
-        const int x = px + 2 * (int)(t % cx), y = py + 2 * (int)((t / cx) % cy), z = pz + 2 * (int)(t / ((long)cx * cy));
-        const long v = x + (long)vx * (y + (long)vy * z);
-        if (!vact[v]) continue;
-        T Au[3];
-        st_node_sum<T, T, true>(x, y, z, vx, vy, vz, nv, st, u, v, Au);
-        T S[9];
-        const T* sb = st + StAddr<T>::base(v);
+    const int nc = cx * cy * cz;
+    const int lane = threadIdx.x & 31, q = lane / NPW;
+    const int stride = gridDim.x * 4 * NPW;
+    for (int t0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * NPW; t0 < nc; t0 += stride) {
+        const int t = t0 + lane % NPW;
+        T Au[3] = {T(0), T(0), T(0)}, S[9], F[3], uu[3];
+        long v = 0;
+        bool act = false;
+        if (t < nc) {
+            const int x = px + 2 * (t % cx), y = py + 2 * (t / cx % cy), z = pz + 2 * (t / (cx * cy));
+            v = x + (long)vx * (y + (long)vy * z);
+            act = vact[v];
+            const T* sb = st + StAddr<T>::base(v);
+            if (act && q == 0) {
 #pragma unroll
-        for (int i = 0; i < 9; i++) S[i] = st_centre<T>(sb, rs, i);
-        const T F[3] = {f[v], f[nv + v], f[2 * nv + v]};
-        T uu[3] = {u[v], u[nv + v], u[2 * nv + v]};
+                for (int i = 0; i < 9; i++) S[i] = st_centre<T>(sb, rs, i);
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    F[c] = f[c * nv + v];
+                    uu[c] = u[c * nv + v];
+                }
+            }
+            if (act)
+#pragma unroll
+                for (int kk = 0; kk < (27 + LPN - 1) / LPN; kk++) {
+                    const int k = q + LPN * kk;
+                    const int jx = x + k % 3 - 1, jy = y + (k / 3) % 3 - 1, jz = z + k / 9 - 1;
+                    if (k >= 27 || k == 13 || jx < 0 || jy < 0 || jz < 0 || jx >= vx || jy >= vy || jz >= vz) continue;
+                    const long nj = jx + (long)vx * (jy + (long)vy * jz);
+                    const T u0 = u[nj], u1 = u[nv + nj], u2 = u[2 * nv + nj];
+#pragma unroll
+                    for (int r = 0; r < 3; r++) {
+                        const T* s = sb + (long)(k * 9 + 3 * r) * rs;
+                        Au[r] += s[0] * u0 + s[rs] * u1 + s[2 * rs] * u2;
+                    }
+                }
+        }
+#pragma unroll
+        for (int o = NPW; o < 32; o <<= 1)
+#pragma unroll
+            for (int r = 0; r < 3; r++) Au[r] += __shfl_xor_sync(0xffffffffu, Au[r], o);
+        if (!act || q != 0) continue;
         if (!backward) {
             uu[0] = (F[0] - S[1] * uu[1] - S[2] * uu[2] - Au[0]) / S[0];
             uu[1] = (F[1] - S[3] * uu[0] - S[5] * uu[2] - Au[1]) / S[4];
@@ -1107,9 +1112,14 @@ int st_gs(rt_hier* h, int lvl, T* u, const T* f, bool backward) {
         int col = backward ? 7 - cc : cc;
         long ncol = (long)((L.vx - (col & 1) + 1) / 2) * ((L.vy - ((col >> 1) & 1) + 1) / 2) *
                     ((L.vz - ((col >> 2) & 1) + 1) / 2);
+        if (ncol == 0) continue;
         RT_CHECK(rt_launch(h->ctx, LVL_NAME(lvl, sizeof(T) == 8, "st_gs"), [&] {
-            k_st_gs<T><<<grid_for(h->ctx, ncol, ST_BS), ST_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward,
-                                                                                    L.vact, stp<T>(L), u, f);
+            if (ncol * 4 > (long)h->ctx->sm_count * 512)
+                k_st_gs<T, 4><<<grid_for(h->ctx, 4 * ncol, 128), 128, 0, h->ctx->stream>>>(
+                    L.vx, L.vy, L.vz, col, backward, L.vact, stp<T>(L), u, f);
+            else
+                k_st_gs<T, 32><<<grid_for(h->ctx, 32 * ncol, 128), 128, 0, h->ctx->stream>>>(
+                    L.vx, L.vy, L.vz, col, backward, L.vact, stp<T>(L), u, f);
         }));
     }
     return RT_OK;

@@ -23,52 +23,14 @@ __device__ __forceinline__ void load_KE(T* sKE, const T* __restrict__ KEg) {
     __syncthreads();
 }
 
-// Sum over incident elements.  SELF: 0 = include own column block,
-// 1 = skip it and accumulate the diagonal block into S (GS / Jacobi form).
-template <typename T, bool WS, bool DIAG, bool SKIPSELF>
-__device__ __forceinline__ void fine_node_sum(int x, int y, int z, int vx, int vy, int nx, int ny, int nz, long nv,
-                                              const float* __restrict__ w, const uint8_t* __restrict__ vfix,
-                                              const T* __restrict__ u, const T* __restrict__ sKE, T KU[3], T S[9],
-                                              int& ne) {
-    KU[0] = KU[1] = KU[2] = T(0);
-    if (DIAG)
-#pragma unroll
-        for (int i = 0; i < 9; i++) S[i] = T(0);
-    ne = 0;
-#pragma unroll 1
-    for (int i = 0; i < 8; i++) {
-        const int ex = x + (i & 1) - 1, ey = y + ((i >> 1) & 1) - 1, ez = z + (i >> 2) - 1;
-        if (ex < 0 || ey < 0 || ez < 0 || ex >= nx || ey >= ny || ez >= nz) continue;
-        const long e = ex + (long)nx * (ey + (long)ny * ez);
-        const float we = w[e];
-        if (we == 0.f) continue;
-        ne++;
-        const int vi = 7 - i;
-        if (DIAG) {
-#pragma unroll
-            for (int a = 0; a < 3; a++)
-#pragma unroll
-                for (int b = 0; b < 3; b++) S[a * 3 + b] += T(we) * sKE[(vi * 3 + a) * 24 + vi * 3 + b];
-        }
-        T acc[3] = {T(0), T(0), T(0)};
-#pragma unroll
-        for (int vj = 0; vj < 8; vj++) {
-            const long nj = (long)(ex + (vj & 1)) + (long)vx * ((ey + ((vj >> 1) & 1)) + (long)vy * (ez + (vj >> 2)));
-            if (SKIPSELF && vj == vi) continue;
-            if (WS && vfix[nj]) continue;
-            const T u0 = u[nj], u1 = u[nv + nj], u2 = u[2 * nv + nj];
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const T* kr = sKE + (vi * 3 + r) * 24 + vj * 3;
-                acc[r] += kr[0] * u0 + kr[1] * u1 + kr[2] * u2;
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 3; r++) KU[r] += T(we) * acc[r];
-    }
-}
+// the 3 x 21 couplings of an element's vertex 0 to its other vertices (KE rows 0..2); the other vertices' follow by
+// reflection: KE[v][v ^ m][r][c] = s_r s_c KE[0][m][r][c], s_t = -1 where v has bit t, else 1
+template <typename T>
+struct VertexRow {
+    T k[7][3][3];
+    T diag_a, diag_b;  // KE[v][v] = a I + b (s s^T - I)
+};
 
-// MODE 0: r = f - K u (fixed rows: K u = 0); MODE 1: out = K u (fixed rows: u)
 template <typename T>
 __device__ __forceinline__ void block_gs(const T S[9], const T F[3], const T KU[3], T uu[3], bool backward) {
     if (!backward) {
@@ -82,34 +44,82 @@ __device__ __forceinline__ void block_gs(const T S[9], const T F[3], const T KU[
     }
 }
 
-// one colour of the 8-colour point-block GS; colour c = x%2 + 2(y%2) + 4(z%2)
+// one colour of the 8-colour point-block GS; colour c = x%2 + 2(y%2) + 4(z%2).  8 lanes per node, one per incident
+// element (lane = 4 * element + node, 4 nodes of a row per warp): a colour of a small grid has too few nodes to fill
+// the GPU with a thread each, and a lane's 21 loads are all in flight at once.  With the reflected vertex row the 63
+// products take their matrix entries from the kernel parameters, whichever vertex the node is.
+// 64x32x32, FP64: 27 us per colour with a thread per node, 7 us here.
 template <typename T, bool WS>
 __global__ void __launch_bounds__(FINE_BS) k_fine_gs(int nx, int ny, int nz, int color, bool backward,
-                                                      const uint8_t* __restrict__ vact, const float* __restrict__ w,
-                                                      const uint8_t* __restrict__ vfix, const T* __restrict__ KEg,
-                                                      T* __restrict__ u, const T* __restrict__ f) {
-    __shared__ T sKE[576];
-    load_KE(sKE, KEg);
+                                                      const uint8_t* __restrict__ code, const float* __restrict__ w,
+                                                      const VertexRow<T> kr, T* __restrict__ u,
+                                                      const T* __restrict__ f) {
     const int vx = nx + 1, vy = ny + 1, vz = nz + 1;
-    const long nv = (long)vx * vy * vz;
+    const long plane = (long)vx * vy, nv = plane * vz;
     const int px = color & 1, py = (color >> 1) & 1, pz = (color >> 2) & 1;
-    const int cx = (vx - px + 1) / 2, cy = (vy - py + 1) / 2, cz = (vz - pz + 1) / 2;
-    const long nc = (long)cx * cy * cz;
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < nc; t += (long)gridDim.x * blockDim.x) {
-        const int x = px + 2 * (int)(t % cx), y = py + 2 * (int)((t / cx) % cy), z = pz + 2 * (int)(t / ((long)cx * cy));
-        const long v = x + (long)vx * (y + (long)vy * z);
-        if (!vact[v]) continue;
-        T KU[3], S[9];
-        int ne;
-        fine_node_sum<T, WS, true, true>(x, y, z, vx, vy, nx, ny, nz, nv, w, vfix, u, sKE, KU, S, ne);
-        if (WS && vfix[v]) {
+    const unsigned cx = (vx - px + 1) / 2, cy = (vy - py + 1) / 2, cz = (vz - pz + 1) / 2;
+    const unsigned nc = cx * cy * cz;
+    const int lane = threadIdx.x & 31, e = lane >> 2;
+    const int dx = e & 1 ? 1 : -1, dy = e & 2 ? 1 : -1, dz = e & 4 ? 1 : -1;  // the element's side of the node
+    const T sx = T(dx), sy = T(dy), sz = T(dz);
+    const unsigned stride = gridDim.x * (FINE_BS / 8);
+    for (unsigned t0 = blockIdx.x * (FINE_BS / 8) + (threadIdx.x >> 5) * 4; t0 < nc; t0 += stride) {
+        const unsigned t = t0 + (lane & 3);
+        T KU[3] = {T(0), T(0), T(0)}, sw = T(0), F[3], uu[3];
+        uint32_t cd = 0;
+        long v = 0;
+        if (t < nc) {
+            const int x = px + 2 * (int)(t % cx), y = py + 2 * (int)(t / cx % cy), z = pz + 2 * (int)(t / (cx * cy));
+            v = x + (long)vx * y + plane * z;
+            const int ex = x + (dx - 1) / 2, ey = y + (dy - 1) / 2, ez = z + (dz - 1) / 2;
+            float wv = 0.f;
+            if (ex >= 0 && ey >= 0 && ez >= 0 && ex < nx && ey < ny && ez < nz)
+                wv = w[ex + (long)nx * (ey + (long)ny * ez)];
+            cd = code[v];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                F[c] = f[c * nv + v];
+                uu[c] = u[c * nv + v];
+            }
+            if (wv != 0.f) {
+                T p[3][3] = {};
+#pragma unroll
+                for (int m = 1; m < 8; m++) {
+                    const long n = v + (m & 1 ? dx : 0) + (m & 2 ? dy * (long)vx : 0) + (m & 4 ? dz * plane : 0);
+                    const bool fixed = WS && code[n] > 1;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        T un = u[c * nv + n];
+                        if (fixed) un = T(0);
+#pragma unroll
+                        for (int r = 0; r < 3; r++) p[r][c] += kr.k[m - 1][r][c] * un;
+                    }
+                }
+                sw = T(wv);
+                KU[0] = sw * (p[0][0] + sx * (sy * p[0][1] + sz * p[0][2]));
+                KU[1] = sw * (p[1][1] + sy * (sx * p[1][0] + sz * p[1][2]));
+                KU[2] = sw * (p[2][2] + sz * (sx * p[2][0] + sy * p[2][1]));
+            }
+        }
+        T sxy = sw * sx * sy, sxz = sw * sx * sz, syz = sw * sy * sz;
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) {
+#pragma unroll
+            for (int c = 0; c < 3; c++) KU[c] += __shfl_xor_sync(0xffffffffu, KU[c], o);
+            sw += __shfl_xor_sync(0xffffffffu, sw, o);
+            sxy += __shfl_xor_sync(0xffffffffu, sxy, o);
+            sxz += __shfl_xor_sync(0xffffffffu, sxz, o);
+            syz += __shfl_xor_sync(0xffffffffu, syz, o);
+        }
+        if (e != 0 || cd == 0) continue;
+        T S[9] = {kr.diag_a * sw,  kr.diag_b * sxy, kr.diag_b * sxz, kr.diag_b * sxy, kr.diag_a * sw,
+                  kr.diag_b * syz, kr.diag_b * sxz, kr.diag_b * syz, kr.diag_a * sw};
+        if (WS && cd > 1u) {
 #pragma unroll
             for (int i = 0; i < 9; i++) S[i] = T(0);
-            S[0] = S[4] = S[8] = T(ne);
+            S[0] = S[4] = S[8] = T(cd >> 2);
             KU[0] = KU[1] = KU[2] = T(0);
         }
-        T F[3] = {f[v], f[nv + v], f[2 * nv + v]};
-        T uu[3] = {u[v], u[nv + v], u[2 * nv + v]};
         block_gs(S, F, KU, uu, backward);
         u[v] = uu[0]; u[nv + v] = uu[1]; u[2 * nv + v] = uu[2];
     }
@@ -166,13 +176,6 @@ unsigned fine_grid(rt_ctx* c, long n) {
     return (unsigned)(b < cap ? b : cap);
 }
 
-template <typename T>
-const T* KEptr(rt_hier* h);
-template <>
-const double* KEptr<double>(rt_hier* h) { return h->KE_dev; }
-template <>
-const float* KEptr<float>(rt_hier* h) { return h->KE32_dev; }
-
 }  // namespace
 
 namespace rtk {
@@ -189,18 +192,25 @@ template <typename T>
 int fine_gs(rt_hier* h, T* u, const T* f, bool backward) {
     rt_level& L = h->L[0];
     const char* nm = sizeof(T) == 8 ? "fine_gs_f64" : "fine_gs_f32";
+    VertexRow<T> kr;
+    for (int m = 1; m < 8; m++)
+        for (int r = 0; r < 3; r++)
+            for (int c = 0; c < 3; c++) kr.k[m - 1][r][c] = (T)h->KE[r * 24 + 3 * m + c];
+    kr.diag_a = (T)h->KE[0];
+    kr.diag_b = (T)h->KE[1];
     for (int cc = 0; cc < 8; cc++) {
         int col = backward ? 7 - cc : cc;
         long ncol = (long)((L.vx - (col & 1) + 1) / 2) * ((L.vy - ((col >> 1) & 1) + 1) / 2) *
                     ((L.vz - ((col >> 2) & 1) + 1) / 2);
+        if (ncol == 0) continue;
         RT_CHECK(rt_launch(h->ctx, nm, [&] {
-            unsigned g = fine_grid(h->ctx, ncol);
+            unsigned g = fine_grid(h->ctx, 8 * ncol);
             if (h->has_support)
-                k_fine_gs<T, true><<<g, FINE_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, L.vact, h->w,
-                                                                      h->vfix, KEptr<T>(h), u, f);
+                k_fine_gs<T, true><<<g, FINE_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, h->ncode, h->w,
+                                                                      kr, u, f);
             else
-                k_fine_gs<T, false><<<g, FINE_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, L.vact, h->w,
-                                                                       h->vfix, KEptr<T>(h), u, f);
+                k_fine_gs<T, false><<<g, FINE_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, h->ncode, h->w,
+                                                                       kr, u, f);
         }));
     }
     return RT_OK;

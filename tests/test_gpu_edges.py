@@ -137,3 +137,23 @@ def test_transfer_edges(dims):
     assert rel_err(G[0].getDisplacement(), uf) < 1e-13
     G.close()
     ctx.close()
+
+
+# both lane counts of the stencil levels' Gauss-Seidel: a warp per node, and 4 lanes once a colour has ~19k nodes
+@pytest.mark.parametrize("dims", [(20, 12, 10), (130, 98, 98)])
+def test_level_gauss_seidel_lane_counts(dims):
+    ctx, G, eact, rho, vfix, r = _hier(*dims, seed=3, skip=0)
+    H = O.Hierarchy(eact, rho, vfix, p=P, E=E, nu=NU, skip=False)
+    G.update_stencil()
+    st = G[1].getStencil()
+    H.arrs[1]["st"][:] = st
+    u, f = r.standard_normal(3 * G[1].nv), r.standard_normal(3 * G[1].nv)
+    for smoother, back in ((rb.SMOOTH_GS, 0), (rb.SMOOTH_SGS, 1)):
+        G[1].setDisplacement(u)
+        G[1].setForce(f)
+        G[1].smooth(smoother, 1)
+        uo = u.copy()
+        O.lib().or_st_gs(H.lv(1), O.ptr(uo), O.ptr(f), back)
+        assert rel_err(G[1].getDisplacement(), uo) < 1e-10
+    G.close()
+    ctx.close()

@@ -2393,28 +2393,14 @@ extern "C" int rt_sensitivity(rt_hier* h, int filt) {
 extern "C" int rt_oc_update(rt_hier* h, float vgoal, float* lambda_out, int* trials_out) {
     if (!h) return RT_EINVAL;
     RT_NOT_WORKSPACE(h);
-    rt_level& L = h->L[0];
-    RT_CHECK(rtk::oc_maxabs(h, nullptr));
-    double gmax;
-    RT_CHECK(read_scalars(h, 50, 1, &gmax));
-    float lo = 0, hi = (float)gmax, thr = (lo + hi) / 2, V = 2;
-    const double nact = (double)L.n_act_elems;
-    int itn = 0, trials = 0;
-    do {
-        thr = (lo + hi) / 2;
-        RT_CHECK(rtk::oc_try(h, thr, h->ftmp, h->scal + 51));
-        double vs;
-        RT_CHECK(read_scalars(h, 51, 1, &vs));
-        V = (float)(vs / nact);
-        trials++;
-        if (V > vgoal) lo = thr;
-        else if (V < vgoal) hi = thr;
-    } while (std::fabs(V - vgoal) > 1e-4f && itn++ < 30);
-    RT_CHECK(rtk::oc_try(h, thr, h->rho, h->scal + 51));
+    RT_CHECK(rtk::oc_update(h, vgoal, h->scal + 50));
     h->stencil_ready = false;
     h->design_epoch++;
-    if (lambda_out) *lambda_out = thr;
-    if (trials_out) *trials_out = trials;
+    if (!lambda_out && !trials_out) return RT_OK;
+    double r[2];
+    RT_CHECK(read_scalars(h, 50, 2, r));
+    if (lambda_out) *lambda_out = (float)r[0];
+    if (trials_out) *trials_out = (int)r[1];
     return RT_OK;
 }
 

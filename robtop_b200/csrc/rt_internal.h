@@ -353,8 +353,7 @@ int tridiag_max_eig(rt_hier* h, int k, const double* alpha_dev, const double* be
 int sensitivity(rt_hier* h, const double* u);
 int element_compliance(rt_hier* h, const double* u, float* out);
 int filter(rt_hier* h, float radius);
-int oc_try(rt_hier* h, float thr, float* out, double* vol_dev);
-int oc_maxabs(rt_hier* h, float* out_dev);
+int oc_update(rt_hier* h, float vgoal, double* res_dev);  // res: multiplier, trials
 // setup
 int node_active(rt_ctx* c, int nx, int ny, int nz, const uint8_t* eact, uint8_t* vact);
 int coarsen_elements(rt_ctx* c, int nx, int ny, int nz, int ratio, const uint8_t* ef, uint8_t* ec);

@@ -157,3 +157,36 @@ def test_level_gauss_seidel_lane_counts(dims):
         assert rel_err(G[1].getDisplacement(), uo) < 1e-10
     G.close()
     ctx.close()
+
+
+# the filter's shared-memory tiles (32 x 8 x 8 elements, radius up to 3 elements) and the general kernel past them; the
+# OC update's vector loads (element counts with every remainder of 4), the default damping and another
+@pytest.mark.parametrize("dims", [(33, 9, 9), (31, 7, 17), (13, 7, 5), (64, 16, 8)])
+@pytest.mark.parametrize("radius", [1.0, 1.6, 2.0, 3.2, 4.5])
+def test_filter_and_oc_edges(dims, radius):
+    import ctypes as C
+
+    damp = 0.5 if radius < 3 else 0.8
+    ctx, G, eact, rho, vfix, r = _hier(*dims, seed=5, design_step=0.03, damp_ratio=damp)
+    nx, ny, nz = dims
+    act = G[0].getEact()
+    sens = -np.exp(r.standard_normal(rho.size)).astype(np.float32)
+    sens[r.random(rho.size) < 0.05] *= -1
+    G[0].setSens(sens)
+    G[0].filterSensitivity(radius)
+    fo = np.zeros_like(sens)
+    O.lib().or_filter(nx, ny, nz, O.ptr(act), radius, O.ptr(sens), O.ptr(fo))
+    # a tap's FP32 weight 1 - 6 t^2 + 8 t^3 - 3 t^4 is a sum of terms up to 8, contracted on one side: up to 4 roundings
+    # of 2^-24 x 8 = 2e-6; the weights add up to at least 1 (the centre's), and the errors of the taps rarely add
+    assert rel_err(G[0].getSens(), fo) < 1e-5
+    goal = float(rho.mean()) - 0.005
+    G[0].setSens(fo)
+    lam, trials, it = C.c_float(), C.c_int(), np.zeros(1, np.int32)
+    rb._capi.check(rb.lib().rt_oc_update(G.handle, goal, C.byref(lam), C.byref(trials)), ctx.handle)
+    ro, tmp = rho.ravel().copy(), np.zeros(rho.size, np.float32)
+    lo = O.lib().or_oc_update(ro.size, O.ptr(act), None, O.ptr(ro), O.ptr(fo), goal, 0.03, damp, 1e-3, int(act.sum()),
+                              O.ptr(it), O.ptr(tmp))
+    # a power rounded differently moves the volume by 1e-7; the bisection stops at 1e-4 of it
+    assert np.abs(G[0].getRho() - ro).max() <= 1e-4 and abs(lam.value - lo) <= 1e-3 * abs(lo)
+    G.close()
+    ctx.close()

@@ -4,8 +4,8 @@
 // factors it on the host with Eigen::BDCSVD (Grid::buildCoarsestSystem,
 // grid/Grid.cpp:1884-1939), then does a D2H / svd.solve / H2D round trip every
 // V-cycle (Grid::solve_fem_host, grid/Grid.cpp:1981-2043).  Here the dense
-// matrix is assembled, inverted (Gauss-Jordan, one cooperative launch with a
-// grid barrier per pivot) and applied (GEMV) without leaving the GPU.
+// matrix is assembled, inverted (blocked Gauss-Jordan, one cooperative launch with a
+// grid barrier per 32 pivots) and applied (GEMV) without leaving the GPU.
 // Without supports the matrix is singular with the rigid modes as null space;
 // the minimum-norm solve of BDCSVD is reproduced as A^+ = (A + a R R^T)^-1 - R R^T / a.
 #include <cooperative_groups.h>
@@ -58,44 +58,122 @@ __global__ void k_trace(int n, const double* __restrict__ A, double* __restrict_
     if (threadIdx.x == 0) out[0] = sh[0] / n;
 }
 
-// In-place Gauss-Jordan inversion of an SPD matrix (no pivoting needed).
-// colbuf/rowbuf hold the pivot column and row of the current step; the
-// threads that produce the next step's column/row write them during the
-// update, so one grid barrier per step suffices.  status[0] != 0 reports a
-// non-positive pivot.
-__global__ void k_gauss_jordan(int n, double* __restrict__ A, double* __restrict__ colbuf,
-                               double* __restrict__ rowbuf, int* __restrict__ status) {
+// In-place blocked Gauss-Jordan inversion of an SPD matrix (no pivoting needed), one grid barrier per GJ_B columns.
+// With the step's panels C = A(:, K), R = A(K, :) as they were and P = A(K, K)^-1, every tile is independent:
+//   A(i, j) -= (C_i P) R_j,  A(K, j) = P R_j,  A(i, K) = -C_i P,  A(K, K) = P.
+// Every block inverts the 32 x 32 pivot block itself (cheaper than a second barrier), takes strips of one tile row,
+// so that C_i P is formed once per strip, and writes the parts of the next step's panels that it updated into the
+// other pair of panel buffers.  status[0] != 0 reports a non-positive pivot.  n = 1260: a barrier and a pass over
+// the matrix per column took 14.6 ms, 0.4 ms here.
+constexpr int GJ_B = 32, GJ_T = 256;
+
+__global__ void __launch_bounds__(GJ_T) k_gauss_jordan(int n, double* __restrict__ A, double* __restrict__ panels,
+                                                       int* __restrict__ status) {
     cg::grid_group grid = cg::this_grid();
-    const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const long nth = (long)gridDim.x * blockDim.x;
-    const long nn = (long)n * n;
-    // step 0 buffers
-    for (long i = tid; i < n; i += nth) {
-        colbuf[i] = A[i * n + 0];
-        rowbuf[i] = A[i];
+    __shared__ double P[GJ_B][GJ_B + 1], Ct[GJ_B][GJ_B + 1], W[GJ_B][GJ_B + 1], Rt[GJ_B][GJ_B];
+    __shared__ int bad;
+    const int tid = threadIdx.x, lane = tid & 31, wr = (tid >> 5) * 4;  // a thread's column and first of its 4 rows
+    const int nb = (n + GJ_B - 1) / GJ_B;
+    const long pn = (long)n * GJ_B;  // one panel: C [n][32], R [32][n]
+    const int strips = (int)gridDim.x / nb > 0 ? (int)gridDim.x / nb : 1;  // per tile row
+    const int per = (nb + strips - 1) / strips;                           // tiles of a strip
+    const int items = nb * strips;
+    for (long t = blockIdx.x * (long)GJ_T + tid; t < pn; t += (long)gridDim.x * GJ_T) {
+        const int i = (int)(t / GJ_B), k = (int)(t % GJ_B);
+        panels[t] = k < n ? A[(long)i * n + k] : 0.0;
+        panels[pn + t] = t / n < n ? A[t] : 0.0;  // rows 0..31
     }
     grid.sync();
-    for (int k = 0; k < n; k++) {
-        const double* col = colbuf + (long)(k & 1) * n;
-        const double* row = rowbuf + (long)(k & 1) * n;
-        double* ncol = colbuf + (long)((k + 1) & 1) * n;
-        double* nrow = rowbuf + (long)((k + 1) & 1) * n;
-        const double pivot = row[k];
-        if (!(pivot > 0)) {
-            if (tid == 0) status[0] = k + 1;
-            return;  // uniform across the grid: every thread read the same pivot
+    for (int kb = 0; kb < nb; kb++) {
+        const double *C = panels + 2 * pn * (kb & 1), *R = C + pn;
+        double *Cn = panels + 2 * pn * ((kb + 1) & 1), *Rn = Cn + pn;
+        const int k0 = kb * GJ_B, kw = min(GJ_B, n - k0);
+        // P = inverse of the pivot block (the identity past the matrix's end)
+        for (int i = tid; i < GJ_B * GJ_B; i += GJ_T) {
+            const int r = i / GJ_B, c = i % GJ_B;
+            P[r][c] = r < kw && c < kw ? C[(long)(k0 + r) * GJ_B + c] : (r == c ? 1.0 : 0.0);
         }
-        const double ip = 1.0 / pivot;
-        for (long t = tid; t < nn; t += nth) {
-            const int i = (int)(t / n), j = (int)(t % n);
-            double v;
-            if (i == k && j == k) v = ip;
-            else if (i == k) v = row[j] * ip;
-            else if (j == k) v = -col[i] * ip;
-            else v = A[t] - col[i] * row[j] * ip;
-            A[t] = v;
-            if (j == k + 1) ncol[i] = v;
-            if (i == k + 1) nrow[j] = v;
+        if (tid == 0) bad = 0;
+        __syncthreads();
+        for (int k = 0; k < kw; k++) {
+            const double pv = P[k][k];
+            double row = P[k][lane], col[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) col[q] = P[wr + q][k];
+            if (!(pv > 0)) {
+                if (tid == 0) bad = k0 + k + 1;
+                break;  // uniform: every thread of every block reads the same pivot
+            }
+            const double ip = 1.0 / pv;
+            row *= ip;
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int r = wr + q;
+                if (r == k) P[r][lane] = lane == k ? ip : row;
+                else P[r][lane] = lane == k ? -col[q] * ip : P[r][lane] - col[q] * row;
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+        if (bad != 0) {
+            if (blockIdx.x == 0 && tid == 0) status[0] = bad;
+            return;
+        }
+        for (int it = blockIdx.x; it < items; it += gridDim.x) {
+            const int ib = it / strips, j0 = (it - ib * strips) * per, j1 = min(j0 + per, nb);
+            const int i0 = ib * GJ_B;
+            if (j0 >= j1) continue;
+            __syncthreads();
+            if (ib == kb) {  // this tile row becomes P R_j
+                for (int i = tid; i < GJ_B * GJ_B; i += GJ_T) W[i / GJ_B][i % GJ_B] = P[i / GJ_B][i % GJ_B];
+            } else {  // W = C_i P
+                for (int i = tid; i < GJ_B * GJ_B; i += GJ_T) {
+                    const int r = i / GJ_B, c = i % GJ_B;
+                    Ct[r][c] = i0 + r < n && c < kw ? C[(long)(i0 + r) * GJ_B + c] : 0.0;
+                }
+                __syncthreads();
+                double w[4] = {0, 0, 0, 0};
+                for (int k = 0; k < GJ_B; k++) {
+                    const double b = P[k][lane];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) w[q] += Ct[wr + q][k] * b;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) W[wr + q][lane] = w[q];
+            }
+            for (int jb = j0; jb < j1; jb++) {
+                const int j = jb * GJ_B + lane;
+                __syncthreads();
+                for (int i = tid; i < GJ_B * GJ_B; i += GJ_T) {
+                    const int r = i / GJ_B, c = i % GJ_B;
+                    Rt[r][c] = r < kw && jb * GJ_B + c < n ? R[(long)r * n + jb * GJ_B + c] : 0.0;
+                }
+                double a[4], s[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    a[q] = ib != kb && jb != kb && i0 + wr + q < n && j < n ? A[(long)(i0 + wr + q) * n + j] : 0.0;
+                __syncthreads();
+                if (jb == kb) {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) s[q] = W[wr + q][lane];
+                } else {
+                    for (int k = 0; k < GJ_B; k++) {
+                        const double b = Rt[k][lane];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) s[q] += W[wr + q][k] * b;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int i = i0 + wr + q;
+                    if (i >= n || j >= n) continue;
+                    const double v = ib == kb ? s[q] : a[q] - s[q];
+                    A[(long)i * n + j] = v;
+                    if (jb == kb + 1) Cn[(long)i * GJ_B + lane] = v;
+                    if (ib == kb + 1) Rn[(long)(wr + q) * n + j] = v;
+                }
+            }
         }
         grid.sync();
     }
@@ -164,11 +242,10 @@ int coarsest_setup(rt_hier* h) {
     RT_CUDA(c, cudaStreamSynchronize(c->stream));
     for (int i = 0; i < na; i++) rowof_h[aidx_h[i]] = i;
     int* rowof = nullptr;
-    double *colbuf = nullptr, *rowbuf = nullptr, *R = nullptr;
+    double *panels = nullptr, *R = nullptr;
     int* status = nullptr;
     RT_CUDA(c, cudaMallocAsync(&rowof, sizeof(int) * L.nv, c->stream));
-    RT_CUDA(c, cudaMallocAsync(&colbuf, sizeof(double) * 2 * n, c->stream));
-    RT_CUDA(c, cudaMallocAsync(&rowbuf, sizeof(double) * 2 * n, c->stream));
+    RT_CUDA(c, cudaMallocAsync(&panels, sizeof(double) * 4 * GJ_B * n, c->stream));
     RT_CUDA(c, cudaMallocAsync(&status, sizeof(int), c->stream));
     RT_CUDA(c, cudaMemcpyAsync(rowof, rowof_h.data(), sizeof(int) * L.nv, cudaMemcpyHostToDevice, c->stream));
     RT_CUDA(c, cudaMemsetAsync(status, 0, sizeof(int), c->stream));
@@ -210,17 +287,17 @@ int coarsest_setup(rt_hier* h) {
     }
     // cooperative Gauss-Jordan
     int dev = c->device, nb_per_sm = 0;
-    RT_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb_per_sm, k_gauss_jordan, 256, 0));
+    RT_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb_per_sm, k_gauss_jordan, GJ_T, 0));
     int coop = 0;
     RT_CUDA(c, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop || nb_per_sm < 1) return rt_fail(c, RT_ECUDA, "cooperative launch unavailable");
-    unsigned gblocks = (unsigned)std::min<long>((long)c->sm_count * std::min(nb_per_sm, 2), ((long)n * n + 255) / 256);
-    if (gblocks < 1) gblocks = 1;
+    const long tiles = (long)((n + GJ_B - 1) / GJ_B) * ((n + GJ_B - 1) / GJ_B);
+    const unsigned gblocks = (unsigned)std::min<long>((long)c->sm_count * std::min(nb_per_sm, 2), tiles);
     double* Aptr = L.ainv;
     int nn_ = n;
-    void* args[] = {&nn_, &Aptr, &colbuf, &rowbuf, &status};
+    void* args[] = {&nn_, &Aptr, &panels, &status};
     RT_CHECK(rt_launch(c, "coarsest_gauss_jordan", [&] {
-        cudaLaunchCooperativeKernel((void*)k_gauss_jordan, gblocks, 256, args, 0, c->stream);
+        cudaLaunchCooperativeKernel((void*)k_gauss_jordan, gblocks, GJ_T, args, 0, c->stream);
     }));
     if (no_support) {
         RT_CHECK(rt_launch(c, "coarsest_sub_rrt",
@@ -230,8 +307,7 @@ int coarsest_setup(rt_hier* h) {
     int st_h = 0;
     RT_CUDA(c, cudaMemcpyAsync(&st_h, status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     RT_CUDA(c, cudaFreeAsync(rowof, c->stream));
-    RT_CUDA(c, cudaFreeAsync(colbuf, c->stream));
-    RT_CUDA(c, cudaFreeAsync(rowbuf, c->stream));
+    RT_CUDA(c, cudaFreeAsync(panels, c->stream));
     RT_CUDA(c, cudaFreeAsync(status, c->stream));
     RT_CUDA(c, cudaStreamSynchronize(c->stream));
     if (st_h != 0) return rt_fail(c, RT_ENAN, "coarsest matrix not positive definite (pivot %d)", st_h - 1);

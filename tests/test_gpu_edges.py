@@ -190,3 +190,33 @@ def test_filter_and_oc_edges(dims, radius):
     assert np.abs(G[0].getRho() - ro).max() <= 1e-4 and abs(lam.value - lo) <= 1e-3 * abs(lo)
     G.close()
     ctx.close()
+
+
+# the blocked inverse of the coarsest matrix: n = 3 (nodes) below, at and above multiples of its 32-column blocks,
+# against the solve of the assembled matrix
+@pytest.mark.parametrize("dims,limit", [((5, 4, 4), 4), ((9, 5, 4), 30), ((8, 8, 4), 60), ((31, 17, 9), 100),
+                                        ((40, 24, 24), 400)])
+def test_coarsest_inverse_block_edges(dims, limit):
+    ctx, G, eact, rho, vfix, r = _hier(*dims, seed=2, coarsest_elements=limit)
+    G.update_stencil()
+    g = G[G.n_grid() - 1]
+    nv, vx, vy, vz = g.nv, g.nx + 1, g.ny + 1, g.nz + 1
+    st = g.getStencil().reshape(27, 3, 3, vz, vy, vx)
+    A = np.zeros((nv, 3, nv, 3))
+    ids = np.arange(nv).reshape(vz, vy, vx)
+    for k in range(27):
+        d = (k // 9 - 1, k // 3 % 3 - 1, k % 3 - 1)
+        a = tuple(slice(max(0, -s), n - max(0, s)) for s, n in zip(d, (vz, vy, vx)))
+        b = tuple(slice(max(0, s), n - max(0, -s)) for s, n in zip(d, (vz, vy, vx)))
+        i, j = ids[a].ravel(), ids[b].ravel()
+        A[i, :, j, :] = st[(k, slice(None), slice(None)) + a].reshape(3, 3, -1).transpose(2, 0, 1)
+    A = A.reshape(3 * nv, 3 * nv)
+    f = r.standard_normal((3, nv))
+    want = np.linalg.solve(A, f.T.ravel()).reshape(nv, 3).T
+    g.setForce(f.ravel())
+    g.solve_fem_host()
+    got = g.getDisplacement().reshape(3, nv)
+    # two FP64 inversions differ by about eps cond(A)
+    assert np.abs(got - want).max() <= 1e-14 * np.linalg.cond(A) * np.abs(want).max() + 1e-12 * np.abs(want).max()
+    G.close()
+    ctx.close()

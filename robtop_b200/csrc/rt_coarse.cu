@@ -856,146 +856,196 @@ __global__ void __launch_bounds__(ST_BS) k_prolong(int fvx, int fvy, int fvz, in
 }
 
 // ---------------------------------------------------------------------------
-// Galerkin assembly of the first coarse level directly from the elements:
-// for every coarse cell M = sum_e rho_e^p Q_pos(e), Q_pos = P_pos^T KE P_pos,
-// then M's 3x3 blocks are added into the 8 corner nodes' stencils.  Cells are
-// processed in 8 parity colours so no two cells of one launch share a node
-// (deterministic, no atomics).  Elements touching a fixed node take the
-// Dirichlet form of grid/Grid.cu:465-490 and are computed explicitly.
+// Galerkin assembly of the first coarse level directly from the elements: a coarse cell's matrix is
+// M = sum_pos w_pos Q_pos, Q_pos = P_pos^T KE P_pos over its R^3 element positions, and the stencil of a node is the
+// sum of its row blocks of the 8 cells around it.  k_galerkin_nodes computes it by nodes: the 8 corners of a cell
+// partition the rows of M, so nothing is computed twice, and every stencil entry is written once, coalesced.  A block
+// owns 32 x 2 nodes (x, y) of a layer with the weights of the 33 x 3 x 2 cells around them in shared memory; lane =
+// node column, and a warp owns whole neighbours k (8 cell-neighbour pairs each), so that a Q block is loaded once for
+// 64 nodes.  FP64 FMA bound (576 R^3 per node).  Elements touching a fixed node have weight 0 here and are added by
+// k_galerkin_fixed.  160x144x96: 4.5 ms with cell matrices scattered through 8 colours, 0.25 ms here.
 // ---------------------------------------------------------------------------
-constexpr int GAL_CELLS = 8;
-constexpr int GAL_BS = 288;  // 2 entries of the 576-entry cell matrix per thread
+constexpr int GN_BS = 256;
+
+// neighbour k of warp w: the centre (8 cells), 2 faces (4 each), 4 edges (2 each), 8 corners (1 each); -1 ends a list
+__constant__ int8_t GN_K[8][9] = {{13, -1, -1, -1, -1, -1, -1, -1, -1}, {4, 22, -1, -1, -1, -1, -1, -1, -1},
+                                  {10, 16, -1, -1, -1, -1, -1, -1, -1}, {12, 14, -1, -1, -1, -1, -1, -1, -1},
+                                  {1, 3, 5, 7, -1, -1, -1, -1, -1},     {9, 11, 15, 17, -1, -1, -1, -1, -1},
+                                  {19, 21, 23, 25, -1, -1, -1, -1, -1}, {0, 2, 6, 8, 18, 20, 24, 26, -1}};
 
 __device__ __forceinline__ double interp_w(int off, int corner, int R) {
     return (double)(R - abs(off - R * corner)) / (double)R;
 }
 
+// Qp: [corner m][corner n][pos][10] (9 entries of block (m, n) of Q_pos, one of padding)
 template <int R>
-__global__ void __launch_bounds__(GAL_BS) k_galerkin_cells(int fnx, int fny, int fnz, int cnx, int cny, int cnz,
-                                                           int color, const uint8_t* __restrict__ ceact,
-                                                           const float* __restrict__ w,
-                                                           const uint8_t* __restrict__ vfix,
-                                                           const double* __restrict__ Q, const double* __restrict__ KEg,
-                                                           double* __restrict__ st) {
-    constexpr int NP = R * R * R;
-    __shared__ double sw[GAL_CELLS][NP];
-    __shared__ int scell[GAL_CELLS];
-    __shared__ int sfixed[GAL_CELLS];
+__global__ void __launch_bounds__(GN_BS) k_galerkin_nodes(int fnx, int fny, int fnz, int cnx, int cny, int cnz,
+                                                          const float* __restrict__ w, const double* __restrict__ Qp,
+                                                          double* __restrict__ st) {
+    constexpr int NP = R * R * R, CX = 33, CW = CX * 3 * 2;
+    extern __shared__ double sw[];  // [NP][2 z][3 y][33 x]
+    const int cvx = cnx + 1, cvy = cny + 1, cvz = cnz + 1;
+    const long nvc = (long)cvx * cvy * cvz;
+    const int X0 = blockIdx.x * 32, Y0 = blockIdx.y * 2, Z = blockIdx.z;
+    for (int i = threadIdx.x; i < CX * R * 3 * R * 2 * R; i += GN_BS) {
+        const int ix = i % (CX * R), iy = i / (CX * R) % (3 * R), iz = i / (CX * R * 3 * R);
+        const int ex = R * (X0 - 1) + ix, ey = R * (Y0 - 1) + iy, ez = R * (Z - 1) + iz;
+        double v = 0;
+        if (ex >= 0 && ey >= 0 && ez >= 0 && ex < fnx && ey < fny && ez < fnz)
+            v = fmaxf(w[ex + (long)fnx * (ey + (long)fny * ez)], 0.f);  // a NaN density is left to the solve to report
+        const int pos = ix % R + R * (iy % R + R * (iz % R));
+        sw[pos * CW + (iz / R * 3 + iy / R) * CX + ix / R] = v;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int li = 0; li < 8; li++) {
+        const int k = GN_K[wid][li];
+        if (k < 0) break;
+        const int kx = k % 3 - 1, ky = k / 3 % 3 - 1, kz = k / 9 - 1;
+        double acc[2][9];
+#pragma unroll
+        for (int q = 0; q < 9; q++) acc[0][q] = acc[1][q] = 0;
+        for (int m = 0; m < 8; m++) {  // the node is corner m of the cell, its neighbour corner n
+            const int nxb = (m & 1) + kx, nyb = ((m >> 1) & 1) + ky, nzb = (m >> 2) + kz;
+            if (nxb < 0 || nxb > 1 || nyb < 0 || nyb > 1 || nzb < 0 || nzb > 1) continue;
+            const double2* q2 = reinterpret_cast<const double2*>(Qp + ((m * 8 + nxb + 2 * nyb + 4 * nzb) * (long)NP) * 10);
+            const double* wc = sw + ((1 - (m >> 2)) * 3 + 1 - ((m >> 1) & 1)) * CX + lane + 1 - (m & 1);
+#pragma unroll 4
+            for (int pos = 0; pos < NP; pos++) {
+                const double2 a = q2[5 * pos], b = q2[5 * pos + 1], c = q2[5 * pos + 2], d = q2[5 * pos + 3],
+                              e = q2[5 * pos + 4];
+                const double w0 = wc[pos * CW], w1 = wc[pos * CW + CX];
+                const double q[9] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x};
+#pragma unroll
+                for (int t = 0; t < 9; t++) {
+                    acc[0][t] += w0 * q[t];
+                    acc[1][t] += w1 * q[t];
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            if (X0 + lane >= cvx || Y0 + j >= cvy) continue;
+            const long v = X0 + lane + (long)cvx * (Y0 + j + (long)cvy * Z);
+#pragma unroll
+            for (int t = 0; t < 9; t++) st[(long)(k * 9 + t) * nvc + v] = acc[j][t];
+        }
+    }
+}
+
+// the weights without the elements that touch a fixed node, and flags of the cells that hold such elements
+template <int R>
+__global__ void k_free_weights(int nx, int ny, int nz, int cnx, int cny, const float* __restrict__ w,
+                               const uint8_t* __restrict__ vfix, float* __restrict__ wfree,
+                               uint8_t* __restrict__ cfix) {
+    const int vx = nx + 1, vy = ny + 1;
+    const long ne = (long)nx * ny * nz;
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < ne; e += (long)gridDim.x * blockDim.x) {
+        const int x = (int)(e % nx), y = (int)((e / nx) % ny), z = (int)(e / ((long)nx * ny));
+        const long v = x + (long)vx * (y + (long)vy * z);
+        bool fx = false;
+#pragma unroll
+        for (int j = 0; j < 8; j++) fx |= vfix[v + (j & 1) + (j & 2 ? vx : 0) + (j & 4 ? (long)vx * vy : 0)] != 0;
+        const float we = w[e];
+        wfree[e] = fx ? 0.f : we;
+        if (fx && we != 0.f) cfix[x / R + (long)cnx * (y / R + (long)cny * (z / R))] = 1;
+    }
+}
+
+// adds the elements with fixed nodes in their Dirichlet form K' (grid/Grid.cu:465-490): rows and columns of fixed nodes
+// dropped, 1e6 on the fixed diagonal; P^T K' P of an element is T = K' P, then P^T T, 8 terms per entry and step.  One
+// parity colour of cells per launch, so that no two cells share a node; a block looks at GF_CELLS cells and leaves at
+// once where none is flagged.
+constexpr int GF_BS = 288;  // 2 entries of the 576-entry cell matrix per thread
+constexpr int GF_CELLS = 4;
+
+template <int R>
+__global__ void __launch_bounds__(GF_BS) k_galerkin_fixed(int fnx, int fny, int fnz, int cnx, int cny, int cnz,
+                                                          int color, const uint8_t* __restrict__ cfix,
+                                                          const float* __restrict__ w,
+                                                          const uint8_t* __restrict__ vfix,
+                                                          const double* __restrict__ KEg, double* __restrict__ st) {
+    __shared__ double T[576], sP[R * R * R][8][8];  // sP[pos][element vertex][cell corner]
+    __shared__ int cell[GF_CELLS];
     const int fvx = fnx + 1, fvy = fny + 1;
     const int cvx = cnx + 1, cvy = cny + 1, cvz = cnz + 1;
     const long nvc = (long)cvx * cvy * cvz;
     const int px = color & 1, py = (color >> 1) & 1, pz = (color >> 2) & 1;
     const int ccx = (cnx - px + 1) / 2, ccy = (cny - py + 1) / 2, ccz = (cnz - pz + 1) / 2;
-    const long ncells = (long)ccx * ccy * ccz;
-    const long ngroups = (ncells + GAL_CELLS - 1) / GAL_CELLS;
-    for (long g = blockIdx.x; g < ngroups; g += gridDim.x) {
-        __syncthreads();
-        if (threadIdx.x < GAL_CELLS) {
-            long t = g * GAL_CELLS + threadIdx.x;
-            int cid = -1;
-            if (t < ncells) {
-                int X = px + 2 * (int)(t % ccx), Y = py + 2 * (int)((t / ccx) % ccy), Z = pz + 2 * (int)(t / ((long)ccx * ccy));
-                if (ceact[X + (long)cnx * (Y + (long)cny * Z)]) cid = X + cnx * (Y + cny * Z);
-            }
-            scell[threadIdx.x] = cid;
-            sfixed[threadIdx.x] = 0;
+    const int ncells = ccx * ccy * ccz;
+    if (threadIdx.x < GF_CELLS) {
+        const int t = blockIdx.x * GF_CELLS + threadIdx.x;
+        int cid = -1;
+        if (t < ncells) {
+            cid = px + 2 * (t % ccx) + cnx * (py + 2 * (t / ccx % ccy) + cny * (pz + 2 * (t / (ccx * ccy))));
+            if (!cfix[cid]) cid = -1;
         }
-        __syncthreads();
-        for (int i = threadIdx.x; i < GAL_CELLS * NP; i += blockDim.x) {
-            const int c = i / NP, pos = i % NP;
-            double wv = 0;
-            const int cid = scell[c];
-            if (cid >= 0) {
-                const int X = cid % cnx, Y = (cid / cnx) % cny, Z = cid / (cnx * cny);
-                const int a = pos % R, b = (pos / R) % R, cc = pos / (R * R);
-                const int ex = R * X + a, ey = R * Y + b, ez = R * Z + cc;
-                if (ex < fnx && ey < fny && ez < fnz) {
-                    wv = w[ex + (long)fnx * (ey + (long)fny * ez)];
-                    if (vfix != nullptr && wv != 0) {
-                        bool fx = false;
-                        for (int j = 0; j < 8; j++)
-                            fx |= vfix[(ex + (j & 1)) + (long)fvx * ((ey + ((j >> 1) & 1)) + (long)fvy * (ez + (j >> 2)))] != 0;
-                        if (fx) { sfixed[c] = 1; wv = -1.0 - wv; }  // marker: handled explicitly below
-                    }
+        cell[threadIdx.x] = cid;
+    }
+    if (!__syncthreads_or(threadIdx.x < GF_CELLS && cell[threadIdx.x < GF_CELLS ? threadIdx.x : 0] >= 0)) return;
+    for (int i = threadIdx.x; i < R * R * R * 64; i += GF_BS) {
+        const int pos = i / 64, j = i / 8 % 8, m = i % 8;
+        sP[pos][j][m] = interp_w(pos % R + (j & 1), m & 1, R) * interp_w(pos / R % R + ((j >> 1) & 1), (m >> 1) & 1, R) *
+                        interp_w(pos / (R * R) + (j >> 2), m >> 2, R);
+    }
+    // the thread's entries (3 m + row) * 24 + 3 n + col, half 0 and 1
+    int m[2], n[2], row[2], col[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int t = threadIdx.x + h * GF_BS;
+        m[h] = t / 72;
+        row[h] = t / 24 % 3;
+        n[h] = t % 24 / 3;
+        col[h] = t % 3;
+    }
+    for (int li = 0; li < GF_CELLS; li++) {
+        const int cid = cell[li];
+        if (cid < 0) continue;
+        const int X = cid % cnx, Y = cid / cnx % cny, Z = cid / (cnx * cny);
+        double acc[2] = {0, 0};
+        for (int pos = 0; pos < R * R * R; pos++) {
+            const int ex = R * X + pos % R, ey = R * Y + pos / R % R, ez = R * Z + pos / (R * R);
+            if (ex >= fnx || ey >= fny || ez >= fnz) continue;
+            const double pen = w[ex + (long)fnx * (ey + (long)fny * ez)];
+            if (pen == 0 || pen <= -1) continue;
+            unsigned fm = 0;
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                fm |= (vfix[(ex + (j & 1)) + (long)fvx * ((ey + ((j >> 1) & 1)) + (long)fvy * (ez + (j >> 2)))] != 0) << j;
+            if (fm == 0) continue;
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < 2; h++) {  // row 3 j + row of K' times column n of P, j = m[h]
+                const int j = m[h];
+                double s = 0;
+                for (int k = 0; k < 8; k++) {
+                    double kk = 0;
+                    if ((fm >> j & 1) || (fm >> k & 1)) kk = j == k && row[h] == col[h] ? 1e6 : 0.0;
+                    else kk = pen * KEg[(3 * j + row[h]) * 24 + 3 * k + col[h]];
+                    s += kk * sP[pos][k][n[h]];
                 }
+                T[threadIdx.x + h * GF_BS] = s;
             }
-            sw[c][pos] = wv;
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                for (int j = 0; j < 8; j++) acc[h] += sP[pos][j][m[h]] * T[(3 * j + row[h]) * 24 + 3 * n[h] + col[h]];
         }
-        __syncthreads();
-        // dense part: M[c][t] = sum_pos w[c][pos] Q[pos][t] over non-fixed elements
-        double acc[GAL_CELLS][2];
+        // corner m of the cell, neighbour k(n - m)
 #pragma unroll
-        for (int c = 0; c < GAL_CELLS; c++) acc[c][0] = acc[c][1] = 0;
-        const int t0 = threadIdx.x, t1 = threadIdx.x + GAL_BS;
-        for (int pos = 0; pos < NP; pos++) {
-            const double q0 = Q[(long)pos * 576 + t0], q1 = Q[(long)pos * 576 + t1];
-#pragma unroll
-            for (int c = 0; c < GAL_CELLS; c++) {
-                const double wv = sw[c][pos] > 0 ? sw[c][pos] : 0.0;
-                acc[c][0] += wv * q0;
-                acc[c][1] += wv * q1;
-            }
-        }
-        // elements with fixed nodes: rows/cols dropped, 1e6 * P^T P diagonal
-        for (int c = 0; c < GAL_CELLS; c++) {
-            if (!sfixed[c]) continue;
-            const int cid = scell[c];
-            const int X = cid % cnx, Y = (cid / cnx) % cny, Z = cid / (cnx * cny);
-            for (int pos = 0; pos < NP; pos++) {
-                const double wm = sw[c][pos];
-                if (wm >= 0) continue;
-                const double pen = -1.0 - wm;
-                const int a = pos % R, b = (pos / R) % R, cc = pos / (R * R);
-                const int ex = R * X + a, ey = R * Y + b, ez = R * Z + cc;
-#pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    const int t = half ? t1 : t0;
-                    const int mrow = t / 24, ncol = t % 24;
-                    const int m = mrow / 3, row = mrow % 3, n = ncol / 3, col = ncol % 3;
-                    double s = 0;
-                    for (int j = 0; j < 8; j++) {
-                        const int oj[3] = {a + (j & 1), b + ((j >> 1) & 1), cc + (j >> 2)};
-                        const double pj = interp_w(oj[0], m & 1, R) * interp_w(oj[1], (m >> 1) & 1, R) *
-                                          interp_w(oj[2], m >> 2, R);
-                        if (pj == 0) continue;
-                        const bool fj = vfix[(ex + (j & 1)) + (long)fvx * ((ey + ((j >> 1) & 1)) + (long)fvy * (ez + (j >> 2)))];
-                        for (int k = 0; k < 8; k++) {
-                            const int ok[3] = {a + (k & 1), b + ((k >> 1) & 1), cc + (k >> 2)};
-                            const double pk = interp_w(ok[0], n & 1, R) * interp_w(ok[1], (n >> 1) & 1, R) *
-                                              interp_w(ok[2], n >> 2, R);
-                            if (pk == 0) continue;
-                            const bool fk = vfix[(ex + (k & 1)) + (long)fvx * ((ey + ((k >> 1) & 1)) + (long)fvy * (ez + (k >> 2)))];
-                            double kk;
-                            if (fj || fk) kk = (j == k && row == col) ? 1e6 : 0.0;
-                            else kk = pen * KEg[(3 * j + row) * 24 + 3 * k + col];
-                            s += pj * kk * pk;
-                        }
-                    }
-                    acc[c][half] += s;
-                }
-            }
-        }
-        // scatter: entry t = (3m+row)*24 + 3n+col -> node corner m, neighbour k(n-m)
-#pragma unroll
-        for (int c = 0; c < GAL_CELLS; c++) {
-            const int cid = scell[c];
-            if (cid < 0) continue;
-            const int X = cid % cnx, Y = (cid / cnx) % cny, Z = cid / (cnx * cny);
-#pragma unroll
-            for (int half = 0; half < 2; half++) {
-                const int t = half ? t1 : t0;
-                const int mrow = t / 24, ncol = t % 24;
-                const int m = mrow / 3, row = mrow % 3, n = ncol / 3, col = ncol % 3;
-                const int dx = (n & 1) - (m & 1), dy = ((n >> 1) & 1) - ((m >> 1) & 1), dz = (n >> 2) - (m >> 2);
-                const int k = (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
-                const long vc = (X + (m & 1)) + (long)cvx * ((Y + ((m >> 1) & 1)) + (long)cvy * (Z + (m >> 2)));
-                st[(long)(k * 9 + row * 3 + col) * nvc + vc] += acc[c][half];
-            }
+        for (int h = 0; h < 2; h++) {
+            const int dx = (n[h] & 1) - (m[h] & 1), dy = ((n[h] >> 1) & 1) - ((m[h] >> 1) & 1), dz = (n[h] >> 2) - (m[h] >> 2);
+            const int k = (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
+            const long vc = (X + (m[h] & 1)) + (long)cvx * ((Y + ((m[h] >> 1) & 1)) + (long)cvy * (Z + (m[h] >> 2)));
+            st[(long)(k * 9 + row[h] * 3 + col[h]) * nvc + vc] += acc[h];
         }
     }
 }
 
-// A_c = P^T A_f P for a dyadic (ratio 2) level from the finer stencil
+// A_c = P^T A_f P for a dyadic (ratio 2) level from the finer stencil.  A warp per coarse node and block entry: lane i
+// takes fine node i of the node's 3^3 support, reads that node's 27 entries and restricts them along each axis to the
+// 3^3 coarse neighbours (the weights of an axis depend on the lane's offset on it), then the lanes are summed.  A
+// thread per coarse node and entry looped over 729 products with 27 candidates each: 500 us a level, 40 us here.
 __global__ void __launch_bounds__(ST_BS) k_galerkin_dyadic(int fnx, int fny, int fnz, int cnx, int cny, int cnz,
                                                            const uint8_t* __restrict__ fvact,
                                                            const uint8_t* __restrict__ cvact,
@@ -1003,39 +1053,58 @@ __global__ void __launch_bounds__(ST_BS) k_galerkin_dyadic(int fnx, int fny, int
     const int fvx = fnx + 1, fvy = fny + 1, fvz = fnz + 1;
     const int cvx = cnx + 1, cvy = cny + 1, cvz = cnz + 1;
     const long nvf = (long)fvx * fvy * fvz, nvc = (long)cvx * cvy * cvz;
-    const double wtab[4] = {1.0, 0.5, 0.25, 0.125};
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < nvc * 9; t += (long)gridDim.x * blockDim.x) {
-        const long vc = t % nvc;
-        const int rc = (int)(t / nvc);
+    const int lane = threadIdx.x & 31;
+    const int d[3] = {lane % 3 - 1, lane / 3 % 3 - 1, lane / 9 - 1};
+    // weight of fine offset e = d + j - 1 in coarse neighbour s - 1: 1 - |2 (s - 1) - e| / 2 where positive
+    double wt[3][3][3];
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const int g = abs(2 * (q - 1) - (d[ax] + j - 1));
+                wt[ax][j][q] = g < 2 ? 0.5 * (2 - g) : 0.0;
+            }
+    const double wi = (d[0] ? 0.5 : 1.0) * (d[1] ? 0.5 : 1.0) * (d[2] ? 0.5 : 1.0);
+    for (long t = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; t < nvc * 9; t += (long)gridDim.x * (ST_BS / 32)) {
+        const long vc = t / 9;
+        const int rc = (int)(t - vc * 9);
         const int X = (int)(vc % cvx), Y = (int)((vc / cvx) % cvy), Z = (int)(vc / ((long)cvx * cvy));
-        double acc[27];
+        double b[27];
 #pragma unroll
-        for (int s = 0; s < 27; s++) acc[s] = 0;
-        if (cvact[vc]) {
-            for (int i = 0; i < 27; i++) {
-                const int dx = i % 3 - 1, dy = (i / 3) % 3 - 1, dz = i / 9 - 1;
-                const int x = 2 * X + dx, y = 2 * Y + dy, z = 2 * Z + dz;
-                if (x < 0 || y < 0 || z < 0 || x >= fvx || y >= fvy || z >= fvz) continue;
-                const long vn = x + (long)fvx * (y + (long)fvy * z);
-                if (!fvact[vn]) continue;
-                const double wi = wtab[abs(dx) + abs(dy) + abs(dz)];
+        for (int j = 0; j < 27; j++) b[j] = 0;
+        const int x = 2 * X + d[0], y = 2 * Y + d[1], z = 2 * Z + d[2];
+        if (lane < 27 && cvact[vc] && x >= 0 && y >= 0 && z >= 0 && x < fvx && y < fvy && z < fvz) {
+            const long vn = x + (long)fvx * (y + (long)fvy * z);
+            if (fvact[vn]) {
+#pragma unroll
                 for (int j = 0; j < 27; j++) {
-                    const int mx = x + j % 3 - 1, my = y + (j / 3) % 3 - 1, mz = z + j / 9 - 1;
-                    if (mx < 0 || my < 0 || mz < 0 || mx >= fvx || my >= fvy || mz >= fvz) continue;
-                    const double kij = stf[(long)(j * 9 + rc) * nvf + vn] * wi;
-                    if (kij == 0) continue;
-#pragma unroll
-                    for (int s = 0; s < 27; s++) {
-                        const int ax = abs(2 * (X + s % 3 - 1) - mx), ay = abs(2 * (Y + (s / 3) % 3 - 1) - my),
-                                  az = abs(2 * (Z + s / 9 - 1) - mz);
-                        if (ax >= 2 || ay >= 2 || az >= 2) continue;
-                        acc[s] += wtab[ax + ay + az] * kij;
-                    }
+                    const int mx = x + j % 3 - 1, my = y + j / 3 % 3 - 1, mz = z + j / 9 - 1;
+                    if (mx >= 0 && my >= 0 && mz >= 0 && mx < fvx && my < fvy && mz < fvz)
+                        b[j] = stf[(long)(j * 9 + rc) * nvf + vn] * wi;
                 }
+#pragma unroll
+                for (int ax = 0, str = 1; ax < 3; ax++, str *= 3)
+#pragma unroll
+                    for (int l = 0; l < 9; l++) {
+                        const int o = ax == 0 ? 3 * l : ax == 1 ? l % 3 + 9 * (l / 3) : l;
+                        const double a0 = b[o], a1 = b[o + str], a2 = b[o + 2 * str];
+#pragma unroll
+                        for (int q = 0; q < 3; q++)
+                            b[o + q * str] = wt[ax][0][q] * a0 + wt[ax][1][q] * a1 + wt[ax][2][q] * a2;
+                    }
             }
         }
+        double mine = 0;
 #pragma unroll
-        for (int s = 0; s < 27; s++) stc[(long)(s * 9 + rc) * nvc + vc] = acc[s];
+        for (int q = 0; q < 27; q++) {
+            double v = b[q];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == q) mine = v;
+        }
+        if (lane < 27) stc[(long)(lane * 9 + rc) * nvc + vc] = mine;
     }
 }
 
@@ -1308,10 +1377,10 @@ int prolong_add(rt_hier* h, int lvl, const T* uc, T* uf) {
     });
 }
 
-// Q_pos = P_pos^T KE P_pos for every element position in a coarse cell
+// Q_pos = P_pos^T KE P_pos for every element position in a coarse cell, as [corner m][corner n][pos][10]
 static int build_Q(rt_hier* h, int R, double** Qdev) {
     const int NP = R * R * R;
-    std::vector<double> Qh((size_t)NP * 576);
+    std::vector<double> Qh((size_t)NP * 640);
     for (int pos = 0; pos < NP; pos++) {
         int a = pos % R, b = (pos / R) % R, c = pos / (R * R);
         double P[8][8];
@@ -1334,7 +1403,7 @@ static int build_Q(rt_hier* h, int R, double** Qdev) {
                             for (int k = 0; k < 8; k++)
                                 s += P[j][m] * h->KE[(3 * j + row) * 24 + 3 * k + col] * P[k][n];
                         }
-                        Qh[(size_t)pos * 576 + (3 * m + row) * 24 + 3 * n + col] = s;
+                        Qh[((size_t)(m * 8 + n) * NP + pos) * 10 + 3 * row + col] = s;
                     }
     }
     RT_CUDA(h->ctx, cudaMalloc(Qdev, sizeof(double) * Qh.size()));
@@ -1342,6 +1411,8 @@ static int build_Q(rt_hier* h, int R, double** Qdev) {
                                     h->ctx->stream));
     return RT_OK;
 }
+
+static constexpr size_t gn_smem(int R) { return sizeof(double) * R * R * R * 33 * 3 * 2; }
 
 int galerkin_from_elements(rt_hier* h) {
     rt_level& F = h->L[0];
@@ -1353,24 +1424,44 @@ int galerkin_from_elements(rt_hier* h) {
         RT_CHECK(build_Q(h, R, &h->Qgal));
         h->Qgal_ratio = R;
     }
-    const double* Q = h->Qgal;
-    RT_CUDA(h->ctx, cudaMemsetAsync(Cc.st, 0, sizeof(double) * 243 * Cc.nv, h->ctx->stream));
-    for (int color = 0; color < 8; color++) {
-        long ccells = (long)((Cc.nx - (color & 1) + 1) / 2) * ((Cc.ny - ((color >> 1) & 1) + 1) / 2) *
-                      ((Cc.nz - (color >> 2) + 1) / 2);
-        long groups = (ccells + GAL_CELLS - 1) / GAL_CELLS;
-        if (groups == 0) continue;
-        unsigned g = (unsigned)(groups < (long)h->ctx->sm_count * 8 ? groups : (long)h->ctx->sm_count * 8);
-        RT_CHECK(rt_launch(h->ctx, "galerkin_cells", [&] {
-            const uint8_t* vf = h->has_support ? h->vfix : nullptr;
+    rt_ctx* c = h->ctx;
+    const float* w = h->w;
+    uint8_t* cfix = nullptr;
+    if (h->has_support) {  // ftmp: element scratch of the filter
+        RT_CUDA(c, cudaMallocAsync(&cfix, (size_t)Cc.ne, c->stream));
+        RT_CUDA(c, cudaMemsetAsync(cfix, 0, (size_t)Cc.ne, c->stream));
+        RT_CHECK(rt_launch(c, "galerkin_weights", [&] {
+            const unsigned g = grid_for(c, F.ne, ST_BS);
             if (R == 4)
-                k_galerkin_cells<4><<<g, GAL_BS, 0, h->ctx->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, color,
-                                                                      Cc.eact, h->w, vf, Q, h->KE_dev, Cc.st);
+                k_free_weights<4><<<g, ST_BS, 0, c->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, h->w, h->vfix, h->ftmp, cfix);
             else
-                k_galerkin_cells<2><<<g, GAL_BS, 0, h->ctx->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, color,
-                                                                      Cc.eact, h->w, vf, Q, h->KE_dev, Cc.st);
+                k_free_weights<2><<<g, ST_BS, 0, c->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, h->w, h->vfix, h->ftmp, cfix);
+        }));
+        w = h->ftmp;
+    }
+    RT_CHECK(rt_launch(c, "galerkin_nodes", [&] {
+        const dim3 g((Cc.vx + 31) / 32, (Cc.vy + 1) / 2, Cc.vz);
+        if (R == 4)
+            k_galerkin_nodes<4><<<g, GN_BS, gn_smem(4), c->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, w, h->Qgal, Cc.st);
+        else
+            k_galerkin_nodes<2><<<g, GN_BS, gn_smem(2), c->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, w, h->Qgal, Cc.st);
+    }));
+    if (!cfix) return RT_OK;
+    for (int color = 0; color < 8; color++) {
+        const long ccells = (long)((Cc.nx - (color & 1) + 1) / 2) * ((Cc.ny - ((color >> 1) & 1) + 1) / 2) *
+                            ((Cc.nz - (color >> 2) + 1) / 2);
+        if (ccells == 0) continue;
+        RT_CHECK(rt_launch(c, "galerkin_fixed", [&] {
+            const unsigned g = (unsigned)((ccells + GF_CELLS - 1) / GF_CELLS);
+            if (R == 4)
+                k_galerkin_fixed<4><<<g, GF_BS, 0, c->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, color, cfix, h->w,
+                                                                h->vfix, h->KE_dev, Cc.st);
+            else
+                k_galerkin_fixed<2><<<g, GF_BS, 0, c->stream>>>(F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, color, cfix, h->w,
+                                                                h->vfix, h->KE_dev, Cc.st);
         }));
     }
+    RT_CUDA(c, cudaFreeAsync(cfix, c->stream));
     return RT_OK;
 }
 
@@ -1378,7 +1469,7 @@ int galerkin_from_stencil(rt_hier* h, int lvl) {
     rt_level& F = h->L[lvl - 1];
     rt_level& Cc = h->L[lvl];
     return rt_launch(h->ctx, "galerkin_dyadic", [&] {
-        k_galerkin_dyadic<<<grid_for(h->ctx, Cc.nv * 9, ST_BS), ST_BS, 0, h->ctx->stream>>>(
+        k_galerkin_dyadic<<<grid_for(h->ctx, Cc.nv * 9 * 32, ST_BS), ST_BS, 0, h->ctx->stream>>>(
             F.nx, F.ny, F.nz, Cc.nx, Cc.ny, Cc.nz, F.vact, Cc.vact, F.st, Cc.st);
     });
 }
@@ -1389,7 +1480,8 @@ int d2f(rt_hier* h, long n, const double* a, float* b) {
 
 // dynamic shared-memory limits of the bulk-copy stencil kernels, set once per device
 int init_stencil_kernels(rt_ctx* c) {
-    cudaError_t e[5] = {
+    cudaError_t e[6] = {
+        cudaFuncSetAttribute(k_galerkin_nodes<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gn_smem(4)),
         cudaFuncSetAttribute(k_st_bulk<float, 0, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sb_smem<float, float>()),
         cudaFuncSetAttribute(k_st_bulk<float, 2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -220,3 +220,20 @@ def test_coarsest_inverse_block_edges(dims, limit):
     assert np.abs(got - want).max() <= 1e-14 * np.linalg.cond(A) * np.abs(want).max() + 1e-12 * np.abs(want).max()
     G.close()
     ctx.close()
+
+
+# Galerkin stencils: 32 x 2 nodes per block (33 and 34 coarse nodes in x, odd rows), both coarsening ratios, fixed
+# nodes inside and on the faces; dyadic levels below
+@pytest.mark.parametrize("dims,skip", [((127, 9, 7), 1), ((131, 6, 13), 1), ((63, 7, 6), 0), ((20, 18, 14), 0)])
+def test_galerkin_edges(dims, skip):
+    ctx, G, eact, rho, vfix, r = _hier(*dims, seed=11, skip=skip)
+    vfix[r.random(vfix.shape) < 0.01] = 1
+    G.set_support(vfix)
+    G.update_stencil()
+    H = O.Hierarchy(eact, rho, vfix, p=P, E=E, nu=NU, skip=bool(skip))
+    H.set_weights(G[0].getPenalty())
+    H.update_stencil()
+    for i in range(1, H.nlev):
+        assert rel_err(G[i].getStencil(), H.arrs[i]["st"]) < 1e-11, f"level {i}"
+    G.close()
+    ctx.close()

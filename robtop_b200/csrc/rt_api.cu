@@ -314,7 +314,7 @@ static void free_workspace(rt_hier* w) {
         cudaFree(L.u); cudaFree(L.f); cudaFree(L.r); cudaFree(L.u32); cudaFree(L.f32); cudaFree(L.r32);
         cudaFree(L.d); cudaFree(L.d32); cudaFree(L.dvec);
     }
-    cudaFree(w->x); cudaFree(w->rr); cudaFree(w->z); cudaFree(w->p); cudaFree(w->q); cudaFree(w->rold);
+    cudaFree(w->x); cudaFree(w->rr); cudaFree(w->z); cudaFree(w->p); cudaFree(w->q);
     cudaFree(w->partials); cudaFree(w->scal);
     if (w->pcg_exec) cudaGraphExecDestroy(w->pcg_exec);
     if (w->pcg_graph) cudaGraphDestroy(w->pcg_graph);
@@ -322,7 +322,7 @@ static void free_workspace(rt_hier* w) {
     if (w->pcg_graph_alt) cudaGraphDestroy(w->pcg_graph_alt);
     if (w->pcg32_exec) cudaGraphExecDestroy(w->pcg32_exec);
     if (w->pcg32_graph) cudaGraphDestroy(w->pcg32_graph);
-    cudaFree(w->p32k); cudaFree(w->q32k); cudaFree(w->d32k); cudaFree(w->ro32k);
+    cudaFree(w->p32k); cudaFree(w->q32k); cudaFree(w->d32k);
     rt_ctx* c = w->ctx;
     delete w;
     rt_ctx_release(c);
@@ -357,7 +357,7 @@ static void free_hier(rt_hier* h) {
     if (h->pcg_graph_alt) cudaGraphDestroy(h->pcg_graph_alt);
     if (h->pcg32_exec) cudaGraphExecDestroy(h->pcg32_exec);
     if (h->pcg32_graph) cudaGraphDestroy(h->pcg32_graph);
-    cudaFree(h->p32k); cudaFree(h->q32k); cudaFree(h->d32k); cudaFree(h->ro32k);
+    cudaFree(h->p32k); cudaFree(h->q32k); cudaFree(h->d32k);
     rt_ctx* c = h->ctx;
     delete h;
     rt_ctx_release(c);
@@ -1473,11 +1473,8 @@ extern "C" int rt_relative_residual(rt_hier* h, double* rel) {
 
 // ---------------------------------------------------------------------------
 // MG-preconditioned flexible CG on level 0: x = L0.u (initial guess), b = L0.f
-// scal slots: 10..13 r.z / rold.z (two parities), 20 p.q, 21 r.r, 22 b.b
+// scal slots: 10 z.r, 11 z.q, 12 the previous z.r, 20 p.q, 21 r.r, 22 b.b
 // ---------------------------------------------------------------------------
-// z = B r (the V-cycle, plus the learned correction when attached).  When dots is given and the
-// form allows it, the FP32 path also leaves (z.r, z.rold) in dots[0..1] (fused with the widening
-// of z) and returns with *dots_done set.
 // the FP32 right-hand side of the V-cycle comes out of the x / r update (scaled by the r.r
 // before that update, kept in scal[23]) instead of a separate conversion pass
 static bool fused_f32_rhs(const rt_hier* h) { return h->P.precision == RT_FP32 && !h->P.krylov_fp32; }
@@ -1540,22 +1537,18 @@ static int learned_if(rt_hier* h, F&& fn) {
     return RT_OK;
 }
 
-// z = M^-1 r.  rr_dev: the scale (r.r of the residual the FP32 copy was made from);
-// f32_ready: level 0's FP32 right-hand side already holds r / sqrt(rr_dev)
-static int precondition(rt_hier* h, const double* r, double* z, const double* rr_dev, double* dots = nullptr,
-                        bool* dots_done = nullptr, bool f32_ready = false) {
+// z = M^-1 r (the V-cycle, plus the learned correction when attached).  rr_dev: the scale (r.r of the residual the
+// FP32 copy was made from); f32_ready: level 0's FP32 right-hand side already holds r / sqrt(rr_dev); widen: false
+// leaves an FP32 V-cycle's result in level 0's u32 (z = sqrt(rr_dev) u32) and z unwritten
+static int precondition(rt_hier* h, const double* r, double* z, const double* rr_dev, bool f32_ready = false,
+                        bool widen = true) {
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
-    if (dots_done) *dots_done = false;
     if (h->P.precision == RT_FP32) {
         if (!f32_ready) RT_CHECK(rtk::d2f_scaled(h, n, r, L.f32, rr_dev));
         RT_CHECK(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 0, true));
-        if (dots) {
-            RT_CHECK(rtk::f2d_scaled_dot2(h, n, L.u32, z, rr_dev, r, h->rold, dots));
-            *dots_done = true;
-        } else {
-            RT_CHECK(rtk::f2d_scaled(h, n, L.u32, z, rr_dev));
-        }
+        if (!widen) return RT_OK;
+        RT_CHECK(rtk::f2d_scaled(h, n, L.u32, z, rr_dev));
     } else if (h->P.precision == RT_FP64_FINE && h->L.size() > 1) {
         // FP64 smoothing and residual on the finest level (on r / z themselves), the coarse
         // V-cycle in FP32 on the restricted residual scaled by 1 / |r|, its correction added back
@@ -1591,8 +1584,7 @@ static int precondition(rt_hier* h, const double* r, double* z, const double* rr
         L.u = saved_u;
         RT_CHECK(s);
     }
-    // learned correction z += N(rho, r, z), run only while the gate in scal[28] is on; the dots
-    // the widening of z already produced are recomputed for the corrected z.  Once the gate has
+    // learned correction z += N(rho, r, z), run only while the gate in scal[28] is on.  Once the gate has
     // judged the network off for this design, the loop is captured without it: a conditional
     // node inside the captured loop body slows every iteration's launches, even when it skips
     if (h->unet && !h->unet_off)
@@ -1612,19 +1604,9 @@ static int precondition(rt_hier* h, const double* r, double* z, const double* rr
                 L.u = saved_u;
                 RT_CHECK(st);
             }
-            return (dots_done && *dots_done) ? rtk::dot2(h, n, z, r, h->rold, dots) : RT_OK;
+            return RT_OK;
         }));
     return RT_OK;
-}
-
-// p = z + beta p, flexible beta = (z.r - z.rold) / rz_prev; beta = 0 on the first iteration
-__global__ void k_pcg_p_it(long n, const double* __restrict__ s, const double* __restrict__ it, double* __restrict__ p,
-                           const double* __restrict__ z) {
-    const bool first = it[0] == 0.0;
-    const double den = s[2];
-    const double beta = (first || den == 0.0) ? 0.0 : (s[0] - s[1]) / den;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        p[i] = first ? z[i] : z[i] + beta * p[i];
 }
 
 // end of an iteration: it += 1, rz_prev = rz; optionally set the WHILE condition of the graph
@@ -1656,27 +1638,29 @@ __global__ void k_pcg_tail(double* __restrict__ scal, cudaGraphConditionalHandle
     }
 }
 
-// one MG-PCG iteration, all scalars on the device (graph-capturable):
-// scal[10] z.r, [11] z.rold, [12] previous z.r, [20] p.q, [21] r.r, [24] iteration
+// one MG-PCG iteration, all scalars on the device (graph-capturable); the iteration's step of x is taken by the next
+// one, the last by pcg_x_last
 static int pcg_body(rt_hier* h, double* x, double* r, bool no_support, cudaGraphConditionalHandle cond,
                     int use_cond = 0) {
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
     rt_ctx* c = h->ctx;
-    bool dots_done = false;
     const bool fz = fused_f32_rhs(h);
-    // the projection of z (no supports) must precede its dots: no fusion then
-    RT_CHECK(precondition(h, r, h->z, h->scal + (fz ? 23 : 21), no_support ? nullptr : h->scal + 10, &dots_done, fz));
+    const double* zscale = h->scal + (fz ? 23 : 21);
+    // the projection of z (no supports) and the learned correction work on the FP64 z
+    const bool narrow = h->P.precision == RT_FP32 && !no_support && !(h->unet && !h->unet_off);
+    RT_CHECK(precondition(h, r, h->z, zscale, fz, !narrow));
     if (no_support) RT_CHECK(rtk::displacement_project(h, h->z));
-    if (!dots_done) RT_CHECK(rtk::dot2(h, n, h->z, r, h->rold, h->scal + 10));
-    RT_CHECK(rt_launch(c, "pcg_update_p", [&] {
-        k_pcg_p_it<<<(unsigned)std::min<long>((n + 255) / 256, (long)c->sm_count * 16), 256, 0, c->stream>>>(
-            n, h->scal + 10, h->scal + 24, h->p, h->z);
-    }));
+    if (narrow) {
+        RT_CHECK(rtk::pcg_zdots(h, n, L.u32, zscale, r, h->q, h->scal + 10));
+        RT_CHECK(rtk::pcg_update_xp(h, n, L.u32, zscale, h->p, x));
+    } else {
+        RT_CHECK(rtk::pcg_zdots(h, n, h->z, r, h->q, h->scal + 10));
+        RT_CHECK(rtk::pcg_update_xp(h, n, h->z, h->p, x));
+    }
     RT_CHECK(rtk::fine_applyK<double>(h, h->p, h->q));
     RT_CHECK(rtk::dot(h, n, h->p, h->q, h->scal + 20));
-    RT_CHECK(rtk::pcg_update_xr_rr(h, n, h->scal + 10, h->scal + 20, x, r, h->p, h->q, h->rold, h->scal + 21,
-                                   fz ? L.f32 : nullptr, h->scal + 23));
+    RT_CHECK(rtk::pcg_update_r_rr(h, n, r, h->q, fz ? L.f32 : nullptr));
     return rt_launch(c, "pcg_tail", [&] { k_pcg_tail<<<1, 32, 0, c->stream>>>(h->scal, cond, use_cond); });
 }
 
@@ -1757,7 +1741,7 @@ static int pcg_graph_run(rt_hier* h, double* x, double* r, bool no_support) {
     return RT_OK;
 }
 
-// r = b - K x (identity rows on supports), rold = 0, scal[22] = b.b, scal[21] = r.r (graph-capturable)
+// r = b - K x (identity rows on supports), scal[22] = b.b, scal[21] = r.r (graph-capturable)
 static int pcg_prologue(rt_hier* h, double* x, const double* b) {
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
@@ -1766,7 +1750,6 @@ static int pcg_prologue(rt_hier* h, double* x, const double* b) {
     RT_CUDA(h->ctx, cudaMemcpyAsync(r, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->ctx->stream));
     RT_CHECK(rtk::axpy(h, n, -1.0, h->q, r));
     RT_CHECK(rtk::mask_copy(h, n, r, r));
-    RT_CUDA(h->ctx, cudaMemsetAsync(h->rold, 0, sizeof(double) * n, h->ctx->stream));
     RT_CHECK(rtk::dot(h, n, b, b, h->scal + 22));
     RT_CHECK(rtk::dot(h, n, r, r, h->scal + 21));
     if (!fused_f32_rhs(h)) return RT_OK;
@@ -1804,8 +1787,7 @@ static int ensure_krylov32(rt_hier* h) {
     const size_t n = 3 * (size_t)h->L[0].nv;
     RT_CHECK(dalloc(h->ctx, &h->p32k, n));
     RT_CHECK(dalloc(h->ctx, &h->q32k, n));
-    RT_CHECK(dalloc(h->ctx, &h->d32k, n));
-    return dalloc(h->ctx, &h->ro32k, n);
+    return dalloc(h->ctx, &h->d32k, n);
 }
 
 // one inner iteration: z = V(res) (res is level 0's FP32 right-hand side, z its FP32 solution),
@@ -1815,12 +1797,11 @@ static int pcg32_body(rt_hier* h, cudaGraphConditionalHandle cond, int use_cond)
     const long n = 3 * L.nv;
     rt_ctx* c = h->ctx;
     RT_CHECK(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 0, true));
-    RT_CHECK(rtk::dot32_2(h, n, L.u32, L.f32, h->ro32k, h->scal + 10));
-    RT_CHECK(rtk::pcg32_update_p(h, n, h->scal + 10, h->scal + 24, h->p32k, L.u32));
+    RT_CHECK(rtk::pcg_zdots32(h, n, L.u32, L.f32, h->q32k, h->scal + 10));
+    RT_CHECK(rtk::pcg32_update_xp(h, n, L.u32, h->p32k, h->d32k));
     RT_CHECK(rtk::fine_applyK<float>(h, h->p32k, h->q32k));
     RT_CHECK(rtk::dot32(h, n, h->p32k, h->q32k, h->scal + 20));
-    RT_CHECK(rtk::pcg32_update_xr_rr(h, n, h->scal + 10, h->scal + 20, h->d32k, L.f32, h->p32k, h->q32k, h->ro32k,
-                                     h->scal + 21));
+    RT_CHECK(rtk::pcg32_update_r_rr(h, n, L.f32, h->q32k));
     return rt_launch(c, "pcg_tail", [&] { k_pcg_tail<<<1, 32, 0, c->stream>>>(h->scal, cond, use_cond); });
 }
 
@@ -1904,7 +1885,6 @@ static int pcg32_core(rt_hier* h, double* x, const double* b, double tol, int ma
         RT_CHECK(rtk::d2f_scaled(h, n, h->rr, L.f32, h->scal + 21));
         RT_CUDA(c, cudaMemcpyAsync(h->scal + 23, h->scal + 21, sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
         RT_CUDA(c, cudaMemsetAsync(h->d32k, 0, sizeof(float) * n, c->stream));
-        RT_CUDA(c, cudaMemsetAsync(h->ro32k, 0, sizeof(float) * n, c->stream));
         // inner loop state: scal[24..29] iteration count, tolerance, budget, no learned
         // correction (ratio, gate, previous r.r); scal[21..22] the unit right-hand side's r.r
         // and b.b; scal[90..93] stall detection as in pcg_core
@@ -2019,6 +1999,7 @@ static int pcg_core(rt_hier* h, double* x, const double* b, double tol, int maxi
                 if (!std::isfinite(s2[0]) || std::sqrt(s2[0]) / bn <= tol || stall != 0.0) break;
             }
         }
+        RT_CHECK(rtk::pcg_x_last(h, 3 * h->L[0].nv, x));
         double s3[4], stall = 0;
         RT_CHECK(read_scalars(h, 21, 4, s3));  // rr, bb, (unused), it
         RT_CHECK(read_scalars(h, 92, 1, &stall));
@@ -2803,7 +2784,7 @@ static int make_workspace(rt_hier* p, rt_hier** out) {
     }
     const size_t n3 = 3 * (size_t)p->L[0].nv;
     RT_CHECK(dalloc(c, &w->x, n3)); RT_CHECK(dalloc(c, &w->rr, n3)); RT_CHECK(dalloc(c, &w->z, n3));
-    RT_CHECK(dalloc(c, &w->p, n3)); RT_CHECK(dalloc(c, &w->q, n3)); RT_CHECK(dalloc(c, &w->rold, n3));
+    RT_CHECK(dalloc(c, &w->p, n3)); RT_CHECK(dalloc(c, &w->q, n3));
     RT_CHECK(dalloc(c, &w->partials, RT_PARTIALS));
     RT_CHECK(dalloc(c, &w->scal, RT_NSCAL));
     RT_CUDA(c, cudaMemsetAsync(w->scal, 0, sizeof(double) * RT_NSCAL, c->stream));
@@ -2914,6 +2895,18 @@ static int build_batch_graph_(rt_ctx* c, rt_hier* const* hs, int n, double tol, 
             e = cudaStreamEndCapture(c->stream, &captured);
         }
         iter_kernels->push_back(c->launches - lb);
+        if (e == cudaSuccess && s == RT_OK) {  // the last iteration's step of x
+            cudaGraph_t tg = nullptr;
+            e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+            if (e == cudaSuccess) {
+                s = rtk::pcg_x_last(h, 3 * h->L[0].nv, x);
+                e = cudaStreamEndCapture(c->stream, &tg);
+            }
+            cudaGraphNode_t n4 = nullptr;
+            if (e == cudaSuccess && s == RT_OK) e = cudaGraphAddChildGraphNode(&n4, g, &n3, 1, tg);
+            if (tg) cudaGraphDestroy(tg);
+            (*once_kernels)[i]++;
+        }
         if (s != RT_OK || e != cudaSuccess) {
             c->launches = l0;
             cudaGraphDestroy(g);

@@ -144,7 +144,7 @@ struct rt_hier {
     // reductions
     double* partials = nullptr;  // [RT_RED_BLOCKS * 8]
     // FP32 Krylov vectors of the refinement form (rt_params.krylov_fp32), allocated on first use
-    float *p32k = nullptr, *q32k = nullptr, *d32k = nullptr, *ro32k = nullptr;
+    float *p32k = nullptr, *q32k = nullptr, *d32k = nullptr;
     cudaGraph_t pcg32_graph = nullptr;
     cudaGraphExec_t pcg32_exec = nullptr;
     uint64_t pcg32_key = 0;
@@ -235,6 +235,7 @@ static inline unsigned rt_blocks(long n, int bs) { return (unsigned)((n + bs - 1
 #define RT_CHEBY_HI_FRAC 1.1
 #define RT_SCAL_ERR 295   // set to 1 by a stencil kernel whose bounded copy wait ran out
 #define RT_SCAL_LMAX 300  // device scalar slots holding lmax(D^-1 A) per level
+#define RT_SCAL_TICKET 496  // ticket counter of the grid reductions (u32, zero between launches)
 #define RT_SCAL_GBAR 480  // per level: the grid barrier of the fused Chebyshev sweeps (arrivals, generation as 2 x u32)
 // (a_k, b_k), k < RT_CHEBY_MAXK, per level at RT_SCAL_CHEB + 2 RT_CHEBY_MAXK lvl (levels 0..14);
 // the 16th table serves kernel timing before any stencil exists
@@ -315,7 +316,6 @@ template <typename T>
 int coarsest_solve(rt_hier* h, const T* f, T* u);
 // BLAS-1 / reductions
 int dot(rt_hier* h, long n, const double* a, const double* b, double* out_dev);
-int dot2(rt_hier* h, long n, const double* a, const double* b, const double* c, double* out_dev);
 int axpy(rt_hier* h, long n, double a, const double* x, double* y);
 int d2f(rt_hier* h, long n, const double* a, float* b);
 int stencil_copies(rt_hier* h, int lvl);
@@ -323,21 +323,19 @@ int f2d(rt_hier* h, long n, const float* a, double* b);
 int d2f_scaled(rt_hier* h, long n, const double* a, float* b, const double* s_dev);
 int f2d_scaled(rt_hier* h, long n, const float* a, double* b, const double* s_dev);
 int f2d_scaled_add(rt_hier* h, long n, const float* a, double* b, const double* s_dev);
-// fused passes of the PCG iteration: x, r update with r.r; widening of z with (z.r, z.rold)
-int pcg_update_xr_rr(rt_hier* h, long n, const double* num, const double* den, double* x, double* r, const double* p,
-                     const double* q, double* rold, double* rr_out, float* r32 = nullptr, double* scale_out = nullptr);
+// vector passes of the PCG iteration (rt_misc.cu: k_pcg_*): the scalars are h->scal's slots 10..24; z is the V-cycle's
+// FP32 result times sqrt(s), or an FP64 vector
+int pcg_zdots(rt_hier* h, long n, const float* z, const double* s, const double* r, const double* q, double* out);
+int pcg_zdots(rt_hier* h, long n, const double* z, const double* r, const double* q, double* out);
+int pcg_zdots32(rt_hier* h, long n, const float* z, const float* r, const float* q, double* out);
+int pcg_update_xp(rt_hier* h, long n, const float* z, const double* s, double* p, double* x);
+int pcg_update_xp(rt_hier* h, long n, const double* z, double* p, double* x);
+int pcg32_update_xp(rt_hier* h, long n, const float* z, float* p, float* d);
+int pcg_update_r_rr(rt_hier* h, long n, double* r, const double* q, float* r32);
+int pcg32_update_r_rr(rt_hier* h, long n, float* r, const float* q);
+int pcg_x_last(rt_hier* h, long n, double* x);
 int dot32(rt_hier* h, long n, const float* a, const float* b, double* out);
-int dot32_2(rt_hier* h, long n, const float* a, const float* b, const float* c, double* out);
-int pcg32_update_p(rt_hier* h, long n, const double* s, const double* it, float* p, const float* z);
-int pcg32_update_xr_rr(rt_hier* h, long n, const double* num, const double* den, float* d, float* r, const float* p,
-                       const float* q, float* rold, double* rr_out);
 int axpy_f32_scaled(rt_hier* h, long n, double* x, const float* d, const double* s);
-int f2d_scaled_dot2(rt_hier* h, long n, const float* a, double* z, const double* s_dev, const double* r,
-                    const double* rold, double* out);
-int pcg_update_xr(rt_hier* h, long n, const double* scal_alpha_num, const double* scal_alpha_den, double* x,
-                  double* r, const double* p, const double* q, double* rold);
-int pcg_update_p(rt_hier* h, long n, const double* s_num, const double* s_den, double* p, const double* z,
-                 bool first);
 int mask_copy(rt_hier* h, long n, const double* src, double* dst);
 // worst case
 int rng_uniform(rt_hier* h, uint64_t seed, long n, double* out);

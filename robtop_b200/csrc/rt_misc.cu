@@ -29,9 +29,20 @@ unsigned gridN(rt_ctx* c, long n, int bs = 256) {
     return (unsigned)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
+struct RedOut {
+    double* partials;  // one set per block
+    double* out;
+    unsigned* ticket;
+};
+
+// blocks of a reduction: 2 per SM, fewer for short vectors
+unsigned red_grid(long n) { return (unsigned)(n < (long)RT_RED_BLOCKS * RB ? (n + RB - 1) / RB > 0 ? (n + RB - 1) / RB : 1 : RT_RED_BLOCKS); }
+
+// block sums of v[0..NV) in thread 0
 template <int NV>
-__device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* __restrict__ partials) {
+__device__ __forceinline__ void block_reduce(double (&v)[NV]) {
     __shared__ double sh[NV][RB / 32];
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < NV; k++) {
         double x = v[k];
@@ -46,45 +57,44 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* __re
             double x = threadIdx.x < RB / 32 ? sh[k][threadIdx.x] : 0.0;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            if (threadIdx.x == 0) partials[blockIdx.x * NV + k] = x;
+            v[k] = x;
         }
     }
 }
 
-// sum NV interleaved partial arrays in a fixed order (deterministic)
+// the grid's sums of v[0..NV) in out: every block stores its own, and the last one to finish (a ticket counter, left
+// at zero again) adds them in a fixed order, so that the sum does not depend on which block that is.  One launch
+// where a second one added the partial sums (6 us, three times a PCG iteration).
 template <int NV>
-__global__ void k_final_sum(int nblocks, const double* __restrict__ partials, double* __restrict__ out) {
-    __shared__ double sh[NV][32];
+__device__ __forceinline__ void grid_reduce(double (&v)[NV], const RedOut& o) {
+    __shared__ bool last;
+    block_reduce<NV>(v);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) o.partials[blockIdx.x * NV + k] = v[k];
+        __threadfence();
+        last = atomicInc(o.ticket, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t[NV];
+#pragma unroll
     for (int k = 0; k < NV; k++) {
-        double x = 0;
-        for (int b = threadIdx.x; b < nblocks; b += 32) x += partials[b * NV + k];
-        sh[k][threadIdx.x] = x;
+        t[k] = 0;
+        for (int b = threadIdx.x; b < (int)gridDim.x; b += RB) t[k] += __ldcg(o.partials + (long)b * NV + k);
     }
-    __syncwarp();
-    if (threadIdx.x < NV) {
-        double s = 0;
-        for (int i = 0; i < 32; i++) s += sh[threadIdx.x][i];
-        out[threadIdx.x] = s;
-    }
+    block_reduce<NV>(t);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int k = 0; k < NV; k++) o.out[k] = t[k];
 }
 
 __global__ void __launch_bounds__(RB) k_dot(long n, const double* __restrict__ a, const double* __restrict__ b,
-                                            double* __restrict__ partials) {
+                                            RedOut ro) {
     double v[1] = {0};
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) v[0] += a[i] * b[i];
-    block_reduce_store<1>(v, partials);
-}
-
-// (a.b, a.c) in one pass
-__global__ void __launch_bounds__(RB) k_dot2(long n, const double* __restrict__ a, const double* __restrict__ b,
-                                             const double* __restrict__ c, double* __restrict__ partials) {
-    double v[2] = {0, 0};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const double x = a[i];
-        v[0] += x * b[i];
-        v[1] += x * c[i];
-    }
-    block_reduce_store<2>(v, partials);
+    grid_reduce<1>(v, ro);
 }
 
 __global__ void k_axpy(long n, double a, const double* __restrict__ x, double* __restrict__ y) {
@@ -115,159 +125,134 @@ __global__ void k_f2d_scaled_add(long n, const float* __restrict__ a, double* __
         b[i] += (double)a[i] * sc;
 }
 
-// x += alpha p, r -= alpha q, rold = r(before);  alpha = num / den read on the device
-__global__ void k_pcg_xr(long n, const double* __restrict__ num, const double* __restrict__ den, double* __restrict__ x,
-                         double* __restrict__ r, const double* __restrict__ p, const double* __restrict__ q,
-                         double* __restrict__ rold) {
-    const double alpha = den[0] != 0.0 ? num[0] / den[0] : 0.0;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const double ri = r[i];
-        rold[i] = ri;
-        x[i] += alpha * p[i];
-        r[i] = ri - alpha * q[i];
-    }
-}
+// ---------------------------------------------------------------------------
+// Vector passes of the PCG iteration, FP64 or FP32 vectors (T; dots summed in FP64).  z = sc * zs: the FP32 V-cycle's
+// result is widened where it is used instead of being stored.  The flexible beta = (z.r - z.r_old) / rz_old is
+// -(z.q) / (p.q), since r = r_old - alpha q with alpha = rz_old / (p.q), so no copy of the old residual is kept.  The
+// step of x waits for the next iteration's pass over p (and one pass after the loop).  Per entry, FP64 vectors with
+// an FP32 V-cycle: 84 bytes in 3 passes where 128 in 5 were moved (511x256x256: 2.2 -> 1.4 ms per iteration).
+// scal: 10 z.r, 11 z.q, 12 the previous z.r, 20 p.q, 21 r.r, 24 the iteration.
+// ---------------------------------------------------------------------------
+template <typename TZ>
+__device__ __forceinline__ double z_scale(const double* s) { return s ? sqrt(fmax(s[0], 1e-300)) : 1.0; }
 
-// k_pcg_xr and r.r of the updated r in the same pass (partials as k_dot's: same grid, same order)
-// r32 (optional): the new residual scaled by 1 / sqrt(rr_old) and rounded to FP32, the right-hand
-// side of the next FP32 V-cycle; rr_old (the r.r before this update) is kept in scale_out
-__global__ void __launch_bounds__(RB) k_pcg_xr_rr(long n, const double* __restrict__ num, const double* __restrict__ den,
-                                                  double* __restrict__ x, double* __restrict__ r,
-                                                  const double* __restrict__ p, const double* __restrict__ q,
-                                                  double* __restrict__ rold, double* __restrict__ partials,
-                                                  float* __restrict__ r32, const double* __restrict__ rr_old,
-                                                  double* __restrict__ scale_out) {
-    const double alpha = den[0] != 0.0 ? num[0] / den[0] : 0.0;
-    const double inv = r32 ? 1.0 / sqrt(fmax(rr_old[0], 1e-300)) : 0.0;
-    if (r32 && blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = rr_old[0];
-    double v[1] = {0};
-    // the reduction grid is small (2 blocks per SM): XR_U grid strides per trip keep enough loads in
-    // flight; the sum still runs over each thread's elements in stride order, as in k_dot
-    const long st = (long)gridDim.x * blockDim.x;
-    for (long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x; i0 < n; i0 += XR_U * st) {
-        double ri[XR_U], pi[XR_U], qi[XR_U], xi[XR_U];
-#pragma unroll
-        for (int k = 0; k < XR_U; k++) {
-            const long i = i0 + k * st;
-            if (i < n) { ri[k] = r[i]; pi[k] = p[i]; qi[k] = q[i]; xi[k] = x[i]; }
-        }
-#pragma unroll
-        for (int k = 0; k < XR_U; k++) {
-            const long i = i0 + k * st;
-            if (i >= n) break;
-            rold[i] = ri[k];
-            x[i] = xi[k] + alpha * pi[k];
-            const double rn = ri[k] - alpha * qi[k];
-            r[i] = rn;
-            if (r32) r32[i] = (float)(rn * inv);
-            v[0] += rn * rn;
-        }
-    }
-    block_reduce_store<1>(v, partials);
-}
-
-// z = a * sqrt(s) widened to FP64, with (z.r, z.rold) in the same pass (partials as k_dot2's)
-__global__ void __launch_bounds__(RB) k_f2d_scaled_dot2(long n, const float* __restrict__ a, double* __restrict__ z,
-                                                        const double* __restrict__ s, const double* __restrict__ r,
-                                                        const double* __restrict__ rold,
-                                                        double* __restrict__ partials) {
-    const double sc = sqrt(fmax(s[0], 1e-300));
+// (z.r, z.q)
+template <typename TZ, typename T>
+__global__ void __launch_bounds__(RB) k_pcg_zdots(long n, const TZ* __restrict__ zs, const double* __restrict__ s,
+                                                  const T* __restrict__ r, const T* __restrict__ q, RedOut ro) {
+    const double sc = z_scale<TZ>(s);
     double v[2] = {0, 0};
     const long st = (long)gridDim.x * blockDim.x;
     for (long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x; i0 < n; i0 += XR_U * st) {
-        float ai[XR_U];
-        double ri[XR_U], oi[XR_U];
+        TZ a[XR_U];
+        T ri[XR_U], qi[XR_U];
 #pragma unroll
         for (int k = 0; k < XR_U; k++) {
             const long i = i0 + k * st;
-            if (i < n) { ai[k] = a[i]; ri[k] = r[i]; oi[k] = rold[i]; }
+            if (i < n) { a[k] = zs[i]; ri[k] = r[i]; qi[k] = q[i]; }
+        }
+#pragma unroll
+        for (int k = 0; k < XR_U; k++) {
+            if (i0 + k * st >= n) break;
+            const double z = (double)a[k] * sc;
+            v[0] += z * (double)ri[k];
+            v[1] += z * (double)qi[k];
+        }
+    }
+    grid_reduce<2>(v, ro);
+}
+
+// x += alpha p (the previous iteration's step), then p = z + beta p
+template <typename TZ, typename T>
+__global__ void __launch_bounds__(RB) k_pcg_xp(long n, const double* __restrict__ scal, const TZ* __restrict__ zs,
+                                               const double* __restrict__ s, T* __restrict__ p, T* __restrict__ x) {
+    const bool first = scal[24] == 0.0;
+    const double sc = z_scale<TZ>(s), pq = scal[20];
+    const T beta = first || pq == 0.0 ? T(0) : (T)(-scal[11] / pq), alpha = first || pq == 0.0 ? T(0) : (T)(scal[12] / pq);
+    const long st = (long)gridDim.x * blockDim.x;
+    for (long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x; i0 < n; i0 += XR_U * st) {
+        TZ a[XR_U];
+        T pi[XR_U], xi[XR_U];
+#pragma unroll
+        for (int k = 0; k < XR_U; k++) {
+            const long i = i0 + k * st;
+            if (i >= n) break;
+            a[k] = zs[i];
+            if (!first) { pi[k] = p[i]; xi[k] = x[i]; }
         }
 #pragma unroll
         for (int k = 0; k < XR_U; k++) {
             const long i = i0 + k * st;
             if (i >= n) break;
-            const double x = (double)ai[k] * sc;
-            z[i] = x;
-            v[0] += x * ri[k];
-            v[1] += x * oi[k];
+            const T z = (T)((double)a[k] * sc);
+            if (first) {
+                p[i] = z;
+            } else {
+                x[i] = xi[k] + alpha * pi[k];
+                p[i] = z + beta * pi[k];
+            }
         }
     }
-    block_reduce_store<2>(v, partials);
+}
+
+// r -= alpha q and r.r.  r32 (optional): the new residual scaled by 1 / sqrt(rr_old) and rounded to FP32, the
+// right-hand side of the next FP32 V-cycle; rr_old (the r.r before this update) is kept in scale_out
+template <typename T>
+__global__ void __launch_bounds__(RB) k_pcg_r_rr(long n, const double* __restrict__ num, const double* __restrict__ den,
+                                                 T* __restrict__ r, const T* __restrict__ q, float* __restrict__ r32,
+                                                 const double* rr_old, double* __restrict__ scale_out, RedOut ro) {
+    const T alpha = den[0] != 0.0 ? (T)(num[0] / den[0]) : T(0);
+    const double old = r32 ? rr_old[0] : 0.0, inv = r32 ? 1.0 / sqrt(fmax(old, 1e-300)) : 0.0;
+    if (r32 && blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = old;
+    double v[1] = {0};
+    // the reduction grid is small (2 blocks per SM): XR_U grid strides per trip keep enough loads in flight
+    const long st = (long)gridDim.x * blockDim.x;
+    for (long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x; i0 < n; i0 += XR_U * st) {
+        T ri[XR_U], qi[XR_U];
+#pragma unroll
+        for (int k = 0; k < XR_U; k++) {
+            const long i = i0 + k * st;
+            if (i < n) { ri[k] = r[i]; qi[k] = q[i]; }
+        }
+#pragma unroll
+        for (int k = 0; k < XR_U; k++) {
+            const long i = i0 + k * st;
+            if (i >= n) break;
+            const T rn = ri[k] - alpha * qi[k];
+            r[i] = rn;
+            if (r32) r32[i] = (float)((double)rn * inv);
+            v[0] += (double)rn * (double)rn;
+        }
+    }
+    grid_reduce<1>(v, ro);
+}
+
+// after the loop: the last iteration's step of x (none if the loop did not run)
+__global__ void k_pcg_x_last(long n, const double* __restrict__ scal, const double* __restrict__ p, double* __restrict__ x) {
+    if (scal[24] == 0.0 || scal[20] == 0.0) return;
+    const double alpha = scal[12] / scal[20];
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) x[i] += alpha * p[i];
 }
 
 // ---- FP32 Krylov vectors (FP64 accumulation of every dot product) ----------------------
 __global__ void __launch_bounds__(RB) k_dot32(long n, const float* __restrict__ a, const float* __restrict__ b,
-                                              double* __restrict__ partials) {
+                                              RedOut ro) {
     double v[1] = {0};
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
         v[0] += (double)a[i] * (double)b[i];
-    block_reduce_store<1>(v, partials);
+    grid_reduce<1>(v, ro);
 }
 
-__global__ void __launch_bounds__(RB) k_dot32_2(long n, const float* __restrict__ a, const float* __restrict__ b,
-                                                const float* __restrict__ c, double* __restrict__ partials) {
-    double v[2] = {0, 0};
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const double x = a[i];
-        v[0] += x * (double)b[i];
-        v[1] += x * (double)c[i];
-    }
-    block_reduce_store<2>(v, partials);
-}
-
-// p = z + beta p (flexible beta as k_pcg_p_it), FP32 vectors
-__global__ void k_pcg32_p(long n, const double* __restrict__ s, const double* __restrict__ it, float* __restrict__ p,
-                          const float* __restrict__ z) {
-    const bool first = it[0] == 0.0;
-    const double den = s[2];
-    const float beta = (first || den == 0.0) ? 0.f : (float)((s[0] - s[1]) / den);
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        p[i] = first ? z[i] : z[i] + beta * p[i];
-}
-
-// d += alpha p, rold = r, r -= alpha q, r.r (FP64 sum) with alpha = num / den
-__global__ void __launch_bounds__(RB) k_pcg32_xr_rr(long n, const double* __restrict__ num, const double* __restrict__ den,
-                                                    float* __restrict__ d, float* __restrict__ r,
-                                                    const float* __restrict__ p, const float* __restrict__ q,
-                                                    float* __restrict__ rold, double* __restrict__ partials) {
-    const float alpha = den[0] != 0.0 ? (float)(num[0] / den[0]) : 0.f;
-    double v[1] = {0};
-    const long st = (long)gridDim.x * blockDim.x;
-    for (long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x; i0 < n; i0 += XR_U * st) {
-        float ri[XR_U], pi[XR_U], qi[XR_U], di[XR_U];
-#pragma unroll
-        for (int k = 0; k < XR_U; k++) {
-            const long i = i0 + k * st;
-            if (i < n) { ri[k] = r[i]; pi[k] = p[i]; qi[k] = q[i]; di[k] = d[i]; }
-        }
-#pragma unroll
-        for (int k = 0; k < XR_U; k++) {
-            const long i = i0 + k * st;
-            if (i >= n) break;
-            rold[i] = ri[k];
-            d[i] = di[k] + alpha * pi[k];
-            const float rn = ri[k] - alpha * qi[k];
-            r[i] = rn;
-            v[0] += (double)rn * (double)rn;
-        }
-    }
-    block_reduce_store<1>(v, partials);
-}
-
-// x += sqrt(s) d (the FP32 correction of a refinement step, scaled back to the FP64 residual)
+// x += sqrt(s) (d + alpha p): the FP32 correction of a refinement step with its last iteration's step, scaled back to
+// the FP64 residual
 __global__ void k_axpy_f32_scaled(long n, double* __restrict__ x, const float* __restrict__ d,
-                                  const double* __restrict__ s) {
+                                  const double* __restrict__ s, const double* __restrict__ scal,
+                                  const float* __restrict__ p) {
     const double sc = sqrt(fmax(s[0], 0.0));
+    const bool step = scal[24] != 0.0 && scal[20] != 0.0;
+    const float alpha = step ? (float)(scal[12] / scal[20]) : 0.f;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        x[i] += sc * (double)d[i];
-}
-
-// p = z + beta p with flexible beta = (r.z - rold.z) / rz_old; scalars: s[0]=r.z, s[1]=rold.z, den=rz_old
-__global__ void k_pcg_p(long n, const double* __restrict__ s, const double* __restrict__ den, double* __restrict__ p,
-                        const double* __restrict__ z, int first) {
-    const double beta = first ? 0.0 : (s[0] - s[1]) / den[0];
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        p[i] = first ? z[i] : z[i] + beta * p[i];
+        x[i] += sc * (double)(step ? d[i] + alpha * p[i] : d[i]);
 }
 
 __global__ void k_scale(long n, double* __restrict__ x, const double* __restrict__ s, int inv_sqrt) {
@@ -320,7 +305,7 @@ __global__ void k_sub_modes(long n, int nrig, const double* __restrict__ Rd, con
 }
 // six dots against the rigid modes in one pass
 __global__ void __launch_bounds__(RB) k_dot6(long n, int nrig, const double* __restrict__ Rd,
-                                             const double* __restrict__ x, double* __restrict__ partials) {
+                                             const double* __restrict__ x, RedOut ro) {
     double v[6] = {0, 0, 0, 0, 0, 0};
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const double xi = x[i];
@@ -328,7 +313,7 @@ __global__ void __launch_bounds__(RB) k_dot6(long n, int nrig, const double* __r
         for (int k = 0; k < 6; k++)
             if (k < nrig) v[k] += Rd[k * n + i] * xi;
     }
-    block_reduce_store<6>(v, partials);
+    grid_reduce<6>(v, ro);
 }
 
 // largest eigenvalue of the symmetric tridiagonal (alpha, beta) by Sturm counts, one warp: each round the 32 lanes
@@ -584,10 +569,10 @@ __global__ void __launch_bounds__(RB) k_oc_update(long ne, const uint8_t* __rest
     }
 }
 
-__global__ void __launch_bounds__(RB) k_count_u8(long n, const uint8_t* __restrict__ a, double* __restrict__ partials) {
+__global__ void __launch_bounds__(RB) k_count_u8(long n, const uint8_t* __restrict__ a, RedOut ro) {
     double v[1] = {0};
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) v[0] += a[i] ? 1.0 : 0.0;
-    block_reduce_store<1>(v, partials);
+    grid_reduce<1>(v, ro);
 }
 
 __global__ void k_node_active(int nx, int ny, int nz, const uint8_t* __restrict__ eact, uint8_t* __restrict__ vact) {
@@ -724,24 +709,13 @@ __global__ void k_mask_copy(long n, long nv, const uint8_t* __restrict__ vact, c
 
 namespace rtk {
 
-static int final_sum(rt_hier* h, int nv_, double* out) {
-    return rt_launch(h->ctx, "reduce_final", [&] {
-        switch (nv_) {
-            case 1: k_final_sum<1><<<1, 32, 0, h->ctx->stream>>>(RT_RED_BLOCKS, h->partials, out); break;
-            case 2: k_final_sum<2><<<1, 32, 0, h->ctx->stream>>>(RT_RED_BLOCKS, h->partials, out); break;
-            default: k_final_sum<6><<<1, 32, 0, h->ctx->stream>>>(RT_RED_BLOCKS, h->partials, out); break;
-        }
-    });
+// the hierarchy's reduction buffers (its launches are ordered on one stream)
+static RedOut red(rt_hier* h, double* out) {
+    return RedOut{h->partials, out, reinterpret_cast<unsigned*>(h->scal + RT_SCAL_TICKET)};
 }
 
 int dot(rt_hier* h, long n, const double* a, const double* b, double* out) {
-    RT_CHECK(rt_launch(h->ctx, "dot", [&] { k_dot<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, a, b, h->partials); }));
-    return final_sum(h, 1, out);
-}
-
-int dot2(rt_hier* h, long n, const double* a, const double* b, const double* c, double* out) {
-    RT_CHECK(rt_launch(h->ctx, "dot2", [&] { k_dot2<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, a, b, c, h->partials); }));
-    return final_sum(h, 2, out);
+    return rt_launch(h->ctx, "dot", [&] { k_dot<<<red_grid(n), RB, 0, h->ctx->stream>>>(n, a, b, red(h, out)); });
 }
 
 int axpy(rt_hier* h, long n, double a, const double* x, double* y) {
@@ -765,62 +739,65 @@ int f2d_scaled_add(rt_hier* h, long n, const float* a, double* b, const double* 
                      [&] { k_f2d_scaled_add<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, a, b, s); });
 }
 
-int pcg_update_xr(rt_hier* h, long n, const double* num, const double* den, double* x, double* r, const double* p,
-                  const double* q, double* rold) {
-    return rt_launch(h->ctx, "pcg_update_xr",
-                     [&] { k_pcg_xr<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, num, den, x, r, p, q, rold); });
+int pcg_zdots(rt_hier* h, long n, const float* z, const double* s, const double* r, const double* q, double* out) {
+    return rt_launch(h->ctx, "pcg_zdots", [&] {
+        k_pcg_zdots<float, double><<<red_grid(n), RB, 0, h->ctx->stream>>>(n, z, s, r, q, red(h, out));
+    });
+}
+int pcg_zdots(rt_hier* h, long n, const double* z, const double* r, const double* q, double* out) {
+    return rt_launch(h->ctx, "pcg_zdots", [&] {
+        k_pcg_zdots<double, double><<<red_grid(n), RB, 0, h->ctx->stream>>>(n, z, nullptr, r, q, red(h, out));
+    });
+}
+int pcg_zdots32(rt_hier* h, long n, const float* z, const float* r, const float* q, double* out) {
+    return rt_launch(h->ctx, "pcg32_zdots", [&] {
+        k_pcg_zdots<float, float><<<red_grid(n), RB, 0, h->ctx->stream>>>(n, z, nullptr, r, q, red(h, out));
+    });
 }
 
-int pcg_update_xr_rr(rt_hier* h, long n, const double* num, const double* den, double* x, double* r, const double* p,
-                     const double* q, double* rold, double* rr_out, float* r32, double* scale_out) {
-    RT_CHECK(rt_launch(h->ctx, "pcg_update_xr", [&] {
-        k_pcg_xr_rr<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, num, den, x, r, p, q, rold, h->partials, r32, rr_out,
-                                                               scale_out);
-    }));
-    return final_sum(h, 1, rr_out);
+int pcg_update_xp(rt_hier* h, long n, const float* z, const double* s, double* p, double* x) {
+    return rt_launch(h->ctx, "pcg_update_xp", [&] {
+        k_pcg_xp<float, double><<<gridN(h->ctx, n), RB, 0, h->ctx->stream>>>(n, h->scal, z, s, p, x);
+    });
+}
+int pcg_update_xp(rt_hier* h, long n, const double* z, double* p, double* x) {
+    return rt_launch(h->ctx, "pcg_update_xp", [&] {
+        k_pcg_xp<double, double><<<gridN(h->ctx, n), RB, 0, h->ctx->stream>>>(n, h->scal, z, nullptr, p, x);
+    });
+}
+int pcg32_update_xp(rt_hier* h, long n, const float* z, float* p, float* d) {
+    return rt_launch(h->ctx, "pcg32_update_xp", [&] {
+        k_pcg_xp<float, float><<<gridN(h->ctx, n), RB, 0, h->ctx->stream>>>(n, h->scal, z, nullptr, p, d);
+    });
 }
 
-int f2d_scaled_dot2(rt_hier* h, long n, const float* a, double* z, const double* s, const double* r,
-                    const double* rold, double* out) {
-    RT_CHECK(rt_launch(h->ctx, "f2d_scaled", [&] {
-        k_f2d_scaled_dot2<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, a, z, s, r, rold, h->partials);
-    }));
-    return final_sum(h, 2, out);
+int pcg_update_r_rr(rt_hier* h, long n, double* r, const double* q, float* r32) {
+    return rt_launch(h->ctx, "pcg_update_r", [&] {
+        k_pcg_r_rr<double><<<red_grid(n), RB, 0, h->ctx->stream>>>(n, h->scal + 10, h->scal + 20, r, q, r32, h->scal + 21,
+                                                                   h->scal + 23, red(h, h->scal + 21));
+    });
+}
+int pcg32_update_r_rr(rt_hier* h, long n, float* r, const float* q) {
+    return rt_launch(h->ctx, "pcg32_update_r", [&] {
+        k_pcg_r_rr<float><<<red_grid(n), RB, 0, h->ctx->stream>>>(n, h->scal + 10, h->scal + 20, r, q, nullptr, nullptr,
+                                                                  nullptr, red(h, h->scal + 21));
+    });
+}
+
+int pcg_x_last(rt_hier* h, long n, double* x) {
+    return rt_launch(h->ctx, "pcg_x_last", [&] {
+        k_pcg_x_last<<<gridN(h->ctx, n), RB, 0, h->ctx->stream>>>(n, h->scal, h->p, x);
+    });
 }
 
 int dot32(rt_hier* h, long n, const float* a, const float* b, double* out) {
-    RT_CHECK(rt_launch(h->ctx, "dot32", [&] { k_dot32<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, a, b, h->partials); }));
-    return final_sum(h, 1, out);
-}
-
-int dot32_2(rt_hier* h, long n, const float* a, const float* b, const float* c, double* out) {
-    RT_CHECK(rt_launch(h->ctx, "dot32_2", [&] {
-        k_dot32_2<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, a, b, c, h->partials);
-    }));
-    return final_sum(h, 2, out);
-}
-
-int pcg32_update_p(rt_hier* h, long n, const double* s, const double* it, float* p, const float* z) {
-    return rt_launch(h->ctx, "pcg32_update_p",
-                     [&] { k_pcg32_p<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, s, it, p, z); });
-}
-
-int pcg32_update_xr_rr(rt_hier* h, long n, const double* num, const double* den, float* d, float* r, const float* p,
-                       const float* q, float* rold, double* rr_out) {
-    RT_CHECK(rt_launch(h->ctx, "pcg32_update_xr", [&] {
-        k_pcg32_xr_rr<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, num, den, d, r, p, q, rold, h->partials);
-    }));
-    return final_sum(h, 1, rr_out);
+    return rt_launch(h->ctx, "dot32", [&] { k_dot32<<<red_grid(n), RB, 0, h->ctx->stream>>>(n, a, b, red(h, out)); });
 }
 
 int axpy_f32_scaled(rt_hier* h, long n, double* x, const float* d, const double* s) {
-    return rt_launch(h->ctx, "axpy_f32",
-                     [&] { k_axpy_f32_scaled<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, x, d, s); });
-}
-
-int pcg_update_p(rt_hier* h, long n, const double* s, const double* den, double* p, const double* z, bool first) {
-    return rt_launch(h->ctx, "pcg_update_p",
-                     [&] { k_pcg_p<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, s, den, p, z, first ? 1 : 0); });
+    return rt_launch(h->ctx, "axpy_f32", [&] {
+        k_axpy_f32_scaled<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, x, d, s, h->scal, h->p32k);
+    });
 }
 
 int scale(rt_hier* h, long n, double* x, const double* s, bool inv_sqrt) {
@@ -864,9 +841,8 @@ int project_load(rt_hier* h, double* f) {
         }));
     if (h->nrig > 0 && n > 0) {
         RT_CHECK(rt_launch(h->ctx, "dot6", [&] {
-            k_dot6<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, h->nrig, h->Rd, h->fs, h->partials);
+            k_dot6<<<red_grid(n), RB, 0, h->ctx->stream>>>(n, h->nrig, h->Rd, h->fs, red(h, h->scal + 40));
         }));
-        RT_CHECK(final_sum(h, 6, h->scal + 40));
         RT_CHECK(rt_launch(h->ctx, "sub_modes", [&] {
             k_sub_modes<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, h->nrig, h->Rd, h->scal + 40, h->fs);
         }));
@@ -878,8 +854,9 @@ int project_load(rt_hier* h, double* f) {
 int displacement_project(rt_hier* h, double* u) {
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
-    RT_CHECK(rt_launch(h->ctx, "dot6", [&] { k_dot6<<<RT_RED_BLOCKS, RB, 0, h->ctx->stream>>>(n, 6, h->Ru, u, h->partials); }));
-    RT_CHECK(final_sum(h, 6, h->scal + 40));
+    RT_CHECK(rt_launch(h->ctx, "dot6", [&] {
+        k_dot6<<<red_grid(n), RB, 0, h->ctx->stream>>>(n, 6, h->Ru, u, red(h, h->scal + 40));
+    }));
     return rt_launch(h->ctx, "sub_modes",
                      [&] { k_sub_modes<<<gridN(h->ctx, n), 256, 0, h->ctx->stream>>>(n, 6, h->Ru, h->scal + 40, u); });
 }
@@ -954,10 +931,12 @@ int oc_update(rt_hier* h, float vgoal, double* res) {
 }
 
 int count_u8(rt_ctx* c, long n, const uint8_t* a, double* out) {
-    double* part = nullptr;
-    RT_CUDA(c, cudaMallocAsync(&part, sizeof(double) * RT_RED_BLOCKS, c->stream));
-    RT_CHECK(rt_launch(c, "count_u8", [&] { k_count_u8<<<RT_RED_BLOCKS, RB, 0, c->stream>>>(n, a, part); }));
-    RT_CHECK(rt_launch(c, "reduce_final", [&] { k_final_sum<1><<<1, 32, 0, c->stream>>>(RT_RED_BLOCKS, part, out); }));
+    double* part = nullptr;  // partial sums and, after them, the ticket
+    RT_CUDA(c, cudaMallocAsync(&part, sizeof(double) * (RT_RED_BLOCKS + 1), c->stream));
+    RT_CUDA(c, cudaMemsetAsync(part + RT_RED_BLOCKS, 0, sizeof(double), c->stream));
+    RT_CHECK(rt_launch(c, "count_u8", [&] {
+        k_count_u8<<<RT_RED_BLOCKS, RB, 0, c->stream>>>(n, a, RedOut{part, out, reinterpret_cast<unsigned*>(part + RT_RED_BLOCKS)});
+    }));
     RT_CUDA(c, cudaFreeAsync(part, c->stream));
     return RT_OK;
 }

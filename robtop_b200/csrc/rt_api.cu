@@ -315,7 +315,7 @@ static void free_workspace(rt_hier* w) {
         cudaFree(L.d); cudaFree(L.d32); cudaFree(L.dvec);
     }
     cudaFree(w->x); cudaFree(w->rr); cudaFree(w->z); cudaFree(w->p); cudaFree(w->q);
-    cudaFree(w->partials); cudaFree(w->scal);
+    cudaFree(w->partials); cudaFree(w->scal); cudaFree(w->kpart);
     if (w->pcg_exec) cudaGraphExecDestroy(w->pcg_exec);
     if (w->pcg_graph) cudaGraphDestroy(w->pcg_graph);
     if (w->pcg_exec_alt) cudaGraphExecDestroy(w->pcg_exec_alt);
@@ -350,7 +350,7 @@ static void free_hier(rt_hier* h) {
     cudaFree(h->sens); cudaFree(h->ftmp); cudaFree(h->eshell); cudaFree(h->load_nodes); cudaFree(h->load_normal);
     cudaFree(h->Rd); cudaFree(h->Ru); cudaFree(h->fs); cudaFree(h->fs_old); cudaFree(h->x); cudaFree(h->rr);
     cudaFree(h->z); cudaFree(h->p); cudaFree(h->q); cudaFree(h->rold); cudaFree(h->Q); cudaFree(h->partials);
-    cudaFree(h->scal); cudaFree(h->Qgal); cudaFree(h->dinv64); cudaFree(h->dinv32); cudaFree(h->ncode);
+    cudaFree(h->scal); cudaFree(h->kpart); cudaFree(h->Qgal); cudaFree(h->dinv64); cudaFree(h->dinv32); cudaFree(h->ncode);
     if (h->pcg_exec) cudaGraphExecDestroy(h->pcg_exec);
     if (h->pcg_graph) cudaGraphDestroy(h->pcg_graph);
     if (h->pcg_exec_alt) cudaGraphExecDestroy(h->pcg_exec_alt);
@@ -529,6 +529,7 @@ static int build_hier(rt_ctx* c, const rt_params* p, int nx, int ny, int nz, uin
     RT_CHECK(dalloc(c, &h->x, n3)); RT_CHECK(dalloc(c, &h->rr, n3)); RT_CHECK(dalloc(c, &h->z, n3));
     RT_CHECK(dalloc(c, &h->p, n3)); RT_CHECK(dalloc(c, &h->q, n3)); RT_CHECK(dalloc(c, &h->rold, n3));
     RT_CHECK(dalloc(c, &h->partials, RT_PARTIALS));
+    RT_CHECK(dalloc(c, &h->kpart, rtk::face_dot_partials(L0.vx, L0.vy, L0.vz)));
     RT_CHECK(dalloc(c, &h->scal, RT_NSCAL));
     RT_CUDA(c, cudaMemsetAsync(h->scal, 0, sizeof(double) * RT_NSCAL, c->stream));
     RT_CHECK(upload_KE(h));
@@ -1609,42 +1610,12 @@ static int precondition(rt_hier* h, const double* r, double* z, const double* rr
     return RT_OK;
 }
 
-// end of an iteration: it += 1, rz_prev = rz; optionally set the WHILE condition of the graph
-__global__ void k_pcg_tail(double* __restrict__ scal, cudaGraphConditionalHandle cond, int use_cond) {
-    if (threadIdx.x != 0) return;
-    const double it = scal[24] + 1.0;
-    scal[24] = it;
-    scal[12] = scal[10];
-    // learned-correction fallback: off for the rest of the solve once an iteration's residual
-    // norm did not drop below ratio x the previous one
-    if (scal[28] != 0.0 && scal[29] > 0.0 && !(scal[21] <= scal[27] * scal[27] * scal[29])) scal[28] = 0.0;
-    scal[29] = scal[21];
-    // precision fallback: the loop ends once |r| has not halved within scal[93] iterations (0: off);
-    // scal[90] is the last halving's r.r, scal[91] its iteration, scal[92] the flag
-    bool stalled = false;
-    if (scal[93] > 0.0) {
-        if (scal[21] <= 0.25 * scal[90]) {
-            scal[90] = scal[21];
-            scal[91] = it;
-        } else if (it - scal[91] >= scal[93]) {
-            scal[92] = 1.0;
-            stalled = true;
-        }
-    }
-    if (use_cond) {
-        const double rr = scal[21], bb = scal[22] > 0 ? scal[22] : 1.0;
-        const bool go = isfinite(rr) && sqrt(rr) > scal[25] * sqrt(bb) && it < scal[26] && !stalled;
-        cudaGraphSetConditional(cond, go ? 1u : 0u);
-    }
-}
-
 // one MG-PCG iteration, all scalars on the device (graph-capturable); the iteration's step of x is taken by the next
 // one, the last by pcg_x_last
 static int pcg_body(rt_hier* h, double* x, double* r, bool no_support, cudaGraphConditionalHandle cond,
                     int use_cond = 0) {
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
-    rt_ctx* c = h->ctx;
     const bool fz = fused_f32_rhs(h);
     const double* zscale = h->scal + (fz ? 23 : 21);
     // the projection of z (no supports) and the learned correction work on the FP64 z
@@ -1658,10 +1629,8 @@ static int pcg_body(rt_hier* h, double* x, double* r, bool no_support, cudaGraph
         RT_CHECK(rtk::pcg_zdots(h, n, h->z, r, h->q, h->scal + 10));
         RT_CHECK(rtk::pcg_update_xp(h, n, h->z, h->p, x));
     }
-    RT_CHECK(rtk::fine_applyK<double>(h, h->p, h->q));
-    RT_CHECK(rtk::dot(h, n, h->p, h->q, h->scal + 20));
-    RT_CHECK(rtk::pcg_update_r_rr(h, n, r, h->q, fz ? L.f32 : nullptr));
-    return rt_launch(c, "pcg_tail", [&] { k_pcg_tail<<<1, 32, 0, c->stream>>>(h->scal, cond, use_cond); });
+    RT_CHECK(rtk::fine_applyK_dot<double>(h, h->p, h->q, h->scal + 20));
+    return rtk::pcg_update_r_rr(h, n, r, h->q, fz ? L.f32 : nullptr, cond, use_cond);
 }
 
 // the whole iteration loop as one graph: a WHILE conditional node whose body is one
@@ -1795,14 +1764,11 @@ static int ensure_krylov32(rt_hier* h) {
 static int pcg32_body(rt_hier* h, cudaGraphConditionalHandle cond, int use_cond) {
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
-    rt_ctx* c = h->ctx;
     RT_CHECK(vcycle_T<float>(h, h->P.smoother, h->P.pre_sweeps, h->P.post_sweeps, h->P.jacobi_omega, 0, true));
     RT_CHECK(rtk::pcg_zdots32(h, n, L.u32, L.f32, h->q32k, h->scal + 10));
     RT_CHECK(rtk::pcg32_update_xp(h, n, L.u32, h->p32k, h->d32k));
-    RT_CHECK(rtk::fine_applyK<float>(h, h->p32k, h->q32k));
-    RT_CHECK(rtk::dot32(h, n, h->p32k, h->q32k, h->scal + 20));
-    RT_CHECK(rtk::pcg32_update_r_rr(h, n, L.f32, h->q32k));
-    return rt_launch(c, "pcg_tail", [&] { k_pcg_tail<<<1, 32, 0, c->stream>>>(h->scal, cond, use_cond); });
+    RT_CHECK(rtk::fine_applyK_dot<float>(h, h->p32k, h->q32k, h->scal + 20));
+    return rtk::pcg32_update_r_rr(h, n, L.f32, h->q32k, cond, use_cond);
 }
 
 // the inner loop as one graph with a WHILE conditional node (as pcg_graph_run)
@@ -2786,6 +2752,7 @@ static int make_workspace(rt_hier* p, rt_hier** out) {
     RT_CHECK(dalloc(c, &w->x, n3)); RT_CHECK(dalloc(c, &w->rr, n3)); RT_CHECK(dalloc(c, &w->z, n3));
     RT_CHECK(dalloc(c, &w->p, n3)); RT_CHECK(dalloc(c, &w->q, n3));
     RT_CHECK(dalloc(c, &w->partials, RT_PARTIALS));
+    RT_CHECK(dalloc(c, &w->kpart, rtk::face_dot_partials(w->L[0].vx, w->L[0].vy, w->L[0].vz)));
     RT_CHECK(dalloc(c, &w->scal, RT_NSCAL));
     RT_CUDA(c, cudaMemsetAsync(w->scal, 0, sizeof(double) * RT_NSCAL, c->stream));
     ws_sync(w);

@@ -42,11 +42,12 @@ __device__ __forceinline__ T face_rcp(T x) {
 // MODE 2: unew = u + omega D^-1 (f - K u)     MODE 3: Chebyshev step kstep: d = a_k d + b_k D^-1 (f - K u), unew = u + d
 // (fixed nodes in MODE 2/3: unew = f / n_e, d = 0; inactive nodes: 0)
 // code: per node, bit 0 active, bit 1 fixed (supports), for fixed nodes n_e << 2
-template <typename T, bool WS, int MODE, int R, int W, int MINB>
+template <typename T, bool WS, int MODE, int R, int W, int MINB, bool DOT>
 __global__ void __launch_bounds__(32 * W, MINB)
     k_fine_face(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code, const float* __restrict__ wgt,
                 const rte::KtVals<T> kt, const T* __restrict__ u, const T* __restrict__ f, T* __restrict__ out, T omega,
-                T* __restrict__ dvec, const double* __restrict__ coef, int kstep) {
+                T* __restrict__ dvec, const double* __restrict__ coef, int kstep, double* __restrict__ partials,
+                double* __restrict__ dot_out, unsigned* __restrict__ ticket) {
     constexpr int NX = MODE >= 2 ? 8 : 6;  // values handed to the next warp
     __shared__ T S[2][W][NX][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
         }
     };
 
+    double pq = 0;  // DOT: the thread's part of u . out
     T F[R][12];  // forward face data of node layer t
     T G[R][12];  // inverse z output of element layer t - 1 toward node layer t
     uint32_t co[R];
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
             for (int c = 0; c < 3; c++) {
                 fv[r][c] = (MODE != 1 && ld) ? f[c * nv + v] : T(0);
                 dv[r][c] = (MODE == 3 && ld && kstep > 0) ? dvec[c * nv + v] : T(0);
-                uo[r][c] = ((MODE >= 2 || (WS && MODE == 1 && co[r] > 1u)) && ld) ? u[c * nv + v] : T(0);  // in L1: layer t was fetched two layers ago
+                uo[r][c] = ((MODE >= 2 || DOT || (WS && MODE == 1 && co[r] > 1u)) && ld) ? u[c * nv + v] : T(0);  // in L1: layer t was fetched two layers ago
             }
         }
         if (MODE >= 2) {
@@ -229,7 +231,10 @@ __global__ void __launch_bounds__(32 * W, MINB)
                     for (int c = 0; c < 3; c++) o[c] = act ? (fixed ? fv[r][c] : fv[r][c] - acc[c]) : T(0);
                 } else if (MODE == 1) {
 #pragma unroll
-                    for (int c = 0; c < 3; c++) o[c] = act ? (fixed ? uo[r][c] : acc[c]) : T(0);
+                    for (int c = 0; c < 3; c++) {
+                        o[c] = act ? (fixed ? uo[r][c] : acc[c]) : T(0);
+                        if (DOT) pq += (double)uo[r][c] * (double)o[c];
+                    }
                 } else if (fixed) {
 #pragma unroll
                     for (int c = 0; c < 3; c++) o[c] = fv[r][c] / T(co[r] >> 2);
@@ -267,6 +272,35 @@ __global__ void __launch_bounds__(32 * W, MINB)
                 for (int q = 0; q < 4; q++) Qp[r][q] = Q[q];
             co[r] = cn[r];
         }
+    }
+    if (DOT) {  // block sums, added by the last block in their order (no second launch and no second read of u and out)
+        __shared__ double sd[W];
+        __shared__ bool last;
+        auto block_sum = [&](double x) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+            __syncthreads();
+            if (lane == 0) sd[w] = x;
+            __syncthreads();
+            double a = 0;
+#pragma unroll
+            for (int i = 0; i < W; i++) a += sd[i];
+            return a;
+        };
+        const double b = block_sum(pq);
+        const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+        if (threadIdx.x == 0) {
+            partials[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = b;
+            __threadfence();
+            last = atomicInc(ticket, nb - 1) == nb - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        double a = 0;
+        for (unsigned i = threadIdx.x; i < nb; i += 32 * W) a += __ldcg(partials + i);
+        a = block_sum(a);
+        if (threadIdx.x == 0) dot_out[0] = a;
     }
 }
 
@@ -352,16 +386,17 @@ __global__ void k_node_code(int nx, int ny, int nz, const uint8_t* __restrict__ 
     }
 }
 
-template <typename T, bool WS, int MODE, int R, int W, int MINB>
+template <typename T, bool WS, int MODE, int R, int W, int MINB, bool DOT>
 int launch_face_rw(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
-                   const double* coef, int kstep) {
+                   const double* coef, int kstep, double* dot_out) {
     rt_level& L = h->L[0];
     const int zc = h->tune[sizeof(T) == 8 ? 1 : 0][MODE].zchunk;
     const dim3 grid((L.vx + FACE_NX - 1) / FACE_NX, (L.vy + W * R - 2) / (W * R - 1), (L.vz + zc - 1) / zc);
     const rte::KtVals<T> kt = rte::make_kt<T>(h);
     return rt_launch(h->ctx, name, [&] {
-        k_fine_face<T, WS, MODE, R, W, MINB><<<grid, 32 * W, 0, h->ctx->stream>>>(
-            L.nx, L.ny, L.nz, zc, h->ncode, h->w, kt, u, f, out, (T)omega, dvec, coef, kstep);
+        k_fine_face<T, WS, MODE, R, W, MINB, DOT><<<grid, 32 * W, 0, h->ctx->stream>>>(
+            L.nx, L.ny, L.nz, zc, h->ncode, h->w, kt, u, f, out, (T)omega, dvec, coef, kstep, h->kpart, dot_out,
+            reinterpret_cast<unsigned*>(h->scal + RT_SCAL_TICKET));
     });
 }
 
@@ -400,18 +435,46 @@ template int fine_smooth0<float>(rt_hier*, const float*, float*, double, float*,
 // the block shape of ty element rows per warp (measured on 511x256x256, where a spill costs more than a block):
 // FP32 1 row 8 warps, 2 rows 4 warps; FP64 1 row, 12 warps in one block per SM, 8 where the smoothing step needs
 // the registers (845 us residual and 1526 us Chebyshev step; two blocks of 8 warps with spills: 1287 and 2431 us)
+template <typename T, bool WS, int MODE, bool DOT>
+static int launch_face_shape(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
+                             const double* coef, int kstep, double* dot_out) {
+    if constexpr (sizeof(T) == 8) {
+        constexpr int W = face_warps(true, MODE, 1);
+        return launch_face_rw<T, WS, MODE, 1, W, 1, DOT>(h, u, f, out, omega, name, dvec, coef, kstep, dot_out);
+    } else {
+        if (h->tune[0][MODE].ty == 1)
+            return launch_face_rw<T, WS, MODE, 1, 8, 3, DOT>(h, u, f, out, omega, name, dvec, coef, kstep, dot_out);
+        return launch_face_rw<T, WS, MODE, 2, 4, 4, DOT>(h, u, f, out, omega, name, dvec, coef, kstep, dot_out);
+    }
+}
+
 template <typename T, bool WS, int MODE>
 int launch_face(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
                 const double* coef, int kstep) {
-    if constexpr (sizeof(T) == 8) {
-        constexpr int W = face_warps(true, MODE, 1);
-        return launch_face_rw<T, WS, MODE, 1, W, 1>(h, u, f, out, omega, name, dvec, coef, kstep);
-    } else {
-        if (h->tune[0][MODE].ty == 1)
-            return launch_face_rw<T, WS, MODE, 1, 8, 3>(h, u, f, out, omega, name, dvec, coef, kstep);
-        return launch_face_rw<T, WS, MODE, 2, 4, 4>(h, u, f, out, omega, name, dvec, coef, kstep);
-    }
+    return launch_face_shape<T, WS, MODE, false>(h, u, f, out, omega, name, dvec, coef, kstep, nullptr);
 }
+
+// partial sums of K u's dot product: one per block of the smallest launch shape (7 rows, one layer)
+size_t face_dot_partials(int vx, int vy, int vz) {
+    return (size_t)((vx + FACE_NX - 1) / FACE_NX) * ((vy + 6) / 7) * vz;
+}
+
+// out = K u and dot_dev = u . out
+template <typename T>
+int fine_applyK_dot(rt_hier* h, const T* u, T* out, double* dot_dev) {
+    const rt_tile_cfg& tn = h->tune[sizeof(T) == 8 ? 1 : 0][1];
+    const long n = 3 * h->L[0].nv;
+    if (tn.variant != 8 || n >= (1L << 31)) {  // the other kernels leave the dot product to a pass of its own
+        RT_CHECK(fine_applyK<T>(h, u, out));
+        if constexpr (sizeof(T) == 8) return dot(h, n, u, out, dot_dev);
+        else return dot32(h, n, u, out, dot_dev);
+    }
+    const char* nm = sizeof(T) == 8 ? "fine_applyK_f64" : "fine_applyK_f32";
+    return h->has_support ? launch_face_shape<T, true, 1, true>(h, u, nullptr, out, 0.0, nm, nullptr, nullptr, 0, dot_dev)
+                          : launch_face_shape<T, false, 1, true>(h, u, nullptr, out, 0.0, nm, nullptr, nullptr, 0, dot_dev);
+}
+template int fine_applyK_dot<double>(rt_hier*, const double*, double*, double*);
+template int fine_applyK_dot<float>(rt_hier*, const float*, float*, double*);
 
 // the launch shape used before rt_autotune ran: the z-chunk whose waves of blocks march through the fewest layers
 // (a chunk of zc layers takes zc + 2 steps).  64x32x32: 2, 129x97x85: 16, 255x256x128: 16, as the sweep found best

@@ -142,6 +142,7 @@ struct rt_hier {
     double* Q = nullptr;
     int Qcap = 0;
     // reductions
+    double* kpart = nullptr;     // block sums of fine_applyK_dot
     double* partials = nullptr;  // [RT_RED_BLOCKS * 8]
     // FP32 Krylov vectors of the refinement form (rt_params.krylov_fp32), allocated on first use
     float *p32k = nullptr, *q32k = nullptr, *d32k = nullptr;
@@ -265,6 +266,9 @@ int fine_residual(rt_hier* h, const T* u, const T* f, T* r);
 template <typename T>
 int fine_applyK(rt_hier* h, const T* u, T* out);
 template <typename T>
+int fine_applyK_dot(rt_hier* h, const T* u, T* out, double* dot_dev);  // and u . out
+size_t face_dot_partials(int vx, int vy, int vz);
+template <typename T>
 int fine_gs(rt_hier* h, T* u, const T* f, bool backward);
 template <typename T>
 int fine_jacobi(rt_hier* h, const T* u, const T* f, T* unew, double omega);
@@ -331,8 +335,9 @@ int pcg_zdots32(rt_hier* h, long n, const float* z, const float* r, const float*
 int pcg_update_xp(rt_hier* h, long n, const float* z, const double* s, double* p, double* x);
 int pcg_update_xp(rt_hier* h, long n, const double* z, double* p, double* x);
 int pcg32_update_xp(rt_hier* h, long n, const float* z, float* p, float* d);
-int pcg_update_r_rr(rt_hier* h, long n, double* r, const double* q, float* r32);
-int pcg32_update_r_rr(rt_hier* h, long n, float* r, const float* q);
+// r -= alpha q, r.r and the end of the iteration (iteration count, stall and correction gates, the loop condition)
+int pcg_update_r_rr(rt_hier* h, long n, double* r, const double* q, float* r32, cudaGraphConditionalHandle cond, int use_cond);
+int pcg32_update_r_rr(rt_hier* h, long n, float* r, const float* q, cudaGraphConditionalHandle cond, int use_cond);
 int pcg_x_last(rt_hier* h, long n, double* x);
 int dot32(rt_hier* h, long n, const float* a, const float* b, double* out);
 int axpy_f32_scaled(rt_hier* h, long n, double* x, const float* d, const double* s);

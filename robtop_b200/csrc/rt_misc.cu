@@ -66,7 +66,7 @@ __device__ __forceinline__ void block_reduce(double (&v)[NV]) {
 // at zero again) adds them in a fixed order, so that the sum does not depend on which block that is.  One launch
 // where a second one added the partial sums (6 us, three times a PCG iteration).
 template <int NV>
-__device__ __forceinline__ void grid_reduce(double (&v)[NV], const RedOut& o) {
+__device__ __forceinline__ bool grid_reduce(double (&v)[NV], const RedOut& o) {
     __shared__ bool last;
     block_reduce<NV>(v);
     if (threadIdx.x == 0) {
@@ -76,7 +76,7 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NV], const RedOut& o) {
         last = atomicInc(o.ticket, gridDim.x - 1) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last) return;
+    if (!last) return false;
     __threadfence();
     double t[NV];
 #pragma unroll
@@ -88,6 +88,7 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NV], const RedOut& o) {
     if (threadIdx.x == 0)
 #pragma unroll
         for (int k = 0; k < NV; k++) o.out[k] = t[k];
+    return true;  // in the block that holds the sums
 }
 
 __global__ void __launch_bounds__(RB) k_dot(long n, const double* __restrict__ a, const double* __restrict__ b,
@@ -195,12 +196,41 @@ __global__ void __launch_bounds__(RB) k_pcg_xp(long n, const double* __restrict_
     }
 }
 
-// r -= alpha q and r.r.  r32 (optional): the new residual scaled by 1 / sqrt(rr_old) and rounded to FP32, the
+// end of an iteration, by one thread: it += 1, rz_prev = rz; optionally set the WHILE condition of the graph
+__device__ __forceinline__ void pcg_end(double* scal, cudaGraphConditionalHandle cond, int use_cond) {
+    const double it = scal[24] + 1.0;
+    scal[24] = it;
+    scal[12] = scal[10];
+    // learned-correction fallback: off for the rest of the solve once an iteration's residual
+    // norm did not drop below ratio x the previous one
+    if (scal[28] != 0.0 && scal[29] > 0.0 && !(scal[21] <= scal[27] * scal[27] * scal[29])) scal[28] = 0.0;
+    scal[29] = scal[21];
+    // precision fallback: the loop ends once |r| has not halved within scal[93] iterations (0: off);
+    // scal[90] is the last halving's r.r, scal[91] its iteration, scal[92] the flag
+    bool stalled = false;
+    if (scal[93] > 0.0) {
+        if (scal[21] <= 0.25 * scal[90]) {
+            scal[90] = scal[21];
+            scal[91] = it;
+        } else if (it - scal[91] >= scal[93]) {
+            scal[92] = 1.0;
+            stalled = true;
+        }
+    }
+    if (use_cond) {
+        const double rr = scal[21], bb = scal[22] > 0 ? scal[22] : 1.0;
+        const bool go = isfinite(rr) && sqrt(rr) > scal[25] * sqrt(bb) && it < scal[26] && !stalled;
+        cudaGraphSetConditional(cond, go ? 1u : 0u);
+    }
+}
+
+// r -= alpha q, r.r and the end of the iteration (by the last block, which has the sum).  r32 (optional): the new residual scaled by 1 / sqrt(rr_old) and rounded to FP32, the
 // right-hand side of the next FP32 V-cycle; rr_old (the r.r before this update) is kept in scale_out
 template <typename T>
 __global__ void __launch_bounds__(RB) k_pcg_r_rr(long n, const double* __restrict__ num, const double* __restrict__ den,
                                                  T* __restrict__ r, const T* __restrict__ q, float* __restrict__ r32,
-                                                 const double* rr_old, double* __restrict__ scale_out, RedOut ro) {
+                                                 const double* rr_old, double* __restrict__ scale_out, RedOut ro,
+                                                 double* scal, cudaGraphConditionalHandle cond, int use_cond) {
     const T alpha = den[0] != 0.0 ? (T)(num[0] / den[0]) : T(0);
     const double old = r32 ? rr_old[0] : 0.0, inv = r32 ? 1.0 / sqrt(fmax(old, 1e-300)) : 0.0;
     if (r32 && blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = old;
@@ -224,7 +254,7 @@ __global__ void __launch_bounds__(RB) k_pcg_r_rr(long n, const double* __restric
             v[0] += (double)rn * (double)rn;
         }
     }
-    grid_reduce<1>(v, ro);
+    if (grid_reduce<1>(v, ro) && threadIdx.x == 0) pcg_end(scal, cond, use_cond);
 }
 
 // after the loop: the last iteration's step of x (none if the loop did not run)
@@ -771,16 +801,17 @@ int pcg32_update_xp(rt_hier* h, long n, const float* z, float* p, float* d) {
     });
 }
 
-int pcg_update_r_rr(rt_hier* h, long n, double* r, const double* q, float* r32) {
+int pcg_update_r_rr(rt_hier* h, long n, double* r, const double* q, float* r32, cudaGraphConditionalHandle cond,
+                    int use_cond) {
     return rt_launch(h->ctx, "pcg_update_r", [&] {
         k_pcg_r_rr<double><<<red_grid(n), RB, 0, h->ctx->stream>>>(n, h->scal + 10, h->scal + 20, r, q, r32, h->scal + 21,
-                                                                   h->scal + 23, red(h, h->scal + 21));
+                                                                   h->scal + 23, red(h, h->scal + 21), h->scal, cond, use_cond);
     });
 }
-int pcg32_update_r_rr(rt_hier* h, long n, float* r, const float* q) {
+int pcg32_update_r_rr(rt_hier* h, long n, float* r, const float* q, cudaGraphConditionalHandle cond, int use_cond) {
     return rt_launch(h->ctx, "pcg32_update_r", [&] {
         k_pcg_r_rr<float><<<red_grid(n), RB, 0, h->ctx->stream>>>(n, h->scal + 10, h->scal + 20, r, q, nullptr, nullptr,
-                                                                  nullptr, red(h, h->scal + 21));
+                                                                  nullptr, red(h, h->scal + 21), h->scal, cond, use_cond);
     });
 }
 

@@ -345,6 +345,7 @@ static void free_hier(rt_hier* h) {
         cudaFree(L.u32); cudaFree(L.f32); cudaFree(L.r32); cudaFree(L.st); cudaFree(L.st32); cudaFree(L.st16);
         cudaFree(L.d); cudaFree(L.d32);
         cudaFree(L.aidx); cudaFree(L.ainv); cudaFree(L.dvec);
+        cudaFree(L.crow); cudaFree(L.cpanels); cudaFree(L.cstatus); cudaFree(L.crigid); cudaFree(L.cfix);
     }
     cudaFree(h->KE_dev); cudaFree(h->KE32_dev); cudaFree(h->rho); cudaFree(h->w); cudaFree(h->vfix);
     cudaFree(h->sens); cudaFree(h->ftmp); cudaFree(h->eshell); cudaFree(h->load_nodes); cudaFree(h->load_normal);

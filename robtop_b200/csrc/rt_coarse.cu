@@ -1440,7 +1440,8 @@ int galerkin_from_elements(rt_hier* h) {
     const float* w = h->w;
     uint8_t* cfix = nullptr;
     if (h->has_support) {  // ftmp: element scratch of the filter
-        RT_CUDA(c, cudaMallocAsync(&cfix, (size_t)Cc.ne, c->stream));
+        if (!Cc.cfix) RT_CUDA(c, cudaMalloc(&Cc.cfix, (size_t)Cc.ne));
+        cfix = Cc.cfix;
         RT_CUDA(c, cudaMemsetAsync(cfix, 0, (size_t)Cc.ne, c->stream));
         RT_CHECK(rt_launch(c, "galerkin_weights", [&] {
             const unsigned g = grid_for(c, F.ne, ST_BS);
@@ -1473,7 +1474,6 @@ int galerkin_from_elements(rt_hier* h) {
                                                                 h->vfix, h->KE_dev, Cc.st);
         }));
     }
-    RT_CUDA(c, cudaFreeAsync(cfix, c->stream));
     return RT_OK;
 }
 

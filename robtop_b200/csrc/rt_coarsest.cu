@@ -269,33 +269,26 @@ __global__ void __launch_bounds__(256) k_coarsest(int na, int nv, const int* __r
 
 namespace rtk {
 
-int coarsest_setup(rt_hier* h) {
+// what the coarsest set-up needs besides the matrix, made once per hierarchy: the stream-ordered allocations and the
+// host round trip of the index map that every call made here took 1 ms and, where the pool had given its memory back
+// to the system, up to a second
+static int coarsest_workspace(rt_hier* h, bool rigid) {
     rt_ctx* c = h->ctx;
     rt_level& L = h->L.back();
     const int na = L.na, n = 3 * na;
-    if (na == 0) return rt_fail(c, RT_ESTATE, "coarsest level has no active node");
-    // rowof on device (node -> active index)
+    if (L.crow && (L.crigid || !rigid)) return RT_OK;
     std::vector<int> aidx_h(na), rowof_h(L.nv, -1);
     RT_CUDA(c, cudaMemcpyAsync(aidx_h.data(), L.aidx, sizeof(int) * na, cudaMemcpyDeviceToHost, c->stream));
     RT_CUDA(c, cudaStreamSynchronize(c->stream));
     for (int i = 0; i < na; i++) rowof_h[aidx_h[i]] = i;
-    int* rowof = nullptr;
-    double *panels = nullptr, *R = nullptr;
-    int* status = nullptr;
-    RT_CUDA(c, cudaMallocAsync(&rowof, sizeof(int) * L.nv, c->stream));
-    RT_CUDA(c, cudaMallocAsync(&panels, sizeof(double) * 4 * GJ_B * n, c->stream));
-    RT_CUDA(c, cudaMallocAsync(&status, sizeof(int), c->stream));
-    RT_CUDA(c, cudaMemcpyAsync(rowof, rowof_h.data(), sizeof(int) * L.nv, cudaMemcpyHostToDevice, c->stream));
-    RT_CUDA(c, cudaMemsetAsync(status, 0, sizeof(int), c->stream));
-    RT_CUDA(c, cudaMemsetAsync(L.ainv, 0, sizeof(double) * (size_t)n * n, c->stream));
-    RT_CHECK(rt_launch(c, "coarsest_assemble", [&] {
-        long tot = (long)na * 243;
-        unsigned g = (unsigned)std::min<long>((tot + 255) / 256, (long)c->sm_count * 8);
-        k_assemble_dense<<<g, 256, 0, c->stream>>>(L.vx, L.vy, L.vz, L.nv, na, L.aidx, rowof, L.st, L.ainv);
-    }));
-    const bool no_support = (h->P.mode == RT_MODE_NSCF || h->P.mode == RT_MODE_NSFF);
-    unsigned gnn = (unsigned)std::min<long>(((long)n * n + 255) / 256, (long)c->sm_count * 8);
-    if (no_support) {
+    if (!L.cpanels) RT_CUDA(c, cudaMalloc(&L.cpanels, sizeof(double) * 4 * GJ_B * n));
+    if (!L.cstatus) RT_CUDA(c, cudaMalloc(&L.cstatus, sizeof(int)));
+    if (!L.crow) {
+        RT_CUDA(c, cudaMalloc(&L.crow, sizeof(int) * L.nv));
+        RT_CUDA(c, cudaMemcpyAsync(L.crow, rowof_h.data(), sizeof(int) * L.nv, cudaMemcpyHostToDevice, c->stream));
+        RT_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
+    if (rigid && !L.crigid) {
         // orthonormal rigid modes at the coarsest active nodes (positions are static)
         std::vector<double> Rh((size_t)6 * n, 0.0);
         for (int i = 0; i < na; i++) {
@@ -317,8 +310,32 @@ int coarsest_setup(rt_hier* h) {
             nn = std::sqrt(nn);
             for (int q = 0; q < n; q++) Rh[(size_t)a * n + q] /= nn;
         }
-        RT_CUDA(c, cudaMallocAsync(&R, sizeof(double) * 6 * n, c->stream));
-        RT_CUDA(c, cudaMemcpyAsync(R, Rh.data(), sizeof(double) * 6 * n, cudaMemcpyHostToDevice, c->stream));
+        RT_CUDA(c, cudaMalloc(&L.crigid, sizeof(double) * 6 * n));
+        RT_CUDA(c, cudaMemcpyAsync(L.crigid, Rh.data(), sizeof(double) * 6 * n, cudaMemcpyHostToDevice, c->stream));
+        RT_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
+    return RT_OK;
+}
+
+int coarsest_setup(rt_hier* h) {
+    rt_ctx* c = h->ctx;
+    rt_level& L = h->L.back();
+    const int na = L.na, n = 3 * na;
+    if (na == 0) return rt_fail(c, RT_ESTATE, "coarsest level has no active node");
+    const bool no_support = (h->P.mode == RT_MODE_NSCF || h->P.mode == RT_MODE_NSFF);
+    RT_CHECK(coarsest_workspace(h, no_support));
+    const int* rowof = L.crow;
+    double *panels = L.cpanels, *R = L.crigid;
+    int* status = L.cstatus;
+    RT_CUDA(c, cudaMemsetAsync(status, 0, sizeof(int), c->stream));
+    RT_CUDA(c, cudaMemsetAsync(L.ainv, 0, sizeof(double) * (size_t)n * n, c->stream));
+    RT_CHECK(rt_launch(c, "coarsest_assemble", [&] {
+        long tot = (long)na * 243;
+        unsigned g = (unsigned)std::min<long>((tot + 255) / 256, (long)c->sm_count * 8);
+        k_assemble_dense<<<g, 256, 0, c->stream>>>(L.vx, L.vy, L.vz, L.nv, na, L.aidx, rowof, L.st, L.ainv);
+    }));
+    unsigned gnn = (unsigned)std::min<long>(((long)n * n + 255) / 256, (long)c->sm_count * 8);
+    if (no_support) {
         RT_CHECK(rt_launch(c, "coarsest_trace", [&] { k_trace<<<1, 256, 0, c->stream>>>(n, L.ainv, h->scal + 60); }));
         RT_CHECK(rt_launch(c, "coarsest_add_rrt",
                            [&] { k_add_rrt_dev<<<gnn, 256, 0, c->stream>>>(n, 6, R, h->scal + 60, L.ainv); }));
@@ -340,13 +357,9 @@ int coarsest_setup(rt_hier* h) {
     if (no_support) {
         RT_CHECK(rt_launch(c, "coarsest_sub_rrt",
                            [&] { k_sub_rrt<<<gnn, 256, 0, c->stream>>>(n, 6, R, h->scal + 60, L.ainv); }));
-        RT_CUDA(c, cudaFreeAsync(R, c->stream));
     }
     int st_h = 0;
     RT_CUDA(c, cudaMemcpyAsync(&st_h, status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    RT_CUDA(c, cudaFreeAsync(rowof, c->stream));
-    RT_CUDA(c, cudaFreeAsync(panels, c->stream));
-    RT_CUDA(c, cudaFreeAsync(status, c->stream));
     RT_CUDA(c, cudaStreamSynchronize(c->stream));
     if (st_h != 0) return rt_fail(c, RT_ENAN, "coarsest matrix not positive definite (pivot %d)", st_h - 1);
     return RT_OK;

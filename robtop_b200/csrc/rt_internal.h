@@ -80,6 +80,13 @@ struct rt_level {
     int* aidx = nullptr;
     double* ainv = nullptr;  // [3na][3na]
     double* dvec = nullptr;  // [3na] gather buffer
+    // set-up workspace, made by the first rt_update_stencil and kept: node -> active index, pivot panels, status,
+    // orthonormal rigid modes (no-support modes); level 1: flags of the cells with fixed elements
+    int* crow = nullptr;
+    double* cpanels = nullptr;
+    int* cstatus = nullptr;
+    double* crigid = nullptr;
+    uint8_t* cfix = nullptr;
 };
 
 // launch shape of a finest-level operator kernel (chosen by rt_autotune)

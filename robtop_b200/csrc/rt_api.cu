@@ -1105,78 +1105,92 @@ __global__ void k_lmax_finish(const double* __restrict__ xx, double* __restrict_
     }
 }
 
+__global__ void k_zero_fixed(long n, long nv, const uint8_t* __restrict__ vact, const uint8_t* __restrict__ vfix,
+                             int ws, double* __restrict__ f) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+        const long v = i % nv;
+        if (!vact[v] || (ws && vfix[v])) f[i] = 0.0;
+    }
+}
+
 // the tables belong to the operator: a workspace reads its parent's
 static double* cheby_table(rt_hier* h, int lvl) {
     return (h->parent ? h->parent->scal : h->scal) + RT_SCAL_CHEB + 2 * RT_CHEBY_MAXK * lvl;
 }
 
-// v /= s and r /= s with s = sqrt(max(-v.r, tiny)) in slot out (the A-norm of v when r = -A v)
-__global__ void k_anorm_scale(long n, const double* __restrict__ vr, double* __restrict__ out, double* __restrict__ v,
-                              double* __restrict__ r) {
-    const double s = sqrt(fmax(-vr[0], 1e-300));
-    if (blockIdx.x == 0 && threadIdx.x == 0 && out) out[0] = s;
-    const double is = 1.0 / s;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        v[i] *= is;
-        r[i] *= is;
-    }
-}
-
-// Lanczos step update: w = -w - alpha v - beta_prev vp
-__global__ void k_lanczos_w(long n, double* __restrict__ w, const double* __restrict__ v,
-                            const double* __restrict__ vp, const double* __restrict__ alpha,
-                            const double* __restrict__ beta_prev) {
-    const double a = alpha[0], b = beta_prev ? beta_prev[0] : 0.0;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        w[i] = -w[i] - a * v[i] - b * vp[i];
-}
-
 #define RT_LMAX_STEPS 30
+
+// Raw scalars of the Lanczos steps below: sw[j] = s_j . D^-1 s_j and ws[j] = w_j . (A w_j) (ws[-1]: of the start
+// vector), for vectors that are not normalised.  The A-norm of v_j is lz_norm(ws[j - 1]).
+__device__ __forceinline__ double lz_norm(double sgn, double ws) { return sqrt(fmax(sgn * ws, 1e-300)); }
+
+// w = M v_j - alpha_j v_j - beta_{j-1} v_{j-1} from w = sgn D^-1 (A v_j), v and vp, all with their norms still in them
+__global__ void k_lanczos_w(long n, double sgn, int j, double* __restrict__ w, const double* __restrict__ v,
+                            const double* __restrict__ vp, const double* __restrict__ sw, const double* __restrict__ ws) {
+    const double b = lz_norm(sgn, ws[j - 1]), bp = j > 0 ? lz_norm(sgn, ws[j - 2]) : 1.0;
+    const double c = sgn / b, a = sw[j] / (b * b) / b, p = j > 0 ? b / bp : 0.0;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        w[i] = c * w[i] - a * v[i] - (j > 0 ? p * vp[i] : 0.0);
+}
+
+// the tridiagonal matrix: alpha_j = sw_j / |v_j|^2, beta_j = |w_j|
+__global__ void k_lanczos_coef(int steps, double sgn, const double* __restrict__ sw, const double* __restrict__ ws,
+                               double* __restrict__ alpha, double* __restrict__ beta) {
+    const int j = threadIdx.x;
+    if (j >= steps) return;
+    const double b = lz_norm(sgn, ws[j - 1]);
+    alpha[j] = sw[j] / (b * b);
+    beta[j] = lz_norm(sgn, ws[j]);
+}
 
 // lmax(D^-1 A) of a smoothed level by RT_LMAX_STEPS Lanczos steps in the A inner product, in which
 // M = D^-1 A is self-adjoint (no re-orthogonalisation: only the extreme Ritz value is used).
-// r = f - A v with f = 0 gives -A v; one Jacobi step from u = 0 (omega = 1) gives D^-1 r = -M v.
-// Step j, with v_j and r_j = -A v_j: w = -D^-1 r_j, alpha_j = r_j . D^-1 r_j,
-// w -= alpha_j v_j + beta_{j-1} v_{j-1}, beta_j = |w|_A, v_{j+1} = w / beta_j.  Supported rows
-// drop out (r = f = 0 there).  The largest eigenvalue of the tridiagonal matrix and the level's
-// Chebyshev table stay on the device.
+// Step j, with s_j = A v_j: w = D^-1 s_j, alpha_j = s_j . w, w -= alpha_j v_j + beta_{j-1} v_{j-1},
+// beta_j = |w|_A, v_{j+1} = w / beta_j.  The vectors keep their norms, which only the scalars carry along, so that no
+// pass scales them; on the finest level both dot products come out of the kernels that make their second vector
+// (3 passes per step; 6 before).  On the stencil levels the residual of f = 0 gives s = -A v (sgn).  Supported rows
+// drop out: zero in the start vector there, and D^-1 keeps them zero.  The largest eigenvalue of the tridiagonal
+// matrix and the level's Chebyshev table stay on the device.
 static int estimate_lmax(rt_hier* h, int lvl) {
     rt_level& L = h->L[lvl];
     rt_ctx* c = h->ctx;
     const long n = 3 * L.nv;
-    double *vp = h->x, *v = h->rold, *r = h->q, *w = h->z, *r2 = h->rr, *zero = h->p;
+    const double sgn = lvl == 0 ? 1.0 : -1.0;
+    double *vp = h->x, *v = h->rold, *s = h->q, *w = h->z, *s2 = h->rr, *zero = h->p;
     double* alpha = h->scal + 100;  // [RT_LMAX_STEPS] (the Lanczos eigen-solve's slots; not in use here)
     double* beta = h->scal + 164;
+    double* sw = h->scal + 132;     // raw scalars: sw[0 .. STEPS - 1], ws[-1 .. STEPS - 1]
+    double* ws = h->scal + 197;
     const unsigned g = (unsigned)std::min<long>((n + 255) / 256, (long)c->sm_count * 16);
-    auto residual = [&](const double* x, double* out) {
-        return lvl == 0 ? rtk::fine_residual<double>(h, x, zero, out) : rtk::st_residual<double>(h, lvl, x, zero, out);
+    // out = sgn A x and x . out
+    auto apply = [&](const double* x, double* out, double* dot_out) -> int {
+        if (lvl == 0) return rtk::fine_applyK_dot<double>(h, x, out, dot_out);
+        RT_CHECK(rtk::st_residual<double>(h, lvl, x, zero, out));
+        return rtk::dot(h, n, x, out, dot_out);
     };
-    auto jacobi = [&](const double* f, double* out) {
-        return lvl == 0 ? rtk::fine_smooth0<double>(h, f, out, 1.0, nullptr, nullptr)
-                        : rtk::st_smooth0<double>(h, lvl, f, out, 1.0, nullptr, nullptr);
+    auto diag = [&](const double* f, double* out, double* dot_out) -> int {
+        if (lvl == 0) return rtk::fine_smooth0<double>(h, f, out, 1.0, nullptr, nullptr, dot_out);
+        RT_CHECK(rtk::st_smooth0<double>(h, lvl, f, out, 1.0, nullptr, nullptr));
+        return rtk::dot(h, n, f, out, dot_out);
     };
-    RT_CUDA(c, cudaMemsetAsync(zero, 0, sizeof(double) * n, c->stream));
-    RT_CUDA(c, cudaMemsetAsync(vp, 0, sizeof(double) * n, c->stream));
+    if (lvl > 0) RT_CUDA(c, cudaMemsetAsync(zero, 0, sizeof(double) * n, c->stream));
     RT_CHECK(rtk::rng_uniform(h, 0x51ab + lvl, n, v));
-    RT_CHECK(residual(v, r));
-    RT_CHECK(rtk::dot(h, n, v, r, h->scal + 292));
-    RT_CHECK(rt_launch(c, "lmax_anorm", [&] { k_anorm_scale<<<g, 256, 0, c->stream>>>(n, h->scal + 292, nullptr, v, r); }));
-    for (int it = 0; it < RT_LMAX_STEPS; it++) {
-        RT_CHECK(jacobi(r, w));
-        RT_CHECK(rtk::dot(h, n, r, w, alpha + it));
-        RT_CHECK(rt_launch(c, "lmax_lanczos_w", [&] {
-            k_lanczos_w<<<g, 256, 0, c->stream>>>(n, w, v, vp, alpha + it, it > 0 ? beta + it - 1 : nullptr);
+    if (lvl == 0 && h->has_support)
+        RT_CHECK(rt_launch(c, "zero_fixed", [&] {
+            k_zero_fixed<<<g, 256, 0, c->stream>>>(n, L.nv, L.vact, h->vfix, 1, v);
         }));
-        RT_CHECK(residual(w, r2));
-        RT_CHECK(rtk::dot(h, n, w, r2, h->scal + 292));
-        RT_CHECK(rt_launch(c, "lmax_anorm",
-                           [&] { k_anorm_scale<<<g, 256, 0, c->stream>>>(n, h->scal + 292, beta + it, w, r2); }));
-        // rotate: v_{j-1} <- v_j, v_j <- w, r_j <- r2
+    RT_CHECK(apply(v, s, ws - 1));
+    for (int j = 0; j < RT_LMAX_STEPS; j++) {
+        RT_CHECK(diag(s, w, sw + j));
+        RT_CHECK(rt_launch(c, "lmax_lanczos_w", [&] { k_lanczos_w<<<g, 256, 0, c->stream>>>(n, sgn, j, w, v, vp, sw, ws); }));
+        if (j + 1 < RT_LMAX_STEPS) RT_CHECK(apply(w, s2, ws + j));  // beta of the last step is not used
+        // rotate: v_{j-1} <- v_j, v_j <- w, s_j <- s2
         std::swap(vp, v);
         std::swap(v, w);
-        std::swap(r, r2);
+        std::swap(s, s2);
     }
     double* lmax = h->scal + RT_SCAL_LMAX + lvl;
+    RT_CHECK(rt_launch(c, "lmax_coef", [&] { k_lanczos_coef<<<1, 32, 0, c->stream>>>(RT_LMAX_STEPS, sgn, sw, ws, alpha, beta); }));
     RT_CHECK(rtk::tridiag_max_eig(h, RT_LMAX_STEPS, alpha, beta, lmax));
     return rt_launch(c, "lmax_finish", [&] {
         k_lmax_finish<<<1, 32, 0, c->stream>>>(nullptr, lmax, cheby_table(h, lvl));
@@ -3275,14 +3289,6 @@ extern "C" int rt_hier_learned_stats(rt_hier* h, long long* applied, int* judged
     if (applied) *applied = h->unet_applied;
     if (judged_off) *judged_off = h->unet_off ? 1 : 0;
     return RT_OK;
-}
-
-__global__ void k_zero_fixed(long n, long nv, const uint8_t* __restrict__ vact, const uint8_t* __restrict__ vfix,
-                             int ws, double* __restrict__ f) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const long v = i % nv;
-        if (!vact[v] || (ws && vfix[v])) f[i] = 0.0;
-    }
 }
 
 // one training sample from the solver: a random load on the free nodes, k PCG iterations

@@ -38,6 +38,41 @@ __device__ __forceinline__ T face_rcp(T x) {
     else return T(1) / x;
 }
 
+// the grid's sum of x in out[0]: block sums, added by the last block to finish in their order (the ticket counter is
+// left at zero); W warps per block
+template <int W>
+__device__ __forceinline__ void face_grid_sum(double x, double* __restrict__ partials, double* __restrict__ out,
+                                              unsigned* __restrict__ ticket) {
+    __shared__ double sd[W];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto block_sum = [&](double v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        __syncthreads();
+        if (lane == 0) sd[w] = v;
+        __syncthreads();
+        double a = 0;
+#pragma unroll
+        for (int i = 0; i < W; i++) a += sd[i];
+        return a;
+    };
+    const double b = block_sum(x);
+    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = b;
+        __threadfence();
+        last = atomicInc(ticket, nb - 1) == nb - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double a = 0;
+    for (unsigned i = threadIdx.x; i < nb; i += 32 * W) a += __ldcg(partials + i);
+    a = block_sum(a);
+    if (threadIdx.x == 0) out[0] = a;
+}
+
 // MODE 0: r = f - K u (fixed rows: r = f)     MODE 1: out = K u (fixed rows: u)
 // MODE 2: unew = u + omega D^-1 (f - K u)     MODE 3: Chebyshev step kstep: d = a_k d + b_k D^-1 (f - K u), unew = u + d
 // (fixed nodes in MODE 2/3: unew = f / n_e, d = 0; inactive nodes: 0)
@@ -273,50 +308,27 @@ __global__ void __launch_bounds__(32 * W, MINB)
             co[r] = cn[r];
         }
     }
-    if (DOT) {  // block sums, added by the last block in their order (no second launch and no second read of u and out)
-        __shared__ double sd[W];
-        __shared__ bool last;
-        auto block_sum = [&](double x) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-            __syncthreads();
-            if (lane == 0) sd[w] = x;
-            __syncthreads();
-            double a = 0;
-#pragma unroll
-            for (int i = 0; i < W; i++) a += sd[i];
-            return a;
-        };
-        const double b = block_sum(pq);
-        const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
-        if (threadIdx.x == 0) {
-            partials[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = b;
-            __threadfence();
-            last = atomicInc(ticket, nb - 1) == nb - 1;
-        }
-        __syncthreads();
-        if (!last) return;
-        __threadfence();
-        double a = 0;
-        for (unsigned i = threadIdx.x; i < nb; i += 32 * W) a += __ldcg(partials + i);
-        a = block_sum(a);
-        if (threadIdx.x == 0) dot_out[0] = a;
-    }
+    // no second launch and no second read of u and out for p.q
+    if (DOT) face_grid_sum<W>(pq, partials, dot_out, ticket);
 }
 
 // The smoothing step from u = 0, where K u needs no evaluation: out = omega D^-1 f (MODE 2) or out = d = b_0 D^-1 f
 // (MODE 3), fixed nodes f / n_e (d = 0).  A thread marches one node column through a z-chunk with the weight sums of
 // the element layer below; 33 B (MODE 2) or 45 B per node in FP32 instead of the full step's 66.
-template <typename T, int MODE>
+template <typename T, int MODE, bool DOT>
 __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code,
                                                    const float* __restrict__ wgt, T diag_a, T diag_b,
                                                    const T* __restrict__ f, T* __restrict__ out, T omega,
-                                                   T* __restrict__ dvec, const double* __restrict__ coef) {
+                                                   T* __restrict__ dvec, const double* __restrict__ coef,
+                                                   double* __restrict__ partials, double* __restrict__ dot_out,
+                                                   unsigned* __restrict__ ticket) {
+    double fo = 0;  // DOT: the thread's part of f . out
     const int vx = nx + 1, vy = ny + 1, vz = nz + 1;
     const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (x >= vx || y >= vy) return;
+    const bool col_ok = x < vx && y < vy;
+    if (!DOT && !col_ok) return;
     const T scale = MODE == 3 ? (T)coef[1] : omega;
-    const int Z0 = blockIdx.z * zchunk, Z1 = min(Z0 + zchunk, vz);
+    const int Z0 = blockIdx.z * zchunk, Z1 = col_ok ? min(Z0 + zchunk, vz) : 0;
     const long plane = (long)vx * vy, nv = plane * vz, eplane = (long)nx * ny;
     const long col = x + (long)vx * y, ecol = x + (long)nx * y;
     const bool x0 = x > 0, x1 = x < nx, y0 = y > 0, y1 = y < ny;
@@ -357,10 +369,12 @@ __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int z
                 out[q * nv + v] = o[q];
                 if (MODE == 3) dvec[q * nv + v] = c == 1u ? o[q] : T(0);
             }
+            if (DOT) fo += (double)f0 * (double)o[0] + (double)f1 * (double)o[1] + (double)f2 * (double)o[2];
         }
 #pragma unroll
         for (int q = 0; q < 4; q++) Qp[q] = Q[q];
     }
+    if (DOT) face_grid_sum<8>(fo, partials, dot_out, ticket);
 }
 
 // node codes read by k_fine_face: bit 0 active, bit 1 fixed, bits 2.. the number of elements of non-zero weight
@@ -412,25 +426,27 @@ int node_codes(rt_hier* h) {
     });
 }
 
-// one smoothing step from u = 0: Jacobi (coef null) or the first Chebyshev step
+// one smoothing step from u = 0: Jacobi (coef null) or the first Chebyshev step; dot_out (optional, Jacobi) f . out
 template <typename T>
-int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const double* coef) {
+int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const double* coef, double* dot_out) {
     rt_level& L = h->L[0];
     int zc = 32;  // 1/32 of the weight layers read twice; shorter chunks where blocks are few
     const long xy = (long)((L.vx + 31) / 32) * ((L.vy + 7) / 8);
     while (zc > 4 && xy * ((L.vz + zc - 1) / zc) < 8L * h->ctx->sm_count) zc /= 2;
     const dim3 grid((L.vx + 31) / 32, (L.vy + 7) / 8, (L.vz + zc - 1) / zc);
+    unsigned* ticket = reinterpret_cast<unsigned*>(h->scal + RT_SCAL_TICKET);
     return rt_launch(h->ctx, sizeof(T) == 8 ? "fine_smooth0_f64" : "fine_smooth0_f32", [&] {
-        if (coef)
-            k_fine_diag<T, 3><<<grid, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, zc, h->ncode, h->w, (T)h->KE[0],
-                                                                (T)h->KE[1], f, out, T(0), dvec, coef);
-        else
-            k_fine_diag<T, 2><<<grid, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, zc, h->ncode, h->w, (T)h->KE[0],
-                                                                (T)h->KE[1], f, out, (T)omega, nullptr, nullptr);
+        auto go = [&](auto kern, T om, T* d, const double* cf) {
+            kern<<<grid, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, zc, h->ncode, h->w, (T)h->KE[0], (T)h->KE[1], f, out,
+                                                   om, d, cf, h->kpart, dot_out, ticket);
+        };
+        if (coef) go(k_fine_diag<T, 3, false>, T(0), dvec, coef);
+        else if (dot_out) go(k_fine_diag<T, 2, true>, (T)omega, (T*)nullptr, (const double*)nullptr);
+        else go(k_fine_diag<T, 2, false>, (T)omega, (T*)nullptr, (const double*)nullptr);
     });
 }
-template int fine_smooth0<double>(rt_hier*, const double*, double*, double, double*, const double*);
-template int fine_smooth0<float>(rt_hier*, const float*, float*, double, float*, const double*);
+template int fine_smooth0<double>(rt_hier*, const double*, double*, double, double*, const double*, double*);
+template int fine_smooth0<float>(rt_hier*, const float*, float*, double, float*, const double*, double*);
 
 // the block shape of ty element rows per warp (measured on 511x256x256, where a spill costs more than a block):
 // FP32 1 row 8 warps, 2 rows 4 warps; FP64 1 row, 12 warps in one block per SM, 8 where the smoothing step needs

@@ -283,7 +283,7 @@ template <typename T>
 int fine_cheby(rt_hier* h, const T* u, const T* f, T* unew, T* d, const double* coef, int kstep);
 // one smoothing step from u = 0 (its operator product is zero): Jacobi (coef null) or the first Chebyshev step
 template <typename T>
-int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const double* coef);
+int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const double* coef, double* dot_out = nullptr);
 template <typename T>
 int st_smooth0(rt_hier* h, int lvl, const T* f, T* out, double omega, T* dvec, const double* coef);
 template <typename T>

@@ -1270,6 +1270,11 @@ static int mg_cycle(rt_hier* h, int i, int smoother, int pre, int post, double o
     if (i == nl - 1) return rtk::coarsest_solve<T>(h, LvlVec<T>::f(h->L[i]), LvlVec<T>::u(h->L[i]));
     const int cs = h->P.coarse_sweeps;
     const int npre = (i > 0 && cs > 0) ? cs : pre, npost = (i > 0 && cs > 0) ? cs : post;
+    if constexpr (sizeof(T) == 4) {
+        if (zero && rtk::tail_cycle_ok(h, i, smoother, npre) &&
+            (smoother == RT_SMOOTH_JACOBI || (npre <= RT_CHEBY_MAXK && npost <= RT_CHEBY_MAXK)))
+            return rtk::tail_cycle(h, i, smoother, npre, npost, omega, cheby_table(h, i));
+    }
     RT_CHECK(level_smooth<T>(h, i, smoother, npre, omega, false, zero));
     const int gl = h->P.cycle_gamma_levels;
     const int reps = (i > 0 && i + 1 < nl - 1 && h->P.cycle_gamma > 1 && (gl <= 0 || i <= gl)) ? h->P.cycle_gamma : 1;

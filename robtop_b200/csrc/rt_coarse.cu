@@ -671,6 +671,221 @@ __global__ void __launch_bounds__(SB_BS) k_st_bulk(int nx, int ny, int nz, const
     }
 }
 
+// ---------------------------------------------------------------------------
+// The two coarsest levels of an FP32 cycle in one launch: smoothing from zero, residual, restriction, the coarsest
+// product, prolongation and smoothing on the last smoothed level.  That level has a few thousand nodes at most, so a
+// step is all launch and memory latency (3 us each, 20 of them per V-cycle with 8 smoothing steps); here one cluster
+// of 16 blocks runs through them with a hardware cluster barrier in between.  Block b keeps the stencils of nodes
+// [b npc, (b + 1) npc) in shared memory for the whole cycle (read through L1 from their usual place, every step cost
+// as much as a launch), LPN lanes a node, with the node's inverse diagonal row and right-hand side in registers; the
+// vectors, which other blocks write, go through L2 (ld.cg).  A PCG iteration of 97x61x45 (882 nodes, 8 steps)
+// 279 -> 244 us, of 96x96x48 (1183 nodes) 344 -> 311 us.
+// ---------------------------------------------------------------------------
+constexpr int TC_CTAS = 16, TC_BS = 640;  // 640 threads: 96 registers, with 64 the products spill
+constexpr long TC_MAX_N = 1300;  // rows of the coarsest inverse: 16 SMs read n^2 doubles (13 MB) in ~7 us
+constexpr size_t TC_MAX_SMEM = 227 * 1024;
+
+// lanes per node for npc nodes in a block, and the stride of a coefficient's nodes in shared memory: an odd multiple of
+// the nodes in a warp, so that the LPN x 32 / LPN words of one load lie in 32 banks
+__host__ __device__ constexpr int tc_lpn(int npc) { return npc <= TC_BS / 8 ? 8 : 4; }
+__host__ __device__ constexpr int tc_stride(int npc, int lpn) {
+    return ((npc + 32 / lpn - 1) / (32 / lpn) | 1) * (32 / lpn);
+}
+constexpr size_t tc_smem(int npc, long n) {
+    return sizeof(float) * 243 * tc_stride(npc, tc_lpn(npc)) + sizeof(double) * n;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+struct TailArgs {
+    int vx, vy, vz, cvx, cvy, cvz;  // smoothed level, coarsest level
+    int npc;                        // nodes of the smoothed level per block
+    int na, npre, npost;
+    bool cheby;
+    float omega;
+    const uint8_t *vact, *cvact;
+    const float *st, *f;
+    float *u, *r, *fc, *uc;
+    const double *coef, *ainv;
+    const int* aidx;
+};
+
+template <int LPN>
+__global__ void __launch_bounds__(TC_BS) k_tail_cycle(const TailArgs a) {
+    extern __shared__ double sd[];  // the coarsest right-hand side, then the block's stencils [243][stride]
+    float* ss = reinterpret_cast<float*>(sd + 3 * a.na);
+    const int tid = threadIdx.x, lane = tid & 31, q = tid % LPN, stride = tc_stride(a.npc, LPN);
+    const int gid = blockIdx.x * TC_BS + tid;
+    const int nv = a.vx * a.vy * a.vz, nvc = a.cvx * a.cvy * a.cvz;
+    const int vb = blockIdx.x * a.npc, i = tid / LPN;  // the block's first node, the group's node in it
+    const int v = i < a.npc && vb + i < nv ? vb + i : -1;
+    const bool act = v >= 0 && a.vact[v];
+    for (int c = tid / 32; c < 243; c += TC_BS / 32) {
+        // 4-node pieces of a 128 B line
+#pragma unroll 4
+        for (int j = lane; j < a.npc; j += 32)
+            if (vb + j < nv) ss[c * stride + j] = a.st[StAddr<float>::base(vb + j) + c * 32];
+    }
+    float f0 = 0.f, f1 = 0.f, f2 = 0.f, i0 = 0.f, i1 = 0.f, i2 = 0.f, dl = 0.f;
+    if (act && q < 3) {
+        f0 = __ldcg(a.f + v);
+        f1 = __ldcg(a.f + nv + v);
+        f2 = __ldcg(a.f + 2 * nv + v);
+    }
+    __syncthreads();
+    if (act && q < 3) {
+        float m[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) m[k] = ss[(117 + k) * stride + i];
+        const float A = m[4] * m[8] - m[5] * m[7], B = m[5] * m[6] - m[3] * m[8], C = m[3] * m[7] - m[4] * m[6];
+        const float id = 1.f / (m[0] * A + m[1] * B + m[2] * C);
+        i0 = id * (q == 0 ? A : q == 1 ? B : C);
+        i1 = id * (q == 0 ? m[2] * m[7] - m[1] * m[8] : q == 1 ? m[0] * m[8] - m[2] * m[6] : m[1] * m[6] - m[0] * m[7]);
+        i2 = id * (q == 0 ? m[1] * m[5] - m[2] * m[4] : q == 1 ? m[2] * m[3] - m[0] * m[5] : m[0] * m[4] - m[1] * m[3]);
+    }
+    const int x = max(v, 0) % a.vx, y = max(v, 0) / a.vx % a.vy, z = max(v, 0) / (a.vx * a.vy);
+    // A u of the group's node (every lane of it)
+    auto product = [&](const float* src, float (&Au)[3]) {
+        Au[0] = Au[1] = Au[2] = 0.f;
+        if (act) {
+            constexpr int NK = (27 + LPN - 1) / LPN;
+#pragma unroll
+            for (int k0 = 0; k0 < NK; k0 += 4) {  // 12 loads in flight
+                float un[4][3];
+#pragma unroll
+                for (int kk = k0; kk < min(k0 + 4, NK); kk++) {
+                    const int k = q + LPN * kk;
+                    const int jx = x + k % 3 - 1, jy = y + (k / 3) % 3 - 1, jz = z + k / 9 - 1;
+                    const bool in = k < 27 && jx >= 0 && jy >= 0 && jz >= 0 && jx < a.vx && jy < a.vy && jz < a.vz;
+                    const int nj = jx + a.vx * (jy + a.vy * jz);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) un[kk - k0][c] = in ? __ldcg(src + c * nv + nj) : 0.f;
+                }
+#pragma unroll
+                for (int kk = k0; kk < min(k0 + 4, NK); kk++) {
+                    const int k = q + LPN * kk;
+                    if (k >= 27) break;
+                    const float* s = ss + k * 9 * stride + i;
+#pragma unroll
+                    for (int r = 0; r < 3; r++)
+                        Au[r] += s[(3 * r) * stride] * un[kk - k0][0] + s[(3 * r + 1) * stride] * un[kk - k0][1] +
+                                 s[(3 * r + 2) * stride] * un[kk - k0][2];
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+            for (int o = 1; o < LPN; o <<= 1) Au[r] += __shfl_xor_sync(0xffffffffu, Au[r], o);
+    };
+    // smoothing step k, src -> dst; from zero: src is not read
+    auto smooth = [&](int k, const float* src, float* dst, bool zero) {
+        const float ca = a.cheby ? (float)a.coef[2 * k] : 0.f, cb = a.cheby ? (float)a.coef[2 * k + 1] : a.omega;
+        float Au[3] = {0.f, 0.f, 0.f};
+        if (!zero) product(src, Au);
+        if (v >= 0 && q < 3) {
+            float res = 0.f;
+            if (act) {
+                const float zz = i0 * (f0 - Au[0]) + i1 * (f1 - Au[1]) + i2 * (f2 - Au[2]);
+                const float old = zero ? 0.f : __ldcg(src + q * nv + v);
+                dl = (k > 0 && a.cheby ? ca * dl : 0.f) + cb * zz;
+                res = old + dl;
+            }
+            dst[q * nv + v] = res;
+        }
+        cluster_barrier();
+    };
+    // from zero the first step writes the vector that leaves the result in u
+    const bool swap = a.npre % 2 == 1;
+    for (int k = 0; k < a.npre; k++) {
+        const bool even = (k % 2 == 0) != swap;
+        smooth(k, even ? a.u : a.r, even ? a.r : a.u, k == 0);
+    }
+    {  // residual
+        float Au[3];
+        product(a.u, Au);
+        if (v >= 0 && q < 3) a.r[q * nv + v] = act ? (q == 0 ? f0 - Au[0] : q == 1 ? f1 - Au[1] : f2 - Au[2]) : 0.f;
+    }
+    cluster_barrier();
+    // restriction, 8 lanes per coarse node (as k_restrict2)
+    for (int t0 = gid / 8; t0 < (nvc + TC_CTAS * TC_BS / 8 - 1) / (TC_CTAS * TC_BS / 8) * (TC_CTAS * TC_BS / 8);
+         t0 += TC_CTAS * TC_BS / 8) {
+        float s[3] = {0.f, 0.f, 0.f};
+        if (t0 < nvc && a.cvact[t0]) {
+            const int X = t0 % a.cvx, Y = t0 / a.cvx % a.cvy, Z = t0 / (a.cvx * a.cvy);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int k = (tid & 7) + 8 * i;
+                if (k >= 27) break;
+                const int dx = k % 3 - 1, dy = k / 3 % 3 - 1, dz = k / 9 - 1;
+                const int fx = 2 * X + dx, fy = 2 * Y + dy, fz = 2 * Z + dz;
+                if (fx < 0 || fy < 0 || fz < 0 || fx >= a.vx || fy >= a.vy || fz >= a.vz) continue;
+                const int n = fx + a.vx * (fy + a.vy * fz);
+                const float w = 0.125f * (float)((2 - abs(dx)) * (2 - abs(dy)) * (2 - abs(dz)));
+                s[0] += w * __ldcg(a.r + n);
+                s[1] += w * __ldcg(a.r + nv + n);
+                s[2] += w * __ldcg(a.r + 2 * nv + n);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            s[c] += __shfl_xor_sync(0xffffffffu, s[c], 1);
+            s[c] += __shfl_xor_sync(0xffffffffu, s[c], 2);
+            s[c] += __shfl_xor_sync(0xffffffffu, s[c], 4);
+        }
+        if (t0 < nvc && (tid & 7) < 3) a.fc[(tid & 7) * nvc + t0] = (tid & 7) == 0 ? s[0] : (tid & 7) == 1 ? s[1] : s[2];
+    }
+    cluster_barrier();
+    // coarsest solve (as k_coarsest)
+    const int n = 3 * a.na;
+    for (int k = tid; k < a.na; k += TC_BS) {
+        const int vc = a.aidx[k];
+        sd[3 * k] = (double)__ldcg(a.fc + vc);
+        sd[3 * k + 1] = (double)__ldcg(a.fc + nvc + vc);
+        sd[3 * k + 2] = (double)__ldcg(a.fc + 2 * nvc + vc);
+    }
+    for (int vc = gid; vc < nvc; vc += TC_CTAS * TC_BS)
+        if (!a.cvact[vc]) a.uc[vc] = a.uc[nvc + vc] = a.uc[2 * nvc + vc] = 0.f;
+    __syncthreads();
+    for (int k = gid / 32; k < n; k += TC_CTAS * TC_BS / 32) {
+        const double* row = a.ainv + (long)k * n;
+        double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (int j0 = lane; j0 < n; j0 += 256) {
+            double b[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) b[k] = j0 + 32 * k < n ? row[j0 + 32 * k] : 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (j0 + 32 * k < n) s[k] += b[k] * sd[j0 + 32 * k];
+        }
+        double t = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) a.uc[(k % 3) * nvc + a.aidx[k / 3]] = (float)t;
+    }
+    cluster_barrier();
+    // prolongation to the group's node
+    if (act && q < 3) {
+        const int ox = x & 1, oy = y & 1, oz = z & 1;
+        const int c = x / 2 + a.cvx * (y / 2 + a.cvy * (z / 2));
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int bx = k & 1, by = (k >> 1) & 1, bz = k >> 2;
+            const int w = (bx ? ox : 2 - ox) * (by ? oy : 2 - oy) * (bz ? oz : 2 - oz);
+            // a corner without a weight may lie outside the coarse box
+            if (w != 0) s += 0.125f * (float)w * __ldcg(a.uc + q * nvc + c + bx + a.cvx * (by + a.cvy * bz));
+        }
+        a.u[q * nv + v] = __ldcg(a.u + q * nv + v) + s;
+    }
+    cluster_barrier();
+    for (int k = 0; k < a.npost; k++) smooth(k, k % 2 == 0 ? a.u : a.r, k % 2 == 0 ? a.r : a.u, false);
+    // the last step wrote r: every lane copies what it wrote
+    if (a.npost % 2 == 1 && v >= 0 && q < 3) a.u[q * nv + v] = __ldcg(a.r + q * nv + v);
+}
+
 // smoother copies of level stencils (layout above); one thread per (node, row group)
 __global__ void k_st_to_f32(long nv, long nvpad, const double* __restrict__ st, float* __restrict__ out) {
     const long n = nvpad * 243;
@@ -1486,6 +1701,47 @@ int galerkin_from_stencil(rt_hier* h, int lvl) {
     });
 }
 
+// one cluster with smem bytes of dynamic shared memory per block
+static cudaLaunchConfig_t tail_config(size_t smem, cudaStream_t stream, cudaLaunchAttribute* at) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = TC_CTAS;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(TC_CTAS);
+    cfg.blockDim = dim3(TC_BS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// the last smoothed level and the coarsest one in one launch (k_tail_cycle): FP32 Jacobi or Chebyshev cycles from zero
+// whose level fits the cluster and whose coarsest inverse 16 SMs can read in the time of a launch of all of them
+bool tail_cycle_ok(rt_hier* h, int lvl, int smoother, int pre) {
+    const int nl = (int)h->L.size();
+    if (!h->ctx->tail_cluster || lvl != nl - 2 || lvl < 1 || pre < 1 || h->P.coarse_bf16 || ((h->cheby_fused >> lvl) & 1u)) return false;
+    if (smoother != RT_SMOOTH_JACOBI && smoother != RT_SMOOTH_CHEBY) return false;
+    const long n = 3L * h->L[lvl + 1].na, npc = (h->L[lvl].nv + TC_CTAS - 1) / TC_CTAS;
+    return npc <= TC_BS / 4 && n <= TC_MAX_N && tc_smem((int)npc, n) <= TC_MAX_SMEM;
+}
+
+int tail_cycle(rt_hier* h, int lvl, int smoother, int pre, int post, double omega, const double* coef) {
+    rt_level &L = h->L[lvl], &Cc = h->L[lvl + 1];
+    const int npc = (int)((L.nv + TC_CTAS - 1) / TC_CTAS);
+    TailArgs a{L.vx, L.vy, L.vz, Cc.vx, Cc.vy, Cc.vz, npc, Cc.na, pre, post, smoother == RT_SMOOTH_CHEBY, (float)omega, L.vact,
+               Cc.vact, L.st32, L.f32, L.u32, L.r32, Cc.f32, Cc.u32, coef, Cc.ainv, Cc.aidx};
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = tail_config(tc_smem(npc, 3L * Cc.na), h->ctx->stream, &at);
+    cudaError_t e = cudaSuccess;
+    RT_CHECK(rt_launch(h->ctx, "tail_cycle_f32", [&] {
+        if (tc_lpn(npc) == 8) e = cudaLaunchKernelEx(&cfg, k_tail_cycle<8>, a);
+        else e = cudaLaunchKernelEx(&cfg, k_tail_cycle<4>, a);
+    }));
+    if (e != cudaSuccess) return rt_fail(h->ctx, RT_ECUDA, "cluster launch failed: %s", cudaGetErrorString(e));
+    return RT_OK;
+}
+
 int d2f(rt_hier* h, long n, const double* a, float* b) {
     return rt_launch(h->ctx, "d2f", [&] { k_d2f<<<grid_for(h->ctx, n, 256), 256, 0, h->ctx->stream>>>(n, a, b); });
 }
@@ -1506,6 +1762,19 @@ int init_stencil_kernels(rt_ctx* c) {
                              (int)sb_smem<float, uint16_t>())};
     for (cudaError_t x : e)
         if (x != cudaSuccess) return rt_fail(c, RT_ECUDA, "stencil kernel attributes: %s", cudaGetErrorString(x));
+    // a cluster of 16 is above the portable size: where it does not fit, the levels run in separate launches
+    c->tail_cluster = true;
+    for (auto k : {k_tail_cycle<8>, k_tail_cycle<4>}) {
+        cudaLaunchAttribute at;
+        cudaLaunchConfig_t cfg = tail_config(TC_MAX_SMEM, c->stream, &at);
+        int n = 0;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_MAX_SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            c->tail_cluster = false;
+        }
+    }
     return RT_OK;
 }
 

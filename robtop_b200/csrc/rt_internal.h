@@ -26,6 +26,7 @@ struct rt_ctx {
     bool own_stream = false;
     std::string err;
     int sm_count = 148;
+    bool tail_cluster = false;  // the device runs k_tail_cycle's cluster
     long long launches = 0;
     // polls of a bounded device wait on another block (the grid barrier of the fused sweeps);
     // rt_ctx_set_wait_limit lowers it so a test can make a wait run out
@@ -292,6 +293,9 @@ int st_cheby(rt_hier* h, int lvl, const T* u, const T* f, T* unew, T* d, const d
 // the result in u); false from st_cheby_fused_ok when the device cannot co-schedule the grid
 int st_cheby_fused(rt_hier* h, int lvl, float* u, const float* f, float* tmp, float* d, const double* coef, int nsteps);
 bool st_cheby_fused_ok(rt_hier* h);
+// the FP32 cycle's two coarsest levels from u = 0 in one launch
+bool tail_cycle_ok(rt_hier* h, int lvl, int smoother, int pre);
+int tail_cycle(rt_hier* h, int lvl, int smoother, int pre, int post, double omega, const double* coef);
 int penalty_weights(rt_hier* h);
 int init_tile_kernels(rt_ctx* c);
 int init_sf_kernels(rt_ctx* c);

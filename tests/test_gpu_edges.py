@@ -12,7 +12,7 @@ import robtop_b200 as rb  # noqa: E402
 from gpu_common import E, NU, P, rel_err  # noqa: E402
 
 
-def _perforated(nx, ny, nz, seed, sup):
+def _perforated(nx, ny, nz, seed, sup, skip=1):
     """A box with voids and scattered supports, and its oracle hierarchy."""
     r = np.random.default_rng(seed)
     eact = (r.random((nz, ny, nx)) < 0.85).astype(np.uint8)
@@ -23,11 +23,12 @@ def _perforated(nx, ny, nz, seed, sup):
         vfix[r.random(vfix.shape) < 0.03] = 1
     ctx = rb.Context(0)
     G = rb.HierarchyGrid(ctx, rb.default_params(mode=rb.MODE_WSFF if sup else rb.MODE_NSFF, youngs_modulus=E,
-                                                poisson_ratio=NU, power_penalty=P))
+                                                poisson_ratio=NU, power_penalty=P, skip_layer1=skip))
     G.genFromBox(eact)
     G[0].setRho(rho.ravel())
     G.set_support(vfix)
-    H = O.Hierarchy(eact, rho, vfix if sup else None, p=P, E=E, nu=NU, no_support=not sup)
+    H = O.Hierarchy(eact, rho, vfix if sup else None, p=P, E=E, nu=NU, no_support=not sup,
+                    skip=bool(skip))
     G.update_stencil()
     H.set_weights(G[0].getPenalty())  # the device's FP32 powf weights
     H.update_stencil()
@@ -235,5 +236,46 @@ def test_galerkin_edges(dims, skip):
     H.update_stencil()
     for i in range(1, H.nlev):
         assert rel_err(G[i].getStencil(), H.arrs[i]["st"]) < 1e-11, f"level {i}"
+    G.close()
+    ctx.close()
+
+
+# the two coarsest levels of an FP32 cycle in one cluster launch: 8 lanes per node up to 1280 nodes (672, 1224), 4 up
+# to 2560 (1440, 1710, 2420), both parities of the sweep counts, odd sides
+@pytest.mark.parametrize("dims,skip,pre,post,cs", [((21, 13, 11), 0, 2, 2, 8), ((21, 13, 11), 0, 1, 3, 0),
+                                                   ((32, 16, 14), 0, 3, 1, 0), ((33, 17, 14), 0, 2, 2, 1),
+                                                   ((38, 20, 20), 0, 2, 1, 0), ((70, 33, 30), 1, 2, 2, 3)])
+@pytest.mark.parametrize("sup", [True, False])
+@pytest.mark.parametrize("jacobi", [False, True])
+def test_tail_cycle_edges(dims, skip, pre, post, cs, sup, jacobi):
+    ctx, G, H, r = _perforated(*dims, sum(dims), sup, skip)
+    params = G.params
+    params.smoother = rb.SMOOTH_JACOBI if jacobi else rb.SMOOTH_CHEBY
+    params.pre_sweeps, params.post_sweeps, params.coarse_sweeps, params.jacobi_omega = pre, post, cs, 0.5
+    act = np.tile(G[0].getVact(), 3).astype(bool)
+    b = r.standard_normal(3 * G[0].nv) * act
+    if sup:
+        b[np.tile(H.arrs[0]["vfix"], 3).astype(bool)] = 0
+    else:
+        Ru = np.zeros(6 * b.size)
+        O.lib().or_rigid_nodes(H.lv(0), O.ptr(Ru))
+        O.lib().or_displacement_project(b.size // 3, O.ptr(Ru), O.ptr(b))
+    x = {}
+    for prec in (rb.FP64, rb.FP32):
+        params.precision = prec
+        G.set_params(params)
+        G.update_stencil()
+        G[0].setForce(b)
+        G[0].reset_displacement()
+        if prec == rb.FP32:
+            ctx.profile(True)
+            ctx.profile_reset()
+        G.pcg(1e-14, 1)
+        if prec == rb.FP32:
+            assert "tail_cycle_f32" in ctx.profile_stats()
+            ctx.profile(False)
+        x[prec] = G[0].getDisplacement()
+    # one preconditioned step in FP32 against FP64: 81 terms a row x 40 steps x 2^-24, of values up to 5 times the result
+    assert rel_err(x[rb.FP32], x[rb.FP64]) < 1e-3
     G.close()
     ctx.close()

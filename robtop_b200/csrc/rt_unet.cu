@@ -270,8 +270,9 @@ static int unet_backward(rt_unet* u, const float* tgt) {
         rtu::k_mse<<<ew_blocks(c, 3 * V0), 256, 0, c->stream>>>(u->out, tgt, 3 * V0, u->g_out, u->dloss);
     }));
     RT_CHECK(rt_launch(c, "unet_head_bwd", [&] {
-        rtu::k_head_bwd<<<(unsigned)std::min<long>((V0 + 255) / 256, 512), 256, 0, c->stream>>>(
-            u->d0, HEAD_C, V0, u->P + u->head_w, u->g_out, u->g_d0, u->G + u->head_w, u->G + u->head_b);
+        static_assert(HEAD_C == 16, "k_head_bwd keeps 16 channels in registers");
+        rtu::k_head_bwd<<<(unsigned)std::min<long>((V0 + 127) / 128, 148 * 4), 128, 0, c->stream>>>(
+            u->d0, V0, u->P + u->head_w, u->g_out, u->g_d0, u->G + u->head_w, u->G + u->head_b);
     }));
     // level 0 decoder
     RT_CHECK(unet_conv_bwd(u, 13, 0, u->d0a, 16, u->d0, 16, u->g_d0, 16, u->g_y));

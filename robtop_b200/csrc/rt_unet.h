@@ -49,8 +49,8 @@ __global__ void k_weights_bf16(const float* w, int cin, int cout, __nv_bfloat16*
 __global__ void k_adam(long n, float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float c1,
                        float c2, float eps);
 __global__ void k_head(const __nv_bfloat16* in, int C, long V, const float* hw, const float* hb, float* out);
-__global__ void k_head_bwd(const __nv_bfloat16* in, int C, long V, const float* hw, const float* gout, float* gin,
-                           float* dhw, float* dhb);
+__global__ void k_head_bwd(const __nv_bfloat16* in, long V, const float* hw, const float* gout, float* gin, float* dhw,
+                           float* dhb);  // 16 channels
 __global__ void k_mse(const float* out, const float* tgt, long n, float* gout, double* loss);
 }  // namespace rtu
 

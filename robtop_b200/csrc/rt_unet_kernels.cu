@@ -299,8 +299,11 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3_halo(ConvArgs a, int P, 
 }
 
 // planes per CTA (P), taps per weight stage (G) and shared memory of k_conv3_halo: the largest
-// P, then the largest G, whose halo and weight stages fit in 200 KB; P = 0 if nothing fits
-static int halo_plan(int cin, int cout, int* G, size_t* smem) {
+// P, then the largest G, whose halo and weight stages fit in 200 KB; P = 0 if nothing fits.  More planes re-read
+// less of the halo, but a box of xy patches x Z planes is cut into no fewer CTAs than the GPU has SMs where it can be:
+// on a 33^3 training crop, 8 planes left half of the SMs idle and each CTA's loads and MMAs in series (37 us a
+// convolution, 17 us with the rule)
+static int halo_plan(int cin, int cout, long xy, int Z, int sms, int* G, size_t* smem) {
     static const int gs[4] = {27, 9, 3, 1};
     // first pass: plans that leave two CTAs per SM (one loads its halo while the other multiplies);
     // second pass: anything within 200 KB
@@ -308,6 +311,7 @@ static int halo_plan(int cin, int cout, int* G, size_t* smem) {
     for (int pass = 0; pass < 2; pass++) {
         for (int P = 8; P >= 1; P /= 2) {
             if (P * cout > 512 || (pass == 0 && 2 * rttc::tmem_cols(P * cout) > 512)) continue;
+            if (P > 1 && xy * ((Z + P - 1) / P) < sms) continue;
             for (int gi = 0; gi < 4; gi++) {
                 const int nst = gs[gi] == 27 ? 1 : 2;
                 const size_t need =
@@ -358,7 +362,8 @@ int conv3(rt_ctx* c, const ConvArgs& a) {
                        a.cin, a.cout);
     size_t hsmem = 0;
     int G = 1;
-    const int P = g_conv_variant ? halo_plan(a.cin, a.cout, &G, &hsmem) : 0;
+    const long xy = (long)((a.X + 7) / 8) * ((a.Y + 15) / 16);
+    const int P = g_conv_variant ? halo_plan(a.cin, a.cout, xy, a.Z, c->sm_count, &G, &hsmem) : 0;
     if (P > 0) {
         const dim3 grid((unsigned)((a.X + 7) / 8), (unsigned)((a.Y + 15) / 16), (unsigned)((a.Z + P - 1) / P));
         return rt_launch(c, "unet_conv3_halo",
@@ -609,28 +614,39 @@ __global__ void k_head(const __nv_bfloat16* __restrict__ in, int C, long V, cons
     }
 }
 
-// head backward: gin[v][c] = sum_k hw[k][c] gout[v][k]; block partials of dhw, dhb
-__global__ void k_head_bwd(const __nv_bfloat16* __restrict__ in, int C, long V, const float* __restrict__ hw,
-                           const float* __restrict__ gout, float* __restrict__ gin, float* __restrict__ dhw,
-                           float* __restrict__ dhb) {
-    __shared__ float sw[3 * 64 + 3];
+// head backward: gin[v][c] = sum_k hw[k][c] gout[v][k]; dhw, dhb by warp sums, one shared atomic per warp and value, one
+// global atomic per block.  C = 16 is the head's width: with a run-time C the 51 sums lived in local memory (130 us on
+// 33^3, 10 us here).
+__global__ void __launch_bounds__(128) k_head_bwd(const __nv_bfloat16* __restrict__ in, long V,
+                                                  const float* __restrict__ hw, const float* __restrict__ gout,
+                                                  float* __restrict__ gin, float* __restrict__ dhw,
+                                                  float* __restrict__ dhb) {
+    constexpr int C = 16;
+    __shared__ float sw[3 * C + 3];
     for (int i = threadIdx.x; i < 3 * C + 3; i += blockDim.x) sw[i] = 0.f;
     __syncthreads();
-    float lw[3 * 16], lb[3] = {0.f, 0.f, 0.f};  // C <= 16
-    for (int i = 0; i < 3 * C; i++) lw[i] = 0.f;
+    float lw[3 * C + 3];
+#pragma unroll
+    for (int i = 0; i < 3 * C + 3; i++) lw[i] = 0.f;
     for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {
-        const float g0 = gout[3 * v], g1 = gout[3 * v + 1], g2 = gout[3 * v + 2];
-        lb[0] += g0; lb[1] += g1; lb[2] += g2;
+        const float g[3] = {gout[3 * v], gout[3 * v + 1], gout[3 * v + 2]};
+#pragma unroll
+        for (int k = 0; k < 3; k++) lw[3 * C + k] += g[k];
+#pragma unroll
         for (int c = 0; c < C; c++) {
             const float x = bf(in[v * C + c]);
-            gin[v * C + c] = hw[c] * g0 + hw[C + c] * g1 + hw[2 * C + c] * g2;
-            lw[c] += g0 * x;
-            lw[C + c] += g1 * x;
-            lw[2 * C + c] += g2 * x;
+            gin[v * C + c] = hw[c] * g[0] + hw[C + c] * g[1] + hw[2 * C + c] * g[2];
+#pragma unroll
+            for (int k = 0; k < 3; k++) lw[k * C + c] += g[k] * x;
         }
     }
-    for (int i = 0; i < 3 * C; i++) atomicAdd(&sw[i], lw[i]);
-    for (int k = 0; k < 3; k++) atomicAdd(&sw[3 * C + k], lb[k]);
+#pragma unroll
+    for (int i = 0; i < 3 * C + 3; i++) {
+        float x = lw[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sw[i], x);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < 3 * C; i += blockDim.x) atomicAdd(&dhw[i], sw[i]);
     for (int k = threadIdx.x; k < 3; k += blockDim.x) atomicAdd(&dhb[k], sw[3 * C + k]);

@@ -11,6 +11,8 @@
 // (residual) or n_e * I (GS).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "rt_element.cuh"
 #include "rt_internal.h"
 
@@ -26,96 +28,132 @@ struct VertexRow {
     T diag_a, diag_b;  // KE[v][v] = a I + b (s s^T - I)
 };
 
+// diag: the common diagonal entry of the node's block, off: its entries xy, xz, yz
 template <typename T>
-__device__ __forceinline__ void block_gs(const T S[9], const T F[3], const T KU[3], T uu[3], bool backward) {
+__device__ __forceinline__ void block_gs(T diag, const T (&off)[3], const T (&F)[3], const T (&KU)[3], T (&uu)[3],
+                                         bool backward) {
+    const T id = T(1) / diag;  // off the chain of the three updates
     if (!backward) {
-        uu[0] = (F[0] - S[1] * uu[1] - S[2] * uu[2] - KU[0]) / S[0];
-        uu[1] = (F[1] - S[3] * uu[0] - S[5] * uu[2] - KU[1]) / S[4];
-        uu[2] = (F[2] - S[6] * uu[0] - S[7] * uu[1] - KU[2]) / S[8];
+        uu[0] = (F[0] - off[0] * uu[1] - off[1] * uu[2] - KU[0]) * id;
+        uu[1] = (F[1] - off[0] * uu[0] - off[2] * uu[2] - KU[1]) * id;
+        uu[2] = (F[2] - off[1] * uu[0] - off[2] * uu[1] - KU[2]) * id;
     } else {
-        uu[2] = (F[2] - S[6] * uu[0] - S[7] * uu[1] - KU[2]) / S[8];
-        uu[1] = (F[1] - S[3] * uu[0] - S[5] * uu[2] - KU[1]) / S[4];
-        uu[0] = (F[0] - S[1] * uu[1] - S[2] * uu[2] - KU[0]) / S[0];
+        uu[2] = (F[2] - off[1] * uu[0] - off[2] * uu[1] - KU[2]) * id;
+        uu[1] = (F[1] - off[0] * uu[0] - off[2] * uu[2] - KU[1]) * id;
+        uu[0] = (F[0] - off[0] * uu[1] - off[1] * uu[2] - KU[0]) * id;
     }
 }
 
-// one colour of the 8-colour point-block GS; colour c = x%2 + 2(y%2) + 4(z%2).  8 lanes per node, one per incident
-// element (lane = 4 * element + node, 4 nodes of a row per warp): a colour of a small grid has too few nodes to fill
-// the GPU with a thread each, and a lane's 21 loads are all in flight at once.  With the reflected vertex row the 63
-// products take their matrix entries from the kernel parameters, whichever vertex the node is.
-// 64x32x32, FP64: 27 us per colour with a thread per node, 7 us here.
+// x with its sign bit flipped where mask has bit 31
+__device__ __forceinline__ double flip_sign(double x, unsigned mask) {
+    return __hiloint2double((int)((unsigned)__double2hiint(x) ^ mask), __double2loint(x));
+}
+__device__ __forceinline__ float flip_sign(float x, unsigned mask) {
+    return __uint_as_float(__float_as_uint(x) ^ mask);
+}
+
+// one colour of the 8-colour point-block GS; colour c = x%2 + 2(y%2) + 4(z%2).  4 lanes per node (lane = 8 * quadrant +
+// node, 8 nodes of a row per warp), each with the two elements of its (y, z) quadrant: a colour of a small grid has too
+// few nodes to fill the GPU with a thread each, and the two elements share a face, so that a lane loads 11 neighbours
+// where two lanes with an element each load 14.  A warp's load touches 4 rows; with 8 lanes per node, one per element,
+// it touched 8, and the L1's wavefronts were the bound.  The loads depend on the box alone, not on the weights, which
+// only select.  With the reflected vertex row the products take their matrix entries from the kernel parameters,
+// whichever vertex the node is.
+// FP64, per colour with the launch: 64x32x32 10.7 us with 8 lanes, 9.8 with 4; 128x48x40 19.0, 13.9; 65x41x33 without
+// supports 12.5, 8.9.  Blocks per SM: without supports the compiler keeps all 33 loads in flight and spills at 4 blocks
+// (10.7 us); with them 3 blocks take 16.2 us on 128x48x40.
+constexpr int GS_BS = 128;
+
 template <typename T, bool WS>
-__global__ void __launch_bounds__(FINE_BS) k_fine_gs(int nx, int ny, int nz, int color, bool backward,
-                                                      const uint8_t* __restrict__ code, const float* __restrict__ w,
-                                                      const VertexRow<T> kr, T* __restrict__ u,
-                                                      const T* __restrict__ f) {
+__global__ void __launch_bounds__(GS_BS, WS ? 4 : 3) k_fine_gs(int nx, int ny, int nz, int color, bool backward,
+                                                       const uint8_t* __restrict__ code, const float* __restrict__ w,
+                                                       const VertexRow<T> kr, T* __restrict__ u,
+                                                       const T* __restrict__ f) {
     const int vx = nx + 1, vy = ny + 1, vz = nz + 1;
     const long plane = (long)vx * vy, nv = plane * vz;
     const int px = color & 1, py = (color >> 1) & 1, pz = (color >> 2) & 1;
     const unsigned cx = (vx - px + 1) / 2, cy = (vy - py + 1) / 2, cz = (vz - pz + 1) / 2;
     const unsigned nc = cx * cy * cz;
-    const int lane = threadIdx.x & 31, e = lane >> 2;
-    const int dx = e & 1 ? 1 : -1, dy = e & 2 ? 1 : -1, dz = e & 4 ? 1 : -1;  // the element's side of the node
-    const T sx = T(dx), sy = T(dy), sz = T(dz);
-    const unsigned stride = gridDim.x * (FINE_BS / 8);
-    for (unsigned t0 = blockIdx.x * (FINE_BS / 8) + (threadIdx.x >> 5) * 4; t0 < nc; t0 += stride) {
-        const unsigned t = t0 + (lane & 3);
-        T KU[3] = {T(0), T(0), T(0)}, sw = T(0), F[3], uu[3];
+    const int lane = threadIdx.x & 31, quad = lane >> 3;
+    const int dy = quad & 1 ? 1 : -1, dz = quad & 2 ? 1 : -1;  // the quadrant's side of the node
+    const unsigned my = dy < 0 ? 0x80000000u : 0u, mz = dz < 0 ? 0x80000000u : 0u;
+    const unsigned stride = gridDim.x * (GS_BS / 4);
+    for (unsigned t0 = blockIdx.x * (GS_BS / 4) + (threadIdx.x >> 5) * 8; t0 < nc; t0 += stride) {
+        const unsigned t = t0 + (lane & 7);
+        T KU[3] = {T(0), T(0), T(0)}, F[3] = {T(0), T(0), T(0)}, uu[3] = {T(0), T(0), T(0)};
+        T sw = T(0), swx = T(0);  // sums of the two weights, and with the sign of x
         uint32_t cd = 0;
         long v = 0;
         if (t < nc) {
             const int x = px + 2 * (int)(t % cx), y = py + 2 * (int)(t / cx % cy), z = pz + 2 * (int)(t / (cx * cy));
             v = x + (long)vx * y + plane * z;
-            const int ex = x + (dx - 1) / 2, ey = y + (dy - 1) / 2, ez = z + (dz - 1) / 2;
-            float wv = 0.f;
-            if (ex >= 0 && ey >= 0 && ez >= 0 && ex < nx && ey < ny && ez < nz)
-                wv = w[ex + (long)nx * (ey + (long)ny * ez)];
-            cd = code[v];
+            if (quad == 0) {
+                cd = code[v];
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                F[c] = f[c * nv + v];
-                uu[c] = u[c * nv + v];
-            }
-            if (wv != 0.f) {
-                T p[3][3] = {};
-#pragma unroll
-                for (int m = 1; m < 8; m++) {
-                    const long n = v + (m & 1 ? dx : 0) + (m & 2 ? dy * (long)vx : 0) + (m & 4 ? dz * plane : 0);
-                    const bool fixed = WS && code[n] > 1;
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        T un = u[c * nv + n];
-                        if (fixed) un = T(0);
-#pragma unroll
-                        for (int r = 0; r < 3; r++) p[r][c] += kr.k[m - 1][r][c] * un;
-                    }
+                for (int c = 0; c < 3; c++) {
+                    F[c] = f[c * nv + v];
+                    uu[c] = u[c * nv + v];
                 }
-                sw = T(wv);
-                KU[0] = sw * (p[0][0] + sx * (sy * p[0][1] + sz * p[0][2]));
-                KU[1] = sw * (p[1][1] + sy * (sx * p[1][0] + sz * p[1][2]));
-                KU[2] = sw * (p[2][2] + sz * (sx * p[2][0] + sy * p[2][1]));
+            }
+            const int ey = y + (dy - 1) / 2, ez = z + (dz - 1) / 2;
+            if (ey >= 0 && ez >= 0 && ey < ny && ez < nz) {
+                const float* we = w + x + (long)nx * (ey + (long)ny * ez);
+                const bool in[2] = {x > 0, x < nx};
+                const float wv[2] = {in[0] ? we[-1] : 0.f, in[1] ? we[0] : 0.f};
+                // rows of KE in the vertex's reflected frame: sx u0, sy u1, sz u2 of the shared nodes apart from u0, whose sign
+                // depends on the side
+                T sh0[3] = {}, sh[3] = {}, p[2][3] = {};
+                // vertex m of the node's elements on side d; nodes without an element, and fixed ones, count as zero
+                auto vertex = [&](int m, int d, bool load, bool use, T (&acc0)[3], T (&acc)[3]) {
+                    const long n = v + (m & 1 ? 2 * d - 1 : 0) + (m & 2 ? dy * (long)vx : 0) + (m & 4 ? dz * plane : 0);
+                    T un[3] = {T(0), T(0), T(0)};
+                    if (load) {
+                        if (WS) use = use && code[n] <= 1;
+#pragma unroll
+                        for (int c = 0; c < 3; c++) un[c] = u[c * nv + n];
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; c++) un[c] = use ? un[c] : T(0);
+                    if (d == 0 && (m & 1)) un[0] = -un[0];
+                    un[1] = flip_sign(un[1], my);
+                    un[2] = flip_sign(un[2], mz);
+#pragma unroll
+                    for (int r = 0; r < 3; r++) {
+                        acc0[r] += kr.k[m - 1][r][0] * un[0];
+                        acc[r] += kr.k[m - 1][r][1] * un[1];
+                        acc[r] += kr.k[m - 1][r][2] * un[2];
+                    }
+                };
+#pragma unroll
+                for (int m = 2; m < 8; m += 2) vertex(m, 0, true, wv[0] != 0.f || wv[1] != 0.f, sh0, sh);
+#pragma unroll
+                for (int d = 0; d < 2; d++)
+#pragma unroll
+                    for (int m = 1; m < 8; m += 2) vertex(m, d, in[d], wv[d] != 0.f, p[d], p[d]);
+                const T w0 = T(wv[0]), w1 = T(wv[1]);
+                sw = w0 + w1;
+                swx = w1 - w0;
+                KU[0] = w1 * (p[1][0] + (sh[0] + sh0[0])) - w0 * (p[0][0] + (sh[0] - sh0[0]));
+                KU[1] = flip_sign(w1 * (p[1][1] + (sh[1] + sh0[1])) + w0 * (p[0][1] + (sh[1] - sh0[1])), my);
+                KU[2] = flip_sign(w1 * (p[1][2] + (sh[2] + sh0[2])) + w0 * (p[0][2] + (sh[2] - sh0[2])), mz);
             }
         }
-        T sxy = sw * sx * sy, sxz = sw * sx * sz, syz = sw * sy * sz;
+        T S[4] = {sw, flip_sign(swx, my), flip_sign(swx, mz), flip_sign(sw, my ^ mz)};  // sums of w, w sx sy, w sx sz, w sy sz
 #pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
+        for (int o = 8; o < 32; o <<= 1) {
 #pragma unroll
             for (int c = 0; c < 3; c++) KU[c] += __shfl_xor_sync(0xffffffffu, KU[c], o);
-            sw += __shfl_xor_sync(0xffffffffu, sw, o);
-            sxy += __shfl_xor_sync(0xffffffffu, sxy, o);
-            sxz += __shfl_xor_sync(0xffffffffu, sxz, o);
-            syz += __shfl_xor_sync(0xffffffffu, syz, o);
-        }
-        if (e != 0 || cd == 0) continue;
-        T S[9] = {kr.diag_a * sw,  kr.diag_b * sxy, kr.diag_b * sxz, kr.diag_b * sxy, kr.diag_a * sw,
-                  kr.diag_b * syz, kr.diag_b * sxz, kr.diag_b * syz, kr.diag_a * sw};
-        if (WS && cd > 1u) {
 #pragma unroll
-            for (int i = 0; i < 9; i++) S[i] = T(0);
-            S[0] = S[4] = S[8] = T(cd >> 2);
-            KU[0] = KU[1] = KU[2] = T(0);
+            for (int c = 0; c < 4; c++) S[c] += __shfl_xor_sync(0xffffffffu, S[c], o);
         }
-        block_gs(S, F, KU, uu, backward);
+        if (quad != 0 || cd == 0) continue;
+        if (WS && cd > 1u) {  // n_e u = f
+#pragma unroll
+            for (int c = 0; c < 3; c++) uu[c] = F[c] / T(cd >> 2);
+        } else {
+            const T off[3] = {kr.diag_b * S[1], kr.diag_b * S[2], kr.diag_b * S[3]};
+            block_gs(kr.diag_a * S[0], off, F, KU, uu, backward);
+        }
         u[v] = uu[0]; u[nv + v] = uu[1]; u[2 * nv + v] = uu[2];
     }
 }
@@ -214,12 +252,12 @@ int fine_gs(rt_hier* h, T* u, const T* f, bool backward) {
                     ((L.vz - ((col >> 2) & 1) + 1) / 2);
         if (ncol == 0) continue;
         RT_CHECK(rt_launch(h->ctx, nm, [&] {
-            unsigned g = fine_grid(h->ctx, 8 * ncol);
+            const unsigned g = (unsigned)std::min<long>((4 * ncol + GS_BS - 1) / GS_BS, (long)h->ctx->sm_count * 64);
             if (h->has_support)
-                k_fine_gs<T, true><<<g, FINE_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, h->ncode, h->w,
+                k_fine_gs<T, true><<<g, GS_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, h->ncode, h->w,
                                                                       kr, u, f);
             else
-                k_fine_gs<T, false><<<g, FINE_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, h->ncode, h->w,
+                k_fine_gs<T, false><<<g, GS_BS, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, col, backward, h->ncode, h->w,
                                                                        kr, u, f);
         }));
     }

@@ -140,6 +140,28 @@ def test_transfer_edges(dims):
     ctx.close()
 
 
+# finest Gauss-Seidel: 8 nodes of a colour per warp, 32 per block; colours with odd and even row lengths, nodes on every
+# face with and without an element on either side, NaN in nodes that no element holds
+@pytest.mark.parametrize("nx,ny,nz", [(15, 7, 8), (16, 8, 7), (17, 9, 9), (40, 7, 7)])
+@pytest.mark.parametrize("sup", [True, False])
+def test_fine_gauss_seidel_edges(nx, ny, nz, sup):
+    ctx, G, H, r = _perforated(nx, ny, nz, nx + nz, sup)
+    act = np.tile(G[0].getVact(), 3).astype(bool)
+    u = r.standard_normal(3 * G[0].nv)
+    u[~act] = np.nan
+    f = r.standard_normal(3 * G[0].nv) * act
+    for smoother, back in ((rb.SMOOTH_GS, 0), (rb.SMOOTH_SGS, 1)):
+        G[0].setDisplacement(u)
+        G[0].setForce(f)
+        G[0].smooth(smoother, 1)
+        uo = np.where(act, u, 0.0)
+        O.lib().or_fine_gs(H.lv(0), O.ptr(H.KE), O.ptr(uo), O.ptr(f), back)
+        # 168 terms per row and 8 colours in a chain, each product to 2^-53
+        assert rel_err(G[0].getDisplacement()[act], uo[act]) < 1e-10
+    G.close()
+    ctx.close()
+
+
 # both lane counts of the stencil levels' Gauss-Seidel: a warp per node, and 4 lanes once a colour has ~19k nodes
 @pytest.mark.parametrize("dims", [(20, 12, 10), (130, 98, 98)])
 def test_level_gauss_seidel_lane_counts(dims):

@@ -287,10 +287,10 @@ int rt_autotune(rt_hier* h, int reps);
  * two elements per thread in packed FP32, 5 sum-factorised row marching (the element grid's Hadamard stages shared between
  * neighbouring elements, one warp per node row, one barrier per layer; ty 4, 8 or 16 node rows), 6 and 7 variant 3 with
  * TMA-staged node layers, 8 (the default) element columns marched through z with the transforms of faces carried in
- * registers (ty = element rows per warp: 1, or 2 in FP32) */
+ * registers (ty = element rows per warp: 1) */
 int rt_tuning_info(rt_hier* h, int precision, int mode, int* variant, int* ty, int* zchunk, double* us);
 /* set a finest-level kernel's launch shape explicitly (ty: 2, 4 or 8 rows for variants 0, 1, 3, 4; 2 or 4 for
- * variant 2; 4, 8 or 16 for variant 5; 1 or, in FP32, 2 for variant 8) */
+ * variant 2; 4, 8 or 16 for variant 5; 1 for variant 8) */
 int rt_set_tuning(rt_hier* h, int precision, int mode, int variant, int ty, int zchunk);
 /* time reps launches of one finest-level kernel at its current shape on random data
  * (device time per launch in microseconds, CUDA events on the context stream) */

@@ -2461,8 +2461,7 @@ extern "C" int rt_autotune(rt_hier* h, int reps) {
     // the face-carrying march, and the tile kernels that were the fastest before it (511x256x256, 255x256x128,
     // 129x97x85 and 64x32x32: the march won every kernel there, by 1.1 to 2.5 times)
     std::vector<rt_tile_cfg> cands;
-    for (int ty : {1, 2})  // 2: FP32 only
-        for (int zc : {2, 4, 8, 16, 32, 64}) cands.push_back(rt_tile_cfg{8, ty, zc});
+    for (int zc : {2, 4, 8, 16, 32, 64}) cands.push_back(rt_tile_cfg{8, 1, zc});
     cands.push_back(rt_tile_cfg{0, 4, 8});
     cands.push_back(rt_tile_cfg{3, 8, 16});
     if (h->L[0].vx % 16 == 0) {  // TMA-staged node layers: the flags' row pitch must be a multiple of 16 bytes
@@ -2475,7 +2474,6 @@ extern "C" int rt_autotune(rt_hier* h, int reps) {
             double best = 1e30;
             for (const rt_tile_cfg& cfg : cands) {
                 if (cfg.zchunk > 2 * L.vz && cfg.zchunk != 4) continue;
-                if (cfg.variant == 8 && cfg.ty == 2 && prec == 1) continue;
                 h->tune[prec][mode] = cfg;
                 const double t = time_fine_kernel(h, prec, mode, reps);
                 if (t < best) { best = t; best_cfg = cfg; }
@@ -2507,8 +2505,7 @@ extern "C" int rt_set_tuning(rt_hier* h, int precision, int mode, int variant, i
     RT_NOT_WORKSPACE(h);
     if (variant == 4 && precision == RT_FP64) return rt_fail(h->ctx, RT_EINVAL, "variant 4 (packed FP32 pairs) is FP32 only");
     if (variant == 8) {
-        if (ty != 1 && !(ty == 2 && precision != RT_FP64))
-            return rt_fail(h->ctx, RT_EINVAL, "face-march element rows per warp must be 1 or (FP32) 2");
+        if (ty != 1) return rt_fail(h->ctx, RT_EINVAL, "face-march element rows per warp must be 1");
     } else if (variant == 5) {
         if (ty != 4 && ty != 8 && ty != 16) return rt_fail(h->ctx, RT_EINVAL, "sum-factorised rows per tile must be 4, 8 or 16");
     } else if (variant == 6 || variant == 7) {

@@ -10,11 +10,17 @@
 //    x stage of an edge serves 4 elements, the y stage of a face 2 (the element below keeps it in registers for
 //    the element above), only the z stage is per element: 6 + 12 + 24 adds instead of 72, and the same on the
 //    way back, where neighbours' results are added between the stages, so that no scatter remains.
-//  * A lane owns element column X0 - 1 + lane and node column X0 - 1 + lane, a warp R consecutive element rows.
-//    x neighbours meet by shuffles, the rows of a warp in registers.  Only the upper edge of a warp's last row
-//    crosses warps, 6 values (and 2 weight sums) per lane and layer through shared memory, with one barrier per
-//    layer.  Lanes 1..30 finish nodes; a block of W warps finishes 30 x (W R - 1) nodes per layer.
-//  * The loads of the next layer and of this layer's output stage are issued before the arithmetic.
+//  * A lane owns element column X0 - 1 + lane and node column X0 - 1 + lane, a warp one element row.  x neighbours
+//    meet by shuffles; the upper edge of a warp's row goes to the next warp, 6 values (and 2 weight sums) per lane and
+//    layer through shared memory, with one barrier per layer.  Lanes 1..30 finish nodes; a block of W warps finishes
+//    30 x (W - 1) nodes per layer.
+//  * The loads of the next layer and of this layer's output stage are issued before the arithmetic (FP32 Chebyshev on
+//    511x256x256: 874 us with them behind it, 666).
+//  * FP64 K u, with 12 warps per SM, waits longest at the barrier: there a warp arrives at an mbarrier when its edge of
+//    layer t is written, and waits (with a limit) before the output of layer t, which follows the x stage and the loads
+//    of layer t + 1 (511x256x256: 897 us with __syncthreads, 766 us).  The other forms hold the inputs of the output
+//    stage as well and got slower with it (FP64 residual 850, 938 us with it; FP32 residual 490, 600 us).
+//  * Two element rows per warp, with the edge between them in registers, need 128 registers in FP32: Chebyshev 736 us.
 //  * The 3x3 diagonal block of a node needs four signed sums of its 8 weights, factorised the same way.
 //
 // Fixed and inactive nodes enter the element products as zero (the reference's WS rule); out[] follows
@@ -25,12 +31,15 @@
 
 #include "rt_element.cuh"
 #include "rt_internal.h"
+#include "rt_tc.cuh"
 
 namespace {
 
 constexpr int FACE_NX = 30;  // node columns a warp finishes (lanes 1..30)
 
-constexpr int face_warps(bool f64, int mode, int rows) { return f64 ? (mode < 2 ? 12 : 8) : rows == 1 ? 8 : 4; }
+// warps per block: FP64 12, one block per SM (registers), 8 for the smoothing steps (two blocks of 8 with spills: residual
+// 1287 us, Chebyshev 2431 us on 511x256x256); FP32 8, three blocks
+constexpr int face_warps(bool f64, int mode) { return f64 && mode < 2 ? 12 : 8; }
 
 template <typename T>
 __device__ __forceinline__ T face_rcp(T x) {
@@ -77,14 +86,16 @@ __device__ __forceinline__ void face_grid_sum(double x, double* __restrict__ par
 // MODE 2: unew = u + omega D^-1 (f - K u)     MODE 3: Chebyshev step kstep: d = a_k d + b_k D^-1 (f - K u), unew = u + d
 // (fixed nodes in MODE 2/3: unew = f / n_e, d = 0; inactive nodes: 0)
 // code: per node, bit 0 active, bit 1 fixed (supports), for fixed nodes n_e << 2
-template <typename T, bool WS, int MODE, int R, int W, int MINB, bool DOT>
+template <typename T, bool WS, int MODE, int W, int MINB, bool DOT>
 __global__ void __launch_bounds__(32 * W, MINB)
     k_fine_face(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code, const float* __restrict__ wgt,
                 const rte::KtVals<T> kt, const T* __restrict__ u, const T* __restrict__ f, T* __restrict__ out, T omega,
                 T* __restrict__ dvec, const double* __restrict__ coef, int kstep, double* __restrict__ partials,
-                double* __restrict__ dot_out, unsigned* __restrict__ ticket) {
+                double* __restrict__ dot_out, unsigned* __restrict__ ticket, double* __restrict__ err) {
     constexpr int NX = MODE >= 2 ? 8 : 6;  // values handed to the next warp
+    constexpr bool LATE = sizeof(T) == 8 && MODE == 1;
     __shared__ T S[2][W][NX][32];
+    __shared__ uint64_t bar;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     T cheb_a = T(0), cheb_b = T(0);
     if (MODE == 3) {
@@ -94,23 +105,27 @@ __global__ void __launch_bounds__(32 * W, MINB)
     const int vx = nx + 1, vy = ny + 1, vz = nz + 1;
     const int nv = vx * vy * vz, plane = vx * vy, eplane = nx * ny;  // 3 nv < 2^31 (launch_face checks)
     const int ci = blockIdx.x * FACE_NX - 1 + lane;
-    const int rb = blockIdx.y * (W * R - 1) - 1 + w * R;  // the warp's first element row = first node row
+    const int ri = blockIdx.y * (W - 1) - 1 + w;  // the warp's element row = first node row
     const int Z0 = blockIdx.z * zchunk, Z1 = min(Z0 + zchunk, vz);
-    const bool own_col = lane >= 1 && lane <= FACE_NX && ci < vx;
-    bool n_ok[R + 1], e_ok[R];
-#pragma unroll
-    for (int r = 0; r <= R; r++) n_ok[r] = ci >= 0 && ci < vx && rb + r >= 0 && rb + r < vy;
-#pragma unroll
-    for (int r = 0; r < R; r++) e_ok[r] = ci >= 0 && ci < nx && rb + r >= 0 && rb + r < ny;
+    const bool c_ok = ci >= 0 && ci < vx, n_ok[2] = {c_ok && ri >= 0 && ri < vy, c_ok && ri + 1 >= 0 && ri + 1 < vy};
+    const bool e_ok = ci >= 0 && ci < nx && ri >= 0 && ri < ny;
+    const bool own = lane >= 1 && lane <= FACE_NX && n_ok[0] && w > 0;  // the lane finishes node (ci, ri)
+    if (LATE) {
+        if (threadIdx.x == 0) {
+            rttc::mbar_init(&bar, W);
+            rttc::fence_mbar_init();
+        }
+        __syncthreads();
+    }
 
-    T pu[R + 1][3];    // u of the next node layer, as stored
-    uint32_t pc[R + 1];  // its node codes
-    float pw[R];       // weights of the element layer below it
+    T pu[2][3];      // u of the next node layer, as stored
+    uint32_t pc[2];  // its node codes
+    float pw;        // weight of the element layer below it
     // node layer L (index vn of the lane's first node) and element layer L - 1 (index en)
     auto fetch = [&](int L, int vn, int en) {
         const bool zn = L >= 0 && L < vz, ze = L >= 1 && L <= nz;
 #pragma unroll
-        for (int r = 0; r <= R; r++) {
+        for (int r = 0; r < 2; r++) {
             const int v = vn + r * vx;
             pc[r] = 0;
             if (zn && n_ok[r]) {
@@ -120,10 +135,9 @@ __global__ void __launch_bounds__(32 * W, MINB)
                 pu[r][2] = u[2 * nv + v];
             }
         }
-#pragma unroll
-        for (int r = 0; r < R; r++) pw[r] = ze && e_ok[r] ? wgt[en + r * nx] : 0.f;
+        pw = ze && e_ok ? wgt[en] : 0.f;
     };
-    // x stage of node row r: sums and differences along the edge to the next column (active free nodes only)
+    // x stage of a node row: sums and differences along the edge to the next column (active free nodes only)
     auto x_stage = [&](const T (&p)[3], uint32_t c, T (&E)[6]) {
 #pragma unroll
         for (int q = 0; q < 3; q++) {
@@ -135,178 +149,174 @@ __global__ void __launch_bounds__(32 * W, MINB)
     };
 
     double pq = 0;  // DOT: the thread's part of u . out
-    T F[R][12];  // forward face data of node layer t
-    T G[R][12];  // inverse z output of element layer t - 1 toward node layer t
-    uint32_t co[R];
-    T Qp[R][4];  // signed weight sums of element layer t - 1
-    int vn = ci + vx * rb + plane * (Z0 - 1);  // node (ci, rb) of layer t
-    int en = ci + nx * rb + eplane * (Z0 - 1);
+    T F[12];        // forward face data of node layer t
+    T G[12];        // inverse z output of element layer t - 1 toward node layer t
+    uint32_t cc = 0, co = 0;              // node codes of the next layer and of the output stage's layer
+    T Qp[4] = {T(0), T(0), T(0), T(0)};   // signed weight sums of the element layer below the output stage's layer
+    T X[6], wa = T(0), wb = T(0);         // the output stage's x-edge data and weight sums along x
+    T fv[3], dv[3], uo[3];                // its inputs
+    int vn = ci + vx * ri + plane * (Z0 - 1);  // node (ci, ri) of layer t
+    int en = ci + nx * ri + eplane * (Z0 - 1);
     fetch(Z0 - 1, vn, en - eplane);
     {
         T E0[6], E1[6];
         x_stage(pu[0], pc[0], E0);
+        x_stage(pu[1], pc[1], E1);
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            x_stage(pu[r + 1], pc[r + 1], E1);
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                F[r][q] = E0[q] + E1[q];
-                F[r][6 + q] = E0[q] - E1[q];
-                E0[q] = E1[q];
-            }
-#pragma unroll
-            for (int q = 0; q < 12; q++) G[r][q] = T(0);
-#pragma unroll
-            for (int q = 0; q < 4; q++) Qp[r][q] = T(0);
-            co[r] = 0;
+        for (int q = 0; q < 6; q++) {
+            F[q] = E0[q] + E1[q];
+            F[6 + q] = E0[q] - E1[q];
         }
+#pragma unroll
+        for (int q = 0; q < 12; q++) G[q] = T(0);
     }
     fetch(Z0, vn + plane, en);
 
-    for (int t = Z0 - 1; t < Z1; t++, vn += plane, en += eplane) {
-        // ---- node layer t + 1 into the x stage, then the loads of layer t + 2
-        T E[R + 1][6];
-        uint32_t cn[R];
-        T wv[R];
-#pragma unroll
-        for (int r = 0; r <= R; r++) x_stage(pu[r], pc[r], E[r]);
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            cn[r] = pc[r];
-            wv[r] = (T)pw[r];
+    uint32_t phase = 0;
+    // node layer t (index v of the lane's node) from X, once every warp has written its edge of it.  The other buffer of
+    // S is written next; this one again only after the barrier of that one
+    auto output = [&](int t, int v) {
+        if (!LATE) {
+            __syncthreads();
+        } else {
+            const bool arrived = rttc::mbar_wait(&bar, phase);
+            if (!arrived && lane == 0) *err = 1.0;  // all warps of a block arrive in every layer: not reached
+            phase ^= 1;
         }
-        if (t + 1 < Z1) fetch(t + 2, vn + 2 * plane, en + eplane);
-        const bool lay = t >= Z0;
-        // ---- element layer t, last row first: X[r] collects the x-edge data of node row r
-        T X[R][6], wa[R], wb[R];
-#pragma unroll
-        for (int r = R - 1; r >= 0; r--) {
-            if (MODE >= 2) {
-                const T wl = __shfl_up_sync(0xffffffffu, wv[r], 1);
-                wa[r] = wv[r] + wl;
-                wb[r] = wv[r] - wl;
-            }
-            T h[24], z[24], Ft[12];
-#pragma unroll
-            for (int q = 0; q < 12; q++) {
-                const T hi = q < 6 ? E[r][q] + E[r + 1][q] : E[r][q - 6] - E[r + 1][q - 6];
-                h[q] = F[r][q] + hi;
-                h[12 + q] = F[r][q] - hi;
-                F[r][q] = hi;
-            }
-            // rows 0..2 of Kt (the rigid translations) are empty; a row's first product initialises it
-#pragma unroll
-            for (int k = 0; k < 45; k++) {
-                if (k == 0 || rte::KT_R[k - 1] != rte::KT_R[k]) z[rte::KT_R[k]] = kt.v[k] * h[rte::KT_C[k]];
-                else z[rte::KT_R[k]] += kt.v[k] * h[rte::KT_C[k]];
-            }
-#pragma unroll
-            for (int q = 0; q < 12; q++) {
-                const T s = q < 3 ? z[12 + q] : z[q] + z[12 + q], d = q < 3 ? -z[12 + q] : z[q] - z[12 + q];
-                Ft[q] = G[r][q] + wv[r] * s;  // toward node layer t, with element layer t - 1's part
-                G[r][q] = wv[r] * d;          // toward node layer t + 1
-            }
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                const T up = Ft[q] - Ft[6 + q];
-                X[r][q] = Ft[q] + Ft[6 + q];
-                if (r + 1 < R) X[r + 1 < R ? r + 1 : 0][q] += up;
-                else S[t & 1][w][q][lane] = up;
-            }
-        }
-        // ---- output-stage inputs of node layer t
-        T fv[R][3], dv[R][3], uo[R][3];
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-            const int v = vn + r * vx;
-            const bool ld = lay && own_col && co[r] != 0 && (r > 0 || w > 0);
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                fv[r][c] = (MODE != 1 && ld) ? f[c * nv + v] : T(0);
-                dv[r][c] = (MODE == 3 && ld && kstep > 0) ? dvec[c * nv + v] : T(0);
-                uo[r][c] = ((MODE >= 2 || DOT || (WS && MODE == 1 && co[r] > 1u)) && ld) ? u[c * nv + v] : T(0);  // in L1: layer t was fetched two layers ago
-            }
-        }
-        if (MODE >= 2) {
-            S[t & 1][w][NX - 2][lane] = wa[R - 1];
-            S[t & 1][w][NX - 1][lane] = wb[R - 1];
-        }
-        __syncthreads();
-        // the other buffer is written in the next iteration; this one again only after that one's barrier
         T wa_b = T(0), wb_b = T(0);
         if (w > 0) {
 #pragma unroll
-            for (int q = 0; q < 6; q++) X[0][q] += S[t & 1][w > 0 ? w - 1 : 0][q][lane];
+            for (int q = 0; q < 6; q++) X[q] += S[t & 1][w - 1][q][lane];
             if (MODE >= 2) {
-                wa_b = S[t & 1][w > 0 ? w - 1 : 0][NX - 2][lane];
-                wb_b = S[t & 1][w > 0 ? w - 1 : 0][NX - 1][lane];
+                wa_b = S[t & 1][w - 1][NX - 2][lane];
+                wb_b = S[t & 1][w - 1][NX - 1][lane];
             }
         }
-        // ---- node layer t
+        T acc[3];
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            T acc[3];
+        for (int c = 0; c < 3; c++) acc[c] = X[c] + X[3 + c] + __shfl_up_sync(0xffffffffu, X[c] - X[3 + c], 1);
+        T Q[4];
+        if (MODE >= 2) {
+            Q[0] = wa + wa_b;  // sum w
+            Q[1] = wb - wb_b;  // sum w sx sy
+            Q[2] = wa - wa_b;  // sum w sy
+            Q[3] = wb + wb_b;  // sum w sx
+        }
+        if (t >= Z0 && own) {
+            const bool act = co != 0, fixed = WS && co > 1u;
+            T o[3] = {T(0), T(0), T(0)}, dn[3] = {T(0), T(0), T(0)};
+            if (MODE == 0) {
 #pragma unroll
-            for (int c = 0; c < 3; c++)
-                acc[c] = X[r][c] + X[r][3 + c] + __shfl_up_sync(0xffffffffu, X[r][c] - X[r][3 + c], 1);
-            T Q[4];
-            if (MODE >= 2) {
-                const T ab = r > 0 ? wa[r > 0 ? r - 1 : 0] : wa_b, bb = r > 0 ? wb[r > 0 ? r - 1 : 0] : wb_b;
-                Q[0] = wa[r] + ab;  // sum w
-                Q[1] = wb[r] - bb;  // sum w sx sy
-                Q[2] = wa[r] - ab;  // sum w sy
-                Q[3] = wb[r] + bb;  // sum w sx
-            }
-            if (lay && own_col && n_ok[r] && (r > 0 || w > 0)) {
-                const int v = vn + r * vx;
-                const bool act = co[r] != 0, fixed = WS && co[r] > 1u;
-                T o[3] = {T(0), T(0), T(0)}, dn[3] = {T(0), T(0), T(0)};
-                if (MODE == 0) {
+                for (int c = 0; c < 3; c++) o[c] = act ? (fixed ? fv[c] : fv[c] - acc[c]) : T(0);
+            } else if (MODE == 1) {
 #pragma unroll
-                    for (int c = 0; c < 3; c++) o[c] = act ? (fixed ? fv[r][c] : fv[r][c] - acc[c]) : T(0);
-                } else if (MODE == 1) {
+                for (int c = 0; c < 3; c++) {
+                    o[c] = act ? (fixed ? uo[c] : acc[c]) : T(0);
+                    if (DOT) pq += (double)uo[c] * (double)o[c];
+                }
+            } else if (fixed) {
 #pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        o[c] = act ? (fixed ? uo[r][c] : acc[c]) : T(0);
-                        if (DOT) pq += (double)uo[r][c] * (double)o[c];
-                    }
-                } else if (fixed) {
+                for (int c = 0; c < 3; c++) o[c] = fv[c] / T(co >> 2);
+            } else if (act) {
+                const T sw = Q[0] + Qp[0], sxy = Q[1] + Qp[1], sxz = Q[3] - Qp[3], syz = Q[2] - Qp[2];
+                const T A = kt.diag_a * sw, bxy = kt.diag_b * sxy, bxz = kt.diag_b * sxz, byz = kt.diag_b * syz;
+                // inverse of [[A,bxy,bxz],[bxy,A,byz],[bxz,byz,A]]
+                const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
+                const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
+                const T id = face_rcp(A * c00 + bxy * c01 + bxz * c02);
+                T rr[3];
 #pragma unroll
-                    for (int c = 0; c < 3; c++) o[c] = fv[r][c] / T(co[r] >> 2);
-                } else if (act) {
-                    const T sw = Q[0] + Qp[r][0], sxy = Q[1] + Qp[r][1], sxz = Q[3] - Qp[r][3], syz = Q[2] - Qp[r][2];
-                    const T A = kt.diag_a * sw, bxy = kt.diag_b * sxy, bxz = kt.diag_b * sxz, byz = kt.diag_b * syz;
-                    // inverse of [[A,bxy,bxz],[bxy,A,byz],[bxz,byz,A]]
-                    const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
-                    const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
-                    const T id = face_rcp(A * c00 + bxy * c01 + bxz * c02);
-                    T rr[3];
+                for (int c = 0; c < 3; c++) rr[c] = fv[c] - acc[c];
+                const T zz[3] = {id * (c00 * rr[0] + c01 * rr[1] + c02 * rr[2]),
+                                 id * (c01 * rr[0] + c11 * rr[1] + c12 * rr[2]),
+                                 id * (c02 * rr[0] + c12 * rr[1] + c22 * rr[2])};
 #pragma unroll
-                    for (int c = 0; c < 3; c++) rr[c] = fv[r][c] - acc[c];
-                    const T zz[3] = {id * (c00 * rr[0] + c01 * rr[1] + c02 * rr[2]),
-                                     id * (c01 * rr[0] + c11 * rr[1] + c12 * rr[2]),
-                                     id * (c02 * rr[0] + c12 * rr[1] + c22 * rr[2])};
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        if (MODE == 2) {
-                            o[c] = uo[r][c] + omega * zz[c];
-                        } else {
-                            dn[c] = cheb_a * dv[r][c] + cheb_b * zz[c];  // dv = 0 in step 0
-                            o[c] = uo[r][c] + dn[c];
-                        }
+                for (int c = 0; c < 3; c++) {
+                    if (MODE == 2) {
+                        o[c] = uo[c] + omega * zz[c];
+                    } else {
+                        dn[c] = cheb_a * dv[c] + cheb_b * zz[c];  // dv = 0 in step 0
+                        o[c] = uo[c] + dn[c];
                     }
                 }
-#pragma unroll
-                for (int c = 0; c < 3; c++) out[c * nv + v] = o[c];
-                if (MODE == 3)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) dvec[c * nv + v] = dn[c];
             }
-            if (MODE >= 2)
 #pragma unroll
-                for (int q = 0; q < 4; q++) Qp[r][q] = Q[q];
-            co[r] = cn[r];
+            for (int c = 0; c < 3; c++) out[c * nv + v] = o[c];
+            if (MODE == 3)
+#pragma unroll
+                for (int c = 0; c < 3; c++) dvec[c * nv + v] = dn[c];
         }
+        if (MODE >= 2)
+#pragma unroll
+            for (int q = 0; q < 4; q++) Qp[q] = Q[q];
+    };
+
+    for (int t = Z0 - 1;; t++, vn += plane, en += eplane) {
+        if (!LATE && t == Z1) break;
+        // ---- node layer t + 1 into the x stage, then the loads of layer t + 2
+        T E0[6], E1[6], wv = T(0);
+        uint32_t cn = 0;
+        if (!LATE || t < Z1) {
+            x_stage(pu[0], pc[0], E0);
+            x_stage(pu[1], pc[1], E1);
+            cn = pc[0];
+            wv = (T)pw;
+            if (t + 1 < Z1) fetch(t + 2, vn + 2 * plane, en + eplane);
+        }
+        if (LATE) {
+            if (t >= Z0) output(t - 1, vn - plane);
+            if (t == Z1) break;
+        }
+        co = cc;
+        cc = cn;
+        // inputs of layer t's output stage (u is in L1: the layer was fetched two layers ago)
+        const bool ld = t >= Z0 && own && co != 0;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            fv[c] = (MODE != 1 && ld) ? f[c * nv + vn] : T(0);
+            dv[c] = (MODE == 3 && ld && kstep > 0) ? dvec[c * nv + vn] : T(0);
+            uo[c] = ((MODE >= 2 || DOT || (WS && MODE == 1 && co > 1u)) && ld) ? u[c * nv + vn] : T(0);
+        }
+        // ---- element layer t
+        if (MODE >= 2) {
+            const T wl = __shfl_up_sync(0xffffffffu, wv, 1);
+            wa = wv + wl;
+            wb = wv - wl;
+        }
+        T h[24], z[24], Ft[12];
+#pragma unroll
+        for (int q = 0; q < 12; q++) {
+            const T hi = q < 6 ? E0[q] + E1[q] : E0[q - 6] - E1[q - 6];
+            h[q] = F[q] + hi;
+            h[12 + q] = F[q] - hi;
+            F[q] = hi;
+        }
+        // rows 0..2 of Kt (the rigid translations) are empty; a row's first product initialises it
+#pragma unroll
+        for (int k = 0; k < 45; k++) {
+            if (k == 0 || rte::KT_R[k - 1] != rte::KT_R[k]) z[rte::KT_R[k]] = kt.v[k] * h[rte::KT_C[k]];
+            else z[rte::KT_R[k]] += kt.v[k] * h[rte::KT_C[k]];
+        }
+#pragma unroll
+        for (int q = 0; q < 12; q++) {
+            const T s = q < 3 ? z[12 + q] : z[q] + z[12 + q], d = q < 3 ? -z[12 + q] : z[q] - z[12 + q];
+            Ft[q] = G[q] + wv * s;  // toward node layer t, with element layer t - 1's part
+            G[q] = wv * d;          // toward node layer t + 1
+        }
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+            X[q] = Ft[q] + Ft[6 + q];
+            S[t & 1][w][q][lane] = Ft[q] - Ft[6 + q];
+        }
+        if (MODE >= 2) {
+            S[t & 1][w][NX - 2][lane] = wa;
+            S[t & 1][w][NX - 1][lane] = wb;
+        }
+        if (LATE) {
+            __syncwarp();
+            if (lane == 0) rttc::mbar_arrive(&bar);
+        }
+        if (!LATE) output(t, vn);
     }
     // no second launch and no second read of u and out for p.q
     if (DOT) face_grid_sum<W>(pq, partials, dot_out, ticket);
@@ -400,17 +410,18 @@ __global__ void k_node_code(int nx, int ny, int nz, const uint8_t* __restrict__ 
     }
 }
 
-template <typename T, bool WS, int MODE, int R, int W, int MINB, bool DOT>
-int launch_face_rw(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
-                   const double* coef, int kstep, double* dot_out) {
+template <typename T, bool WS, int MODE, bool DOT>
+int launch_face_dot(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
+                    const double* coef, int kstep, double* dot_out) {
+    constexpr int W = face_warps(sizeof(T) == 8, MODE), MINB = sizeof(T) == 8 ? 1 : 3;
     rt_level& L = h->L[0];
     const int zc = h->tune[sizeof(T) == 8 ? 1 : 0][MODE].zchunk;
-    const dim3 grid((L.vx + FACE_NX - 1) / FACE_NX, (L.vy + W * R - 2) / (W * R - 1), (L.vz + zc - 1) / zc);
+    const dim3 grid((L.vx + FACE_NX - 1) / FACE_NX, (L.vy + W - 2) / (W - 1), (L.vz + zc - 1) / zc);
     const rte::KtVals<T> kt = rte::make_kt<T>(h);
     return rt_launch(h->ctx, name, [&] {
-        k_fine_face<T, WS, MODE, R, W, MINB, DOT><<<grid, 32 * W, 0, h->ctx->stream>>>(
+        k_fine_face<T, WS, MODE, W, MINB, DOT><<<grid, 32 * W, 0, h->ctx->stream>>>(
             L.nx, L.ny, L.nz, zc, h->ncode, h->w, kt, u, f, out, (T)omega, dvec, coef, kstep, h->kpart, dot_out,
-            reinterpret_cast<unsigned*>(h->scal + RT_SCAL_TICKET));
+            reinterpret_cast<unsigned*>(h->scal + RT_SCAL_TICKET), h->scal + RT_SCAL_ERR);
     });
 }
 
@@ -448,26 +459,10 @@ int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const do
 template int fine_smooth0<double>(rt_hier*, const double*, double*, double, double*, const double*, double*);
 template int fine_smooth0<float>(rt_hier*, const float*, float*, double, float*, const double*, double*);
 
-// the block shape of ty element rows per warp (measured on 511x256x256, where a spill costs more than a block):
-// FP32 1 row 8 warps, 2 rows 4 warps; FP64 1 row, 12 warps in one block per SM, 8 where the smoothing step needs
-// the registers (845 us residual and 1526 us Chebyshev step; two blocks of 8 warps with spills: 1287 and 2431 us)
-template <typename T, bool WS, int MODE, bool DOT>
-static int launch_face_shape(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
-                             const double* coef, int kstep, double* dot_out) {
-    if constexpr (sizeof(T) == 8) {
-        constexpr int W = face_warps(true, MODE, 1);
-        return launch_face_rw<T, WS, MODE, 1, W, 1, DOT>(h, u, f, out, omega, name, dvec, coef, kstep, dot_out);
-    } else {
-        if (h->tune[0][MODE].ty == 1)
-            return launch_face_rw<T, WS, MODE, 1, 8, 3, DOT>(h, u, f, out, omega, name, dvec, coef, kstep, dot_out);
-        return launch_face_rw<T, WS, MODE, 2, 4, 4, DOT>(h, u, f, out, omega, name, dvec, coef, kstep, dot_out);
-    }
-}
-
 template <typename T, bool WS, int MODE>
 int launch_face(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec,
                 const double* coef, int kstep) {
-    return launch_face_shape<T, WS, MODE, false>(h, u, f, out, omega, name, dvec, coef, kstep, nullptr);
+    return launch_face_dot<T, WS, MODE, false>(h, u, f, out, omega, name, dvec, coef, kstep, nullptr);
 }
 
 // partial sums of K u's dot product: one per block of the smallest launch shape (7 rows, one layer)
@@ -486,8 +481,8 @@ int fine_applyK_dot(rt_hier* h, const T* u, T* out, double* dot_dev) {
         else return dot32(h, n, u, out, dot_dev);
     }
     const char* nm = sizeof(T) == 8 ? "fine_applyK_f64" : "fine_applyK_f32";
-    return h->has_support ? launch_face_shape<T, true, 1, true>(h, u, nullptr, out, 0.0, nm, nullptr, nullptr, 0, dot_dev)
-                          : launch_face_shape<T, false, 1, true>(h, u, nullptr, out, 0.0, nm, nullptr, nullptr, 0, dot_dev);
+    return h->has_support ? launch_face_dot<T, true, 1, true>(h, u, nullptr, out, 0.0, nm, nullptr, nullptr, 0, dot_dev)
+                          : launch_face_dot<T, false, 1, true>(h, u, nullptr, out, 0.0, nm, nullptr, nullptr, 0, dot_dev);
 }
 template int fine_applyK_dot<double>(rt_hier*, const double*, double*, double*);
 template int fine_applyK_dot<float>(rt_hier*, const float*, float*, double*);
@@ -496,10 +491,10 @@ template int fine_applyK_dot<float>(rt_hier*, const float*, float*, double*);
 // (a chunk of zc layers takes zc + 2 steps).  64x32x32: 2, 129x97x85: 16, 255x256x128: 16, as the sweep found best
 // or within 5 %
 rt_tile_cfg face_default(rt_ctx* c, bool f64, int mode, int vx, int vy, int vz) {
-    const int r = f64 || mode == 0 ? 1 : 2, w = face_warps(f64, mode, r);
-    const long slots = (long)c->sm_count * (f64 ? 1 : r == 1 ? 3 : 4);
-    const long xy = (long)((vx + FACE_NX - 1) / FACE_NX) * ((vy + w * r - 2) / (w * r - 1));
-    rt_tile_cfg best{8, r, 2};
+    const int w = face_warps(f64, mode);
+    const long slots = (long)c->sm_count * (f64 ? 1 : 3);
+    const long xy = (long)((vx + FACE_NX - 1) / FACE_NX) * ((vy + w - 2) / (w - 1));
+    rt_tile_cfg best{8, 1, 2};
     long cost = -1;
     for (int zc = 2; zc <= 64; zc *= 2) {
         const long waves = (xy * ((vz + zc - 1) / zc) + slots - 1) / slots, cz = waves * (zc + 2);

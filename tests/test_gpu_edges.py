@@ -37,15 +37,15 @@ def _perforated(nx, ny, nz, seed, sup, skip=1):
 
 # node columns finished per warp 30, node rows per block 7 (FP32, and FP64 smoothing), 11 (FP64): boxes one below,
 # at and above these, and z-chunks that end inside the box, at its end and beyond it
-@pytest.mark.parametrize("nx,ny,nz,rows,zc", [(29, 6, 9, 1, 1), (30, 7, 16, 1, 2), (31, 13, 8, 2, 3), (59, 10, 7, 2, 64),
-                                              (60, 11, 15, 1, 16), (12, 21, 17, 2, 5), (95, 8, 8, 2, 4)])
+@pytest.mark.parametrize("nx,ny,nz,zc", [(29, 6, 9, 1), (30, 7, 16, 2), (31, 13, 8, 3), (59, 10, 7, 64), (60, 11, 15, 16),
+                                         (12, 21, 17, 5), (95, 8, 8, 4)])
 @pytest.mark.parametrize("sup", [True, False])
-def test_face_march_edges(nx, ny, nz, rows, zc, sup):
+def test_face_march_edges(nx, ny, nz, zc, sup):
     ctx, G, H, r = _perforated(nx, ny, nz, nx + ny, sup)
     L = rb.lib()
     for prec in (rb.FP64, rb.FP32):
         for m in range(4):
-            rb._capi.check(L.rt_set_tuning(G.handle, prec, m, 8, 1 if prec == rb.FP64 else rows, zc), ctx.handle)
+            rb._capi.check(L.rt_set_tuning(G.handle, prec, m, 8, 1, zc), ctx.handle)
     act = np.tile(G[0].getVact(), 3).astype(bool)
     u = r.standard_normal(3 * G[0].nv)
     u[~act] = np.nan  # values of nodes without elements are not read into any result

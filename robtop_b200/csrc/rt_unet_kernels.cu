@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv3_halo(ConvArgs a, int P, 
 // P, then the largest G, whose halo and weight stages fit in 200 KB; P = 0 if nothing fits.  More planes re-read
 // less of the halo, but a box of xy patches x Z planes is cut into no fewer CTAs than the GPU has SMs where it can be:
 // on a 33^3 training crop, 8 planes left half of the SMs idle and each CTA's loads and MMAs in series (37 us a
-// convolution, 17 us with the rule)
+// convolution, 25 us with the rule)
 static int halo_plan(int cin, int cout, long xy, int Z, int sms, int* G, size_t* smem) {
     static const int gs[4] = {27, 9, 3, 1};
     // first pass: plans that leave two CTAs per SM (one loads its halo while the other multiplies);
@@ -616,7 +616,7 @@ __global__ void k_head(const __nv_bfloat16* __restrict__ in, int C, long V, cons
 
 // head backward: gin[v][c] = sum_k hw[k][c] gout[v][k]; dhw, dhb by warp sums, one shared atomic per warp and value, one
 // global atomic per block.  C = 16 is the head's width: with a run-time C the 51 sums lived in local memory (130 us on
-// 33^3, 10 us here).
+// 33^3, 17 us here).
 __global__ void __launch_bounds__(128) k_head_bwd(const __nv_bfloat16* __restrict__ in, long V,
                                                   const float* __restrict__ hw, const float* __restrict__ gout,
                                                   float* __restrict__ gin, float* __restrict__ dhw,

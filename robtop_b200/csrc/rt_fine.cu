@@ -168,8 +168,9 @@ __global__ void k_penalty(long ne, const uint8_t* __restrict__ eact, const float
 // ELEM_C = true: c_e = rho^p u_e.KE u_e (elementCompliance_kernel, grid/Grid.cu:3434-3480).
 // u_e.KE u_e = h.Kt h with h = H u_e the Hadamard transform of the element's displacements (rt_element.cuh): 45
 // products instead of 576.  A thread marches an element column through a z-chunk and keeps the x and y stages of the
-// node layer below, 48 adds and 12 loads per element.  FP64 arithmetic bound: 255x256x128 took 835 us with the dense
-// 24 x 24 product, 150 us here.
+// node layer below, 48 adds and 12 loads per element, issued a layer ahead.  255x256x128: 835 us with the dense 24 x 24
+// product, 288 us with one chain of 45 products and the loads in their own layer, 167 us here.  Latency bound, at three
+// blocks per SM (four, with spills: 197 us).
 template <bool ELEM_C>
 __global__ void __launch_bounds__(128) k_sensitivity(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ eact,
                                                      const float* __restrict__ rho, float p,
@@ -181,12 +182,24 @@ __global__ void __launch_bounds__(128) k_sensitivity(int nx, int ny, int nz, int
     const long plane = (long)vx * vy, nv = plane * (nz + 1);
     const int Z0 = blockIdx.z * zchunk, Z1 = min(Z0 + zchunk, nz);
     long v = x + (long)vx * y + plane * Z0, e = x + (long)nx * (y + (long)ny * Z0);
-    // x and y stages of the four nodes of a layer: index 3 (mx + 2 my) + component
-    auto face = [&](long n, double (&F)[12]) {
+    double raw[12];  // the four nodes of the next layer, loaded a layer ahead
+    float nro = 0.f;
+    bool nact = false;
+    auto load = [&](long n) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             const double* q = u + c * nv + n;
-            const double a = q[0], b = q[1], d = q[vx], g = q[vx + 1];
+            raw[4 * c] = q[0];
+            raw[4 * c + 1] = q[1];
+            raw[4 * c + 2] = q[vx];
+            raw[4 * c + 3] = q[vx + 1];
+        }
+    };
+    // x and y stages of the four nodes of a layer: index 3 (mx + 2 my) + component
+    auto face = [&](double (&F)[12]) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const double a = raw[4 * c], b = raw[4 * c + 1], d = raw[4 * c + 2], g = raw[4 * c + 3];
             F[c] = (a + b) + (d + g);
             F[3 + c] = (a - b) + (d - g);
             F[6 + c] = (a + b) - (d + g);
@@ -194,12 +207,21 @@ __global__ void __launch_bounds__(128) k_sensitivity(int nx, int ny, int nz, int
         }
     };
     double lo[12], hi[12];
-    face(v, lo);
+    load(v);
+    face(lo);
+    load(v + plane);
+    nact = eact[e];
+    nro = rho[e];
     for (int z = Z0; z < Z1; z++, e += (long)nx * ny) {
         v += plane;
-        face(v, hi);
-        const bool act = eact[e];
-        const float ro = rho[e];
+        face(hi);
+        const bool act = nact;
+        const float ro = nro;
+        if (z + 1 < Z1) {
+            load(v + plane);
+            nact = eact[e + (long)nx * ny];
+            nro = rho[e + (long)nx * ny];
+        }
         double h[24];
 #pragma unroll
         for (int q = 0; q < 12; q++) {
@@ -207,10 +229,17 @@ __global__ void __launch_bounds__(128) k_sensitivity(int nx, int ny, int nz, int
             h[12 + q] = lo[q] - hi[q];
             lo[q] = hi[q];
         }
-        double s = 0;
+        // row sums first: 66 products instead of 90, in short chains instead of one of 45
+        double zz[24], t[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-        for (int k = 0; k < 45; k++) s += kt.v[k] * h[rte::KT_R[k]] * h[rte::KT_C[k]];
-        s = fabs(s);  // u.KE u >= 0: where an element moves rigidly, the rounding left over may be negative
+        for (int k = 0; k < 45; k++) {
+            if (k == 0 || rte::KT_R[k - 1] != rte::KT_R[k]) zz[rte::KT_R[k]] = kt.v[k] * h[rte::KT_C[k]];
+            else zz[rte::KT_R[k]] += kt.v[k] * h[rte::KT_C[k]];
+        }
+#pragma unroll
+        for (int r = 3; r < 24; r++) t[r % 3] += h[r] * zz[r];
+        // u.KE u >= 0: where an element moves rigidly, the rounding left over may be negative
+        const double s = fabs(t[0] + t[1] + t[2]);
         if (ELEM_C)
             sens[e] = act ? (float)(s * (double)powf(ro, p)) : 0.f;
         else

@@ -245,6 +245,22 @@ def test_coarsest_inverse_block_edges(dims, limit):
     ctx.close()
 
 
+# sensitivity: columns of 32 x 4 elements, z-chunks of 2 to 16 layers whose next layer is loaded ahead
+@pytest.mark.parametrize("nx,ny,nz", [(31, 5, 8), (32, 4, 9), (33, 9, 17), (65, 41, 33)])
+def test_sensitivity_edges(nx, ny, nz):
+    ctx, G, H, r = _perforated(nx, ny, nz, nx, True)
+    rho = G[0].getRho()
+    u = r.standard_normal(3 * G[0].nv)
+    G[0].setDisplacement(u)
+    rb._capi.check(rb.lib().rt_sensitivity(G.handle, 0), ctx.handle)
+    want = np.zeros(nx * ny * nz, np.float32)
+    O.lib().or_sensitivity(nx, ny, nz, O.ptr(H.arrs[0]["eact"]), O.ptr(rho), float(P), O.ptr(H.KE), O.ptr(u), O.ptr(want))
+    # FP32 results: powf to 2 units in the last place, a product and the rounding of either side
+    assert np.all(np.abs(G[0].getSens() - want) <= 6 * 2.0**-24 * np.abs(want))
+    G.close()
+    ctx.close()
+
+
 # Galerkin stencils: 32 x 2 nodes per block (33 and 34 coarse nodes in x, odd rows), both coarsening ratios, fixed
 # nodes inside and on the faces; dyadic levels below
 @pytest.mark.parametrize("dims,skip", [((127, 9, 7), 1), ((131, 6, 13), 1), ((63, 7, 6), 0), ((20, 18, 14), 0)])

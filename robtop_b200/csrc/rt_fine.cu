@@ -158,10 +158,20 @@ __global__ void __launch_bounds__(GS_BS, WS ? 4 : 3) k_fine_gs(int nx, int ny, i
     }
 }
 
+// four elements per thread (the arrays are allocations of their own): 255x256x128 49 us with one and the launch, 38 us (powf)
 __global__ void k_penalty(long ne, const uint8_t* __restrict__ eact, const float* __restrict__ rho, float p,
                           float* __restrict__ w) {
-    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < ne; e += (long)gridDim.x * blockDim.x)
+    const long n4 = ne / 4, tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    for (long i = tid; i < n4; i += (long)gridDim.x * blockDim.x) {
+        const uchar4 a = reinterpret_cast<const uchar4*>(eact)[i];
+        const float4 r = reinterpret_cast<const float4*>(rho)[i];
+        reinterpret_cast<float4*>(w)[i] = make_float4(a.x ? powf(r.x, p) : 0.f, a.y ? powf(r.y, p) : 0.f,
+                                                      a.z ? powf(r.z, p) : 0.f, a.w ? powf(r.w, p) : 0.f);
+    }
+    if (tid < ne - 4 * n4) {
+        const long e = 4 * n4 + tid;
         w[e] = eact[e] ? powf(rho[e], p) : 0.f;
+    }
 }
 
 // ELEM_C = false: s_e = -p rho^(p-1) u_e.KE u_e (computeSensitivity_kernel, optimization/optimization.cu:44-107);
@@ -260,7 +270,7 @@ namespace rtk {
 int penalty_weights(rt_hier* h) {
     rt_level& L = h->L[0];
     return rt_launch(h->ctx, "penalty_weights", [&] {
-        k_penalty<<<fine_grid(h->ctx, L.ne), FINE_BS, 0, h->ctx->stream>>>(L.ne, L.eact, h->rho, h->P.power_penalty,
+        k_penalty<<<fine_grid(h->ctx, (L.ne + 3) / 4), FINE_BS, 0, h->ctx->stream>>>(L.ne, L.eact, h->rho, h->P.power_penalty,
                                                                           h->w);
     });
 }

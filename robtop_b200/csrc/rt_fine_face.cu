@@ -388,14 +388,15 @@ __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int z
 }
 
 // node codes read by k_fine_face: bit 0 active, bit 1 fixed, bits 2.. the number of elements of non-zero weight
-// around a fixed node (its smoothing rule f / n_e)
+// around a fixed node (its smoothing rule f / n_e).  Four nodes per thread (the arrays are allocations of their own):
+// 255x256x128 37 us with one and the launch, 17 us
 __global__ void k_node_code(int nx, int ny, int nz, const uint8_t* __restrict__ vact, const uint8_t* __restrict__ vfix,
                             const float* __restrict__ w, uint8_t* __restrict__ code) {
     const int vx = nx + 1, vy = ny + 1;
-    const long nv = (long)vx * vy * (nz + 1);
-    for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += (long)gridDim.x * blockDim.x) {
-        uint8_t c = vact[v] ? 1 : 0;
-        if (c && vfix != nullptr && vfix[v]) {
+    const long nv = (long)vx * vy * (nz + 1), n4 = nv / 4, tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    auto node = [&](long v, bool act, bool fix) {
+        uint8_t c = act ? 1 : 0;
+        if (act && fix) {
             const int x = (int)(v % vx), y = (int)((v / vx) % vy), z = (int)(v / ((long)vx * vy));
             int ne = 0;
             for (int i = 0; i < 8; i++) {
@@ -406,7 +407,17 @@ __global__ void k_node_code(int nx, int ny, int nz, const uint8_t* __restrict__ 
             }
             c = (uint8_t)(3 | (ne << 2));
         }
-        code[v] = c;
+        return c;
+    };
+    for (long i = tid; i < n4; i += (long)gridDim.x * blockDim.x) {
+        const uchar4 a = reinterpret_cast<const uchar4*>(vact)[i];
+        const uchar4 f = vfix != nullptr ? reinterpret_cast<const uchar4*>(vfix)[i] : make_uchar4(0, 0, 0, 0);
+        reinterpret_cast<uchar4*>(code)[i] = make_uchar4(node(4 * i, a.x, f.x), node(4 * i + 1, a.y, f.y),
+                                                         node(4 * i + 2, a.z, f.z), node(4 * i + 3, a.w, f.w));
+    }
+    if (tid < nv - 4 * n4) {
+        const long v = 4 * n4 + tid;
+        code[v] = node(v, vact[v], vfix != nullptr && vfix[v]);
     }
 }
 
@@ -432,7 +443,7 @@ namespace rtk {
 int node_codes(rt_hier* h) {
     rt_level& L = h->L[0];
     return rt_launch(h->ctx, "node_codes", [&] {
-        k_node_code<<<(unsigned)std::min<long>((L.nv + 255) / 256, (long)h->ctx->sm_count * 16), 256, 0,
+        k_node_code<<<(unsigned)std::min<long>((L.nv + 1023) / 1024, (long)h->ctx->sm_count * 16), 256, 0,
                       h->ctx->stream>>>(L.nx, L.ny, L.nz, L.vact, h->has_support ? h->vfix : nullptr, h->w, h->ncode);
     });
 }

@@ -347,7 +347,7 @@ static void free_hier(rt_hier* h) {
         cudaFree(L.aidx); cudaFree(L.ainv); cudaFree(L.dvec);
         cudaFree(L.crow); cudaFree(L.cpanels); cudaFree(L.cstatus); cudaFree(L.crigid); cudaFree(L.cfix);
     }
-    cudaFree(h->KE_dev); cudaFree(h->KE32_dev); cudaFree(h->rho); cudaFree(h->w); cudaFree(h->vfix);
+    cudaFree(h->KE_dev); cudaFree(h->rho); cudaFree(h->w); cudaFree(h->vfix);
     cudaFree(h->sens); cudaFree(h->ftmp); cudaFree(h->eshell); cudaFree(h->load_nodes); cudaFree(h->load_normal);
     cudaFree(h->Rd); cudaFree(h->Ru); cudaFree(h->fs); cudaFree(h->fs_old); cudaFree(h->x); cudaFree(h->rr);
     cudaFree(h->z); cudaFree(h->p); cudaFree(h->q); cudaFree(h->rold); cudaFree(h->Q); cudaFree(h->partials);
@@ -383,7 +383,7 @@ static void ws_sync(rt_hier* w) {
         a.n_act_nodes = b.n_act_nodes; a.n_act_elems = b.n_act_elems;
     }
     memcpy(w->KE, p->KE, sizeof(w->KE));
-    w->KE_dev = p->KE_dev; w->KE32_dev = p->KE32_dev;
+    w->KE_dev = p->KE_dev;
     w->rho = p->rho; w->w = p->w; w->vfix = p->vfix; w->has_support = p->has_support;
     w->sens = p->sens; w->ftmp = p->ftmp; w->eshell = p->eshell;
     w->nload = p->nload; w->load_nodes = p->load_nodes; w->load_normal = p->load_normal; w->Rd = p->Rd;
@@ -404,10 +404,7 @@ static void ws_sync(rt_hier* w) {
 
 static int upload_KE(rt_hier* h) {
     template_matrix(h->P.youngs_modulus, h->P.poisson_ratio, h->P.element_length, h->KE);
-    float ke32[576];
-    for (int i = 0; i < 576; i++) ke32[i] = (float)h->KE[i];
     RT_CUDA(h->ctx, cudaMemcpyAsync(h->KE_dev, h->KE, sizeof(double) * 576, cudaMemcpyHostToDevice, h->ctx->stream));
-    RT_CUDA(h->ctx, cudaMemcpyAsync(h->KE32_dev, ke32, sizeof(float) * 576, cudaMemcpyHostToDevice, h->ctx->stream));
     RT_CUDA(h->ctx, cudaStreamSynchronize(h->ctx->stream));
     if (h->Qgal) { cudaFree(h->Qgal); h->Qgal = nullptr; h->Qgal_ratio = 0; }
     h->graph_epoch++;  // the element operator's Hadamard-domain values are kernel parameters
@@ -513,7 +510,6 @@ static int build_hier(rt_ctx* c, const rt_params* p, int nx, int ny, int nz, uin
     }
     rt_level& L0 = h->L[0];
     RT_CHECK(dalloc(c, &h->KE_dev, 576));
-    RT_CHECK(dalloc(c, &h->KE32_dev, 576));
     RT_CHECK(dalloc(c, &h->dinv64, 6 * (size_t)L0.nv));
     RT_CHECK(dalloc(c, &h->dinv32, 6 * (size_t)L0.nv));
     RT_CHECK(dalloc(c, &h->ncode, (size_t)L0.nv));

@@ -60,8 +60,8 @@ __device__ __forceinline__ T st_centre(const S* sb, long rs, int rc) {
 
 // one colour of the point-block GS on a stencil level, LPN lanes per node: lane q sums neighbours k = q, q + LPN, ...
 // (the low lane bits count nodes, so that neighbouring lanes read neighbouring columns).  A colour of the levels below
-// the first has tens to hundreds of nodes, where a thread's 27 x 12 loads one after another took 16 us; 4 lanes where
-// the colour's nodes fill the GPU, a warp per node below that: 5 us.
+// the first has tens to hundreds of nodes, where a thread's 27 x 12 loads one after another took 16 us with the
+// launch; 4 lanes where the colour's nodes fill the GPU, a warp per node below that: 8 us.
 template <typename T, int LPN>
 __global__ void __launch_bounds__(128) k_st_gs(int vx, int vy, int vz, int color, bool backward,
                                                const uint8_t* __restrict__ vact, const T* __restrict__ st,
@@ -932,8 +932,8 @@ __global__ void k_st_to_bf16(long nv, long nvpad, const double* __restrict__ st,
 // threads owns 31 x TY coarse columns of one component: a thread reads one fine column x, a fine plane's 4 TY + 3 rows
 // go into TY row sums, those into the two coarse planes the fine plane touches, and a finished coarse plane is
 // reduced along x through shared memory.  Each fine value is read 1.4 times (y and z overlap of neighbouring blocks,
-// mostly L2 hits) instead of the 5.4 times, in 28-byte pieces, of a gather per coarse node.  511x256x256, FP32:
-// 540 -> 150 us.
+// mostly L2 hits) instead of the 5.4 times, in 28-byte pieces, of a gather per coarse node.  511x256x256, FP32, the 23
+// restrictions of a W-cycle: 740 -> 322 us with their launches.
 // ---------------------------------------------------------------------------
 constexpr int RS_CX = 31;  // coarse columns per block: 4 * 30 + 7 = 127 fine columns
 
@@ -1037,7 +1037,8 @@ __global__ void __launch_bounds__(ST_BS) k_restrict2(int fvx, int fvy, int fvz, 
 
 // u_f += trilinear interpolation of u_c.  A thread marches one fine column through zcells coarse cells, interpolating
 // each coarse plane in x and y once (12 loads) for the R fine planes above and below it, where a thread per fine
-// node gathered 24 coarse values.  511x256x256, FP32: 450 -> 160 us.
+// node gathered 24 coarse values.  511x256x256, FP32, the 23 prolongations of a W-cycle: 654 -> 396 us
+// with their launches.
 template <typename T, int R>
 __global__ void __launch_bounds__(ST_BS) k_prolong(int fvx, int fvy, int fvz, int cvx, int cvy, int cvz, int zcells,
                                                    const uint8_t* __restrict__ fvact, const T* __restrict__ uc,
@@ -1088,7 +1089,8 @@ __global__ void __launch_bounds__(ST_BS) k_prolong(int fvx, int fvy, int fvz, in
 // owns 32 x 2 nodes (x, y) of a layer with the weights of the 33 x 3 x 2 cells around them in shared memory; lane =
 // node column, and a warp owns whole neighbours k (8 cell-neighbour pairs each), so that a Q block is loaded once for
 // 64 nodes.  FP64 FMA bound (576 R^3 per node).  Elements touching a fixed node have weight 0 here and are added by
-// k_galerkin_fixed.  160x144x96: 4.5 ms with cell matrices scattered through 8 colours, 0.25 ms here.
+// k_galerkin_fixed.  160x144x96: 4.5 ms with cell matrices scattered through 8 colours, 0.5 ms here and 0.5 ms for the
+// cells with fixed nodes.
 // ---------------------------------------------------------------------------
 constexpr int GN_BS = 256;
 
@@ -1270,7 +1272,7 @@ __global__ void __launch_bounds__(GF_BS) k_galerkin_fixed(int fnx, int fny, int 
 // A_c = P^T A_f P for a dyadic (ratio 2) level from the finer stencil.  A warp per coarse node and block entry: lane i
 // takes fine node i of the node's 3^3 support, reads that node's 27 entries and restricts them along each axis to the
 // 3^3 coarse neighbours (the weights of an axis depend on the lane's offset on it), then the lanes are summed.  A
-// thread per coarse node and entry looped over 729 products with 27 candidates each: 500 us a level, 40 us here.
+// thread per coarse node and entry looped over 729 products with 27 candidates each: 500 us a level, 79 us here.
 __global__ void __launch_bounds__(ST_BS) k_galerkin_dyadic(int fnx, int fny, int fnz, int cnx, int cny, int cnz,
                                                            const uint8_t* __restrict__ fvact,
                                                            const uint8_t* __restrict__ cvact,

@@ -64,7 +64,7 @@ __global__ void k_trace(int n, const double* __restrict__ A, double* __restrict_
 // Every block inverts the 32 x 32 pivot block itself (cheaper than a second barrier), takes strips of one tile row,
 // so that C_i P is formed once per strip, and writes the parts of the next step's panels that it updated into the
 // other pair of panel buffers.  status[0] != 0 reports a non-positive pivot.  n = 1260: a barrier and a pass over
-// the matrix per column took 14.6 ms, 0.4 ms here.
+// the matrix per column took 14.6 ms, 1.36 ms here.
 constexpr int GJ_B = 32, GJ_T = 256;
 
 __global__ void __launch_bounds__(GJ_T) k_gauss_jordan(int n, double* __restrict__ A, double* __restrict__ panels,
@@ -229,8 +229,8 @@ __global__ void k_gemv_scatter(int na, long nv, const int* __restrict__ aidx, co
 
 // the coarsest solve in one launch, n <= CS_MAXN: every block gathers the right-hand side of the active nodes into
 // shared memory, a warp multiplies a row of the inverse (8 loads in flight per lane), and the inactive nodes are set to
-// zero.  The V-cycle visits it up to 8 times per iteration; gather, memset and product took three launches (11 us,
-// 6 us here).
+// zero.  The V-cycle visits it up to 8 times per iteration; gather, memset and product took three launches.  n = 1260:
+// 14.7 us with the launch.
 constexpr int CS_MAXN = 4096;
 template <typename T>
 __global__ void __launch_bounds__(256) k_coarsest(int na, int nv, const int* __restrict__ aidx,

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(GS_BS, WS ? 4 : 3) k_fine_gs(int nx, int ny, i
                 const float* we = w + x + (long)nx * (ey + (long)ny * ez);
                 const bool in[2] = {x > 0, x < nx};
                 const float wv[2] = {in[0] ? we[-1] : 0.f, in[1] ? we[0] : 0.f};
-                // rows of KE in the vertex's reflected frame: sx u0, sy u1, sz u2 of the shared nodes apart from u0, whose sign
+                // rows of KE in the vertex's reflected frame (sx u0, sy u1, sz u2); the shared nodes' u0 apart, whose sign
                 // depends on the side
                 T sh0[3] = {}, sh[3] = {}, p[2][3] = {};
                 // vertex m of the node's elements on side d; nodes without an element, and fixed ones, count as zero
@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(GS_BS, WS ? 4 : 3) k_fine_gs(int nx, int ny, i
                 KU[2] = flip_sign(w1 * (p[1][2] + (sh[2] + sh0[2])) + w0 * (p[0][2] + (sh[2] - sh0[2])), mz);
             }
         }
-        T S[4] = {sw, flip_sign(swx, my), flip_sign(swx, mz), flip_sign(sw, my ^ mz)};  // sums of w, w sx sy, w sx sz, w sy sz
+        // sums of w, w sx sy, w sx sz, w sy sz
+        T S[4] = {sw, flip_sign(swx, my), flip_sign(swx, mz), flip_sign(sw, my ^ mz)};
 #pragma unroll
         for (int o = 8; o < 32; o <<= 1) {
 #pragma unroll
@@ -158,7 +159,8 @@ __global__ void __launch_bounds__(GS_BS, WS ? 4 : 3) k_fine_gs(int nx, int ny, i
     }
 }
 
-// four elements per thread (the arrays are allocations of their own): 255x256x128 49 us with one and the launch, 38 us (powf)
+// four elements per thread (the arrays are allocations of their own).  255x256x128, with the launch: 49 us with one,
+// 38 us here, powf bound
 __global__ void k_penalty(long ne, const uint8_t* __restrict__ eact, const float* __restrict__ rho, float p,
                           float* __restrict__ w) {
     const long n4 = ne / 4, tid = blockIdx.x * (long)blockDim.x + threadIdx.x;

@@ -37,8 +37,8 @@ namespace {
 
 constexpr int FACE_NX = 30;  // node columns a warp finishes (lanes 1..30)
 
-// warps per block: FP64 12, one block per SM (registers), 8 for the smoothing steps (two blocks of 8 with spills: residual
-// 1287 us, Chebyshev 2431 us on 511x256x256); FP32 8, three blocks
+// warps per block: FP64 12, one block per SM (registers), 8 for the smoothing steps (two blocks of 8 with spills:
+// residual 1287 us, Chebyshev 2431 us on 511x256x256); FP32 8, three blocks
 constexpr int face_warps(bool f64, int mode) { return f64 && mode < 2 ? 12 : 8; }
 
 template <typename T>
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int z
 
 // node codes read by k_fine_face: bit 0 active, bit 1 fixed, bits 2.. the number of elements of non-zero weight
 // around a fixed node (its smoothing rule f / n_e).  Four nodes per thread (the arrays are allocations of their own):
-// 255x256x128 37 us with one and the launch, 17 us
+// 255x256x128, with the launch: 37 us with one, 17 us here
 __global__ void k_node_code(int nx, int ny, int nz, const uint8_t* __restrict__ vact, const uint8_t* __restrict__ vfix,
                             const float* __restrict__ w, uint8_t* __restrict__ code) {
     const int vx = nx + 1, vy = ny + 1;

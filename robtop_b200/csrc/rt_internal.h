@@ -126,7 +126,6 @@ struct rt_hier {
     std::vector<rt_level> L;
     double KE[576];
     double* KE_dev = nullptr;
-    float* KE32_dev = nullptr;
     // level-0 design data
     float* rho = nullptr;
     float* w = nullptr;       // powf(rho, p) or 0

@@ -64,7 +64,7 @@ __device__ __forceinline__ void block_reduce(double (&v)[NV]) {
 
 // the grid's sums of v[0..NV) in out: every block stores its own, and the last one to finish (a ticket counter, left
 // at zero again) adds them in a fixed order, so that the sum does not depend on which block that is.  One launch
-// where a second one added the partial sums (6 us, three times a PCG iteration).
+// where a second one added the partial sums, three times a PCG iteration.
 template <int NV>
 __device__ __forceinline__ bool grid_reduce(double (&v)[NV], const RedOut& o) {
     __shared__ bool last;
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(RB) k_dot6(long n, int nrig, const double* __r
 
 // largest eigenvalue of the symmetric tridiagonal (alpha, beta) by Sturm counts, one warp: each round the 32 lanes
 // count at 32 points of the bracket, which shrinks 33-fold, until it is two neighbouring numbers.  One thread's
-// bisection took 142 us of dependent divisions, 20 us here.
+// bisection took 142 us of dependent divisions, 39 us here (both with the launch).
 __global__ void k_tridiag_max(int k, const double* __restrict__ alpha, const double* __restrict__ beta,
                               double* __restrict__ out) {
     const int lane = threadIdx.x & 31;
@@ -389,7 +389,7 @@ __global__ void k_tridiag_max(int k, const double* __restrict__ alpha, const dou
 // the same filter through shared memory, radius (rounded) RL <= 3: a block of 32 x 8 columns keeps the sensitivities
 // (0 outside the solid) and the activity of its 32 x 8 x 8 elements and their halo, and the list of taps inside the
 // radius with their weights; a thread does 8 elements of a column, so that a tap's entry is read once for them.  Taps
-// in k_filter's order, products in FP32 and their sum in FP64 as there: the same bits.  255x256x128, radius 2:
+// in k_filter's order, products in FP32 and their sum in FP64 as there.  255x256x128, radius 2:
 // 1050 us with 33 bounds-checked gathers per element, 200 us here.
 constexpr int FT_Z = 8;
 template <int RL>

@@ -323,7 +323,7 @@ int rt_fine_kernel_f32(rt_hier* h, int mode, double omega);
  * Overwrites the level's vectors; needs rt_update_stencil. */
 int rt_bench_level_kernel(rt_hier* h, int lvl, int precision, int mode, int reps, double* us_per_launch);
 /* the kernel variant of the FP32 smoother's stencil levels, per stencil copy (stencil_type 0 FP32,
- * 1 BF16): 0 lane-split (4 lanes per node), 1 bulk-copy (each 32-node stencil run staged in shared
+ * 1 BF16): 0 direct loads (9 warps per 32 nodes; reported as lane_split), 1 bulk-copy (each 32-node stencil run staged in shared
  * memory by cp.async.bulk).  rt_autotune times both on level 1 (after rt_update_stencil) and keeps
  * the faster; us_*: its measured Chebyshev-step times (0 before it ran). */
 int rt_level_kernel_info(rt_hier* h, int stencil_type, int* variant, double* us_lane_split, double* us_bulk);

@@ -127,107 +127,109 @@ __global__ void __launch_bounds__(128) k_st_gs(int vx, int vy, int vz, int color
 }
 
 // ---------------------------------------------------------------------------
-// Lane-split stencil kernels: LPN lanes per node, lane q sums neighbours k = q, q + LPN, ..., then the three row sums
-// are combined with shuffles.  MODE 0: r = f - A u;  MODE 2: Jacobi;  MODE 3: Chebyshev step.
-// The large levels (4 lanes) are bound by the stencil stream.  The small ones are bound by the latency of one node:
-// with more lanes each has 1 to 4 neighbours instead of 7, and all its loads, those of the output stage too, are
-// issued before the first is used (a level of 882 nodes: 4.6 -> 2.9 us per step, of which 1.2 us is the launch).
 // ---------------------------------------------------------------------------
-template <typename T, int MODE, typename S, int LPN>
-__global__ void __launch_bounds__(ST_BS, sizeof(T) == 8 || LPN > 4 ? 1 : 3)
-    k_st_split(int vx, int vy, int vz, const uint8_t* __restrict__ vact, const S* __restrict__ st,
-               const T* __restrict__ u, const T* __restrict__ f, T* __restrict__ out, T* __restrict__ d, T omega,
-               const double* __restrict__ coef, int kstep) {
-    constexpr bool EARLY = LPN > 4;
+// Stencil kernels, a block per 32 nodes: warp j sums the three neighbours k = 3 j .. 3 j + 2 of its lane's node, so
+// that every load of a stencil row is a whole line of the blocked layout, and the partial sums meet in shared memory.
+// MODE 0: r = f - A u;  MODE 2: Jacobi;  MODE 3: Chebyshev step.
+// 4 to 32 lanes per node touched 4 to 16 lines a load.  FP32 Chebyshev, 8 steps in a graph: 882 nodes 29 -> 21 us, 5746
+// nodes 43 (4 lanes) -> 23 us; 342k nodes a step 64 us, 5.3 TB/s of stencils, where the bulk-copy form takes 124 us.
+// ---------------------------------------------------------------------------
+template <typename T, int MODE, typename S>
+__global__ void __launch_bounds__(288) k_st_tile(int vx, int vy, int vz, const uint8_t* __restrict__ vact,
+                                                 const S* __restrict__ st, const T* __restrict__ u,
+                                                 const T* __restrict__ f, T* __restrict__ out, T* __restrict__ d,
+                                                 T omega, const double* __restrict__ coef, int kstep) {
+    __shared__ T red[9][3][32];
     T ca = T(0), cb = T(0);
     if (MODE == 3) {
-        const double a_ = coef[2 * kstep], b_ = coef[2 * kstep + 1];
-        ca = (T)a_;
-        cb = (T)b_;
+        ca = (T)coef[2 * kstep];
+        cb = (T)coef[2 * kstep + 1];
     }
     const int nv = vx * vy * vz;  // 243 nv < 2^31
     const long rs = StAddr<S>::stride(nv);
-    const int q = threadIdx.x % LPN;
-    const int ngroups = (int)gridDim.x * (ST_BS / LPN);
-    // every lane runs the same number of trips (the shuffles below use the full mask)
-    const int vend = (nv + ngroups - 1) / ngroups * ngroups;
-    for (int v = (int)((blockIdx.x * ST_BS + threadIdx.x) / LPN); v < vend; v += ngroups) {
-        const bool inb = v < nv;
-        const bool act = inb && vact[v];
-        const S* sb = st + StAddr<S>::base(inb ? v : 0);
-        const int oq = q * nv + v;  // lane q (0..2) owns component q
-        T S9[9], f0 = T(0), f1 = T(0), f2 = T(0), uo = T(0), dl = T(0);
-        auto output_loads = [&] {
-            if (MODE == 0) {
-                f0 = f[oq];
-            } else {
-#pragma unroll
-                for (int i = 0; i < 9; i++) S9[i] = st_centre<T>(sb, rs, i);
-                f0 = f[v];
-                f1 = f[nv + v];
-                f2 = f[2 * nv + v];
-                uo = u[oq];
-                if (MODE == 3 && kstep > 0) dl = d[oq];
-            }
-        };
-        if (EARLY && inb && q < 3) output_loads();
-        T Au[3] = {T(0), T(0), T(0)};
-        if (EARLY ? inb : act) {
-            const int x = v % vx, y = v / vx % vy, z = v / (vx * vy);
-#pragma unroll
-            for (int kk = 0; kk < (27 + LPN - 1) / LPN; kk++) {
-                const int k = q + LPN * kk;
-                const int jx = x + k % 3 - 1, jy = y + (k / 3) % 3 - 1, jz = z + k / 9 - 1;
-                if (k >= 27 || jx < 0 || jy < 0 || jz < 0 || jx >= vx || jy >= vy || jz >= vz) continue;
-                const int nj = jx + vx * (jy + vy * jz);
-                const T u0 = u[nj], u1 = u[nv + nj], u2 = u[2 * nv + nj];
-                const S* s = sb + (long)(k * 9) * rs;
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    T a0 = (T)st_val(s + (3 * r) * rs), a1 = (T)st_val(s + (3 * r + 1) * rs),
-                      a2 = (T)st_val(s + (3 * r + 2) * rs);
-                    if (sizeof(S) == 2 && k == 13) {  // low parts of the BF16 centre block
-                        a0 += (T)st_val(sb + (243 + 3 * r) * rs);
-                        a1 += (T)st_val(sb + (243 + 3 * r + 1) * rs);
-                        a2 += (T)st_val(sb + (243 + 3 * r + 2) * rs);
-                    }
-                    Au[r] += a0 * u0 + a1 * u1 + a2 * u2;
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 3; r++)
-#pragma unroll
-            for (int o = 1; o < LPN; o <<= 1) Au[r] += __shfl_xor_sync(0xffffffffu, Au[r], o);
-        if (!inb || q >= 3) continue;
-        if (!EARLY && (MODE == 0 || act)) output_loads();
+    const int lane = threadIdx.x & 31, j = threadIdx.x >> 5, v = blockIdx.x * 32 + lane;
+    const bool inb = v < nv, act = inb && vact[v];
+    const S* sb = st + StAddr<S>::base(inb ? v : 0);
+    const int oq = j * nv + v;  // warp j (0..2) owns component j
+    T S9[9], f0 = T(0), f1 = T(0), f2 = T(0), uo = T(0), dl = T(0);
+    if (j < 3 && inb) {
         if (MODE == 0) {
-            out[oq] = act ? f0 - (q == 0 ? Au[0] : q == 1 ? Au[1] : Au[2]) : T(0);
-            continue;
+            f0 = f[oq];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 9; i++) S9[i] = st_centre<T>(sb, rs, i);
+            f0 = f[v];
+            f1 = f[nv + v];
+            f2 = f[2 * nv + v];
+            uo = u[oq];
+            if (MODE == 3 && kstep > 0) dl = d[oq];
         }
-        T res = T(0), dn = T(0);
-        if (act) {
-            const T A = S9[4] * S9[8] - S9[5] * S9[7], B = -(S9[3] * S9[8] - S9[5] * S9[6]),
-                    Cc = S9[3] * S9[7] - S9[4] * S9[6];
-            const T id = T(1) / (S9[0] * A + S9[1] * B + S9[2] * Cc);
-            // row q of the inverse (adjugate / determinant)
-            const T i0 = q == 0 ? A : (q == 1 ? B : Cc);
-            const T i1 = q == 0 ? -(S9[1] * S9[8] - S9[2] * S9[7])
-                                : (q == 1 ? (S9[0] * S9[8] - S9[2] * S9[6]) : -(S9[0] * S9[7] - S9[1] * S9[6]));
-            const T i2 = q == 0 ? (S9[1] * S9[5] - S9[2] * S9[4])
-                                : (q == 1 ? -(S9[0] * S9[5] - S9[2] * S9[3]) : (S9[0] * S9[4] - S9[1] * S9[3]));
-            const T r0 = f0 - Au[0], r1 = f1 - Au[1], r2 = f2 - Au[2];
-            const T zq = (i0 * id) * r0 + (i1 * id) * r1 + (i2 * id) * r2;
-            if (MODE == 2) {
-                res = uo + omega * zq;
-            } else {
-                dn = ca * dl + cb * zq;  // dl = 0 in step 0
-                res = uo + dn;
+    }
+    T Au[3] = {T(0), T(0), T(0)};
+    const int x = v % vx, y = v / vx % vy, z = v / (vx * vy), jy = y + j % 3 - 1, jz = z + j / 3 - 1;
+    if (act && jy >= 0 && jz >= 0 && jy < vy && jz < vz) {
+        const int n0 = x + vx * (jy + vy * jz);
+        T un[3][3];  // outside the box zero; the stencil has entries there too
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) un[i][c] = x + i - 1 >= 0 && x + i - 1 < vx ? u[c * nv + n0 + i - 1] : T(0);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int k = 3 * j + i;
+            const S* s = sb + (long)(k * 9) * rs;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                T a[3];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    a[c] = (T)st_val(s + (3 * r + c) * rs);
+                    // low parts of the BF16 centre block
+                    if (sizeof(S) == 2 && k == 13) a[c] += (T)st_val(sb + (243 + 3 * r + c) * rs);
+                }
+                Au[r] += a[0] * un[i][0] + a[1] * un[i][1] + a[2] * un[i][2];
             }
         }
-        out[oq] = res;
-        if (MODE == 3) d[oq] = dn;
     }
+#pragma unroll
+    for (int r = 0; r < 3; r++) red[j][r][lane] = Au[r];
+    __syncthreads();
+    if (j >= 3 || !inb) return;
+    if (MODE == 0) {
+        T a = T(0);
+#pragma unroll
+        for (int i = 0; i < 9; i++) a += red[i][j][lane];
+        out[oq] = act ? f0 - a : T(0);
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        Au[r] = T(0);
+#pragma unroll
+        for (int i = 0; i < 9; i++) Au[r] += red[i][r][lane];
+    }
+    T res = T(0), dn = T(0);
+    if (act) {
+        const T A = S9[4] * S9[8] - S9[5] * S9[7], B = S9[5] * S9[6] - S9[3] * S9[8], C = S9[3] * S9[7] - S9[4] * S9[6];
+        const T id = T(1) / (S9[0] * A + S9[1] * B + S9[2] * C);
+        // row j of the inverse (adjugate / determinant)
+        const T i0 = j == 0 ? A : j == 1 ? B : C;
+        const T i1 = j == 0   ? S9[2] * S9[7] - S9[1] * S9[8]
+                     : j == 1 ? S9[0] * S9[8] - S9[2] * S9[6]
+                              : S9[1] * S9[6] - S9[0] * S9[7];
+        const T i2 = j == 0   ? S9[1] * S9[5] - S9[2] * S9[4]
+                     : j == 1 ? S9[2] * S9[3] - S9[0] * S9[5]
+                              : S9[0] * S9[4] - S9[1] * S9[3];
+        const T zz = id * (i0 * (f0 - Au[0]) + i1 * (f1 - Au[1]) + i2 * (f2 - Au[2]));
+        if (MODE == 2) {
+            res = uo + omega * zz;
+        } else {
+            dn = ca * dl + cb * zz;  // dl = 0 in step 0
+            res = uo + dn;
+        }
+    }
+    out[oq] = res;
+    if (MODE == 3) d[oq] = dn;
 }
 
 // one smoothing step from u = 0: out = omega D^-1 f (MODE 2) or out = d = b_0 D^-1 f (MODE 3), D the centre block;
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(128) k_st_diag(long nv, const uint8_t* __restr
 // launch, the steps separated by a grid barrier instead of a kernel boundary.  The coarse
 // levels below the first are a few thousand nodes: a separate launch per step spends most
 // of its time in launch, ramp-up and drain, not in the 243-entry rows.  Same arithmetic and
-// thread layout as k_st_split (MODE 3, 4 lanes); u is ping-ponged with tmp (u -> tmp -> u ...), so
+// 4 lanes per node, lane q sums neighbours k = q, q + 4, ...; u is ping-ponged with tmp (u -> tmp -> u ...), so
 // after an odd step count a last barrier lets every thread copy its own entries back to u.
 // Values written by other blocks in the previous step are read through L2 (ld.global.cg):
 // L1 is not coherent across SMs.  The barrier is bounded: a block whose wait runs out sets
@@ -1375,17 +1377,9 @@ template <typename T, int MODE, typename S>
 static int launch_split(rt_hier* h, int lvl, const char* name, const S* st, const T* u, const T* f, T* out, T* d,
                         double omega, const double* coef, int kstep) {
     rt_level& L = h->L[lvl];
-    const long lanes = 1024L * h->ctx->sm_count;
-    const int lpn = 32 * L.nv <= lanes ? 32 : 16 * L.nv <= lanes ? 16 : 8 * L.nv <= lanes ? 8 : 4;
     return rt_launch(h->ctx, name, [&] {
-        const unsigned g = grid_for(h->ctx, lpn * L.nv, ST_BS);
-        cudaStream_t s = h->ctx->stream;
-        switch (lpn) {
-            case 32: k_st_split<T, MODE, S, 32><<<g, ST_BS, 0, s>>>(L.vx, L.vy, L.vz, L.vact, st, u, f, out, d, (T)omega, coef, kstep); break;
-            case 16: k_st_split<T, MODE, S, 16><<<g, ST_BS, 0, s>>>(L.vx, L.vy, L.vz, L.vact, st, u, f, out, d, (T)omega, coef, kstep); break;
-            case 8: k_st_split<T, MODE, S, 8><<<g, ST_BS, 0, s>>>(L.vx, L.vy, L.vz, L.vact, st, u, f, out, d, (T)omega, coef, kstep); break;
-            default: k_st_split<T, MODE, S, 4><<<g, ST_BS, 0, s>>>(L.vx, L.vy, L.vz, L.vact, st, u, f, out, d, (T)omega, coef, kstep);
-        }
+        k_st_tile<T, MODE, S><<<(unsigned)((L.nv + 31) / 32), 288, 0, h->ctx->stream>>>(
+            L.vx, L.vy, L.vz, L.vact, st, u, f, out, d, (T)omega, coef, kstep);
     });
 }
 

@@ -317,3 +317,26 @@ def test_tail_cycle_edges(dims, skip, pre, post, cs, sup, jacobi):
     assert rel_err(x[rb.FP32], x[rb.FP64]) < 1e-3
     G.close()
     ctx.close()
+
+
+# stencil levels, 32 nodes per block: 672, 2310, 462 and 540 nodes (remainders 0, 6, 14 and 28), faces on every side
+@pytest.mark.parametrize("dims", [(21, 13, 11), (39, 19, 17), (20, 12, 9), (18, 16, 10)])
+@pytest.mark.parametrize("sup", [True, False])
+def test_stencil_level_edges(dims, sup):
+    ctx, G, H, r = _perforated(*dims, sum(dims) + 2, sup, 0)
+    H.arrs[1]["st"][:] = G[1].getStencil()
+    act = np.tile(G[1].getVact(), 3).astype(bool)
+    u, f = r.standard_normal(3 * G[1].nv) * act, r.standard_normal(3 * G[1].nv) * act
+    G[1].setDisplacement(u)
+    G[1].setForce(f)
+    G[1].update_residual()
+    res = np.zeros_like(u)
+    O.lib().or_st_residual(H.lv(1), O.ptr(u), O.ptr(f), O.ptr(res))
+    assert rel_err(G[1].getResidual(), res) < 1e-12  # 81 terms a row in another order
+    want, tmp = u.copy(), np.zeros_like(u)
+    O.lib().or_st_jacobi(H.lv(1), O.ptr(want), O.ptr(f), 0.6, O.ptr(tmp))
+    G[1].smooth(rb.SMOOTH_JACOBI, 1, 0.6)
+    # the block division amplifies FP64 rounding on the 1e9-contrast stencils
+    assert rel_err(G[1].getDisplacement(), want) < 1e-9
+    G.close()
+    ctx.close()

@@ -691,7 +691,7 @@ extern "C" int rt_set_support(rt_hier* h, const uint8_t* vfix) {
     h->graph_epoch++;  // kernel variants depend on whether supports exist
     h->stencil_ready = false;
     h->design_epoch++;
-    return RT_OK;
+    return rtk::node_codes(h);  // at once: a workspace's calls read them without a refresh
 }
 
 // shell elements (HierarchyGrid::setSolidShellElement, grid/Grid.cpp:67-137 marks them):
@@ -930,6 +930,11 @@ static int convert_layout(rt_hier* h, int field, int lvl, bool to_ref, const voi
     return rt_fail(h->ctx, RT_EINVAL, "field has no reference-order layout");
 }
 
+// fields the finest level's node codes are made from
+static bool in_node_codes(int field, int lvl) {
+    return lvl == 0 && (field == RT_FIELD_VFIX || field == RT_FIELD_VACT || field == RT_FIELD_PENALTY);
+}
+
 extern "C" int rt_put(rt_hier* h, int field, int lvl, int layout, const void* src) {
     if (!h || !src) return RT_EINVAL;
     if (h->parent && field != RT_FIELD_U && field != RT_FIELD_F && field != RT_FIELD_R)
@@ -950,7 +955,7 @@ extern "C" int rt_put(rt_hier* h, int field, int lvl, int layout, const void* sr
         h->stencil_ready = false;
         h->design_epoch++;
     }
-    return RT_OK;
+    return in_node_codes(field, lvl) ? rtk::node_codes(h) : RT_OK;
 }
 
 extern "C" int rt_get(rt_hier* h, int field, int lvl, int layout, void* dst) {
@@ -981,7 +986,7 @@ extern "C" int rt_put_dev(rt_hier* h, int field, int lvl, const void* src) {
         h->stencil_ready = false;
         h->design_epoch++;
     }
-    return RT_OK;
+    return in_node_codes(field, lvl) ? rtk::node_codes(h) : RT_OK;
 }
 
 extern "C" int rt_get_dev(rt_hier* h, int field, int lvl, void* dst) {
@@ -1026,7 +1031,7 @@ static bool reads_dinv(const rt_hier* h) {
 // element weights rho^p, node codes and (where a chosen kernel reads them) the inverted diagonal blocks of
 // the finest level
 static int refresh_fine(rt_hier* h) {
-    if (h->parent) {  // weights and diagonal blocks belong to the parent (refreshed by its own calls)
+    if (h->parent) {  // weights, node codes and diagonal blocks belong to the parent (refreshed by its own calls)
         ws_sync(h);
         return RT_OK;
     }

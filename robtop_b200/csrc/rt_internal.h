@@ -122,7 +122,7 @@ struct rt_hier {
     double* dinv64 = nullptr;        // [6][nv] inverted diagonal blocks of the finest level
     float* dinv32 = nullptr;
     bool dinv_ready = false;         // the diagonal blocks match the weights (made only for kernels that read them)
-    uint8_t* ncode = nullptr;        // [nv] node codes of the finest level: bit 0 active, bit 1 fixed
+    uint8_t* ncode = nullptr;        // [nv] node codes of the finest level (k_node_code), remade when w, vact or vfix change
     std::vector<rt_level> L;
     double KE[576];
     double* KE_dev = nullptr;

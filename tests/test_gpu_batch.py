@@ -10,7 +10,7 @@ import pytest
 
 import oracle as O
 import robtop_b200 as rb
-from gpu_common import CONFIGS, E, NU, P, build_pair
+from gpu_common import CONFIGS, E, NU, P, build_pair, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -71,6 +71,43 @@ def test_workspace_matches_parent():
     info2_w = W.pcg(1e-8, 500)
     assert info2_w.iterations == info2.iterations
     assert np.array_equal(W[0].getDisplacement(), G[0].getDisplacement())
+    G.close()
+    ctx.close()
+
+
+# supports put on the parent reach its workspaces' finest-level calls at once: moved, removed, and put as a field
+@pytest.mark.parametrize("change", ["moved", "none", "put"])
+def test_workspace_follows_supports(change):
+    cfg = CONFIGS["worstcase"]()
+    vfix = np.zeros_like(cfg["vfix"])
+    if change != "none":
+        vfix[:, :, -1] = 1
+    ctx = rb.Context(0)
+    G = _grid(ctx, dict(cfg, load_nodes=None), _params(cfg))
+    W = G.workspace()
+    if change == "put":
+        G[0]._put(rb._capi.FIELD_VFIX, 0, vfix.ravel(), np.uint8)
+    else:
+        G.set_support(vfix)
+    H = O.Hierarchy(cfg["eact"], cfg["rho"], vfix if vfix.any() else None, p=P, E=E, nu=NU, no_support=not vfix.any())
+    H.set_weights(G[0].getPenalty())
+    r = np.random.default_rng(3)
+    act = np.tile(G[0].getVact(), 3).astype(bool)
+    u, f = r.standard_normal(3 * G[0].nv) * act, r.standard_normal(3 * G[0].nv) * act
+    assert rel_err(W[0].applyK(u), H.applyK(u)) < 1e-11
+    W[0].setDisplacement(u)
+    W[0].setForce(f)
+    W[0].update_residual()
+    want = np.zeros_like(u)
+    O.lib().or_fine_residual(H.lv(0), O.ptr(H.KE), O.ptr(u), O.ptr(f), O.ptr(want))
+    assert rel_err(W[0].getResidual(), want) < 1e-11
+    ujac, ugs, tmp = u.copy(), u.copy(), np.zeros_like(u)
+    O.lib().or_fine_jacobi(H.lv(0), O.ptr(H.KE), O.ptr(ujac), O.ptr(f), 0.6, O.ptr(tmp))
+    O.lib().or_fine_gs(H.lv(0), O.ptr(H.KE), O.ptr(ugs), O.ptr(f), 0)
+    for smoother, want in ((rb.SMOOTH_JACOBI, ujac), (rb.SMOOTH_GS, ugs)):
+        W[0].setDisplacement(u)
+        W[0].smooth(smoother, 1, 0.6)
+        assert rel_err(W[0].getDisplacement(), want) < 1e-10
     G.close()
     ctx.close()
 

@@ -41,10 +41,18 @@ constexpr int FACE_NX = 30;  // node columns a warp finishes (lanes 1..30)
 // residual 1287 us, Chebyshev 2431 us on 511x256x256); FP32 8, three blocks
 constexpr int face_warps(bool f64, int mode) { return f64 && mode < 2 ? 12 : 8; }
 
+// 1 / det of a node's block; 0 where all its elements have zero weight (the node keeps its value)
 template <typename T>
-__device__ __forceinline__ T face_rcp(T x) {
-    if constexpr (sizeof(T) == 4) return __frcp_rn(x);
-    else return T(1) / x;
+__device__ __forceinline__ T block_rcp(T det, T sw) {
+    if (sw == T(0)) return T(0);
+    if constexpr (sizeof(T) == 4) return __frcp_rn(det);
+    else return T(1) / det;
+}
+
+// a fixed node's rule f / n_e, from its code; 0 without a weighted element
+template <typename T>
+__device__ __forceinline__ T fixed_value(T f, uint32_t code) {
+    return code >> 2 ? f / T(code >> 2) : T(0);
 }
 
 // the grid's sum of x in out[0]: block sums, added by the last block to finish in their order (the ticket counter is
@@ -84,7 +92,8 @@ __device__ __forceinline__ void face_grid_sum(double x, double* __restrict__ par
 
 // MODE 0: r = f - K u (fixed rows: r = f)     MODE 1: out = K u (fixed rows: u)
 // MODE 2: unew = u + omega D^-1 (f - K u)     MODE 3: Chebyshev step kstep: d = a_k d + b_k D^-1 (f - K u), unew = u + d
-// (fixed nodes in MODE 2/3: unew = f / n_e, d = 0; inactive nodes: 0)
+// (fixed nodes in MODE 2/3: unew = f / n_e, d = 0; inactive nodes: 0; nodes whose elements all have zero weight: D^-1 and
+// f / n_e count as 0, as with the stored blocks)
 // code: per node, bit 0 active, bit 1 fixed (supports), for fixed nodes n_e << 2
 template <typename T, bool WS, int MODE, int W, int MINB, bool DOT>
 __global__ void __launch_bounds__(32 * W, MINB)
@@ -216,14 +225,14 @@ __global__ void __launch_bounds__(32 * W, MINB)
                 }
             } else if (fixed) {
 #pragma unroll
-                for (int c = 0; c < 3; c++) o[c] = fv[c] / T(co >> 2);
+                for (int c = 0; c < 3; c++) o[c] = fixed_value(fv[c], co);
             } else if (act) {
                 const T sw = Q[0] + Qp[0], sxy = Q[1] + Qp[1], sxz = Q[3] - Qp[3], syz = Q[2] - Qp[2];
                 const T A = kt.diag_a * sw, bxy = kt.diag_b * sxy, bxz = kt.diag_b * sxz, byz = kt.diag_b * syz;
                 // inverse of [[A,bxy,bxz],[bxy,A,byz],[bxz,byz,A]]
                 const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
                 const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
-                const T id = face_rcp(A * c00 + bxy * c01 + bxz * c02);
+                const T id = block_rcp(A * c00 + bxy * c01 + bxz * c02, sw);
                 T rr[3];
 #pragma unroll
                 for (int c = 0; c < 3; c++) rr[c] = fv[c] - acc[c];
@@ -365,14 +374,14 @@ __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int z
                 const T A = diag_a * sw, bxy = diag_b * sxy, bxz = diag_b * sxz, byz = diag_b * syz;
                 const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
                 const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
-                const T id = face_rcp(A * c00 + bxy * c01 + bxz * c02) * scale;
+                const T id = block_rcp(A * c00 + bxy * c01 + bxz * c02, sw) * scale;
                 o[0] = id * (c00 * f0 + c01 * f1 + c02 * f2);
                 o[1] = id * (c01 * f0 + c11 * f1 + c12 * f2);
                 o[2] = id * (c02 * f0 + c12 * f1 + c22 * f2);
             } else if (c > 1u) {
-                o[0] = f0 / T(c >> 2);
-                o[1] = f1 / T(c >> 2);
-                o[2] = f2 / T(c >> 2);
+                o[0] = fixed_value(f0, c);
+                o[1] = fixed_value(f1, c);
+                o[2] = fixed_value(f2, c);
             }
 #pragma unroll
             for (int q = 0; q < 3; q++) {

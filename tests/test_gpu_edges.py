@@ -340,3 +340,77 @@ def test_stencil_level_edges(dims, sup):
     assert rel_err(G[1].getDisplacement(), want) < 1e-9
     G.close()
     ctx.close()
+
+
+# elements of zero density inside the box and at a support, so that nodes are left without a weighted element: they keep
+# their values, a fixed one takes 0, and the smoother bounds and solves are those of the body without these elements
+@pytest.mark.parametrize("zc", [0, 3])
+def test_zero_density_pocket(zc):
+    nx, ny, nz = 36, 13, 11
+    ctx, G, eact, rho, vfix, r = _hier(nx, ny, nz, seed=6)
+    hole = np.zeros((nz, ny, nx), bool)
+    hole[3:7, 4:8, 20:25] = True
+    hole[2:5, 2:5, 0:3] = True  # nodes (0, 3, 3), (0, 3, 4), ... of the clamped face
+    rho[hole] = 0
+    G[0].setRho(rho.ravel())
+    G.update_stencil()
+    L = rb.lib()
+    if zc:
+        for prec in (rb.FP64, rb.FP32):
+            for m in range(4):
+                rb._capi.check(L.rt_set_tuning(G.handle, prec, m, 8, 1, zc), ctx.handle)
+    live = np.zeros((nz + 1, ny + 1, nx + 1), bool)
+    for z, y, x in np.argwhere(~hole):
+        live[z:z + 2, y:y + 2, x:x + 2] = True
+    dead, fixed = np.tile(~live.ravel(), 3), np.tile(vfix.ravel().astype(bool), 3)
+    assert (dead & fixed).any() and (dead & ~fixed).any()
+    # n_e of a fixed node counts weighted elements: the oracle gets the body without the others
+    H = O.Hierarchy((~hole).astype(np.uint8), rho, vfix, p=P, E=E, nu=NU)
+    H.set_weights(G[0].getPenalty())
+    lm = [G.smoother_lmax(i) for i in range(H.nlev - 1)]
+    assert np.isfinite(lm).all()
+    H.set_lmax(lm)
+    u, f = r.standard_normal(dead.size), r.standard_normal(dead.size)
+    ujac, ucheb, tmp, d = u.copy(), np.zeros_like(u), np.zeros_like(u), np.zeros_like(u)
+    O.lib().or_fine_jacobi(H.lv(0), O.ptr(H.KE), O.ptr(ujac), O.ptr(f), 0.6, O.ptr(tmp))
+    O.lib().or_fine_cheby(H.lv(0), O.ptr(H.KE), O.ptr(u), O.ptr(f), O.ptr(ucheb), O.ptr(d), 0)
+    keep = np.where(fixed, 0.0, u)
+    G[0].setForce(f)
+    for smoother, m, w in ((rb.SMOOTH_JACOBI, 2, ujac), (rb.SMOOTH_CHEBY, 3, ucheb)):
+        w = np.where(dead, keep, w)
+        G[0].setDisplacement(u)
+        G[0].smooth(smoother, 1, 0.6)
+        assert rel_err(G[0].getDisplacement(), w) < 1e-10
+        G[0].setDisplacement(u)
+        rb._capi.check(L.rt_fine_kernel_f32(G.handle, m, 0.6), ctx.handle)
+        assert rel_err(G[0].getResidual(), w) < 2e-6
+    # the same body with the elements taken out
+    ctx2, G2, *_ = _hier(nx, ny, nz, seed=6)
+    G2.close()
+    G2 = rb.HierarchyGrid(ctx2, G.params)
+    G2.genFromBox((~hole).astype(np.uint8))
+    G2[0].setRho(rho.ravel())
+    G2.set_support(vfix)
+    b = f * ~dead * ~fixed
+    for form in (dict(precision=rb.FP64, smoother=rb.SMOOTH_JACOBI, jacobi_omega=0.5),
+                 dict(precision=rb.FP32, smoother=rb.SMOOTH_CHEBY)):
+        x = []
+        for g in (G, G2):
+            p = g.params
+            p.pre_sweeps = p.post_sweeps = 2
+            for k, v in form.items():
+                setattr(p, k, v)
+            g.set_params(p)
+            g.update_stencil()
+            g[0].setForce(b)
+            g[0].reset_displacement()
+            assert g.pcg(1e-9, 500).rel_residual <= 1e-9
+            x.append(g[0].getDisplacement())
+        assert abs(G.smoother_lmax(0) - G2.smoother_lmax(0)) < 1e-9 * G2.smoother_lmax(0)
+        # two solves to 1e-9 of the residual, amplified by the condition of the 1e3-contrast body; the coarse levels'
+        # corrections leave any values in the nodes without stiffness
+        assert rel_err(x[0][~dead], x[1][~dead]) < 1e-4
+    G2.close()
+    ctx2.close()
+    G.close()
+    ctx.close()

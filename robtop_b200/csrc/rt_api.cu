@@ -407,6 +407,7 @@ static int upload_KE(rt_hier* h) {
     RT_CUDA(h->ctx, cudaMemcpyAsync(h->KE_dev, h->KE, sizeof(double) * 576, cudaMemcpyHostToDevice, h->ctx->stream));
     RT_CUDA(h->ctx, cudaStreamSynchronize(h->ctx->stream));
     if (h->Qgal) { cudaFree(h->Qgal); h->Qgal = nullptr; h->Qgal_ratio = 0; }
+    h->dinv_ready[0] = h->dinv_ready[1] = false;
     h->graph_epoch++;  // the element operator's Hadamard-domain values are kernel parameters
     return RT_OK;
 }
@@ -679,6 +680,8 @@ extern "C" int rt_surface_nodes(rt_hier* h, uint8_t* surf) {
     return s;
 }
 
+static int remake_codes(rt_hier* h);
+
 extern "C" int rt_set_support(rt_hier* h, const uint8_t* vfix) {
     if (!h || !vfix) return RT_EINVAL;
     RT_NOT_WORKSPACE(h);
@@ -691,7 +694,7 @@ extern "C" int rt_set_support(rt_hier* h, const uint8_t* vfix) {
     h->graph_epoch++;  // kernel variants depend on whether supports exist
     h->stencil_ready = false;
     h->design_epoch++;
-    return rtk::node_codes(h);  // at once: a workspace's calls read them without a refresh
+    return remake_codes(h);  // at once: a workspace's calls read them without a refresh
 }
 
 // shell elements (HierarchyGrid::setSolidShellElement, grid/Grid.cpp:67-137 marks them):
@@ -955,7 +958,7 @@ extern "C" int rt_put(rt_hier* h, int field, int lvl, int layout, const void* sr
         h->stencil_ready = false;
         h->design_epoch++;
     }
-    return in_node_codes(field, lvl) ? rtk::node_codes(h) : RT_OK;
+    return in_node_codes(field, lvl) ? remake_codes(h) : RT_OK;
 }
 
 extern "C" int rt_get(rt_hier* h, int field, int lvl, int layout, void* dst) {
@@ -986,7 +989,7 @@ extern "C" int rt_put_dev(rt_hier* h, int field, int lvl, const void* src) {
         h->stencil_ready = false;
         h->design_epoch++;
     }
-    return in_node_codes(field, lvl) ? rtk::node_codes(h) : RT_OK;
+    return in_node_codes(field, lvl) ? remake_codes(h) : RT_OK;
 }
 
 extern "C" int rt_get_dev(rt_hier* h, int field, int lvl, void* dst) {
@@ -1020,27 +1023,41 @@ extern "C" int rt_init_density(rt_hier* h, float rho) {
 // ---------------------------------------------------------------------------
 static int estimate_lmax(rt_hier* h, int lvl);
 
-// the marching kernels (variants 1, 2) smooth with stored inverted diagonal blocks; the others form them
-static bool reads_dinv(const rt_hier* h) {
-    for (int pr = 0; pr < 2; pr++)
-        for (int m = 2; m < 4; m++)
-            if (h->tune[pr][m].variant == 1 || h->tune[pr][m].variant == 2) return true;
+// the marching kernels (variants 1, 2) and the FP32 face march (8) smooth with stored inverted diagonal blocks, the
+// others form them
+static bool reads_dinv(const rt_hier* h, int pr) {
+    for (int m = 2; m < 4; m++) {
+        const int v = h->tune[pr][m].variant;
+        if (v == 1 || v == 2 || (v == 8 && pr == 0)) return true;
+    }
     return false;
 }
 
-// element weights rho^p, node codes and (where a chosen kernel reads them) the inverted diagonal blocks of
-// the finest level
+// the blocks of one precision (0 FP32, 1 FP64) for the current weights, where its smoothing kernels read them
+static int need_dinv(rt_hier* h, int pr) {
+    rt_hier* p = h->parent ? h->parent : h;
+    if (p->dinv_ready[pr] || !reads_dinv(p, pr)) return RT_OK;
+    RT_CHECK(rtk::fine_dinv(p, pr == 1));
+    p->dinv_ready[pr] = true;
+    return RT_OK;
+}
+
+// node codes; the diagonal blocks have to follow
+static int remake_codes(rt_hier* h) {
+    h->dinv_ready[0] = h->dinv_ready[1] = false;
+    return rtk::node_codes(h);
+}
+
+// element weights rho^p and node codes of the finest level, and the blocks that FP64 smoothing and the hierarchy's own
+// solves read; the FP32 calls ask for theirs
 static int refresh_fine(rt_hier* h) {
     if (h->parent) {  // weights, node codes and diagonal blocks belong to the parent (refreshed by its own calls)
         ws_sync(h);
-        return RT_OK;
+        return need_dinv(h, 1);
     }
     RT_CHECK(rtk::penalty_weights(h));
-    RT_CHECK(rtk::node_codes(h));
-    h->dinv_ready = false;
-    if (!reads_dinv(h)) return RT_OK;
-    h->dinv_ready = true;
-    return rtk::fine_dinv(h);
+    RT_CHECK(remake_codes(h));
+    return need_dinv(h, 1);
 }
 
 extern "C" int rt_update_stencil(rt_hier* h) {
@@ -1048,6 +1065,7 @@ extern "C" int rt_update_stencil(rt_hier* h) {
     RT_NOT_WORKSPACE(h);
     RT_CUDA(h->ctx, cudaSetDevice(h->ctx->device));
     RT_CHECK(refresh_fine(h));
+    if (h->P.precision == RT_FP32) RT_CHECK(need_dinv(h, 0));
     const int nl = (int)h->L.size();
     for (int i = 1; i < nl; i++) {
         if (i == 1) RT_CHECK(rtk::galerkin_from_elements(h));
@@ -1346,6 +1364,7 @@ extern "C" int rt_smooth_f32(rt_hier* h, int lvl, int smoother, int sweeps, doub
         return rt_fail(h->ctx, RT_EINVAL, "FP32 smoothing: Jacobi or Chebyshev");
     if (lvl > 0) RT_CHECK(need_stencil(h));
     else RT_CHECK(refresh_fine(h));
+    RT_CHECK(need_dinv(h, 0));
     if (smoother == RT_SMOOTH_CHEBY && !h->stencil_ready) return rt_fail(h->ctx, RT_ESTATE, "rt_update_stencil has not run");
     rt_level& L = h->L[lvl];
     const long n = 3 * L.nv;
@@ -2452,6 +2471,7 @@ extern "C" int rt_autotune(rt_hier* h, int reps) {
     c->profile = false;
     // inputs: random u, f on the solver's scratch vectors (their contents do not persist across calls)
     RT_CHECK(refresh_fine(h));
+    RT_CHECK(need_dinv(h, 0));
     RT_CHECK(rtk::rng_uniform(h, 0xa770, n, h->x));
     RT_CHECK(rtk::rng_uniform(h, 0xa771, n, h->q));
     RT_CHECK(rtk::d2f(h, n, h->x, L.u32));
@@ -2482,6 +2502,7 @@ extern "C" int rt_autotune(rt_hier* h, int reps) {
             h->tune[prec][mode] = best_cfg;
             h->tune_us[prec][mode] = best;
         }
+    RT_CHECK(need_dinv(h, 0));  // the chosen kernel may be the first to read them
     RT_CHECK(autotune_level_kernels(h, reps));
     cudaGetLastError();
     h->graph_epoch++;  // launch shapes are baked into captured graphs
@@ -2519,10 +2540,8 @@ extern "C" int rt_set_tuning(rt_hier* h, int precision, int mode, int variant, i
     if (variant == 2 && ty != 2 && ty != 4) return rt_fail(h->ctx, RT_EINVAL, "prefetching rows per tile must be 2 or 4");
     h->tune[pr][mode] = rt_tile_cfg{variant, ty, zchunk};
     h->graph_epoch++;
-    if (!h->dinv_ready && reads_dinv(h)) {  // the weights' last refresh had no reader for them
-        h->dinv_ready = true;
-        RT_CHECK(rtk::fine_dinv(h));
-    }
+    // the weights' last refresh had no reader for them
+    if (pr == 1 || h->P.precision == RT_FP32) RT_CHECK(need_dinv(h, pr));
     return RT_OK;
 }
 
@@ -2533,6 +2552,7 @@ extern "C" int rt_bench_fine_kernel(rt_hier* h, int precision, int mode, int rep
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;
     RT_CHECK(refresh_fine(h));
+    RT_CHECK(need_dinv(h, 0));
     RT_CHECK(rtk::rng_uniform(h, 0xbe7c, n, h->x));
     RT_CHECK(rtk::rng_uniform(h, 0xbe7d, n, h->q));
     RT_CHECK(rtk::d2f(h, n, h->x, L.u32));
@@ -2550,6 +2570,7 @@ extern "C" int rt_fine_kernel_f32(rt_hier* h, int mode, double omega) {
     if (!h || mode < 0 || mode > 3) return RT_EINVAL;
     RT_NOT_WORKSPACE(h);
     RT_CHECK(refresh_fine(h));
+    RT_CHECK(need_dinv(h, 0));
     if (mode == 3 && !h->stencil_ready) return rt_fail(h->ctx, RT_ESTATE, "rt_update_stencil has not run");
     rt_level& L = h->L[0];
     const long n = 3 * L.nv;

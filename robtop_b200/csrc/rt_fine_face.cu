@@ -11,7 +11,7 @@
 //    the element above), only the z stage is per element: 6 + 12 + 24 adds instead of 72, and the same on the
 //    way back, where neighbours' results are added between the stages, so that no scatter remains.
 //  * A lane owns element column X0 - 1 + lane and node column X0 - 1 + lane, a warp one element row.  x neighbours
-//    meet by shuffles; the upper edge of a warp's row goes to the next warp, 6 values (and 2 weight sums) per lane and
+//    meet by shuffles; the upper edge of a warp's row goes to the next warp, 6 values (in FP64 smoothing 2 weight sums as well) per lane and
 //    layer through shared memory, with one barrier per layer.  Lanes 1..30 finish nodes; a block of W warps finishes
 //    30 x (W - 1) nodes per layer.
 //  * The loads of the next layer and of this layer's output stage are issued before the arithmetic (FP32 Chebyshev on
@@ -21,7 +21,11 @@
 //    of layer t + 1 (511x256x256: 897 us with __syncthreads, 766 us).  The other forms hold the inputs of the output
 //    stage as well and got slower with it (FP64 residual 850, 938 us with it; FP32 residual 490, 600 us).
 //  * Two element rows per warp, with the edge between them in registers, need 128 registers in FP32: Chebyshev 736 us.
-//  * The 3x3 diagonal block of a node needs four signed sums of its 8 weights, factorised the same way.
+//  * The 3x3 diagonal block of a node needs four signed sums of its 8 weights, factorised the same way.  FP64 steps form
+//    and invert it; FP32 steps read the inverse that k_fine_dinv made in FP64.  Inverted in FP32 here, a step from zero
+//    had 2 to 3 times the error, and entries past 1e12 or below 1e-13 left FP32's range in the determinant (511x256x256,
+//    z-chunk 16: Jacobi 637 us so, 715 us read; Chebyshev 686, 715 us); formed here in FP64 it needs registers that are
+//    not there (Jacobi 682 us, Chebyshev 928 us; 768 us with 20 warps per SM instead of 24).
 //
 // Fixed and inactive nodes enter the element products as zero (the reference's WS rule); out[] follows
 // rt_fine_tile.cu's rules for them.
@@ -42,12 +46,7 @@ constexpr int FACE_NX = 30;  // node columns a warp finishes (lanes 1..30)
 constexpr int face_warps(bool f64, int mode) { return f64 && mode < 2 ? 12 : 8; }
 
 // 1 / det of a node's block; 0 where all its elements have zero weight (the node keeps its value)
-template <typename T>
-__device__ __forceinline__ T block_rcp(T det, T sw) {
-    if (sw == T(0)) return T(0);
-    if constexpr (sizeof(T) == 4) return __frcp_rn(det);
-    else return T(1) / det;
-}
+__device__ __forceinline__ double block_rcp(double det, double sw) { return sw == 0.0 ? 0.0 : 1.0 / det; }
 
 // a fixed node's rule f / n_e, from its code; 0 without a weighted element
 template <typename T>
@@ -98,10 +97,11 @@ __device__ __forceinline__ void face_grid_sum(double x, double* __restrict__ par
 template <typename T, bool WS, int MODE, int W, int MINB, bool DOT>
 __global__ void __launch_bounds__(32 * W, MINB)
     k_fine_face(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code, const float* __restrict__ wgt,
-                const rte::KtVals<T> kt, const T* __restrict__ u, const T* __restrict__ f, T* __restrict__ out, T omega,
-                T* __restrict__ dvec, const double* __restrict__ coef, int kstep, double* __restrict__ partials,
+                const rte::KtVals<T> kt, const T* __restrict__ dinv, const T* __restrict__ u, const T* __restrict__ f,
+                T* __restrict__ out, T omega, T* __restrict__ dvec, const double* __restrict__ coef, int kstep, double* __restrict__ partials,
                 double* __restrict__ dot_out, unsigned* __restrict__ ticket, double* __restrict__ err) {
-    constexpr int NX = MODE >= 2 ? 8 : 6;  // values handed to the next warp
+    constexpr bool STORED = sizeof(T) == 4 && MODE >= 2, BLOCK = sizeof(T) == 8 && MODE >= 2;  // inverse blocks read, formed
+    constexpr int NX = BLOCK ? 8 : 6;  // values handed to the next warp
     constexpr bool LATE = sizeof(T) == 8 && MODE == 1;
     __shared__ T S[2][W][NX][32];
     __shared__ uint64_t bar;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
     uint32_t cc = 0, co = 0;              // node codes of the next layer and of the output stage's layer
     T Qp[4] = {T(0), T(0), T(0), T(0)};   // signed weight sums of the element layer below the output stage's layer
     T X[6], wa = T(0), wb = T(0);         // the output stage's x-edge data and weight sums along x
-    T fv[3], dv[3], uo[3];                // its inputs
+    T fv[3], dv[3], uo[3], inv[6];        // its inputs
     int vn = ci + vx * ri + plane * (Z0 - 1);  // node (ci, ri) of layer t
     int en = ci + nx * ri + eplane * (Z0 - 1);
     fetch(Z0 - 1, vn, en - eplane);
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
         if (w > 0) {
 #pragma unroll
             for (int q = 0; q < 6; q++) X[q] += S[t & 1][w - 1][q][lane];
-            if (MODE >= 2) {
+            if (BLOCK) {
                 wa_b = S[t & 1][w - 1][NX - 2][lane];
                 wb_b = S[t & 1][w - 1][NX - 1][lane];
             }
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
 #pragma unroll
         for (int c = 0; c < 3; c++) acc[c] = X[c] + X[3 + c] + __shfl_up_sync(0xffffffffu, X[c] - X[3 + c], 1);
         T Q[4];
-        if (MODE >= 2) {
+        if (BLOCK) {
             Q[0] = wa + wa_b;  // sum w
             Q[1] = wb - wb_b;  // sum w sx sy
             Q[2] = wa - wa_b;  // sum w sy
@@ -227,18 +227,24 @@ __global__ void __launch_bounds__(32 * W, MINB)
 #pragma unroll
                 for (int c = 0; c < 3; c++) o[c] = fixed_value(fv[c], co);
             } else if (act) {
-                const T sw = Q[0] + Qp[0], sxy = Q[1] + Qp[1], sxz = Q[3] - Qp[3], syz = Q[2] - Qp[2];
-                const T A = kt.diag_a * sw, bxy = kt.diag_b * sxy, bxz = kt.diag_b * sxz, byz = kt.diag_b * syz;
-                // inverse of [[A,bxy,bxz],[bxy,A,byz],[bxz,byz,A]]
-                const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
-                const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
-                const T id = block_rcp(A * c00 + bxy * c01 + bxz * c02, sw);
-                T rr[3];
+                T rr[3], zz[3];
 #pragma unroll
                 for (int c = 0; c < 3; c++) rr[c] = fv[c] - acc[c];
-                const T zz[3] = {id * (c00 * rr[0] + c01 * rr[1] + c02 * rr[2]),
-                                 id * (c01 * rr[0] + c11 * rr[1] + c12 * rr[2]),
-                                 id * (c02 * rr[0] + c12 * rr[1] + c22 * rr[2])};
+                if constexpr (STORED) {
+                    zz[0] = inv[0] * rr[0] + inv[1] * rr[1] + inv[2] * rr[2];
+                    zz[1] = inv[1] * rr[0] + inv[3] * rr[1] + inv[4] * rr[2];
+                    zz[2] = inv[2] * rr[0] + inv[4] * rr[1] + inv[5] * rr[2];
+                } else {
+                    const T sw = Q[0] + Qp[0], sxy = Q[1] + Qp[1], sxz = Q[3] - Qp[3], syz = Q[2] - Qp[2];
+                    const T A = kt.diag_a * sw, bxy = kt.diag_b * sxy, bxz = kt.diag_b * sxz, byz = kt.diag_b * syz;
+                    // inverse of [[A,bxy,bxz],[bxy,A,byz],[bxz,byz,A]]
+                    const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
+                    const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
+                    const T id = block_rcp(A * c00 + bxy * c01 + bxz * c02, sw);
+                    zz[0] = id * (c00 * rr[0] + c01 * rr[1] + c02 * rr[2]);
+                    zz[1] = id * (c01 * rr[0] + c11 * rr[1] + c12 * rr[2]);
+                    zz[2] = id * (c02 * rr[0] + c12 * rr[1] + c22 * rr[2]);
+                }
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
                     if (MODE == 2) {
@@ -255,7 +261,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
 #pragma unroll
                 for (int c = 0; c < 3; c++) dvec[c * nv + v] = dn[c];
         }
-        if (MODE >= 2)
+        if (BLOCK)
 #pragma unroll
             for (int q = 0; q < 4; q++) Qp[q] = Q[q];
     };
@@ -286,8 +292,11 @@ __global__ void __launch_bounds__(32 * W, MINB)
             dv[c] = (MODE == 3 && ld && kstep > 0) ? dvec[c * nv + vn] : T(0);
             uo[c] = ((MODE >= 2 || DOT || (WS && MODE == 1 && co > 1u)) && ld) ? u[c * nv + vn] : T(0);
         }
+        if (STORED)
+#pragma unroll
+            for (int q = 0; q < 6; q++) inv[q] = ld ? dinv[q * (long)nv + vn] : T(0);
         // ---- element layer t
-        if (MODE >= 2) {
+        if (BLOCK) {
             const T wl = __shfl_up_sync(0xffffffffu, wv, 1);
             wa = wv + wl;
             wb = wv - wl;
@@ -317,7 +326,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
             X[q] = Ft[q] + Ft[6 + q];
             S[t & 1][w][q][lane] = Ft[q] - Ft[6 + q];
         }
-        if (MODE >= 2) {
+        if (BLOCK) {
             S[t & 1][w][NX - 2][lane] = wa;
             S[t & 1][w][NX - 1][lane] = wb;
         }
@@ -333,10 +342,10 @@ __global__ void __launch_bounds__(32 * W, MINB)
 
 // The smoothing step from u = 0, where K u needs no evaluation: out = omega D^-1 f (MODE 2) or out = d = b_0 D^-1 f
 // (MODE 3), fixed nodes f / n_e (d = 0).  A thread marches one node column through a z-chunk with the weight sums of
-// the element layer below; 33 B (MODE 2) or 45 B per node in FP32 instead of the full step's 66.
+// the element layer below, the block in FP64; 29 B (MODE 2) or 41 B per node in FP32, the full step moves 90.
 template <typename T, int MODE, bool DOT>
 __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code,
-                                                   const float* __restrict__ wgt, T diag_a, T diag_b,
+                                                   const float* __restrict__ wgt, double diag_a, double diag_b,
                                                    const T* __restrict__ f, T* __restrict__ out, T omega,
                                                    T* __restrict__ dvec, const double* __restrict__ coef,
                                                    double* __restrict__ partials, double* __restrict__ dot_out,
@@ -351,33 +360,33 @@ __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int z
     const long plane = (long)vx * vy, nv = plane * vz, eplane = (long)nx * ny;
     const long col = x + (long)vx * y, ecol = x + (long)nx * y;
     const bool x0 = x > 0, x1 = x < nx, y0 = y > 0, y1 = y < ny;
-    T Qp[4] = {T(0), T(0), T(0), T(0)};
+    double Qp[4] = {0, 0, 0, 0};
 #pragma unroll 2
     for (int t = Z0 - 1; t < Z1; t++) {
-        T w00 = T(0), w10 = T(0), w01 = T(0), w11 = T(0);  // element (x - 1 + i, y - 1 + j) of layer t
+        double w00 = 0, w10 = 0, w01 = 0, w11 = 0;  // element (x - 1 + i, y - 1 + j) of layer t
         if (t >= 0 && t < nz) {
             const float* we = wgt + ecol + eplane * t;
-            if (x0 && y0) w00 = (T)we[-1 - nx];
-            if (x1 && y0) w10 = (T)we[-nx];
-            if (x0 && y1) w01 = (T)we[-1];
-            if (x1 && y1) w11 = (T)we[0];
+            if (x0 && y0) w00 = we[-1 - nx];
+            if (x1 && y0) w10 = we[-nx];
+            if (x0 && y1) w01 = we[-1];
+            if (x1 && y1) w11 = we[0];
         }
-        const T a0 = w10 + w00, b0 = w10 - w00, a1 = w11 + w01, b1 = w11 - w01;
-        const T Q[4] = {a1 + a0, b1 - b0, a1 - a0, b1 + b0};  // sums of w, w sx sy, w sy, w sx
+        const double a0 = w10 + w00, b0 = w10 - w00, a1 = w11 + w01, b1 = w11 - w01;
+        const double Q[4] = {a1 + a0, b1 - b0, a1 - a0, b1 + b0};  // sums of w, w sx sy, w sy, w sx
         if (t >= Z0) {
             const long v = col + plane * t;
             const uint32_t c = code[v];
             const T f0 = f[v], f1 = f[nv + v], f2 = f[2 * nv + v];
             T o[3] = {T(0), T(0), T(0)};
             if (c == 1u) {
-                const T sw = Q[0] + Qp[0], sxy = Q[1] + Qp[1], sxz = Q[3] - Qp[3], syz = Q[2] - Qp[2];
-                const T A = diag_a * sw, bxy = diag_b * sxy, bxz = diag_b * sxz, byz = diag_b * syz;
-                const T c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
-                const T c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
-                const T id = block_rcp(A * c00 + bxy * c01 + bxz * c02, sw) * scale;
-                o[0] = id * (c00 * f0 + c01 * f1 + c02 * f2);
-                o[1] = id * (c01 * f0 + c11 * f1 + c12 * f2);
-                o[2] = id * (c02 * f0 + c12 * f1 + c22 * f2);
+                const double sw = Q[0] + Qp[0], sxy = Q[1] + Qp[1], sxz = Q[3] - Qp[3], syz = Q[2] - Qp[2];
+                const double A = diag_a * sw, bxy = diag_b * sxy, bxz = diag_b * sxz, byz = diag_b * syz;
+                const double c00 = A * A - byz * byz, c01 = byz * bxz - bxy * A, c02 = bxy * byz - A * bxz;
+                const double c11 = A * A - bxz * bxz, c12 = bxy * bxz - A * byz, c22 = A * A - bxy * bxy;
+                const double id = block_rcp(A * c00 + bxy * c01 + bxz * c02, sw) * scale;
+                o[0] = (T)(id * (c00 * f0 + c01 * f1 + c02 * f2));
+                o[1] = (T)(id * (c01 * f0 + c11 * f1 + c12 * f2));
+                o[2] = (T)(id * (c02 * f0 + c12 * f1 + c22 * f2));
             } else if (c > 1u) {
                 o[0] = fixed_value(f0, c);
                 o[1] = fixed_value(f1, c);
@@ -440,7 +449,7 @@ int launch_face_dot(rt_hier* h, const T* u, const T* f, T* out, double omega, co
     const rte::KtVals<T> kt = rte::make_kt<T>(h);
     return rt_launch(h->ctx, name, [&] {
         k_fine_face<T, WS, MODE, W, MINB, DOT><<<grid, 32 * W, 0, h->ctx->stream>>>(
-            L.nx, L.ny, L.nz, zc, h->ncode, h->w, kt, u, f, out, (T)omega, dvec, coef, kstep, h->kpart, dot_out,
+            L.nx, L.ny, L.nz, zc, h->ncode, h->w, kt, reinterpret_cast<const T*>(h->dinv32), u, f, out, (T)omega, dvec, coef, kstep, h->kpart, dot_out,
             reinterpret_cast<unsigned*>(h->scal + RT_SCAL_TICKET), h->scal + RT_SCAL_ERR);
     });
 }
@@ -468,7 +477,7 @@ int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const do
     unsigned* ticket = reinterpret_cast<unsigned*>(h->scal + RT_SCAL_TICKET);
     return rt_launch(h->ctx, sizeof(T) == 8 ? "fine_smooth0_f64" : "fine_smooth0_f32", [&] {
         auto go = [&](auto kern, T om, T* d, const double* cf) {
-            kern<<<grid, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, zc, h->ncode, h->w, (T)h->KE[0], (T)h->KE[1], f, out,
+            kern<<<grid, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, zc, h->ncode, h->w, h->KE[0], h->KE[1], f, out,
                                                    om, d, cf, h->kpart, dot_out, ticket);
         };
         if (coef) go(k_fine_diag<T, 3, false>, T(0), dvec, coef);

@@ -284,17 +284,17 @@ int launch_march(rt_hier* h, const T* u, const T* f, T* out, double omega, const
 
 namespace rtk {
 
-int fine_dinv(rt_hier* h) {
+int fine_dinv(rt_hier* h, bool f64) {
     rt_level& L = h->L[0];
     const unsigned g = (unsigned)std::min<long>((L.nv + 255) / 256, (long)h->ctx->sm_count * 16);
     const int ws = h->has_support ? 1 : 0;
-    RT_CHECK(rt_launch(h->ctx, "fine_dinv_f64", [&] {
-        k_fine_dinv<double><<<g, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, L.vact, h->w, h->vfix, ws, h->KE[0],
-                                                           h->KE[1], h->dinv64);
-    }));
-    return rt_launch(h->ctx, "fine_dinv_f32", [&] {
-        k_fine_dinv<float><<<g, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, L.vact, h->w, h->vfix, ws, h->KE[0],
-                                                          h->KE[1], h->dinv32);
+    return rt_launch(h->ctx, f64 ? "fine_dinv_f64" : "fine_dinv_f32", [&] {
+        if (f64)
+            k_fine_dinv<double><<<g, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, L.vact, h->w, h->vfix, ws, h->KE[0],
+                                                               h->KE[1], h->dinv64);
+        else
+            k_fine_dinv<float><<<g, 256, 0, h->ctx->stream>>>(L.nx, L.ny, L.nz, L.vact, h->w, h->vfix, ws, h->KE[0],
+                                                              h->KE[1], h->dinv32);
     });
 }
 

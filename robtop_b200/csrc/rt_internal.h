@@ -121,7 +121,7 @@ struct rt_hier {
     double fused_us[15][2] = {};
     double* dinv64 = nullptr;        // [6][nv] inverted diagonal blocks of the finest level
     float* dinv32 = nullptr;
-    bool dinv_ready = false;         // the diagonal blocks match the weights (made only for kernels that read them)
+    bool dinv_ready[2] = {false, false};  // [FP32, FP64] the blocks match the weights (made for kernels that read them)
     uint8_t* ncode = nullptr;        // [nv] node codes of the finest level (k_node_code), remade when w, vact or vfix change
     std::vector<rt_level> L;
     double KE[576];
@@ -302,7 +302,7 @@ template <typename T, bool WS, int MODE>
 int launch_sf(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec, const double* coef,
               int kstep);
 int init_stencil_kernels(rt_ctx* c);
-int fine_dinv(rt_hier* h);
+int fine_dinv(rt_hier* h, bool f64);
 int node_codes(rt_hier* h);
 template <typename T, bool WS, int MODE>
 int launch_face(rt_hier* h, const T* u, const T* f, T* out, double omega, const char* name, T* dvec, const double* coef,

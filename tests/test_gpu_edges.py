@@ -414,3 +414,70 @@ def test_zero_density_pocket(zc):
     ctx2.close()
     G.close()
     ctx.close()
+
+
+# FP32 block inverse of the finest level: formed in FP64 and rounded once, so that a step from u = 0 has the rounding of
+# its entries and of the result alone, also where a product of three entries of the block leaves FP32's range
+@pytest.mark.parametrize("scale,lo", [(1.0, 0.1), (1e8, 0.1), (1e-8, 1e-3)])
+def test_fp32_block_inverse(scale, lo):
+    nx, ny, nz = 37, 15, 12
+    ctx, G, eact, rho, vfix, r = _hier(nx, ny, nz, seed=8)
+    p = G.params
+    p.youngs_modulus = E * scale
+    G.set_params(p)
+    rho = (lo * 10.0 ** (r.random(eact.shape) * -np.log10(lo))).astype(np.float32)
+    G[0].setRho(rho.ravel())
+    f = r.standard_normal(3 * G[0].nv).astype(np.float32).astype(np.float64)
+    G[0].setForce(f)
+    G[0].reset_displacement()
+    G[0].update_residual()
+    H = O.Hierarchy(eact, rho, vfix, p=P, E=E * scale, nu=NU)
+    H.set_weights(G[0].getPenalty())
+    want, tmp = np.zeros_like(f), np.zeros_like(f)
+    O.lib().or_fine_jacobi(H.lv(0), O.ptr(H.KE), O.ptr(want), O.ptr(f), 1.0, O.ptr(tmp))
+    rb._capi.check(rb.lib().rt_fine_kernel_f32(G.handle, 2, 1.0), ctx.handle)
+    got = G[0].getResidual()
+    n = G[0].nv
+    err = np.abs(got - want).reshape(3, n).max(0) / np.abs(want).reshape(3, n).max(0)
+    # entries, products and sums to 2^-24, the products at most twice the result (condition of the block): 4 units at most
+    assert err.max() < 4 * 2.0**-24, err.max() * 2.0**24
+    G.close()
+    ctx.close()
+
+
+# the stored FP32 blocks are there and current whichever call first needs them: a launch shape chosen after the stencils,
+# a density change, a workspace's smoothing right after new supports
+def test_fp32_blocks_follow():
+    L = rb.lib()
+    ctx, G, eact, rho, vfix, r = _hier(33, 17, 14, seed=9, precision=rb.FP32, smoother=rb.SMOOTH_CHEBY, pre_sweeps=2,
+                                       post_sweeps=2)
+    b = r.standard_normal(3 * G[0].nv) * np.tile(1.0 - vfix.ravel(), 3)
+
+    def step(g, shape=None):
+        if shape:
+            g.set_tiles(*shape)
+        g[0].setForce(b)
+        g[0].reset_displacement()
+        g.pcg(1e-14, 2)
+        return g[0].getDisplacement()
+
+    shape = G.tuning()["chebyshev_f32"]["zchunk"]
+    for new in (rho, (0.1 + 0.9 * r.random(rho.shape)).astype(np.float32)):
+        G[0].setRho(new.ravel())
+        G.set_tiles(3, 8, 16)  # reads no blocks
+        G.update_stencil()
+        late = step(G, (8, 1, shape))
+        G.update_stencil()
+        assert np.array_equal(late, step(G))
+    W = G.workspace()
+    vfix[:, :, -1] = 1
+    G.set_support(vfix)
+    got = []
+    for g in (W, G):
+        g[0].setForce(b)
+        g[0].setDisplacement(b)
+        rb._capi.check(L.rt_smooth_f32(g.handle, 0, rb.SMOOTH_JACOBI, 2, 0.6), ctx.handle)
+        got.append(g[0].getDisplacement())
+    assert np.array_equal(*got)
+    G.close()
+    ctx.close()

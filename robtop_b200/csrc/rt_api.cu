@@ -1768,14 +1768,16 @@ static int pcg_prologue(rt_hier* h, double* x, const double* b) {
     return RT_OK;
 }
 
-// a solve that produced NaN: a stencil kernel whose bounded copy wait ran out writes NaN and
-// flags RT_SCAL_ERR, anything else is a numerical breakdown
+// a solve that produced NaN: a kernel whose bounded wait ran out writes NaN and flags RT_SCAL_ERR, anything else is a
+// numerical breakdown
 static int nan_fail(rt_hier* h, int it) {
     double e = 0;
     RT_CHECK(read_scalars(h, RT_SCAL_ERR, 1, &e));
     if (e != 0.0) {
         RT_CUDA(h->ctx, cudaMemsetAsync(h->scal + RT_SCAL_ERR, 0, sizeof(double), h->ctx->stream));
         RT_CUDA(h->ctx, cudaMemsetAsync(h->scal + RT_SCAL_GBAR, 0, sizeof(double) * RT_MAX_LEVELS, h->ctx->stream));
+        if (e == 4.0)
+            return rt_fail(h->ctx, RT_ECUDA, "a warp of the FP64 product K u gave up waiting for its block's others (iteration %d)", it);
         if (e == 3.0)
             return rt_fail(h->ctx, RT_ECUDA, "a finest-level kernel gave up waiting for its TMA node-layer copies (iteration %d)", it);
         return rt_fail(h->ctx, RT_ECUDA, e == 2.0 ? "a fused Chebyshev sweep gave up at its grid barrier (iteration %d)"

@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "rt_element.cuh"
 #include "rt_internal.h"
@@ -188,8 +189,12 @@ __global__ void __launch_bounds__(32 * W, MINB)
         if (!LATE) {
             __syncthreads();
         } else {
-            const bool arrived = rttc::mbar_wait(&bar, phase);
-            if (!arrived && lane == 0) *err = 1.0;  // all warps of a block arrive in every layer: not reached
+            if (!rttc::mbar_wait(&bar, phase)) {  // not reached: all warps of a block arrive in every layer
+                *err = 4.0;
+#pragma unroll
+                for (int q = 0; q < 6; q++) X[q] = T(NAN);  // in the layer's nodes and u . out, which a solve reports
+                pq = NAN;
+            }
             phase ^= 1;
         }
         T wa_b = T(0), wb_b = T(0);

@@ -241,7 +241,7 @@ static inline unsigned rt_blocks(long n, int bs) { return (unsigned)((n + bs - 1
 // rho_k = 1/(2 sigma - rho_{k-1}), a_k = rho_k rho_{k-1}, b_k = 2 rho_k / delta.
 #define RT_CHEBY_LO_FRAC (1.0 / 30.0)
 #define RT_CHEBY_HI_FRAC 1.1
-#define RT_SCAL_ERR 295   // set to 1 by a stencil kernel whose bounded copy wait ran out
+#define RT_SCAL_ERR 295   // set by a kernel whose bounded wait ran out: 1 stencil copies, 2 grid barrier, 3 TMA layers, 4 FP64 K u
 #define RT_SCAL_LMAX 300  // device scalar slots holding lmax(D^-1 A) per level
 #define RT_SCAL_TICKET 496  // ticket counter of the grid reductions (u32, zero between launches)
 #define RT_SCAL_GBAR 480  // per level: the grid barrier of the fused Chebyshev sweeps (arrivals, generation as 2 x u32)

@@ -28,19 +28,26 @@ struct VertexRow {
     T diag_a, diag_b;  // KE[v][v] = a I + b (s s^T - I)
 };
 
+// x / d from id = 1 / d: the product's remainder added back, which rounds as the division does (Markstein)
+template <typename T>
+__device__ __forceinline__ T quotient(T x, T d, T id) {
+    const T q = x * id;
+    return fma(fma(-d, q, x), id, q);
+}
+
 // diag: the common diagonal entry of the node's block, off: its entries xy, xz, yz
 template <typename T>
 __device__ __forceinline__ void block_gs(T diag, const T (&off)[3], const T (&F)[3], const T (&KU)[3], T (&uu)[3],
                                          bool backward) {
     const T id = T(1) / diag;  // off the chain of the three updates
     if (!backward) {
-        uu[0] = (F[0] - off[0] * uu[1] - off[1] * uu[2] - KU[0]) * id;
-        uu[1] = (F[1] - off[0] * uu[0] - off[2] * uu[2] - KU[1]) * id;
-        uu[2] = (F[2] - off[1] * uu[0] - off[2] * uu[1] - KU[2]) * id;
+        uu[0] = quotient(F[0] - off[0] * uu[1] - off[1] * uu[2] - KU[0], diag, id);
+        uu[1] = quotient(F[1] - off[0] * uu[0] - off[2] * uu[2] - KU[1], diag, id);
+        uu[2] = quotient(F[2] - off[1] * uu[0] - off[2] * uu[1] - KU[2], diag, id);
     } else {
-        uu[2] = (F[2] - off[1] * uu[0] - off[2] * uu[1] - KU[2]) * id;
-        uu[1] = (F[1] - off[0] * uu[0] - off[2] * uu[2] - KU[1]) * id;
-        uu[0] = (F[0] - off[0] * uu[1] - off[1] * uu[2] - KU[0]) * id;
+        uu[2] = quotient(F[2] - off[1] * uu[0] - off[2] * uu[1] - KU[2], diag, id);
+        uu[1] = quotient(F[1] - off[0] * uu[0] - off[2] * uu[2] - KU[1], diag, id);
+        uu[0] = quotient(F[0] - off[0] * uu[1] - off[1] * uu[2] - KU[0], diag, id);
     }
 }
 

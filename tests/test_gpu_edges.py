@@ -481,3 +481,21 @@ def test_fp32_blocks_follow():
     assert np.array_equal(*got)
     G.close()
     ctx.close()
+
+
+# the finest Gauss-Seidel divides by the diagonal: from u = 0 the first colour's first component is f / (KE_00 sum w), and
+# a sum of 8 FP32 weights is exact in FP64, so that any other rounding of the quotient shows
+def test_fine_gauss_seidel_quotient():
+    nx, ny, nz = 25, 13, 11
+    ctx, G, eact, rho, vfix, r = _hier(nx, ny, nz, seed=12, sup=False)
+    f = r.standard_normal((3, nz + 1, ny + 1, nx + 1))
+    G[0].setForce(f.ravel())
+    G[0].reset_displacement()
+    G[0].smooth(rb.SMOOTH_GS, 1)
+    w = np.zeros((nz + 2, ny + 2, nx + 2))
+    w[1:-1, 1:-1, 1:-1] = G[0].getPenalty().reshape(nz, ny, nx)
+    sw = sum(w[k:nz + 1 + k, j:ny + 1 + j, i:nx + 1 + i] for k in (0, 1) for j in (0, 1) for i in (0, 1))
+    want = f[0] / (G.template_matrix().ravel()[0] * sw)
+    assert np.array_equal(G[0].getDisplacement().reshape(f.shape)[0, ::2, ::2, ::2], want[::2, ::2, ::2])
+    G.close()
+    ctx.close()

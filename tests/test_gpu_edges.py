@@ -77,6 +77,37 @@ def test_face_march_edges(nx, ny, nz, zc, sup):
     ctx.close()
 
 
+# the dot products that come with the march (u . K u in both precisions) and with the step from zero (f . D^-1 f), at the
+# same remainders: the smoother bound is 30 of each, and two CG iterations are no further apart than their alpha and beta
+@pytest.mark.parametrize("nx,ny,nz,zc", [(29, 6, 9, 1), (30, 7, 16, 2), (31, 13, 8, 3), (59, 10, 7, 64), (60, 11, 15, 16),
+                                         (12, 21, 17, 5), (95, 8, 8, 4)])
+@pytest.mark.parametrize("sup", [True, False])
+def test_face_march_dots(nx, ny, nz, zc, sup):
+    ctx, G, H, r = _perforated(nx, ny, nz, nx + ny, sup)
+    G.set_tiles(8, 1, zc)
+    G.update_stencil()
+    # the largest Ritz value of the same 30 steps in another order of summation
+    assert abs(G.smoother_lmax(0) - H.LA[0].lmax) <= 1e-6 * H.LA[0].lmax
+    if sup:  # without supports the solves project, which the oracle's do not
+        b = r.standard_normal(3 * G[0].nv) * np.tile(G[0].getVact(), 3) * (1 - np.tile(H.arrs[0]["vfix"], 3))
+        p = G.params
+        p.pre_sweeps = p.post_sweeps = 2
+        p.jacobi_omega = 0.5
+        # FP64: rounding, amplified by the 1e3 contrast; FP32 cycles and vectors: as in test_tail_cycle_edges
+        for prec, krylov, smoother, so, tol in ((rb.FP64, 0, rb.SMOOTH_JACOBI, O.SMOOTH_JACOBI, 1e-9),
+                                                (rb.FP32, 1, rb.SMOOTH_CHEBY, O.SMOOTH_CHEBY, 1e-3)):
+            p.precision, p.krylov_fp32, p.smoother = prec, krylov, smoother
+            G.set_params(p)
+            G.update_stencil()
+            G[0].setForce(b)
+            G[0].reset_displacement()
+            G.pcg(1e-14, 2)
+            want, its, _ = H.pcg(b, tol=1e-14, maxit=2, smoother=so, npre=2, npost=2, omega=0.5)
+            assert its == 2 and rel_err(G[0].getDisplacement(), want) < tol
+    G.close()
+    ctx.close()
+
+
 # the weight-gradient patches are 8 x 16 voxels by 1 to 4 planes: remainders in each axis, one voxel past a patch,
 # and the smallest boxes the network takes
 @pytest.mark.parametrize("dims", [(9, 17, 8), (8, 16, 8), (33, 15, 12), (25, 8, 9)])

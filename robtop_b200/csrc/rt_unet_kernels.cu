@@ -487,9 +487,9 @@ int conv3_dw(rt_ctx* c, const __nv_bfloat16* in, int in_stride, int cin, const _
         return rt_fail(c, RT_EINVAL, "conv3_dw: channel counts must be multiples of 16 in [16, 128]");
     // taps per CTA: at most 256 accumulator columns, so that two CTAs share an SM's TMEM
     const int TG = 256 / cin < 9 ? 256 / cin : 9, groups = (27 + TG - 1) / TG;
-    // planes per patch: the most that let two CTAs share the shared memory (one loads while the other multiplies),
-    // fewer where that would leave SMs without a patch
-    int P = 4;
+    // planes per patch: two, or one where two CTAs would not share the shared memory then (one loads while the other
+    // multiplies) or SMs would be left without a patch.  With four planes the 128 rows of A alone take 128 KB
+    int P = 2;
     size_t smem = 0;
     for (; P >= 1; P /= 2) {
         size_t op = (size_t)(cout / 8) * P * CONV_TM * 16 + (size_t)(P + 2) * HALO_V * 16 * (cin / 8);

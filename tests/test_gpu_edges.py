@@ -108,9 +108,9 @@ def test_face_march_dots(nx, ny, nz, zc, sup):
     ctx.close()
 
 
-# the weight-gradient patches are 8 x 16 voxels by 1 to 4 planes: remainders in each axis, one voxel past a patch,
+# the weight-gradient patches are 8 x 16 voxels by 1 plane, or 2 on the last box: remainders in each axis, one voxel past a patch,
 # and the smallest boxes the network takes
-@pytest.mark.parametrize("dims", [(9, 17, 8), (8, 16, 8), (33, 15, 12), (25, 8, 9)])
+@pytest.mark.parametrize("dims", [(9, 17, 8), (8, 16, 8), (33, 15, 12), (25, 8, 9), (34, 17, 25)])
 def test_unet_weight_gradient_edges(dims):
     import unet_ref
     from robtop_b200 import learned

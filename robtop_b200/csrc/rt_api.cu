@@ -511,8 +511,6 @@ static int build_hier(rt_ctx* c, const rt_params* p, int nx, int ny, int nz, uin
     }
     rt_level& L0 = h->L[0];
     RT_CHECK(dalloc(c, &h->KE_dev, 576));
-    RT_CHECK(dalloc(c, &h->dinv64, 6 * (size_t)L0.nv));
-    RT_CHECK(dalloc(c, &h->dinv32, 6 * (size_t)L0.nv));
     RT_CHECK(dalloc(c, &h->ncode, (size_t)L0.nv));
     for (int pr = 0; pr < 2; pr++)
         for (int m = 0; m < 4; m++) h->tune[pr][m] = rtk::face_default(c, pr == 1, m, L0.vx, L0.vy, L0.vz);
@@ -1033,14 +1031,22 @@ static bool reads_dinv(const rt_hier* h, int pr) {
     return false;
 }
 
-// the blocks of one precision (0 FP32, 1 FP64) for the current weights, where its smoothing kernels read them
-static int need_dinv(rt_hier* h, int pr) {
+// the blocks of one precision (0 FP32, 1 FP64) for the current weights; their memory (24 and 48 B per node) is taken the
+// first time
+static int make_dinv(rt_hier* h, int pr) {
     rt_hier* p = h->parent ? h->parent : h;
-    if (p->dinv_ready[pr] || !reads_dinv(p, pr)) return RT_OK;
+    if (p->dinv_ready[pr]) return RT_OK;
+    const size_t n = 6 * (size_t)p->L[0].nv;
+    if (pr == 1 && !p->dinv64) RT_CHECK(dalloc(p->ctx, &p->dinv64, n));
+    if (pr == 0 && !p->dinv32) RT_CHECK(dalloc(p->ctx, &p->dinv32, n));
     RT_CHECK(rtk::fine_dinv(p, pr == 1));
     p->dinv_ready[pr] = true;
+    ws_sync(h);
     return RT_OK;
 }
+
+// the same where the precision's smoothing kernels read them
+static int need_dinv(rt_hier* h, int pr) { return reads_dinv(h, pr) ? make_dinv(h, pr) : RT_OK; }
 
 // node codes; the diagonal blocks have to follow
 static int remake_codes(rt_hier* h) {
@@ -2473,7 +2479,7 @@ extern "C" int rt_autotune(rt_hier* h, int reps) {
     c->profile = false;
     // inputs: random u, f on the solver's scratch vectors (their contents do not persist across calls)
     RT_CHECK(refresh_fine(h));
-    RT_CHECK(need_dinv(h, 0));
+    RT_CHECK(make_dinv(h, 0));  // for the candidates
     RT_CHECK(rtk::rng_uniform(h, 0xa770, n, h->x));
     RT_CHECK(rtk::rng_uniform(h, 0xa771, n, h->q));
     RT_CHECK(rtk::d2f(h, n, h->x, L.u32));
@@ -2504,7 +2510,6 @@ extern "C" int rt_autotune(rt_hier* h, int reps) {
             h->tune[prec][mode] = best_cfg;
             h->tune_us[prec][mode] = best;
         }
-    RT_CHECK(need_dinv(h, 0));  // the chosen kernel may be the first to read them
     RT_CHECK(autotune_level_kernels(h, reps));
     cudaGetLastError();
     h->graph_epoch++;  // launch shapes are baked into captured graphs

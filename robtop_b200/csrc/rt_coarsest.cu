@@ -36,15 +36,6 @@ __global__ void k_assemble_dense(int vx, int vy, int vz, long nv, int na, const 
     }
 }
 
-__global__ void k_add_rrt(int n, int nr, const double* __restrict__ R, double alpha, double* __restrict__ A) {
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < (long)n * n; t += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / n), j = (int)(t % n);
-        double s = 0;
-        for (int a = 0; a < nr; a++) s += R[(long)a * n + i] * R[(long)a * n + j];
-        A[t] += alpha * s;
-    }
-}
-
 __global__ void k_trace(int n, const double* __restrict__ A, double* __restrict__ out) {
     __shared__ double sh[256];
     double s = 0;

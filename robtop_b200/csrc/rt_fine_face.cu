@@ -449,6 +449,8 @@ int launch_face_dot(rt_hier* h, const T* u, const T* f, T* out, double omega, co
                     const double* coef, int kstep, double* dot_out) {
     constexpr int W = face_warps(sizeof(T) == 8, MODE), MINB = sizeof(T) == 8 ? 1 : 3;
     rt_level& L = h->L[0];
+    if (sizeof(T) == 4 && MODE >= 2 && !h->dinv32)
+        return rt_fail(h->ctx, RT_ESTATE, "%s: the diagonal blocks have not been made", name);
     const int zc = h->tune[sizeof(T) == 8 ? 1 : 0][MODE].zchunk;
     const dim3 grid((L.vx + FACE_NX - 1) / FACE_NX, (L.vy + W - 2) / (W - 1), (L.vz + zc - 1) / zc);
     const rte::KtVals<T> kt = rte::make_kt<T>(h);

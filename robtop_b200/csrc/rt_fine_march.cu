@@ -267,6 +267,7 @@ int launch_march(rt_hier* h, const T* u, const T* f, T* out, double omega, const
                  const double* coef, int kstep) {
     const rt_tile_cfg& tc = h->tune[sizeof(T) == 8 ? 1 : 0][MODE];
     const T* dinv = sizeof(T) == 8 ? (const T*)h->dinv64 : (const T*)h->dinv32;
+    if (MODE >= 2 && !dinv) return rt_fail(h->ctx, RT_ESTATE, "%s: the diagonal blocks have not been made", name);
     if (tc.variant == 2) {
         switch (tc.ty) {
             case 2: return launch_march_ty<T, WS, MODE, 2, true>(h, tc.zchunk, u, f, out, omega, name, dvec, coef, kstep, dinv);

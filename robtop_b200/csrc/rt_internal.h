@@ -119,7 +119,7 @@ struct rt_hier {
     uint32_t cheby_fused = 0;
     uint32_t cheby_stream = 0;  // fused levels held to the streaming form (rt_set_level_fused on = 2)
     double fused_us[15][2] = {};
-    double* dinv64 = nullptr;        // [6][nv] inverted diagonal blocks of the finest level
+    double* dinv64 = nullptr;        // [6][nv] inverted diagonal blocks of the finest level, allocated on first use
     float* dinv32 = nullptr;
     bool dinv_ready[2] = {false, false};  // [FP32, FP64] the blocks match the weights (made for kernels that read them)
     uint8_t* ncode = nullptr;        // [nv] node codes of the finest level (k_node_code), remade when w, vact or vfix change

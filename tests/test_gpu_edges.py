@@ -500,6 +500,16 @@ def test_fp32_blocks_follow():
         late = step(G, (8, 1, shape))
         G.update_stencil()
         assert np.array_equal(late, step(G))
+    # a hierarchy without blocks yet, and its tuner
+    G2 = rb.HierarchyGrid(ctx, G.params)
+    G2.genFromBox(eact)
+    G2[0].setRho(new.ravel())
+    G2.set_support(vfix)
+    G2.set_tiles(3, 8, 16)
+    G2.update_stencil()
+    assert G2.autotune(2)["chebyshev_f32"]["us"] > 0
+    step(G2)
+    G2.close()
     W = G.workspace()
     vfix[:, :, -1] = 1
     G.set_support(vfix)

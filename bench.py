@@ -803,7 +803,7 @@ def run_kernel(args):
             G.set_params(p)
             G.update_stencil()
         variant = None
-        if args.shape and prec == rb.FP32:  # 0 lane-split, 1 bulk-copy
+        if args.shape and prec == rb.FP32:  # 0 direct loads, 1 bulk-copy
             variant = int(args.shape)
             rb._capi.check(rb.lib().rt_set_level_kernel(G.handle, 1 if form == "bf16" else 0, variant), ctx.handle)
         us = C.c_double()

@@ -1995,7 +1995,7 @@ static int pcg_core(rt_hier* h, double* x, const double* b, double tol, int maxi
         // scal[36]: learned corrections run in this solve
         RT_CUDA(h->ctx, cudaMemsetAsync(h->scal + 36, 0, sizeof(double), h->ctx->stream));
         if (h->unet) RT_CHECK(rtu::refresh(h->unet));
-        // scal[90..93]: stall detection of the reduced-precision V-cycles (see k_pcg_tail)
+        // scal[90..93]: stall detection of the reduced-precision V-cycles (pcg_end in rt_misc.cu)
         const bool fallback = h->P.precision != RT_FP64 && h->P.precision_fallback > 0;
         double sd[4] = {s[0], 0.0, 0.0, fallback ? (double)h->P.precision_fallback : 0.0};
         memcpy(h->ctx->hscal + 16, sd, sizeof(sd));
@@ -2646,7 +2646,7 @@ extern "C" int rt_bench_level_kernel(rt_hier* h, int lvl, int precision, int mod
     return RT_OK;
 }
 
-// the lane-split / bulk-copy choice for the FP32 smoother's stencil kernels, timed on the largest
+// the direct-load / bulk-copy choice for the FP32 smoother's stencil kernels, timed on the largest
 // stencil level's Chebyshev step (FP32 stencils, and BF16 ones when they exist)
 // a set of nsteps FP32 Chebyshev steps on stencil level lvl (random u, f), separate launches or one
 // fused launch, captured as a graph as the solver runs it; device time per set in microseconds
@@ -2699,7 +2699,7 @@ static double time_level_sweeps(rt_hier* h, int lvl, bool fused, int nsteps, int
 static int autotune_level_kernels(rt_hier* h, int reps) {
     if (!h->stencil_ready || h->L.size() < 3) return RT_OK;
     // fused Chebyshev sweeps (one cooperative launch per smoothing) per stencil level, timed on
-    // sets of 8 steps against the separate launches of the chosen lane-split / bulk variant.
+    // sets of 8 steps against the separate launches of the chosen direct-load / bulk variant.
     // The timings are recorded, the choice stays with the caller (rt_set_level_fused): alone the
     // fused sets are faster, but inside the solver's conditional-loop graphs the whole solve
     // measured slower with them
@@ -2829,7 +2829,7 @@ __global__ void k_pcg_start(double* __restrict__ scal, double tol, double maxit,
     scal[26] = maxit;
     scal[28] = 0.0;  // batched instances run without the learned correction
     scal[29] = scal[21];
-    scal[90] = scal[21];  // stall detection of reduced-precision V-cycles (k_pcg_tail)
+    scal[90] = scal[21];  // stall detection of reduced-precision V-cycles (pcg_end in rt_misc.cu)
     scal[91] = 0.0;
     scal[92] = 0.0;
     scal[93] = stall;

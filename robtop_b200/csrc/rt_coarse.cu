@@ -127,7 +127,6 @@ __global__ void __launch_bounds__(128) k_st_gs(int vx, int vy, int vz, int color
 }
 
 // ---------------------------------------------------------------------------
-// ---------------------------------------------------------------------------
 // Stencil kernels, a block per 32 nodes: warp j sums the three neighbours k = 3 j .. 3 j + 2 of its lane's node, so
 // that every load of a stencil row is a whole line of the blocked layout, and the partial sums meet in shared memory.
 // MODE 0: r = f - A u;  MODE 2: Jacobi;  MODE 3: Chebyshev step.
@@ -267,8 +266,8 @@ __global__ void __launch_bounds__(128) k_st_diag(long nv, const uint8_t* __restr
 // Fused Chebyshev sweeps of a small stencil level: all nsteps steps in one cooperative
 // launch, the steps separated by a grid barrier instead of a kernel boundary.  The coarse
 // levels below the first are a few thousand nodes: a separate launch per step spends most
-// of its time in launch, ramp-up and drain, not in the 243-entry rows.  Same arithmetic and
-// 4 lanes per node, lane q sums neighbours k = q, q + 4, ...; u is ping-ponged with tmp (u -> tmp -> u ...), so
+// of its time in launch, ramp-up and drain, not in the 243-entry rows.  4 lanes per node, lane q sums
+// neighbours k = q, q + 4, ...; u is ping-ponged with tmp (u -> tmp -> u ...), so
 // after an odd step count a last barrier lets every thread copy its own entries back to u.
 // Values written by other blocks in the previous step are read through L2 (ld.global.cg):
 // L1 is not coherent across SMs.  The barrier is bounded: a block whose wait runs out sets
@@ -1236,7 +1235,7 @@ __global__ void __launch_bounds__(GF_BS) k_galerkin_fixed(int fnx, int fny, int 
             const int ex = R * X + pos % R, ey = R * Y + pos / R % R, ez = R * Z + pos / (R * R);
             if (ex >= fnx || ey >= fny || ez >= fnz) continue;
             const double pen = w[ex + (long)fnx * (ey + (long)fny * ez)];
-            if (pen == 0 || pen <= -1) continue;
+            if (pen == 0) continue;
             unsigned fm = 0;
 #pragma unroll
             for (int j = 0; j < 8; j++)
@@ -1372,9 +1371,9 @@ static int launch_bulk(rt_hier* h, int lvl, const char* name, const S* st, const
     });
 }
 
-// the lane-split kernel: enough lanes per node to give every SM 1024 lanes, 4 at least
+// the direct-load kernel: a block per 32 nodes
 template <typename T, int MODE, typename S>
-static int launch_split(rt_hier* h, int lvl, const char* name, const S* st, const T* u, const T* f, T* out, T* d,
+static int launch_direct(rt_hier* h, int lvl, const char* name, const S* st, const T* u, const T* f, T* out, T* d,
                         double omega, const double* coef, int kstep) {
     rt_level& L = h->L[lvl];
     return rt_launch(h->ctx, name, [&] {
@@ -1388,7 +1387,7 @@ static int launch_f32(rt_hier* h, int lvl, const char* name, const S* st, const 
                       float* d, double omega, const double* coef, int kstep) {
     if (h->st_variant[sizeof(S) == 2 ? 1 : 0] == 1)
         return launch_bulk<MODE, S>(h, lvl, name, st, u, f, out, d, omega, coef, kstep);
-    return launch_split<float, MODE, S>(h, lvl, name, st, u, f, out, d, omega, coef, kstep);
+    return launch_direct<float, MODE, S>(h, lvl, name, st, u, f, out, d, omega, coef, kstep);
 }
 
 template <typename T>
@@ -1398,7 +1397,7 @@ int st_residual(rt_hier* h, int lvl, const T* u, const T* f, T* r) {
         return launch_f32<0, float>(h, lvl, LVL_NAME(lvl, false, "st_residual"), L.st32, u, f, r, nullptr, 0.0,
                                     nullptr, 0);
     else
-        return launch_split<T, 0, T>(h, lvl, LVL_NAME(lvl, true, "st_residual"), L.st, u, f, r, nullptr, 0.0, nullptr, 0);
+        return launch_direct<T, 0, T>(h, lvl, LVL_NAME(lvl, true, "st_residual"), L.st, u, f, r, nullptr, 0.0, nullptr, 0);
 }
 
 template <typename T>
@@ -1437,7 +1436,7 @@ int st_jacobi(rt_hier* h, int lvl, const T* u, const T* f, T* unew, double omega
         return launch_f32<2, float>(h, lvl, LVL_NAME(lvl, false, "st_jacobi"), L.st32, u, f, unew, nullptr, omega,
                                     nullptr, 0);
     } else {
-        return launch_split<T, 2, T>(h, lvl, LVL_NAME(lvl, true, "st_jacobi"), L.st, u, f, unew, nullptr, omega, nullptr, 0);
+        return launch_direct<T, 2, T>(h, lvl, LVL_NAME(lvl, true, "st_jacobi"), L.st, u, f, unew, nullptr, omega, nullptr, 0);
     }
 }
 
@@ -1451,7 +1450,7 @@ int st_cheby(rt_hier* h, int lvl, const T* u, const T* f, T* unew, T* d, const d
         return launch_f32<3, float>(h, lvl, LVL_NAME(lvl, false, "st_cheby"), L.st32, u, f, unew, d, 0.0, coef,
                                     kstep);
     } else {
-        return launch_split<T, 3, T>(h, lvl, LVL_NAME(lvl, true, "st_cheby"), L.st, u, f, unew, d, 0.0, coef, kstep);
+        return launch_direct<T, 3, T>(h, lvl, LVL_NAME(lvl, true, "st_cheby"), L.st, u, f, unew, d, 0.0, coef, kstep);
     }
 }
 template <typename T>

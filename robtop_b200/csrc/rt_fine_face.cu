@@ -11,21 +11,22 @@
 //    the element above), only the z stage is per element: 6 + 12 + 24 adds instead of 72, and the same on the
 //    way back, where neighbours' results are added between the stages, so that no scatter remains.
 //  * A lane owns element column X0 - 1 + lane and node column X0 - 1 + lane, a warp one element row.  x neighbours
-//    meet by shuffles; the upper edge of a warp's row goes to the next warp, 6 values (in FP64 smoothing 2 weight sums as well) per lane and
-//    layer through shared memory, with one barrier per layer.  Lanes 1..30 finish nodes; a block of W warps finishes
-//    30 x (W - 1) nodes per layer.
+//    meet by shuffles; the upper edge of a warp's row goes to the next warp, 6 values (in FP64 smoothing 2 weight sums
+//    as well) per lane and layer through shared memory, with one barrier per layer.  Lanes 1..30 finish nodes; a block
+//    of W warps finishes 30 x (W - 1) nodes per layer.
 //  * The loads of the next layer and of this layer's output stage are issued before the arithmetic (FP32 Chebyshev on
-//    511x256x256: 874 us with them behind it, 666).
+//    511x256x256, when it formed the diagonal block itself: 874 us with them behind it, 666).
 //  * FP64 K u, with 12 warps per SM, waits longest at the barrier: there a warp arrives at an mbarrier when its edge of
 //    layer t is written, and waits (with a limit) before the output of layer t, which follows the x stage and the loads
 //    of layer t + 1 (511x256x256: 897 us with __syncthreads, 766 us).  The other forms hold the inputs of the output
 //    stage as well and got slower with it (FP64 residual 850, 938 us with it; FP32 residual 490, 600 us).
-//  * Two element rows per warp, with the edge between them in registers, need 128 registers in FP32: Chebyshev 736 us.
+//  * Two element rows per warp, with the edge between them in registers, need 128 registers in FP32: that Chebyshev
+//    step 736 us.
 //  * The 3x3 diagonal block of a node needs four signed sums of its 8 weights, factorised the same way.  FP64 steps form
 //    and invert it; FP32 steps read the inverse that k_fine_dinv made in FP64.  Inverted in FP32 here, a step from zero
 //    had 2 to 3 times the error, and entries past 1e12 or below 1e-13 left FP32's range in the determinant (511x256x256,
 //    z-chunk 16: Jacobi 637 us so, 715 us read; Chebyshev 686, 715 us); formed here in FP64 it needs registers that are
-//    not there (Jacobi 682 us, Chebyshev 928 us; 768 us with 20 warps per SM instead of 24).
+//    not there (Jacobi 682 us, Chebyshev 928 us; 773 us with 20 warps per SM instead of 24).
 //
 // Fixed and inactive nodes enter the element products as zero (the reference's WS rule); out[] follows
 // rt_fine_tile.cu's rules for them.
@@ -348,6 +349,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
 // The smoothing step from u = 0, where K u needs no evaluation: out = omega D^-1 f (MODE 2) or out = d = b_0 D^-1 f
 // (MODE 3), fixed nodes f / n_e (d = 0).  A thread marches one node column through a z-chunk with the weight sums of
 // the element layer below, the block in FP64; 29 B (MODE 2) or 41 B per node in FP32, the full step moves 90.
+// FP32 Chebyshev, 511x256x256: 343 us with the block in FP32, 404 us so, 420 us with the stored block read instead.
 template <typename T, int MODE, bool DOT>
 __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code,
                                                    const float* __restrict__ wgt, double diag_a, double diag_b,
@@ -524,8 +526,10 @@ template int fine_applyK_dot<double>(rt_hier*, const double*, double*, double*);
 template int fine_applyK_dot<float>(rt_hier*, const float*, float*, double*);
 
 // the launch shape used before rt_autotune ran: the z-chunk whose waves of blocks march through the fewest layers
-// (a chunk of zc layers takes zc + 2 steps).  64x32x32: 2, 129x97x85: 16, 255x256x128: 16, as the sweep found best
-// or within 5 %
+// (a chunk of zc layers takes zc + 2 steps).  Against the best of 2, 4 .. 64 layers, timed warm on 64x32x32, 129x97x85,
+// 255x256x128 and 511x256x256: FP32 at most 6 % slower.  FP64 at most 2 % on the first two, but 16 layers where 64 are 7
+// to 10 % faster on the last, and on 255x256x128 8 layers for K u, 233 us, and the residual, 251 us, where 64 take 193
+// and 213 us (rt_autotune finds them)
 rt_tile_cfg face_default(rt_ctx* c, bool f64, int mode, int vx, int vy, int vz) {
     const int w = face_warps(f64, mode);
     const long slots = (long)c->sm_count * (f64 ? 1 : 3);

@@ -111,7 +111,7 @@ struct rt_hier {
     rt_tile_cfg tune[2][4];          // [FP32, FP64][residual, applyK, jacobi, chebyshev]
     double tune_us[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};  // measured time of the chosen shape
     // stencil-level kernels of the FP32 smoother [FP32 stencils, BF16 stencils]: 0 direct loads
-    // (4 lanes per node, loads through L1), 1 bulk-copy (32-node stencil runs staged in shared memory)
+    // (9 warps per 32 nodes, loads through L1), 1 bulk-copy (32-node stencil runs staged in shared memory)
     int st_variant[2] = {0, 1};
     double st_us[2][2] = {{0, 0}, {0, 0}};  // [stencil type][variant] level-1 Chebyshev step (rt_autotune)
     // stencil levels whose FP32 Chebyshev sweeps run as one cooperative launch (bit lvl; rt_autotune),

@@ -224,8 +224,9 @@ __device__ __forceinline__ void pcg_end(double* scal, cudaGraphConditionalHandle
     }
 }
 
-// r -= alpha q, r.r and the end of the iteration (by the last block, which has the sum).  r32 (optional): the new residual scaled by 1 / sqrt(rr_old) and rounded to FP32, the
-// right-hand side of the next FP32 V-cycle; rr_old (the r.r before this update) is kept in scale_out
+// r -= alpha q, r.r and the end of the iteration (by the last block, which has the sum).  r32 (optional): the new
+// residual scaled by 1 / sqrt(rr_old) and rounded to FP32, the right-hand side of the next FP32 V-cycle; rr_old (the r.r
+// before this update) is kept in scale_out
 template <typename T>
 __global__ void __launch_bounds__(RB) k_pcg_r_rr(long n, const double* __restrict__ num, const double* __restrict__ den,
                                                  T* __restrict__ r, const T* __restrict__ q, float* __restrict__ r32,

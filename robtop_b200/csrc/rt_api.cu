@@ -1370,7 +1370,7 @@ extern "C" int rt_smooth_f32(rt_hier* h, int lvl, int smoother, int sweeps, doub
         return rt_fail(h->ctx, RT_EINVAL, "FP32 smoothing: Jacobi or Chebyshev");
     if (lvl > 0) RT_CHECK(need_stencil(h));
     else RT_CHECK(refresh_fine(h));
-    RT_CHECK(need_dinv(h, 0));
+    if (lvl == 0) RT_CHECK(need_dinv(h, 0));
     if (smoother == RT_SMOOTH_CHEBY && !h->stencil_ready) return rt_fail(h->ctx, RT_ESTATE, "rt_update_stencil has not run");
     rt_level& L = h->L[lvl];
     const long n = 3 * L.nv;

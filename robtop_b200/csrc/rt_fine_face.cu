@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(32 * W, MINB)
 // The smoothing step from u = 0, where K u needs no evaluation: out = omega D^-1 f (MODE 2) or out = d = b_0 D^-1 f
 // (MODE 3), fixed nodes f / n_e (d = 0).  A thread marches one node column through a z-chunk with the weight sums of
 // the element layer below, the block in FP64; 29 B (MODE 2) or 41 B per node in FP32, the full step moves 90.
-// FP32 Chebyshev, 511x256x256: 343 us with the block in FP32, 404 us so, 420 us with the stored block read instead.
+// FP32 Chebyshev, 511x256x256: 343 us with the block in FP32, 404 us so.
 template <typename T, int MODE, bool DOT>
 __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int zchunk, const uint8_t* __restrict__ code,
                                                    const float* __restrict__ wgt, double diag_a, double diag_b,
@@ -410,6 +410,54 @@ __global__ void __launch_bounds__(256) k_fine_diag(int nx, int ny, int nz, int z
         for (int q = 0; q < 4; q++) Qp[q] = Q[q];
     }
     if (DOT) face_grid_sum<8>(fo, partials, dot_out, ticket);
+}
+
+// The same step from the stored inverse blocks, FP32 only: 53 B (MODE 2) or 65 B per node, but no sums and no division,
+// and two nodes' loads in flight per thread.  Chebyshev, with the launch, against k_fine_diag: 97x61x45 10.7 us (14.7),
+// 255x256x128 96 us (135), 511x256x256 358 us (404); with one node per trip 11.3, 119 and 422 us.
+constexpr int DIAG_U = 2;
+
+template <int MODE>
+__global__ void __launch_bounds__(256) k_fine_diag_stored(long nv, const uint8_t* __restrict__ code,
+                                                          const float* __restrict__ dinv, const float* __restrict__ f,
+                                                          float* __restrict__ out, float omega, float* __restrict__ dvec,
+                                                          const double* __restrict__ coef) {
+    const float scale = MODE == 3 ? (float)coef[1] : omega;
+    const long st = gridDim.x * 256L;
+    for (long v0 = blockIdx.x * 256L + threadIdx.x; v0 < nv; v0 += DIAG_U * st) {
+        uint32_t c[DIAG_U];
+        float inv[DIAG_U][6], r[DIAG_U][3];
+#pragma unroll
+        for (int k = 0; k < DIAG_U; k++) {
+            const long v = v0 + k * st;
+            c[k] = 0;
+            if (v >= nv) break;
+            c[k] = code[v];
+#pragma unroll
+            for (int q = 0; q < 6; q++) inv[k][q] = dinv[q * nv + v];
+#pragma unroll
+            for (int q = 0; q < 3; q++) r[k][q] = f[q * nv + v];
+        }
+#pragma unroll
+        for (int k = 0; k < DIAG_U; k++) {
+            const long v = v0 + k * st;
+            if (v >= nv) break;
+            float o[3] = {0.f, 0.f, 0.f};
+            if (c[k] == 1u) {
+                o[0] = scale * (inv[k][0] * r[k][0] + inv[k][1] * r[k][1] + inv[k][2] * r[k][2]);
+                o[1] = scale * (inv[k][1] * r[k][0] + inv[k][3] * r[k][1] + inv[k][4] * r[k][2]);
+                o[2] = scale * (inv[k][2] * r[k][0] + inv[k][4] * r[k][1] + inv[k][5] * r[k][2]);
+            } else if (c[k] > 1u) {
+#pragma unroll
+                for (int q = 0; q < 3; q++) o[q] = fixed_value(r[k][q], c[k]);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                out[q * nv + v] = o[q];
+                if (MODE == 3) dvec[q * nv + v] = c[k] == 1u ? o[q] : 0.f;
+            }
+        }
+    }
 }
 
 // node codes read by k_fine_face: bit 0 active, bit 1 fixed, bits 2.. the number of elements of non-zero weight
@@ -479,6 +527,19 @@ int node_codes(rt_hier* h) {
 template <typename T>
 int fine_smooth0(rt_hier* h, const T* f, T* out, double omega, T* dvec, const double* coef, double* dot_out) {
     rt_level& L = h->L[0];
+    if constexpr (sizeof(T) == 4) {
+        // where the following steps read the stored blocks they are there, and current; 32 blocks per SM (16: 380 us)
+        const int v = h->tune[0][coef ? 3 : 2].variant;
+        if (v == 8 && h->dinv32 && !dot_out)
+            return rt_launch(h->ctx, "fine_smooth0_f32", [&] {
+                const unsigned g = (unsigned)std::min<long>((L.nv + 255) / 256, (long)h->ctx->sm_count * 32);
+                cudaStream_t s = h->ctx->stream;
+                if (coef)
+                    k_fine_diag_stored<3><<<g, 256, 0, s>>>(L.nv, h->ncode, h->dinv32, f, out, 0.f, dvec, coef);
+                else
+                    k_fine_diag_stored<2><<<g, 256, 0, s>>>(L.nv, h->ncode, h->dinv32, f, out, (float)omega, nullptr, nullptr);
+            });
+    }
     int zc = 32;  // 1/32 of the weight layers read twice; shorter chunks where blocks are few
     const long xy = (long)((L.vx + 31) / 32) * ((L.vy + 7) / 8);
     while (zc > 4 && xy * ((L.vz + zc - 1) / zc) < 8L * h->ctx->sm_count) zc /= 2;

@@ -540,3 +540,29 @@ def test_fine_gauss_seidel_quotient():
     assert np.array_equal(G[0].getDisplacement().reshape(f.shape)[0, ::2, ::2, ::2], want[::2, ::2, ::2])
     G.close()
     ctx.close()
+
+
+# the FP32 step from zero with stored blocks takes a second node per thread past 32 x 256 nodes per SM: one iteration of
+# either precision's cycle, whose first step that is, on a box of 1.3M nodes and supports at both its ends
+@pytest.mark.parametrize("jacobi", [False, True])
+def test_step_from_zero_second_node(jacobi):
+    ctx, G, eact, rho, vfix, r = _hier(133, 103, 97, seed=13)
+    vfix[-1] = 1
+    G.set_support(vfix)
+    p = G.params
+    p.pre_sweeps, p.post_sweeps, p.jacobi_omega = 1, 1, 0.5
+    p.smoother = rb.SMOOTH_JACOBI if jacobi else rb.SMOOTH_CHEBY
+    b = r.standard_normal(3 * G[0].nv) * np.tile(1.0 - vfix.ravel(), 3)
+    x = []
+    for prec in (rb.FP64, rb.FP32):
+        p.precision = prec
+        G.set_params(p)
+        G.update_stencil()
+        G[0].setForce(b)
+        G[0].reset_displacement()
+        G.pcg(1e-14, 1)
+        x.append(G[0].getDisplacement())
+    # as in test_tail_cycle_edges
+    assert rel_err(x[1], x[0]) < 1e-3
+    G.close()
+    ctx.close()

@@ -1054,8 +1054,8 @@ static int remake_codes(rt_hier* h) {
     return rtk::node_codes(h);
 }
 
-// element weights rho^p and node codes of the finest level, and the blocks that FP64 smoothing and the hierarchy's own
-// solves read; the FP32 calls ask for theirs
+// element weights rho^p and node codes of the finest level and, where a chosen kernel reads them, the FP64 blocks; what
+// smooths in FP32 asks for its own
 static int refresh_fine(rt_hier* h) {
     if (h->parent) {  // weights, node codes and diagonal blocks belong to the parent (refreshed by its own calls)
         ws_sync(h);
@@ -1793,6 +1793,14 @@ static int nan_fail(rt_hier* h, int it) {
     return rt_fail(h->ctx, RT_ENAN, "NaN in PCG at iteration %d", it);
 }
 
+// a solve whose first residual is not finite: a wait that ran out in its K u, or the caller's data
+static int start_fail(rt_hier* h) {
+    double e = 0;
+    RT_CHECK(read_scalars(h, RT_SCAL_ERR, 1, &e));
+    if (e != 0.0) return nan_fail(h, 0);
+    return rt_fail(h->ctx, RT_ENAN, "PCG: the right-hand side or the initial residual is not finite");
+}
+
 // ---------------------------------------------------------------------------
 // FP32 Krylov form (rt_params.krylov_fp32 with precision RT_FP32): flexible CG whose vectors,
 // operator products and V-cycles are all FP32 (every dot product summed in FP64), solving
@@ -1885,7 +1893,7 @@ static int pcg32_core(rt_hier* h, double* x, const double* b, double tol, int ma
     RT_CHECK(read_scalars(h, 21, 2, s));
     if (!std::isfinite(s[0]) || !std::isfinite(s[1])) {
         if (info) { info->status = RT_ENAN; info->iterations = 0; }
-        return rt_fail(h->ctx, RT_ENAN, "PCG: the right-hand side or the initial residual is not finite");
+        return start_fail(h);
     }
     const double bn = std::sqrt(s[1]) > 0 ? std::sqrt(s[1]) : 1.0;
     double rel = std::sqrt(s[0]) / bn;
@@ -1976,7 +1984,7 @@ static int pcg_core(rt_hier* h, double* x, const double* b, double tol, int maxi
     RT_CHECK(read_scalars(h, 21, 2, s));
     if (!std::isfinite(s[0]) || !std::isfinite(s[1])) {
         if (info) { info->status = RT_ENAN; info->iterations = 0; }
-        return rt_fail(h->ctx, RT_ENAN, "PCG: the right-hand side or the initial residual is not finite");
+        return start_fail(h);
     }
     const double bn = std::sqrt(s[1]) > 0 ? std::sqrt(s[1]) : 1.0;
     double rel = std::sqrt(s[0]) / bn;
